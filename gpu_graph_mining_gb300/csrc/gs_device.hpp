@@ -19,8 +19,25 @@
 // filtered copy.  Each DFS-tree node also carries gord[row]: the dense rank
 // of the row's graph among the graphs that contain the node's pattern
 // (0..support-1), the index into the node's support bitmaps.
+//
+// Packed rows (databases whose graphs have at most 64 vertices): a row is the
+// embedding itself instead of a chain of back-links, the first graph vertex
+// of its graph and one byte per pattern vertex (graph-local ids), with the
+// row's graph rank: 16 bytes up to 8 pattern vertices, 16 more per further 16
+// (planes of nrows uint4: plane 0 = {first vertex, graph rank, ids 0-3,
+// ids 4-7}, plane p = ids 8 + 16(p - 1) ..).  Neighbour lists are 32-byte
+// blocks, block v = vertex v's list, one DRAM sector: up to 8 entries of 4
+// bytes, ((pair index + 1) << nb_shift) | (neighbour label << 6) |
+// graph-local neighbour, ascending, 0 = none; a list of more than 8 has 7 and
+// in the last word 2^31 | the block that continues it (again up to 8 entries,
+// or 7 and a link).  A wave's extension records are blocks of 32 four-byte
+// items of one tile, (node's key << 11) | (graph-local new vertex << 5) | row
+// in the tile, each with a header {first row of the tile, node, items |
+// counter copy << 8, the node's first key}.
 #pragma once
 #include <cstdint>
+
+#include <cuda_runtime.h>
 
 namespace gsgb {
 
@@ -40,7 +57,29 @@ struct DevDB {
   int32_t adj_sorted;  // 1: each vertex's entries ascend (adj as unsigned 64-bit values)
   const int32_t *root_off;   // [VL+1] first key of each vertex label's (elabel, tolabel) pairs
   const int32_t *pair_code;  // [root_off[VL]] (elabel << 16) | tolabel of each pair
+  const uint4 *nb;           // neighbour blocks (two uint4 each), or nullptr: no packed rows
+  int32_t nb_blocks;         // blocks there is room for
+  int32_t nb_shift;          // 6 + bits of a vertex label
 };
+
+// Whether a database takes packed rows: its graphs' vertices as 6-bit ids,
+// neighbour entries below 2^31, and a node's keys (at most 64 slots of pairs
+// and edge labels) below the items' 2^21.
+inline int32_t packed_shift(int64_t max_graph_vertices, int64_t VL, int64_t EL, int64_t pairs)
+{
+  int32_t bits = 0;
+  while(((int64_t)1 << bits) < VL) bits++;
+  const int32_t sh = 6 + bits;
+  if(max_graph_vertices > 64 || sh > 30 || pairs + 1 >= ((int64_t)1 << (31 - sh)) || 64 * (pairs + EL) >= (1 << 21))
+    return 0;
+  return sh;
+}
+// Neighbour blocks for V vertices and E2 entries: a list of d > 8 entries
+// takes at most d / 7 blocks beside its first; ids of a row address up to 63
+// blocks past its graph's first vertex.
+inline int64_t packed_blocks(int64_t V, int64_t E2) { return V + E2 / 7 + 64; }
+// 16-byte planes of a packed row of k pattern vertices.
+inline int32_t packed_planes(int32_t k) { return k <= 8 ? 1 : 1 + (k - 8 + 15) / 16; }
 
 // Per job of a root phase (the root level of a group of jobs, one launch per
 // kernel): its vertices as 32-vertex warp tiles in the group's tile space, its
@@ -59,7 +98,6 @@ struct RootJob {
 
 // Per DFS-tree node of a wave (a batch of nodes extended together).
 struct NodeDesc {
-  long long row_begin;   // first row in the wave's concatenated row space
   long long tile_begin;  // first 32-row warp tile of the node (tiles never span two nodes)
   long long bm_base;     // first support-bitmap word of the node's key 0
   const int32_t *gord;   // [nrows]
@@ -94,32 +132,44 @@ struct NodeDesc {
   int32_t join_lo;         // first forward key of u
   int32_t join_key;        // the new edge's key (in the parent)
   int32_t join_hi;         // one past u's forward keys
+  // packed rows (rows == nullptr: the node has columns)
+  const uint4 *rows;         // planes of nrows
+  const uint4 *nb;           // its database's neighbour blocks,
+  const int32_t *pair_code;  //   pair codes,
+  int32_t nb_blocks, nb_shift, n_vertices;
+  int32_t planes;
+  int32_t back;              // 1: some slot takes a backward edge
 };
 
-// One right-most-path vertex of a node.
-struct SlotDesc {
+// One right-most-path vertex of a node.  The order rules of the
+// right-most-path edge (el_u, tl_u) that leaves the vertex are single compares:
+//   forward allowed iff (el_u, tl_u) <= (el, tl)  <=>  hi >= frule, with an
+//     adjacency entry's high word hi = (el << 16) | nbr_label (INT32_MIN for
+//     the right-most vertex: no rule), and for packed rows entry >= prule
+//   backward allowed iff el_u < el || (el_u == el && tl_u <= label(right-most))
+//     <=>  el >= bmin
+struct alignas(16) SlotDesc {
   int32_t vertex;    // pattern vertex id
   int32_t vlab;      // its (dense) label
   int32_t fkey_off;  // forward keys of this slot: fkey_off + pair_idx(vlab, el, tl)
-  int32_t fel, ftl;  // forward order rule from the right-most-path edge leaving this
-                     // vertex: allowed iff fel < el || (fel == el && ftl <= tl); fel = -1
-                     // for the right-most vertex (no rule)
   int32_t bkey_off;  // backward keys to this vertex: bkey_off + el; -1 if not a target
-  int32_t bel, blab; // backward order rule: allowed iff bel < el || (bel == el && blab <= label(rightmost))
-  // the same two rules as single compares against an adjacency entry's high
-  // word hi = (el << 16) | nbr_label: forward allowed iff hi >= frule
-  // (INT32_MIN for the right-most vertex); backward allowed iff el >= bmin
   int32_t frule;
   int32_t bmin;
+  int32_t prule;     // packed rows: the least neighbour entry that the forward rule allows
+  int32_t pbase;     // the first pair code of the vertex's label
 };
 
 // Output slots of a child node selected for materialisation.
-struct ChildOut {
-  int2 *col;      // the child's new last column
+struct alignas(16) ChildOut {
+  uint4 *rows;    // packed rows: the child's planes of cap rows (else nullptr)
+  long long word; // packed rows: the key's first support-bitmap word
+  int32_t cap;    // rows allocated (the count pass's embedding count for the key)
+  int32_t kind;   // 0 forward, 1 backward, 2 root
+  int32_t planes; // packed rows: the child's
+  int32_t pad;
+  int2 *col;      // columns: the child's new last column
   int2 *col0;     // root children only: column 0
   int32_t *gord;  // the child's graph ranks
-  int32_t kind;   // 0 forward, 1 backward, 2 root
-  int32_t cap;    // rows allocated (the count pass's embedding count for the key)
 };
 
 }  // namespace gsgb

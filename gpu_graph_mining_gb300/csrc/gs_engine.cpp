@@ -81,6 +81,25 @@ void Database::prepare()
     acc += pair_cnt[a];
   }
   root_keys = acc;
+  index_pairs();
+}
+
+int32_t Database::pair_index(int32_t a, int32_t el, int32_t tl) const
+{
+  if(!pair_tab.empty()) return pair_tab[((int64_t)a * EL + el) * VL + tl];
+  const auto &pr = pairs[a];
+  return (int32_t)(std::lower_bound(pr.begin(), pr.end(), std::make_pair(el, tl)) - pr.begin());
+}
+
+void Database::index_pairs()
+{
+  const int64_t tab = (int64_t)VL * EL * VL;
+  pair_tab.clear();
+  if(tab > 1 << 20) return;
+  pair_tab.assign((size_t)tab, -1);
+  for(int32_t a = 0; a < VL; a++)
+    for(size_t i = 0; i < pairs[a].size(); i++)
+      pair_tab[((int64_t)a * EL + pairs[a][i].first) * VL + pairs[a][i].second] = (int32_t)i;
 }
 
 void Database::upload()
@@ -100,7 +119,15 @@ void Database::upload()
   size_t o_vb = o_ro + al(sizeof(int32_t) * (VL + 1));
   size_t o_ap = o_vb + al(sizeof(int32_t) * (host.n_graphs + 1));
   size_t o_pc = o_ap + al(sizeof(int32_t) * (E2 + 1));
-  size_t total = o_pc + al(sizeof(int32_t) * (root_keys + 1));
+  // neighbour blocks (packed rows), filled by a kernel from the arrays before
+  int32_t maxnv = 0;
+  for(int32_t g = 0; g < host.n_graphs; g++) maxnv = std::max(maxnv, host.graph_nv(g));
+  const int32_t nb_shift = packed_shift(maxnv, VL, EL, root_keys);
+  int64_t nb_blocks = nb_shift ? packed_blocks(V, E2) : 0;
+  if(nb_blocks >= INT32_MAX) nb_blocks = 0;
+  size_t o_nu = o_pc + al(sizeof(int32_t) * (root_keys + 1));
+  size_t o_nb = o_nu + al(sizeof(int32_t));
+  const size_t copied = o_nb;
   std::vector<unsigned long long> adj(E2 + 1, 0);
   parallel_ranges(E2, [&](int64_t b, int64_t e, int) {
     for(int64_t k = b; k < e; k++) {
@@ -143,11 +170,18 @@ void Database::upload()
     }
   });
   std::vector<int32_t> vb(host.n_graphs + 1);
-  int32_t maxnv = 0;
   for(int32_t g = 0; g <= host.n_graphs; g++) vb[g] = (int32_t)host.vbase[g];
-  for(int32_t g = 0; g < host.n_graphs; g++) maxnv = std::max(maxnv, host.graph_nv(g));
-  CK(cudaMalloc(&d_block, total));
+  // without room for the neighbour blocks the database is mined on columns
+  size_t total = copied + al(32 * (size_t)nb_blocks);
+  if(nb_blocks > 0 && cudaMalloc(&d_block, total) != cudaSuccess) {
+    cudaGetLastError();
+    d_block = nullptr;
+    nb_blocks = 0;
+    total = copied;
+  }
+  if(!d_block) CK(cudaMalloc(&d_block, total));
   d_bytes = total;
+  h2d_bytes = copied;
   char *b = (char *)d_block;
   CK(cudaMemcpy(b + o_adj, adj.data(), sizeof(unsigned long long) * (E2 + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b + o_off, off.data(), sizeof(int32_t) * (V + 1), cudaMemcpyHostToDevice));
@@ -182,6 +216,15 @@ void Database::upload()
   d_root_off = (int32_t *)(b + o_ro);
   dev.root_off = d_root_off;
   dev.pair_code = (const int32_t *)(b + o_pc);
+  if(nb_blocks > 0) {
+    dev.nb_shift = nb_shift;
+    dev.nb_blocks = (int32_t)nb_blocks;
+    CK(cudaMemsetAsync(b + o_nu, 0, sizeof(int32_t), cudaStreamLegacy));
+    launch_neighbour_blocks(dev, (uint4 *)(b + o_nb), (int32_t *)(b + o_nu), cudaStreamLegacy);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
+    dev.nb = (const uint4 *)(b + o_nb);
+  }
   resident = true;
 }
 
@@ -576,10 +619,12 @@ struct PNode {
   SmallVec<DFS, 12> code;
   SmallVec<ColRef, 12> cols;  // column c = pattern vertex c
   int32_t last_col = -1;      // the node's reference: its last column (the rest by parent links)
-  int32_t *gord;
-  int32_t gord_blk;
+  int32_t *gord = nullptr;
+  int32_t gord_blk;           // packed rows: the block of the rows
   int64_t nrows;
   int64_t support;
+  uint4 *rows = nullptr;      // packed rows: no columns, the whole embeddings in planes of nrows
+  int32_t nv = 0;             // packed rows: pattern vertices
   // lists strategy (forward children whose parent kept its per-row lists):
   // the parent's lists (a pool block shared by the parent's wave) and the
   // join rule (NodeDesc::join_lo / join_key / join_hi)
@@ -598,6 +643,7 @@ struct JobState {
   std::vector<int32_t> roots;
   std::vector<int32_t> root_keys;  // each root's key (root_off[fl] + pair): the reference's root order
   std::vector<int32_t> stack;  // DFS-tree nodes waiting for a wave (top = back), as node pool ids
+  bool packed = false;         // its nodes have packed rows
   int64_t pending = 0;         // nodes on the stack or in a wave in flight
   int64_t live_bytes = 0;      // embedding-store bytes held by the job's nodes
   int64_t peak_bytes = 0;
@@ -682,6 +728,9 @@ constexpr int kHeadExt = 3;       // embeddings of all keys } the support
 constexpr int kHeadListed = 4;    // keys counted          } selection
 constexpr int kHeadSelBytes = 5;  // algorithmic bytes     }
 constexpr size_t kHeadBytes = 64;
+// A record block of packed rows in int4 units of the record buffer: 32 items
+// of 4 bytes and a 16-byte header.
+constexpr long long kRecBlockInt4 = 9;
 
 // Device scratch and pinned mirrors of one wave in flight.  Two of them let
 // the host prepare one wave's children while the GPU counts the other's.
@@ -803,7 +852,7 @@ struct Engine {
   std::vector<int32_t> free_blocks;
   int64_t pool_limit = 0;
   DBuf<DevDB> d_dbs;
-  DBuf<unsigned long long> d_bytes;   // [0] count bytes, [1] materialise bytes, [2] root bytes, [3] flags
+  DBuf<unsigned long long> d_bytes;   // [0] count bytes, [1] materialise bytes (column kernels), [3] flags
   WaveCtx ctx[kWaveCtx];
   // root phases: the root level of a group of jobs, one launch per kernel
   WaveCtx rootx;
@@ -991,24 +1040,25 @@ void layout_node(const PNode &n, const Database &db, NodeLayout &L)
   int32_t fk = 0;
   for(int s = 0; s <= L.nrm; s++) {
     SlotDesc &sd = L.slots[s];
+    // (el_u, tl_u) <= (el, tl) lexicographically <=> (el_u << 16 | tl_u) <= (el << 16 | tl)
+    int32_t el = -1, tl = 0;  // the right-most-path edge's labels
     if(s < L.nrm) {
       const DFS &e = c[rm[L.nrm - 1 - s]];
       sd.vertex = e.from;
-      sd.fel = e.elabel;
-      sd.ftl = e.tolabel;
+      el = e.elabel;
+      tl = e.tolabel;
     } else {
       sd.vertex = L.maxtoc;
-      sd.fel = -1;
-      sd.ftl = 0;
     }
+    sd.frule = s < L.nrm ? (int32_t)(((uint32_t)el << 16) | (uint32_t)tl) : INT32_MIN;
     sd.vlab = L.vlab[sd.vertex];
     sd.fkey_off = fk;
     fk += db.pair_cnt[sd.vlab];
     sd.bkey_off = -1;
-    sd.bel = sd.blab = 0;
-    // (fel, ftl) <= (el, tl) lexicographically <=> (fel << 16 | ftl) <= (el << 16 | tl)
-    sd.frule = s < L.nrm ? (int32_t)(((uint32_t)sd.fel << 16) | (uint32_t)sd.ftl) : INT32_MIN;
     sd.bmin = INT32_MAX;
+    sd.pbase = db.root_off[sd.vlab];
+    // the path edge is in the database: its pair is the first that the rule allows
+    if(db.dev.nb) sd.prule = ((s < L.nrm ? db.pair_index(sd.vlab, el, tl) : 0) + 1) << db.dev.nb_shift;
   }
   L.nfwd = fk;
   const int32_t rlab = L.vlab[L.maxtoc];
@@ -1020,10 +1070,8 @@ void layout_node(const PNode &n, const Database &db, NodeLayout &L)
     bool joined = false;
     for(const DFS &d : c)
       if((d.from == L.maxtoc && d.to == sd.vertex) || (d.to == L.maxtoc && d.from == sd.vertex)) joined = true;
-    sd.bel = e.elabel;
-    sd.blab = e.tolabel;
     sd.bkey_off = joined ? -1 : fk + s * db.EL;
-    // bel < el || (bel == el && blab <= label(r))  <=>  el >= bel + (blab > label(r))
+    // el_u < el || (el_u == el && tl_u <= label(r))  <=>  el >= el_u + (tl_u > label(r))
     sd.bmin = joined ? INT32_MAX : e.elabel + (e.tolabel > rlab ? 1 : 0);
   }
 }
@@ -1109,6 +1157,11 @@ struct Flight {
   const int2 *const *dc = nullptr;
   const SlotDesc *ds = nullptr;
   const int32_t *dv = nullptr, *dl = nullptr;
+  bool packed = false;       // the wave's nodes have packed rows
+  const int32_t *dt = nullptr;  // packed: first tile of each node
+  int32_t planes = 1;        // packed: the most planes of a node's rows
+  int4 *hdr = nullptr;       // packed: record headers (rec_cap counts the blocks of one region)
+  uint32_t *reg = nullptr;   // packed: the regions' block counters
   bool join = false;         // some node joins its parent's lists (lists strategy)
   int32_t W = 0, kb = 0, kmax = 1;
   bool small = true;
@@ -1182,7 +1235,7 @@ public:
     Database *db = j.db;
     if(!db->resident) {
       db->upload();
-      st_.h2d_bytes += (int64_t)db->d_bytes;
+      st_.h2d_bytes += (int64_t)db->h2d_bytes;
     }
     int32_t slot = -1;
     for(size_t i = 0; i < dbs_.size(); i++)
@@ -1205,6 +1258,8 @@ public:
     JobState &S = *jobs_.back();
     S.job = j;
     S.db_slot = slot;
+    // the lists strategy joins on parent rows: columns
+    S.packed = db->dev.nb != nullptr && wo_.extension == 0;
     active_++;
     order_.push_back(id);
     return id;
@@ -1348,6 +1403,9 @@ private:
     p.code.assign(nullptr, 0);
     p.cols.assign(nullptr, 0);
     p.last_col = -1;
+    p.gord = nullptr;
+    p.rows = nullptr;
+    p.nv = 0;
     p.list_blk = -1;
     p.list_off = nullptr;
     p.list_ent = nullptr;
@@ -1360,9 +1418,13 @@ private:
   // releases a node's columns and graph ranks
   void drop_node(JobState &S, PNode &p)
   {
-    S.live_bytes -= E.unref(p.last_col);
+    if(p.rows) {
+      S.live_bytes -= p.nrows * 16 * packed_planes(p.nv);
+    } else {
+      S.live_bytes -= E.unref(p.last_col);
+      S.live_bytes -= p.nrows * (int64_t)sizeof(int32_t);
+    }
     p.last_col = -1;
-    S.live_bytes -= p.nrows * (int64_t)sizeof(int32_t);
     E.block_unref(p.gord_blk);
     if(p.list_blk >= 0) E.block_unref(p.list_blk);
     p.list_blk = -1;
@@ -1502,8 +1564,7 @@ private:
     CK(cudaMemsetAsync(X.d_bm.p, 0, (size_t)bmw * 4, E.stream));
     CK(cudaMemsetAsync(X.d_cnt.p, 0, (size_t)cntn * 4, E.stream));
     CK(cudaEventRecord(X.ev[0], E.stream));
-    launch_root_count(d_rj, n, tiles, E.d_dbs.p, X.d_bm.p, X.d_cnt.p, X.d_sup.p + keys, keys, E.d_bytes.p + 2,
-                      E.stream);
+    launch_root_count(d_rj, n, tiles, E.d_dbs.p, X.d_bm.p, X.d_cnt.p, X.d_sup.p + keys, keys, E.stream);
     launch_support(d_nd, n, keys, X.d_bm.p, X.d_bmx.p, X.d_sup.p, E.stream);
     CK(cudaEventRecord(X.ev[1], E.stream));
     st_.launches += 3;
@@ -1554,7 +1615,8 @@ private:
           if(!extend) continue;
           const int64_t rows = hcnt[key];
           sel.push_back(Sel{ key, pid, pr.edge, sup, rows });
-          bytes += 2 * Carver::round((size_t)rows * 8) + Carver::round((size_t)rows * 4);
+          bytes += S.packed ? Carver::round((size_t)rows * 16)
+                            : 2 * Carver::round((size_t)rows * 8) + Carver::round((size_t)rows * 4);
         }
       }
       if(sel.empty()) continue;
@@ -1562,10 +1624,17 @@ private:
       const int32_t blk = E.new_block(bytes);
       Carver cv{ (char *)E.blocks[blk].base };
       for(const Sel &s : sel) {
-        int2 *c1 = cv.take<int2>(s.n);
-        int2 *c0 = cv.take<int2>(s.n);
-        int32_t *gord = cv.take<int32_t>(s.n);
-        ChildOut o{ c1, c0, gord, 2, (int32_t)s.n };
+        ChildOut o{};
+        o.cap = (int32_t)s.n;
+        o.kind = 2;
+        if(S.packed) {
+          o.rows = cv.take<uint4>(s.n);
+          o.planes = 1;
+        } else {
+          o.col = cv.take<int2>(s.n);
+          o.col0 = cv.take<int2>(s.n);
+          o.gord = cv.take<int32_t>(s.n);
+        }
         X.h_childmap.p[s.key] = (int32_t)outs.size();
         outs.push_back(o);
         const int32_t nid = pn_new();
@@ -1573,16 +1642,22 @@ private:
         nn.job = id;
         nn.pattern = s.pid;
         nn.code.push_back(s.d);
-        const int32_t id0 = E.new_col(c0, s.n, blk, -1);
-        nn.last_col = E.new_col(c1, s.n, blk, id0, true);
-        nn.cols.push_back(ColRef{ c0, s.n });
-        nn.cols.push_back(ColRef{ c1, s.n });
-        nn.gord = gord;
+        nn.nv = 2;
+        if(S.packed) {
+          nn.rows = o.rows;
+          S.live_bytes += s.n * 16;
+        } else {
+          const int32_t id0 = E.new_col(o.col0, s.n, blk, -1);
+          nn.last_col = E.new_col(o.col, s.n, blk, id0, true);
+          nn.cols.push_back(ColRef{ o.col0, s.n });
+          nn.cols.push_back(ColRef{ o.col, s.n });
+          nn.gord = o.gord;
+          S.live_bytes += s.n * (int64_t)(2 * sizeof(int2) + sizeof(int32_t));
+        }
         nn.gord_blk = blk;
         E.block_ref(blk);
         nn.nrows = s.n;
         nn.support = s.sup;
-        S.live_bytes += s.n * (int64_t)(2 * sizeof(int2) + sizeof(int32_t));
         made[q].push_back(nid);
       }
       S.peak_bytes = std::max(S.peak_bytes, S.live_bytes);
@@ -1695,9 +1770,13 @@ private:
     nodes.clear();
     int64_t rows = 0, words = 0, wkeys = 0;
     bool full = false;
+    int format = -1;  // a wave's nodes all have packed rows or all have columns
     for(size_t oi = 0; oi < order_.size() && !full; oi++) {
       JobState &S = *jobs_[order_[oi]];
       const Database &db = *S.job.db;
+      if(S.stack.empty()) continue;
+      if(format < 0) format = S.packed ? 1 : 0;
+      if(format != (S.packed ? 1 : 0)) continue;
       while(!S.stack.empty() && (int64_t)nodes.size() < limit) {
         const PNode &top = pn_[S.stack.back()];
         if(lays.size() <= nodes.size()) lays.emplace_back();
@@ -1737,8 +1816,9 @@ private:
       any_join = any_join || p.list_off != nullptr;
     }
     size_t off = 0;
-    size_t need = 256 * 7 + sizeof(NodeDesc) * W + sizeof(int2 *) * tot_cols + sizeof(SlotDesc) * tot_slots +
-                  2 * sizeof(int32_t) * tot_cols + 5 * sizeof(int32_t) * tot_edges;
+    const bool packed = format == 1;
+    size_t need = 256 * 8 + sizeof(NodeDesc) * W + sizeof(int2 *) * tot_cols + sizeof(SlotDesc) * tot_slots +
+                  2 * sizeof(int32_t) * tot_cols + 5 * sizeof(int32_t) * tot_edges + sizeof(int32_t) * W;
     X.h_desc.ensure(need);
     X.d_desc.ensure(need);
     char *hb = X.h_desc.p;
@@ -1748,14 +1828,16 @@ private:
     int32_t *hv = carve<int32_t>(hb, off, tot_cols);
     int32_t *hl = carve<int32_t>(hb, off, tot_cols);
     int32_t *hcode = carve<int32_t>(hb, off, 5 * (size_t)tot_edges);
+    int32_t *ht = carve<int32_t>(hb, off, packed ? W : 0);
     const size_t desc_bytes = off;
+    int32_t planes = 1;
     int32_t eo = 0;
     int32_t co = 0, so = 0, kmax = 1;
     bool small = true;  // every database of the wave has graphs of <= 64 vertices
     // adjacency bytes (entries and pair indices) of the wave's databases
     int64_t adj_bytes = 0;
     db_seen_.assign(dbs_.size(), 0);
-    int64_t rb = 0, bb = 0, tb = 0;
+    int64_t bb = 0, tb = 0;
     int32_t kb = 0;
     for(int32_t n = 0; n < W; n++) {
       const PNode &p = pn_[nodes[n]];
@@ -1764,12 +1846,11 @@ private:
       const Database &db = *S.job.db;
       NodeDesc &d = hn[n];
       d = NodeDesc{};
-      d.row_begin = rb;
       d.tile_begin = tb;
       d.bm_base = bb;
       d.gord = p.gord;
       d.nrows = (int32_t)p.nrows;
-      d.k = (int32_t)p.cols.size();
+      d.k = packed ? p.nv : (int32_t)p.cols.size();
       d.col_off = co;
       d.slot_off = so;
       d.vtab_off = co;
@@ -1808,9 +1889,26 @@ private:
       }
       for(size_t s = 0; s < L.slots.size(); s++) {
         hs[so + s] = L.slots[s];
-        if(L.slots[s].bkey_off >= 0) hv[co + L.slots[s].vertex] = (int32_t)s;
+        if(L.slots[s].bkey_off < 0) continue;
+        if(packed) d.back = 1;
+        else hv[co + L.slots[s].vertex] = (int32_t)s;
       }
-      co += d.k;
+      if(packed) {
+        ht[n] = (int32_t)tb;
+        d.rows = p.rows;
+        d.nb = db.dev.nb;
+        d.pair_code = db.dev.pair_code;
+        d.nb_blocks = db.dev.nb_blocks;
+        d.nb_shift = db.dev.nb_shift;
+        d.n_vertices = db.dev.n_vertices;
+        d.planes = packed_planes(p.nv);
+        planes = std::max(planes, d.planes);
+        // algorithmic bytes: the row and one neighbour block per slot (an
+        // extension's bitmap word, counter and record are added with the results)
+        st_.count_bytes += p.nrows * (16 * d.planes + 32 * d.nslot);
+      } else {
+        co += d.k;
+      }
       so += d.nslot;
       kmax = std::max(kmax, d.k);
       small = small && db.dev.max_graph_vertices <= 64;
@@ -1818,7 +1916,6 @@ private:
         db_seen_[S.db_slot] = 1;
         adj_bytes += 12 * db.n_adj();
       }
-      rb += p.nrows;
       tb += (p.nrows + 31) / 32;
       bb += (int64_t)d.nkeys * d.words;
       kb += d.nkeys;
@@ -1830,6 +1927,10 @@ private:
     f.ds = (const SlotDesc *)(db_ + ((char *)hs - hb));
     f.dv = (const int32_t *)(db_ + ((char *)hv - hb));
     f.dl = (const int32_t *)(db_ + ((char *)hl - hb));
+    f.dt = (const int32_t *)(db_ + ((char *)ht - hb));
+    f.packed = packed;
+    f.planes = planes;
+    if(tb >= INT32_MAX) throw Error(ST_ERR_LIMIT, "a wave has 2^36 or more embedding rows");
     const int32_t *dcode = (const int32_t *)(db_ + ((char *)hcode - hb));
     f.join = any_join;
     f.W = W;
@@ -1849,10 +1950,12 @@ private:
     // node's few counters; copies spread them over L2 slices (summed by screening)
     // (records hold a key in 27 bits next to the copy: one copy beyond that)
     const int32_t ccopies =
-        kb >= (1 << 27) ? 1 : (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, ((int64_t)1 << 22) / std::max(kb, 1)));
+        kb >= (1 << 27) ? 1 : (int32_t)std::max<int64_t>(1, std::min<int64_t>(packed ? 4 : 16, ((int64_t)1 << 22) / std::max(kb, 1)));
     const long long cstride = (long long)Carver::round(sizeof(int32_t) * (size_t)std::max(kb, 1)) / 4;
     const size_t cnt_bytes = sizeof(int32_t) * (size_t)cstride * ccopies;
-    const size_t zero_bytes = cnt_bytes + sizeof(uint32_t) * (size_t)std::max<int64_t>(bb, 1);
+    // packed rows: the record regions' counters, behind the embedding counters
+    const size_t reg_bytes = packed ? sizeof(uint32_t) * kRecRegions * kRecRegionStride : 0;
+    const size_t zero_bytes = cnt_bytes + reg_bytes + sizeof(uint32_t) * (size_t)std::max<int64_t>(bb, 1);
     X.d_zero.ensure(zero_bytes);
     X.d_head.ensure(kHeadBytes + sizeof(int4) * (size_t)std::max(kb, 1));
     X.d_bmx.ensure(std::max<int64_t>(bb, 1));
@@ -1862,7 +1965,8 @@ private:
     int32_t *cnt = (int32_t *)X.d_zero.p;
     f.cnt = cnt;
     f.cstride = cstride;
-    f.bm = (uint32_t *)(X.d_zero.p + cnt_bytes);
+    f.reg = packed ? (uint32_t *)(X.d_zero.p + cnt_bytes) : nullptr;
+    f.bm = (uint32_t *)(X.d_zero.p + cnt_bytes + reg_bytes);
     unsigned long long *head = (unsigned long long *)X.d_head.p;
     int4 *sel = (int4 *)(X.d_head.p + kHeadBytes);
     // records: how many the wave appends is not known up front, so keep the
@@ -1886,6 +1990,12 @@ private:
       if(X.d_rec.cap == 0) X.d_rec.ensure((size_t)1 << 22);
       f.rec = X.d_rec.p;
       f.rec_cap = (long long)X.d_rec.cap;
+      if(packed) {
+        // blocks of 32 four-byte items (128 bytes) behind their headers
+        f.rec_cap /= kRecBlockInt4 * kRecRegions;
+        f.hdr = X.d_rec.p;
+        f.rec = X.d_rec.p + f.rec_cap * kRecRegions;
+      }
     }
     // the frequent candidates come back compacted: a prefix sized from earlier
     // waves, the rest (rarely) by a second copy
@@ -1900,7 +2010,11 @@ private:
     q.head = X.d_head.p;
     q.head_host = X.h_head.p;
     q.d2h_bytes = kHeadBytes + sizeof(int4) * (size_t)f.sel_copied;
-    q.count = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
+    if(packed)
+      q.count = rows_count_call(f.dn, f.dt, W, (int32_t)tb, planes, f.ds, f.bm, cnt, ccopies, cstride,
+                                (uint32_t *)f.rec, f.hdr, (int32_t)f.rec_cap, f.reg, err_flag(), wo_.count_grid);
+    else
+      q.count = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
                               err_flag(), f.rec, f.rec_cap, f.rec ? head + kHeadRecords : nullptr,
                               wo_.count_grid, ccopies, cstride, f.join, f.rule_skip);
     int32_t *lnode = nullptr;
@@ -1909,7 +2023,8 @@ private:
       lnode = X.d_lnode.p;
     }
     q.screen = screen_keys_call(f.dn, W, kb, cnt, ccopies, cstride, X.d_childmap.p, X.d_listed.p,
-                                head + kHeadSelected, err_flag(), head + kHeadFlags, lnode);
+                                head + kHeadSelected, err_flag(), head + kHeadFlags, lnode,
+                                f.rec ? f.reg : nullptr, head + kHeadRecords);
     q.listed = count_listed_call(f.dn, X.d_listed.p, f.bm, cnt, X.d_bmx.p, X.d_keyword.p, sel, kb,
                                  head + kHeadSelected, lnode);
     q.with_min = wo_.min_check == 0;
@@ -1972,7 +2087,7 @@ private:
     st_.sel_bytes += (int64_t)hh[kHeadSelBytes];
     // the count kernel's bytes per extension (bitmap word and counter, and the
     // record when records are on), counted here rather than in its inner loop
-    st_.count_bytes += (int64_t)hh[kHeadExt] * (8 + (f.rec ? 16 : 0));
+    st_.count_bytes += (int64_t)hh[kHeadExt] * (8 + (f.rec ? (f.packed ? 4 : 16) : 0));
     if(nsel > kb) throw Error(ST_ERR_STATE, "candidate selection overflow");
     if(nsel > f.sel_copied) {
       // copies the whole list again (growing the pinned buffer drops its
@@ -2104,7 +2219,9 @@ private:
           if(child_edges >= kMaxPatternEdges || (cd.dfs.is_forward() && cd.dfs.to + 1 > 64))
             throw Error(ST_ERR_LIMIT, "pattern exceeds 64 vertices or 127 edges");
           mats.push_back(Mat{ n, ci, pid });
-          bytes += Carver::round((size_t)cd.cnt * 8) + Carver::round((size_t)cd.cnt * 4);
+          bytes += f.packed ? Carver::round((size_t)cd.cnt * 16 *
+                                            packed_planes(p.nv + (cd.dfs.is_forward() ? 1 : 0)))
+                            : Carver::round((size_t)cd.cnt * 8) + Carver::round((size_t)cd.cnt * 4);
         }
         a0 = a1;
       }
@@ -2146,9 +2263,21 @@ private:
           PNode &p = pn_[nodes[m.node]];
           JobState &S = *jobs_[p.job];
           const int64_t rowsn = cd.cnt;
-          int2 *col = cv.take<int2>(rowsn);
-          int32_t *gord = cv.take<int32_t>(rowsn);
-          ChildOut o{ col, nullptr, gord, cd.dfs.is_forward() ? 0 : 1, (int32_t)rowsn };
+          ChildOut o{};
+          o.cap = (int32_t)rowsn;
+          o.kind = cd.dfs.is_forward() ? 0 : 1;
+          const int32_t nv = p.nv + (cd.dfs.is_forward() ? 1 : 0);
+          if(f.packed) {
+            // algorithmic bytes of a child row: its parent's, the rank's bitmap
+            // word and prefix, the row written
+            st_.mat_bytes += rowsn * (16 * packed_planes(p.nv) + 8 + 16 * packed_planes(nv));
+            o.planes = packed_planes(nv);
+            o.rows = cv.take<uint4>((size_t)rowsn * o.planes);
+            o.word = hn[m.node].bm_base + (int64_t)cd.key * hn[m.node].words;
+          } else {
+            o.col = cv.take<int2>(rowsn);
+            o.gord = cv.take<int32_t>(rowsn);
+          }
           pairs.push_back(make_int2(hn[m.node].key_base + cd.key, (int32_t)outs.size()));
           outs.push_back(o);
           const int32_t nid = pn_new();
@@ -2158,13 +2287,20 @@ private:
           nn.code.reserve(p.code.size() + 1);
           nn.code.assign(p.code.data(), p.code.size());
           nn.code.push_back(cd.dfs);
-          // forward children append a column, backward children replace the last
-          const size_t keep = cd.dfs.is_forward() ? p.cols.size() : p.cols.size() - 1;
-          nn.cols.reserve(keep + 1);
-          nn.cols.assign(p.cols.data(), keep);
-          nn.cols.push_back(ColRef{ col, rowsn });
-          nn.last_col = E.new_col(col, rowsn, blk, cd.dfs.is_forward() ? p.last_col : E.cols[p.last_col].parent);
-          nn.gord = gord;
+          nn.nv = nv;
+          if(f.packed) {
+            nn.rows = o.rows;
+            S.live_bytes += rowsn * 16 * o.planes;
+          } else {
+            // forward children append a column, backward children replace the last
+            const size_t keep = cd.dfs.is_forward() ? p.cols.size() : p.cols.size() - 1;
+            nn.cols.reserve(keep + 1);
+            nn.cols.assign(p.cols.data(), keep);
+            nn.cols.push_back(ColRef{ o.col, rowsn });
+            nn.last_col = E.new_col(o.col, rowsn, blk, cd.dfs.is_forward() ? p.last_col : E.cols[p.last_col].parent);
+            nn.gord = o.gord;
+            S.live_bytes += rowsn * (int64_t)(sizeof(int2) + sizeof(int32_t));
+          }
           nn.gord_blk = blk;
           E.block_ref(blk);
           nn.nrows = rowsn;
@@ -2191,7 +2327,6 @@ private:
               }
             }
           }
-          S.live_bytes += rowsn * (int64_t)(sizeof(int2) + sizeof(int32_t));
           S.peak_bytes = std::max(S.peak_bytes, S.live_bytes);
           made.push_back(nid);
         }
@@ -2199,6 +2334,8 @@ private:
       for(int32_t n = 0; n < W; n++) made_at[n + 1] += made_at[n];
     }
     if(!outs.empty()) {
+      // an item and its child map entry per extension
+      if(f.packed) st_.mat_bytes += 8 * (int64_t)hh[kHeadExt];
       // one upload: children's outputs, then the (key, child) pairs
       const size_t outs_bytes = Carver::round(sizeof(ChildOut) * outs.size());
       const size_t pairs_bytes = Carver::round(sizeof(int2) * pairs.size());
@@ -2217,7 +2354,17 @@ private:
       // lists strategy: the records pass also counts the list rows
       ListBuild lb{ X.d_lnode.p, f.dn, (const int32_t *)(X.d_mat.p + outs_bytes + pairs_bytes) };
       if(list_blk >= 0) CK(cudaMemsetAsync(list_off, 0, sizeof(int32_t) * (size_t)(list_rows + 1), st));
-      if(f.rec && nrec <= f.rec_cap) {
+      if(f.packed) {
+        if(f.rec && nrec <= f.rec_cap) {
+          launch_rows_records((const uint32_t *)f.rec, f.hdr, f.reg, (int32_t)f.rec_cap, (int32_t)nrec, f.planes,
+                              f.dn, X.d_childmap.p, f.bm, X.d_bmx.p, f.cnt, f.cstride, douts, err_flag(), st);
+        } else {
+          launch_rows_materialize(f.dn, f.dt, W, (int32_t)f.tb, f.planes, f.ds, f.bm, X.d_bmx.p, X.d_childmap.p,
+                                  X.d_cursor.p, douts, err_flag(), st);
+          if(f.rec)
+            X.wanted_rec = std::max<long long>(X.wanted_rec, (nrec + nrec / 4) * kRecBlockInt4 * kRecRegions);
+        }
+      } else if(f.rec && nrec <= f.rec_cap) {
         // record-driven: one thread per extension record, no graph access
         launch_materialize_records(f.rec, nrec, X.d_childmap.p, X.d_keyword.p, f.bm, X.d_bmx.p, f.cnt, f.cstride,
                                    douts, E.d_bytes.p + 1, err_flag(), list_blk >= 0 ? &lb : nullptr,
@@ -2377,7 +2524,7 @@ int run_jobs_split(std::vector<MineJob> &batch, const MineOptions &wave_opt, Min
   for(auto &j : jobs)
     if(!j.db->resident) {
       j.db->upload();
-      st.h2d_bytes += (int64_t)j.db->d_bytes;
+      st.h2d_bytes += (int64_t)j.db->h2d_bytes;
     }
   std::vector<int32_t> order(jobs.size());
   for(size_t i = 0; i < jobs.size(); i++) order[i] = (int32_t)i;

@@ -706,9 +706,22 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
   const size_t o_ap = o_vb + al(sizeof(int32_t) * (G + 1));
   const size_t o_pc = o_ap + al(sizeof(int32_t) * (E2 + 1));
   const size_t o_in = o_pc + al(sizeof(int32_t) * (nkeys + 1));
-  const size_t total = o_in + al(sizeof(unsigned long long) * (E2 + 1));
+  // neighbour blocks (packed rows)
+  const int32_t nb_shift = packed_shift(mxv, VL, EL, nkeys);
+  int64_t nb_blocks = nb_shift ? packed_blocks(V, E2) : 0;
+  if(nb_blocks >= INT32_MAX) nb_blocks = 0;
+  const size_t o_nu = o_in + al(sizeof(unsigned long long) * (E2 + 1));
+  const size_t o_nb = o_nu + al(sizeof(int32_t));
+  size_t total = o_nb + al(32 * (size_t)nb_blocks);
   char *b = nullptr;
-  if(cudaMallocFromPoolAsync((void **)&b, total, cx.pool, s) != cudaSuccess) {
+  if(nb_blocks > 0 && cudaMallocFromPoolAsync((void **)&b, total, cx.pool, s) != cudaSuccess) {
+    // without room for them the database is mined on columns
+    cudaGetLastError();
+    b = nullptr;
+    nb_blocks = 0;
+    total = o_nb;
+  }
+  if(!b && cudaMallocFromPoolAsync((void **)&b, total, cx.pool, s) != cudaSuccess) {
     cudaGetLastError();
     throw Error(ST_ERR_NOMEM, "device ingest: out of device memory");
   }
@@ -728,6 +741,19 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
     CK(cudaMemcpyAsync(b + o_vg, vgraph, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, s));
     CK(cudaMemcpyAsync(b + o_gb, vgbase, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, s));
     k_narrow<<<blocks_for(G + 1), kThreads, 0, s>>>(vbase, G + 1, (int32_t *)(b + o_vb));
+    DevDB nbd{};
+    if(nb_blocks > 0) {
+      nbd.adj = (const unsigned long long *)(b + o_adj);
+      nbd.adj_off = off;
+      nbd.adj_pair = (const int32_t *)(b + o_ap);
+      nbd.vgbase = vgbase;
+      nbd.n_vertices = (int32_t)V;
+      nbd.nb_shift = nb_shift;
+      nbd.nb_blocks = (int32_t)nb_blocks;
+      CK(cudaMemsetAsync(b + o_nu, 0, sizeof(int32_t), s));
+      launch_neighbour_blocks(nbd, (uint4 *)(b + o_nb), (int32_t *)(b + o_nu), s);
+      nbd.nb = (const uint4 *)(b + o_nb);
+    }
     // host metadata (label values, each label's first pair, the pair codes), one read-back
     int32_t *hm = cx.meta_buf((size_t)(nvl + nel + VL + nkeys + 1));
     int32_t *h_vof = hm, *h_eof = hm + nvl, *hro = hm + nvl + nel, *hpc = hro + VL;
@@ -762,6 +788,7 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
       db.pair_cnt[a] = end - hro[a];
     }
     db.root_keys = (int32_t)nkeys;
+    db.index_pairs();
     db.d_block = b;
     db.pooled = true;
     db.d_bytes = total;
@@ -783,6 +810,9 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
     db.dev.n_vertices = (int32_t)V;
     db.dev.root_off = ro;
     db.dev.pair_code = pc;
+    db.dev.nb = nbd.nb;
+    db.dev.nb_blocks = nbd.nb_blocks;
+    db.dev.nb_shift = nbd.nb_shift;
     db.d_root_off = ro;
     db.resident = true;
     db.device_only = true;

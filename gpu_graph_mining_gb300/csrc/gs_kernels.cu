@@ -38,14 +38,6 @@ __device__ __forceinline__ int find_node_by_key(const NodeDesc *nodes, int n, in
   return lo;
 }
 
-__device__ __forceinline__ void add_bytes(unsigned long long *bytes, unsigned long long mine)
-{
-  if(!bytes) return;
-  // warp-reduce, one atomic per warp
-  for(int o = 16; o > 0; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
-  if((threadIdx.x & 31) == 0 && mine) atomicAdd(bytes, mine);
-}
-
 __device__ __forceinline__ unsigned lanemask_lt()
 {
   unsigned m;
@@ -68,12 +60,11 @@ __device__ __forceinline__ void root_tiles(const RootJob *__restrict__ jobs, int
                                            const DevDB *__restrict__ dbs, uint32_t *bm,
                                            const int32_t *__restrict__ bmx, int32_t *cnt,
                                            const int32_t *__restrict__ childmap, const ChildOut *__restrict__ outs,
-                                           unsigned long long *bytes, unsigned int *err)
+                                           unsigned int *err)
 {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  unsigned long long mine = 0;
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int jn = 0;  // a warp's tiles ascend, so its job index only moves forward
   for(long long tile = gw; tile < tiles; tile += nwarps) {
@@ -87,6 +78,7 @@ __device__ __forceinline__ void root_tiles(const RootJob *__restrict__ jobs, int
     const int32_t *__restrict__ vgraph = dbs[J.db].vgraph;
     const int32_t *__restrict__ adj_pair = dbs[J.db].adj_pair;
     const int32_t *__restrict__ root_off = dbs[J.db].root_off;
+    const int32_t *__restrict__ vgbase = dbs[J.db].vgbase;
     const int n_vertices = dbs[J.db].n_vertices;
     // this warp's copy of the job's root counters (copies spread the hot
     // counters over L2 slices)
@@ -107,7 +99,6 @@ __device__ __forceinline__ void root_tiles(const RootJob *__restrict__ jobs, int
     }
     const int off = incl - W;
     const int T = __shfl_sync(full, incl, 31);
-    if(valid) mine += 16;
     for(int base = 0; base < T; base += 32) {
       const int j = base + lane;
       const bool has = j < T;
@@ -129,14 +120,10 @@ __device__ __forceinline__ void root_tiles(const RootJob *__restrict__ jobs, int
         w = (int)(unsigned)(ent & 0xffffffffull);
         const unsigned hi = (unsigned)(ent >> 32);
         const int wl = (int)(hi & 0xffffu);
-        mine += 8;
         if(fl_o <= wl) key = ro + pr;
       }
       if(!MAT) {
-        if(key >= 0) {
-          atomicOr(&bm[J.bm_base + (long long)key * J.words + (g_o >> 5)], 1u << (g_o & 31));
-          mine += 8;
-        }
+        if(key >= 0) atomicOr(&bm[J.bm_base + (long long)key * J.words + (g_o >> 5)], 1u << (g_o & 31));
         const unsigned peers = __match_any_sync(full, key);
         if(key >= 0 && lane == __ffs(peers) - 1) atomicAdd(&cnt_copy[key], __popc(peers));
       } else {
@@ -152,7 +139,11 @@ __device__ __forceinline__ void root_tiles(const RootJob *__restrict__ jobs, int
           const long long wi = J.bm_base + (long long)key * J.words + (g_o >> 5);
           const int rank = bmx[wi] + __popc(bm[wi] & ((1u << (g_o & 31)) - 1u));
           const ChildOut out = outs[c];
-          if(pos < out.cap) {
+          if(pos < out.cap && out.rows) {
+            // a packed row of two vertices
+            const int gb = __ldg(&vgbase[vt + o]);
+            out.rows[pos] = make_uint4((unsigned)gb, (unsigned)rank, (unsigned)(vt + o - gb) | ((unsigned)(w - gb) << 8), 0u);
+          } else if(pos < out.cap) {
             out.col0[pos] = make_int2((int)(vt + o), -1);
             out.col[pos] = make_int2(w, pos);
             out.gord[pos] = rank;
@@ -163,14 +154,12 @@ __device__ __forceinline__ void root_tiles(const RootJob *__restrict__ jobs, int
       }
     }
   }
-  if(!MAT) add_bytes(bytes, mine);
 }
 
 __global__ void __launch_bounds__(kBlock) k_root_count(const RootJob *__restrict__ jobs, int njobs, long long tiles,
-                                                        const DevDB *__restrict__ dbs, uint32_t *bm, int32_t *cnt,
-                                                        unsigned long long *bytes)
+                                                        const DevDB *__restrict__ dbs, uint32_t *bm, int32_t *cnt)
 {
-  root_tiles<false>(jobs, njobs, tiles, dbs, bm, nullptr, cnt, nullptr, nullptr, bytes, nullptr);
+  root_tiles<false>(jobs, njobs, tiles, dbs, bm, nullptr, cnt, nullptr, nullptr, nullptr);
 }
 
 // Per key of the group, one warp: the job's counter copies turn into the
@@ -214,7 +203,7 @@ __global__ void __launch_bounds__(kBlock) k_root_materialize(const RootJob *__re
                                                               const int32_t *__restrict__ childmap,
                                                               const ChildOut *__restrict__ outs, unsigned int *err)
 {
-  root_tiles<true>(jobs, njobs, tiles, dbs, const_cast<uint32_t *>(bm), bmx, cursor, childmap, outs, nullptr, err);
+  root_tiles<true>(jobs, njobs, tiles, dbs, const_cast<uint32_t *>(bm), bmx, cursor, childmap, outs, err);
 }
 
 __global__ void __launch_bounds__(kBlock) k_support(const NodeDesc *__restrict__ nodes, int nnodes, int total_keys,
@@ -258,7 +247,8 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
                                                          long long cnt_stride, int32_t *childmap, int2 *listed,
                                                          unsigned long long *counters,
                                                          unsigned int *err, unsigned long long *err_copy,
-                                                         int32_t *lnode)
+                                                         int32_t *lnode, const uint32_t *reg,
+                                                         unsigned long long *reg_max)
 {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -267,6 +257,12 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
   // the consistency flags so far (the count pass has finished) travel back
   // with the wave's results
   if(blockIdx.x == 0 && threadIdx.x == 0) *err_copy = *err;
+  if(reg && blockIdx.x == 0 && threadIdx.x < 32) {
+    uint32_t most = 0;
+    for(int r = lane; r < kRecRegions; r += 32) most = max(most, reg[r * kRecRegionStride]);
+    most = __reduce_max_sync(full, most);
+    if(lane == 0) *reg_max = most;
+  }
   // warp-uniform trip count: the list append below is warp-aggregated
   const long long n32 = ((long long)total_keys + 31) & ~31ll;
   for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n32; i += stride) {
@@ -326,8 +322,21 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
     ext += __shfl_down_sync(full, ext, o);
     bytes += __shfl_down_sync(full, bytes, o);
   }
-  if(lane == 0 && ext) atomicAdd(&counters[1], ext);
-  if(lane == 0 && bytes) atomicAdd(&counters[3], bytes);
+  // one add per block: adds to one address complete one after another
+  __shared__ unsigned long long wext[kBlock / 32], wbytes[kBlock / 32];
+  if(lane == 0) {
+    wext[threadIdx.x >> 5] = ext;
+    wbytes[threadIdx.x >> 5] = bytes;
+  }
+  __syncthreads();
+  if(threadIdx.x == 0) {
+    for(int w = 1; w < kBlock / 32; w++) {
+      ext += wext[w];
+      bytes += wbytes[w];
+    }
+    if(ext) atomicAdd(&counters[1], ext);
+    if(bytes) atomicAdd(&counters[3], bytes);
+  }
 }
 
 // A listed key's support: its bitmap words popcounted, their exclusive
@@ -569,9 +578,9 @@ inline int grid_for(long long n)
 }  // namespace
 
 void launch_root_count(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs, uint32_t *bm,
-                       int32_t *cnt, int32_t *tot, int32_t total_keys, unsigned long long *bytes, cudaStream_t s)
+                       int32_t *cnt, int32_t *tot, int32_t total_keys, cudaStream_t s)
 {
-  if(tiles > 0) k_root_count<<<grid_for(tiles * 32), kBlock, 0, s>>>(jobs, njobs, tiles, dbs, bm, cnt, bytes);
+  if(tiles > 0) k_root_count<<<grid_for(tiles * 32), kBlock, 0, s>>>(jobs, njobs, tiles, dbs, bm, cnt);
   if(total_keys > 0)
     k_sum_copies<<<grid_for((long long)total_keys * 32), kBlock, 0, s>>>(jobs, njobs, total_keys, cnt, tot);
 }
@@ -597,7 +606,7 @@ void launch_records_bitmap(const int32_t *keys, const int32_t *gids, long long n
 KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, int32_t *cnt,
                             int32_t cnt_copies, long long cnt_stride, int32_t *childmap, int2 *listed,
                             unsigned long long *counters, unsigned int *err, unsigned long long *err_copy,
-                            int32_t *lnode)
+                            int32_t *lnode, const uint32_t *reg, unsigned long long *reg_max)
 {
   KernelCall c;
   c.func = (const void *)k_screen_keys;
@@ -615,6 +624,8 @@ KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total
   c.arg(err);
   c.arg(err_copy);
   c.arg(lnode);
+  c.arg(reg);
+  c.arg(reg_max);
   return c;
 }
 

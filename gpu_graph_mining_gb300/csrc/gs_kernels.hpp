@@ -63,7 +63,7 @@ private:
 // copy q >= 1 = the count of copies 0..q-1 and copy 0 = 0 (the materialise
 // pass's cursors).  tiles = the group's warp tiles; total_keys = its keys.
 void launch_root_count(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs, uint32_t *bm,
-                       int32_t *cnt, int32_t *tot, int32_t total_keys, unsigned long long *bytes, cudaStream_t s);
+                       int32_t *cnt, int32_t *tot, int32_t total_keys, cudaStream_t s);
 // Writes the two columns and graph ranks of every selected root key of the
 // group (childmap over the group's keys), with the counter copies as cursors.
 void launch_root_materialize(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs,
@@ -92,6 +92,30 @@ void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long to
                              unsigned long long *bytes, unsigned int *err, bool join, bool rule_skip,
                              cudaStream_t s);
 
+// Packed rows (gs_rows.cu).  tile0[] = first 32-row tile of each node; planes =
+// the most planes of the wave's nodes' rows; rec / hdr: record blocks (rec may
+// be null) in kRecRegions regions of blk_cap blocks, reg[r * kRecRegionStride]
+// counts the blocks reserved in region r (zeroed before).
+constexpr int kRecRegions = 64, kRecRegionStride = 32;
+KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
+                           int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, int32_t cnt_copies,
+                           long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
+                           unsigned int *err, int32_t grid_per_sm);
+// Materialise by enumerating again, and from the record blocks (cursor and
+// cursor_stride as for launch_materialize_records).
+void launch_rows_materialize(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
+                             int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
+                             const int32_t *childmap, int32_t *cursor, const ChildOut *outs, unsigned int *err,
+                             cudaStream_t s);
+// most: the most blocks of a region
+void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *reg, int32_t blk_cap, int32_t most,
+                         int32_t planes, const NodeDesc *nodes, const int32_t *childmap, const uint32_t *bm,
+                         const int32_t *bmx, int32_t *cursor, long long cursor_stride, const ChildOut *outs,
+                         unsigned int *err, cudaStream_t s);
+// Fills a database's neighbour blocks from its adjacency (db.nb_blocks,
+// db.nb_shift set; *used zeroed: receives the continuation blocks).
+void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStream_t s);
+
 // Materialise from the count pass's records {wave key, x, y, graph rank}:
 // children whose key is selected get column element (x, y) and their graph
 // rank.  keyword[key] = the key's first support-bitmap word.
@@ -117,10 +141,11 @@ void launch_records_bitmap(const int32_t *keys, const int32_t *gids, long long n
 // counting; listed and sel hold total_keys entries.  *err_copy = *err (the
 // consistency flags after the count pass).
 // lnode (lists strategy, may be null): reset to -1 for every key with extensions
+// reg (packed rows, may be null): *reg_max = the most record blocks of a region
 KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, int32_t *cnt,
                             int32_t cnt_copies, long long cnt_stride, int32_t *childmap, int2 *listed,
                             unsigned long long *counters, unsigned int *err, unsigned long long *err_copy,
-                            int32_t *lnode);
+                            int32_t *lnode, const uint32_t *reg, unsigned long long *reg_max);
 // lnode (lists strategy, may be null): lnode[key] = the key's node for every
 // frequent forward key
 KernelCall count_listed_call(const NodeDesc *nodes, const int2 *listed, const uint32_t *bm, int32_t *cnt,

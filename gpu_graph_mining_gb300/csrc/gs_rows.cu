@@ -1,0 +1,658 @@
+// Extension kernels for packed rows (gs_device.hpp): count (support bitmaps,
+// embedding counts, extension records) and materialise (children's rows), for
+// one wave of DFS-tree nodes.  Same rules and results as the column kernels
+// (gs_wave.cu), which serve graphs of more than 64 vertices, label alphabets
+// too large for the 4-byte entries and the lists strategy.
+//
+// What the format is for: on columns a row cost a chain of k dependent 8-byte
+// loads (a sector each), then two offsets and about 21 bytes of entries per
+// right-most-path vertex, and every step of 32 entries searched owners and
+// emitted few extensions.  250,000 graphs of 40 edges at minsup 0.5% (192 M
+// rows, 760 M extensions, one stream): count kernels 33.3 ms on columns, 12.4
+// here; a large launch 1.30 -> 0.46 ms with 989 M -> 402 M warp instructions
+// and 2.2 -> 0.9 GB of DRAM traffic.  It is bound by issue now (71% of
+// cycles, the integer pipe 69%; 0.24 of the DRAM peak).
+#include "gs_kernels.hpp"
+
+namespace gsgb {
+
+namespace {
+
+#ifndef GS_ROWS_WARPS
+#define GS_ROWS_WARPS 4
+#endif
+#ifndef GS_ROWS_MINB
+#define GS_ROWS_MINB 8
+#endif
+#ifndef GS_ROWS_GRID
+#define GS_ROWS_GRID 64
+#endif
+constexpr int kWarps = GS_ROWS_WARPS;
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kRecBlocks = 4;  // record blocks a warp reserves at a time
+
+struct RowsArgs {
+  const NodeDesc *nodes;
+  const int32_t *tile0;   // first 32-row tile of each node
+  int nnodes;
+  int total_tiles;
+  const SlotDesc *slots;
+  uint32_t *bm;           // count: bitmaps to set; materialise: read
+  const int32_t *bmx;     // materialise: prefix popcounts
+  int32_t *cnt;           // count: embeddings per key, cnt_copies copies cnt_stride apart
+  int cnt_copies;
+  long long cnt_stride;
+  const int32_t *childmap;  // materialise
+  int32_t *cursor;
+  const ChildOut *outs;
+  uint32_t *rec;          // count, optional: record blocks
+  int4 *hdr;
+  int blk_cap;            // blocks of one region
+  uint32_t *reg;          // blocks reserved in each region (may exceed blk_cap: none past it are written)
+  unsigned int *err;
+};
+
+// One warp's shared memory; the right-most path has at most as many slots as
+// the rows have pattern vertices.
+template <int PL> struct RowsSmem {
+  static constexpr int kSlots = PL == 1 ? 8 : PL == 2 ? 24 : 64;
+  uint2 q[32 * 9];      // accepted items waiting for emission (31 and one block per lane):
+                        // {entry, or backward key << 11; owner row | slot << 5 | kBackItem}
+  int4 slot[kSlots];    // {least entry allowed, key of entry 1 << shift, pattern vertex, backward keys or -1}
+  int2 slotb[kSlots];   // {least backward edge label, first pair code}
+  long long bm_base;    // the tile's node, for emission
+  int words, key_base;
+};
+
+__device__ __forceinline__ unsigned lanemask_lt()
+{
+  unsigned m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
+
+constexpr unsigned kBackItem = 1u << 11;
+
+// Inclusive warp sum.
+__device__ __forceinline__ int warp_incl(int x)
+{
+#pragma unroll
+  for(int o = 1; o < 32; o <<= 1)
+    asm volatile("{ .reg .s32 t; .reg .pred p; shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff; @p add.s32 %0, %0, t; }"
+                 : "+r"(x)
+                 : "r"(o));
+  return x;
+}
+
+// Graph-local id of pattern vertex t (the words' unused bytes are 0).
+template <int NW> __device__ __forceinline__ unsigned id_of(const unsigned (&w)[NW], int t)
+{
+  unsigned x = w[0];
+#pragma unroll
+  for(int q = 1; q < NW; q++) x = (t >> 2) == q ? w[q] : x;
+  return (x >> ((t & 3) * 8)) & 0xffu;
+}
+
+// The packed-row part of a child's outputs (two 16-byte loads).
+struct RowsOut {
+  uint4 *rows;
+  long long word;
+  int cap, kind, planes;
+};
+__device__ __forceinline__ RowsOut load_out(const ChildOut *o)
+{
+  const int4 *p = reinterpret_cast<const int4 *>(o);
+  const int4 x = __ldg(p), y = __ldg(p + 1);
+  RowsOut r;
+  r.rows = reinterpret_cast<uint4 *>(((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x);
+  r.word = (long long)(((unsigned long long)(unsigned)x.w << 32) | (unsigned)x.z);
+  r.cap = y.x;
+  r.kind = y.y;
+  r.planes = y.z;
+  return r;
+}
+
+// A child's row: its parent's ids, and for a forward child the new vertex lv
+// as pattern vertex k.
+template <int PL, int NW>
+__device__ __forceinline__ void store_row(const RowsOut &out, int pos, int gb, int rank, unsigned (&w)[NW], int k,
+                                          unsigned lv)
+{
+  if(out.kind == 0) {
+#pragma unroll
+    for(int q = 0; q < NW; q++)
+      if((k >> 2) == q) w[q] |= lv << ((k & 3) * 8);
+  }
+  out.rows[pos] = make_uint4((unsigned)gb, (unsigned)rank, w[0], w[1]);
+#pragma unroll
+  for(int p = 1; p < PL; p++)
+    if(p < out.planes)
+      out.rows[(long long)p * out.cap + pos] = make_uint4(w[4 * p - 2], w[4 * p - 1], w[4 * p], w[4 * p + 1]);
+  // the new vertex is the first of a plane that no row of the wave has
+  if(PL < 5 && out.planes > PL) out.rows[(long long)PL * out.cap + pos] = make_uint4(lv, 0, 0, 0);
+}
+
+// Work layout.  A warp owns a tile of 32 rows of one node, a row per lane: one
+// 16-byte load (per plane) gives the whole embedding.  The right-most path is
+// taken slot by slot; a lane's neighbour block is one aligned 32-byte sector,
+// loaded while the slot before is decided, and its 8 entries are tested in
+// registers: the forward rule and the empty entries are one compare, the
+// embedding is a 64-bit set.  Accepted entries go, ranked by a warp scan, to a
+// queue in shared memory, from which full batches of 32 are emitted: one
+// counter add per distinct key, one bitmap OR per (key, graph), and the batch
+// itself as a record block.
+template <int PL, bool MAT>
+__global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_rows(const RowsArgs a)
+{
+  constexpr int NW = 2 + 4 * (PL - 1);
+  __shared__ RowsSmem<PL> smem[kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  RowsSmem<PL> &S = smem[warp];
+  const int gwarp = blockIdx.x * kWarps + warp, nwarps = gridDim.x * kWarps;
+  const int copy = gwarp % (a.cnt_copies > 0 ? a.cnt_copies : 1);
+  // the warp's reserved record blocks, and (lane 0) those reserved ahead: a
+  // reservation made at the start of a tile arrives while its rows are loaded.
+  // The warps reserve from kRecRegions counters on as many cache lines: adds
+  // to one address complete at about one per 1.6 ns, which bounded the kernel
+  // when one counter served all warps.
+  const int region = gwarp % kRecRegions;
+  int blk = 0, blk_left = 0, blk_next = 0;  // within the region
+  bool ahead = false;
+  auto reserve = [&] {
+    if(lane == 0) blk_next = (int)min(atomicAdd(&a.reg[region * kRecRegionStride], (unsigned)kRecBlocks), 0x7fffff00u);
+    ahead = true;
+  };
+
+  for(int tile = gwarp; tile < a.total_tiles; tile += nwarps) {
+    // ---- the tile's node (tiles never span nodes): a 32-way search
+    int lo = 0, hi = a.nnodes;  // the node is the last in [lo, hi) with tile0 <= tile
+    while(hi - lo > 1) {
+      const int step = (hi - lo + 31) >> 5;
+      const int probe = lo + lane * step;
+      const unsigned ok = __ballot_sync(kFull, probe < hi && __ldg(&a.tile0[probe]) <= tile);
+      lo += (31 - __clz(ok | 1u)) * step;
+      hi = min(hi, lo + step);
+    }
+    const int n = lo;
+    if(!MAT && a.rec && blk_left < kRecBlocks && !ahead) reserve();
+    const NodeDesc &nd = a.nodes[n];
+    const int k = nd.k, nslot = nd.nslot, sh = nd.nb_shift;
+    if(k > RowsSmem<PL>::kSlots || nslot > RowsSmem<PL>::kSlots || k < 2 || nslot < 2 || nd.planes > PL) {
+      if(lane == 0) atomicOr(a.err, 2u);
+      continue;
+    }
+    const int row0 = (tile - __ldg(&a.tile0[n])) * 32;
+    const int i = row0 + lane;
+    bool valid = i < nd.nrows;
+    unsigned w[NW];
+#pragma unroll
+    for(int q = 0; q < NW; q++) w[q] = 0;
+    int gb = 0, g = 0;
+    if(valid) {
+      const uint4 r = __ldg(&nd.rows[i]);
+      gb = (int)r.x;
+      g = (int)r.y;
+      w[0] = r.z;
+      w[1] = r.w;
+#pragma unroll
+      for(int p = 1; p < PL; p++)
+        if(p < nd.planes) {
+          const uint4 x = __ldg(&nd.rows[(long long)p * nd.nrows + i]);
+          w[4 * p - 2] = x.x;
+          w[4 * p - 1] = x.y;
+          w[4 * p] = x.z;
+          w[4 * p + 1] = x.w;
+        }
+    }
+    __syncwarp();  // the previous tile's reads of the tables are done
+    for(int t = lane; t < nslot; t += 32) {
+      const SlotDesc &sd = a.slots[nd.slot_off + t];
+      S.slot[t] = make_int4(sd.prule, sd.fkey_off - 1, sd.vertex, sd.bkey_off);
+      S.slotb[t] = make_int2(sd.bmin, sd.pbase);
+    }
+    if(lane == 0) {
+      S.bm_base = nd.bm_base;
+      S.words = nd.words;
+      S.key_base = nd.key_base;
+    }
+    if(valid && (unsigned)g >= (unsigned)nd.words * 32u) {
+      atomicOr(a.err, 1u);
+      valid = false;
+    }
+    if(valid && (unsigned)gb >= (unsigned)nd.n_vertices) {
+      atomicOr(a.err, 2u);
+      valid = false;
+    }
+    unsigned long long mask = 0;  // the row's vertices
+    if(PL == 1) {
+#pragma unroll
+      for(int t = 0; t < 8; t++)
+        if(t < k) mask |= 1ull << ((w[t >> 2] >> ((t & 3) * 8)) & 63u);
+    } else {
+      for(int t = 0; t < k; t++) mask |= 1ull << (id_of(w, t) & 63u);
+    }
+    __syncwarp();
+    const bool back = nd.back != 0;
+    const uint4 *__restrict__ nb = nd.nb;
+    const unsigned wlm = (1u << sh) - 64u;           // the label field
+    const unsigned minl = (unsigned)nd.minlabel << 6;  // forward targets: label >= minlabel
+
+    uint4 xa = make_uint4(0, 0, 0, 0), xb = xa;
+    auto fetch = [&](int s) {
+      if(valid) {
+        const long long v = (long long)gb + id_of(w, S.slot[s].z);
+        xa = __ldg(&nb[2 * v]);
+        xb = __ldg(&nb[2 * v + 1]);
+      }
+    };
+    int s_n = 0, qn = 0, hops = 0;
+    fetch(0);
+    bool more = true;
+    while(more) {
+      const int s = s_n;
+      const unsigned x[8] = { xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w };
+      // the next blocks: continuations of this slot's lists, then the next slot
+      const unsigned cont = __ballot_sync(kFull, (int)x[7] < 0);
+      if(cont && hops < 16) {  // (a list of 63 entries has 9 blocks)
+        hops++;
+        const unsigned b = x[7] & 0x7fffffffu;
+        const bool ok = (int)x[7] < 0 && b < (unsigned)nd.nb_blocks;
+        xa = xb = make_uint4(0, 0, 0, 0);
+        if(ok) {
+          xa = __ldg(&nb[2ll * b]);
+          xb = __ldg(&nb[2ll * b + 1]);
+        }
+      } else if(++s_n < nslot) {
+        hops = 0;
+        fetch(s_n);
+      } else {
+        more = false;
+      }
+      // ---- this block's entries that are forward extensions
+      const int4 sl = S.slot[s];
+      unsigned acc = 0;
+      if(minl == 0) {
+#pragma unroll
+        for(int u = 0; u < 8; u++)
+          acc |= (int)x[u] >= sl.x && !((unsigned)(mask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
+      } else {
+#pragma unroll
+        for(int u = 0; u < 8; u++)
+          acc |= (int)x[u] >= sl.x && (x[u] & wlm) >= minl && !((unsigned)(mask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
+      }
+      const int c = __popc(acc);
+      const int incl = warp_incl(c);
+      uint2 *at = S.q + (qn + incl - c);
+      qn += __shfl_sync(kFull, incl, 31);
+      const unsigned meta = (unsigned)lane | ((unsigned)s << 5);
+#pragma unroll
+      for(int u = 0; u < 8; u++)
+        if((acc >> u) & 1u) *at++ = make_uint2(x[u], meta);
+      // ---- backward edges from the right-most vertex: entries whose vertex is
+      // a right-most-path vertex of the row that takes one (not accepted above,
+      // so the queue has room: 8 items per lane behind 31)
+      if(back && s == nslot - 1) {
+        unsigned long long bmask = 0;  // the row's vertices that a backward edge may go to
+        for(int t = 0; t + 2 < nslot; t++)
+          if(S.slot[t].w >= 0) bmask |= 1ull << (id_of(w, S.slot[t].z) & 63u);
+        unsigned bb = 0;
+#pragma unroll
+        for(int u = 0; u < 8; u++)
+          bb |= (int)x[u] > 0 && ((unsigned)(bmask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
+        while(__ballot_sync(kFull, bb != 0)) {
+          unsigned item = 0;
+          bool ok = false;
+          if(bb) {
+            const int u = __ffs(bb) - 1;
+            unsigned y = x[0];
+#pragma unroll
+            for(int q = 1; q < 8; q++) y = u == q ? x[q] : y;
+            bb &= bb - 1;
+            const int el = __ldg(&nd.pair_code[S.slotb[s].y + (int)(y >> sh) - 1]) >> 16;
+            for(int t = 0; t + 2 < nslot; t++)
+              if(S.slot[t].w >= 0 && id_of(w, S.slot[t].z) == (y & 63u) && el >= S.slotb[t].x) {
+                item = (unsigned)(S.slot[t].w + el) << 11;
+                ok = true;
+              }
+          }
+          const unsigned m = __ballot_sync(kFull, ok);
+          if(ok) S.q[qn + __popc(m & lanemask_lt())] = make_uint2(item, (unsigned)lane | kBackItem);
+          qn += __popc(m);
+        }
+      }
+      // ---- emission, 32 queued items at a time (all that is left after the
+      // tile's last block), warp converged
+      while(qn >= 32 || (!more && qn > 0)) {
+        __syncwarp();
+        const int m = min(qn, 32);
+        unsigned it = 0;  // the record item: (key << 11) | (new vertex << 5) | row
+        if(lane < m) {
+          const uint2 e = S.q[qn - m + lane];
+          it = e.y & 31u;
+          if(e.y & kBackItem) it |= e.x;
+          else it |= ((unsigned)S.slot[e.y >> 5].y + (e.x >> sh)) << 11 | (e.x & 63u) << 5;
+        }
+        qn -= m;
+        __syncwarp();
+        const int key = lane < m ? (int)(it >> 11) : -1;
+        const int o = (int)(it & 31u);
+        const int g_o = __shfl_sync(kFull, g, o);
+        const int key_base = S.key_base;
+        if(!MAT) {
+          // one counter add per distinct key, into this warp's copy of the
+          // counters (copies spread a node's hot counters over L2 slices); one
+          // bitmap OR per distinct key unless a lane's graph differs from its key
+          // group leader's (a tile's rows mostly share a graph).  Their bytes and
+          // the items' are added on the host from the wave's extension total.
+          const unsigned peers = __match_any_sync(kFull, key);
+          const int leader = __ffs(peers) - 1;
+          const int g_lead = __shfl_sync(kFull, g_o, leader);
+          if(key >= 0 && (lane == leader || g_o != g_lead))
+            atomicOr(&a.bm[S.bm_base + (long long)key * S.words + (g_o >> 5)], 1u << (g_o & 31));
+          if(key >= 0 && lane == leader) atomicAdd(&a.cnt[copy * a.cnt_stride + key_base + key], __popc(peers));
+          if(a.rec) {
+            if(blk_left == 0) {
+              if(!ahead) reserve();
+              blk = __shfl_sync(kFull, blk_next, 0);
+              blk_left = kRecBlocks;
+              ahead = false;
+            }
+            if(blk < a.blk_cap) {  // past the region's end nothing is written
+              const long long b = (long long)region * a.blk_cap + blk;
+              a.rec[b * 32 + lane] = it;
+              if(lane == 0) a.hdr[b] = make_int4(row0, n, m | (copy << 8), key_base);
+            }
+            blk++;
+            blk_left--;
+          }
+        } else {
+          const int c = key >= 0 ? a.childmap[key_base + key] : -1;
+          const unsigned peers = __match_any_sync(kFull, c);
+          const int leader = __ffs(peers) - 1;
+          int pos = 0;
+          if(c >= 0 && lane == leader) pos = atomicAdd(&a.cursor[c], __popc(peers));
+          pos = __shfl_sync(kFull, pos, leader) + __popc(peers & lanemask_lt());
+          const int gb_o = __shfl_sync(kFull, gb, o);
+          unsigned wo[NW];
+#pragma unroll
+          for(int q = 0; q < NW; q++) wo[q] = __shfl_sync(kFull, w[q], o);
+          if(c >= 0) {
+            const RowsOut out = load_out(&a.outs[c]);
+            const long long wi = out.word + (g_o >> 5);
+            const int rank = a.bmx[wi] + __popc(a.bm[wi] & ((1u << (g_o & 31)) - 1u));
+            if(pos < out.cap) store_row<PL>(out, pos, gb_o, rank, wo, k, (it >> 5) & 63u);
+            else atomicOr(a.err, 4u);
+          }
+        }
+      }
+    }
+  }
+  // the reserved blocks that were not needed are empty
+  if(!MAT && a.rec) {
+    int4 *const hdr = a.hdr + (long long)region * a.blk_cap;
+    if(lane < blk_left && blk + lane < a.blk_cap) hdr[blk + lane] = make_int4(0, 0, 0, 0);
+    const int next = __shfl_sync(kFull, blk_next, 0);
+    if(ahead && lane < kRecBlocks && next + lane < a.blk_cap) hdr[next + lane] = make_int4(0, 0, 0, 0);
+  }
+}
+
+// Materialise from the record blocks: a warp takes kB blocks (each one tile of
+// one node) side by side, an item of each per lane.  A key's cursor copies
+// start where the counts of the copies before end.  The chain per item is
+// child map, child, bitmap word and cursor: several blocks per warp and the
+// next ones' items and child map entries loaded ahead keep it in flight.
+#ifndef GS_ROWS_MATB
+#define GS_ROWS_MATB 1
+#endif
+template <int PL, int kB>
+__global__ void __launch_bounds__(256) k_rows_mat(const uint32_t *__restrict__ rec, const int4 *__restrict__ hdr,
+                                                  const uint32_t *__restrict__ reg, int blk_cap, int nblk,
+                                                  const NodeDesc *__restrict__ nodes,
+                                                  const int32_t *__restrict__ childmap,
+                                                  const uint32_t *__restrict__ bm, const int32_t *__restrict__ bmx,
+                                                  int32_t *cursor, long long cursor_stride,
+                                                  const ChildOut *__restrict__ outs, unsigned int *err)
+{
+  constexpr int NW = 2 + 4 * (PL - 1);
+  const int lane = threadIdx.x & 31;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  // Block b is block b / kRecRegions of region b % kRecRegions; a warp stays in
+  // one region (nwarps is a multiple of their number).
+  const int b0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int region = b0 % kRecRegions;
+  const int used = min((int)min(__ldg(&reg[region * kRecRegionStride]), 0x7fffff00u), blk_cap);
+  int4 h1[kB];
+  unsigned it1[kB];
+  int c1[kB];
+  auto load = [&](int b) {
+#pragma unroll
+    for(int q = 0; q < kB; q++) {
+      h1[q] = make_int4(0, 0, 0, 0);
+      it1[q] = 0;
+      const int bq = b + q * nwarps, i = bq / kRecRegions;
+      if(bq < nblk && i < used) {
+        const long long at = (long long)region * blk_cap + i;
+        h1[q] = __ldg(&hdr[at]);
+        it1[q] = __ldg(&rec[at * 32 + lane]);
+      }
+    }
+  };
+  auto child = [&]() {
+#pragma unroll
+    for(int q = 0; q < kB; q++)
+      c1[q] = lane < (h1[q].z & 0xff) ? childmap[h1[q].w + (int)(it1[q] >> 11)] : -1;
+  };
+  load(b0);
+  child();
+  for(int b = b0; b < nblk; b += kB * nwarps) {
+    int4 h[kB];
+    unsigned it[kB];
+    int c[kB];
+    bool any = false;
+#pragma unroll
+    for(int q = 0; q < kB; q++) {
+      h[q] = h1[q];
+      it[q] = it1[q];
+      c[q] = c1[q];
+      any = any || c[q] >= 0;
+    }
+    load(b + kB * nwarps);
+    if(__ballot_sync(kFull, any)) {
+      RowsOut out[kB];
+      uint4 r[kB];
+      unsigned w[kB][NW];
+      int nrows[kB];
+#pragma unroll
+      for(int q = 0; q < kB; q++) {
+        out[q] = RowsOut{};
+        if(c[q] >= 0) out[q] = load_out(&outs[c[q]]);
+        // an empty block's header names node 0: its rows are not used
+        const NodeDesc &nd = nodes[h[q].y];
+        nrows[q] = nd.nrows;
+        const int row = h[q].x + lane;
+        r[q] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for(int t = 0; t < NW; t++) w[q][t] = 0;
+        if(row < nrows[q]) {
+          r[q] = __ldg(&nd.rows[row]);
+          w[q][0] = r[q].z;
+          w[q][1] = r[q].w;
+#pragma unroll
+          for(int p = 1; p < PL; p++)
+            if(p < nd.planes) {
+              const uint4 x = __ldg(&nd.rows[(long long)p * nrows[q] + row]);
+              w[q][4 * p - 2] = x.x;
+              w[q][4 * p - 1] = x.y;
+              w[q][4 * p] = x.z;
+              w[q][4 * p + 1] = x.w;
+            }
+        }
+      }
+      int gb[kB], g[kB], pos[kB], bpre[kB];
+      uint32_t bword[kB];
+#pragma unroll
+      for(int q = 0; q < kB; q++) {
+        const int o = (int)(it[q] & 31u);
+        gb[q] = (int)__shfl_sync(kFull, r[q].x, o);
+        g[q] = (int)__shfl_sync(kFull, r[q].y, o);
+#pragma unroll
+        for(int t = 0; t < NW; t++) w[q][t] = __shfl_sync(kFull, w[q][t], o);
+        // the bitmap word and its prefix are loaded before the cursor add, so
+        // that their latencies overlap
+        bword[q] = 0;
+        bpre[q] = 0;
+        if(c[q] >= 0) {
+          bword[q] = bm[out[q].word + (g[q] >> 5)];
+          bpre[q] = bmx[out[q].word + (g[q] >> 5)];
+        }
+        const unsigned peers = __match_any_sync(kFull, c[q]);
+        const int leader = __ffs(peers) - 1;
+        pos[q] = 0;
+        if(c[q] >= 0 && lane == leader)
+          pos[q] = atomicAdd(&cursor[(h[q].z >> 8) * cursor_stride + h[q].w + (int)(it[q] >> 11)], __popc(peers));
+        pos[q] = __shfl_sync(kFull, pos[q], leader) + __popc(peers & lanemask_lt());
+      }
+      child();
+#pragma unroll
+      for(int q = 0; q < kB; q++)
+        if(c[q] >= 0) {
+          const int rank = bpre[q] + __popc(bword[q] & ((1u << (g[q] & 31)) - 1u));
+          if(pos[q] < out[q].cap) store_row<PL>(out[q], pos[q], gb[q], rank, w[q], nodes[h[q].y].k, (it[q] >> 5) & 63u);
+          else atomicOr(err, 4u);
+        }
+    } else {
+      child();
+    }
+  }
+}
+
+// Neighbour blocks of a database (a thread per vertex, a warp's continuation
+// blocks reserved together).
+__global__ void __launch_bounds__(256) k_neighbour_blocks(const int32_t *__restrict__ adj_off, int V,
+                                                          const unsigned long long *__restrict__ adj,
+                                                          const int32_t *__restrict__ adj_pair,
+                                                          const int32_t *__restrict__ vgbase, int sh, uint4 *nb,
+                                                          int nb_blocks, int *used)
+{
+  const int lane = threadIdx.x & 31;
+  const int stride = gridDim.x * blockDim.x;
+  for(int v0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; v0 < V; v0 += stride) {
+    const int v = v0 + lane;
+    int a0 = 0, d = 0, gb = 0;
+    if(v < V) {
+      a0 = __ldg(&adj_off[v]);
+      d = __ldg(&adj_off[v + 1]) - a0;
+      gb = __ldg(&vgbase[v]);
+    }
+    // continuation blocks: 7 entries and a link each, up to 8 in the last
+    const int need = d <= 8 ? 0 : (d - 7 <= 8 ? 1 : 1 + (d - 7 - 8 + 6) / 7);
+    int incl = need;
+    for(int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(kFull, incl, o);
+      if(lane >= o) incl += t;
+    }
+    const int total = __shfl_sync(kFull, incl, 31);
+    int first = 0;
+    if(total > 0) {
+      if(lane == 0) first = V + atomicAdd(used, total);
+      first = __shfl_sync(kFull, first, 0) + incl - need;
+    }
+    if(v < V) {
+      int at = a0, left = d, next = first;
+      for(long long b = v;;) {
+        const bool link = left > 8;
+        const int here = link ? 7 : left;
+        unsigned x[8];
+#pragma unroll
+        for(int u = 0; u < 8; u++) {
+          x[u] = 0;
+          if(u < here) {
+            const unsigned long long e = __ldg(&adj[at + u]);
+            x[u] = ((unsigned)(__ldg(&adj_pair[at + u]) + 1) << sh) | ((unsigned)((e >> 32) & 0xffffu) << 6) |
+                   (((unsigned)e - (unsigned)gb) & 63u);
+          }
+        }
+        if(link) x[7] = 0x80000000u | (unsigned)next;
+        if(b < nb_blocks) {
+          nb[2 * b] = make_uint4(x[0], x[1], x[2], x[3]);
+          nb[2 * b + 1] = make_uint4(x[4], x[5], x[6], x[7]);
+        }
+        if(!link) break;
+        at += here;
+        left -= here;
+        b = next++;
+      }
+    }
+  }
+}
+
+template <int PL, bool MAT> KernelCall rows_call(const RowsArgs &a, int grid_per_sm)
+{
+  long long blocks = ((long long)a.total_tiles + kWarps - 1) / kWarps;
+  const long long cap = (long long)sm_count() * (grid_per_sm > 0 ? grid_per_sm : GS_ROWS_GRID);
+  blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
+  KernelCall c;
+  c.func = (const void *)k_rows<PL, MAT>;
+  c.grid = dim3((unsigned)blocks);
+  c.block = dim3(kWarps * 32);
+  c.arg(a);
+  return c;
+}
+
+}  // namespace
+
+KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
+                           int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, int32_t cnt_copies,
+                           long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
+                           unsigned int *err, int32_t grid_per_sm)
+{
+  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, bm, nullptr, cnt, cnt_copies, cnt_stride, nullptr,
+                    nullptr, nullptr, rec, hdr, blk_cap, reg, err };
+  if(planes <= 1) return rows_call<1, false>(a, grid_per_sm);
+  if(planes <= 2) return rows_call<2, false>(a, grid_per_sm);
+  return rows_call<5, false>(a, grid_per_sm);
+}
+
+void launch_rows_materialize(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
+                             int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
+                             const int32_t *childmap, int32_t *cursor, const ChildOut *outs, unsigned int *err,
+                             cudaStream_t s)
+{
+  if(total_tiles <= 0) return;
+  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, const_cast<uint32_t *>(bm), bmx, nullptr, 0, 0, childmap,
+                    cursor, outs, nullptr, nullptr, 0, nullptr, err };
+  KernelCall c = planes <= 1 ? rows_call<1, true>(a, 0) : planes <= 2 ? rows_call<2, true>(a, 0) : rows_call<5, true>(a, 0);
+  c.run(s);
+}
+
+void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *reg, int32_t blk_cap, int32_t most,
+                         int32_t planes, const NodeDesc *nodes, const int32_t *childmap, const uint32_t *bm,
+                         const int32_t *bmx, int32_t *cursor, long long cursor_stride, const ChildOut *outs,
+                         unsigned int *err, cudaStream_t s)
+{
+  if(most <= 0) return;
+  static_assert(kRecRegions % 8 == 0, "a block of 8 warps per 8 regions");
+  const int nblk = most * kRecRegions;
+  // a multiple of kRecRegions warps
+  const long long want = nblk / 8, cap = 32LL * sm_count() / (kRecRegions / 8) * (kRecRegions / 8);
+  const int blocks = (int)(want < cap ? want : cap);
+  if(planes <= 1)
+    k_rows_mat<1, GS_ROWS_MATB><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
+                                         cursor_stride, outs, err);
+  else if(planes <= 2)
+    k_rows_mat<2, 1><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
+                                         cursor_stride, outs, err);
+  else
+    k_rows_mat<5, 1><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
+                                         cursor_stride, outs, err);
+}
+
+void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStream_t s)
+{
+  if(db.n_vertices <= 0) return;
+  const long long want = ((long long)db.n_vertices + 255) / 256, cap = 64LL * sm_count();
+  k_neighbour_blocks<<<(int)(want < cap ? want : cap), 256, 0, s>>>(db.adj_off, db.n_vertices, db.adj, db.adj_pair,
+                                                                    db.vgbase, db.nb_shift, nb, db.nb_blocks, used);
+}
+
+}  // namespace gsgb

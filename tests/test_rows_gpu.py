@@ -1,0 +1,105 @@
+"""Packed rows (graphs of at most 64 vertices) against the oracle and against
+the column kernels: neighbour lists that end at and past their 8-entry blocks,
+databases on either side of the rule that chooses the row format, batches of
+both, and the re-enumerating materialise after a record overflow."""
+import random
+
+import pytest
+
+from conftest import run_oracle, to_lines
+
+pytestmark = pytest.mark.gpu
+
+
+def _write(path, graphs):
+    """graphs: (vertex labels, [(a, b, edge label)])"""
+    with open(path, "w") as f:
+        for i, (vl, edges) in enumerate(graphs):
+            f.write("t # %d\n" % i)
+            f.writelines("v %d %d\n" % x for x in enumerate(vl))
+            f.writelines("e %d %d %d\n" % e for e in edges)
+
+
+def _lines(gs, db, s, **kw):
+    return to_lines(gs.mine(db, s, label_style=gs.LABELS_SEQ, **kw)[0], gs)
+
+
+# a list of d entries: one block up to 8, then 7 and a continuation (8 again, or 7 and another)
+@pytest.mark.parametrize("degree", [1, 7, 8, 9, 15, 16, 22, 23, 62, 63])
+def test_list_lengths(gs, oracle, tmp_path, degree):
+    r = random.Random(degree)
+    graphs = []
+    for g in range(6):
+        # a hub with `degree` leaves and some edges between them; the leaves' labels decide
+        # where in the hub's sorted list an entry stands
+        vl = [0] + [r.randrange(1, 5) for _ in range(degree)]
+        edges = [(0, v, r.randrange(3)) for v in range(1, degree + 1)]
+        edges += [(v, v + 1, r.randrange(3)) for v in range(1, degree) if r.random() < 0.3]
+        graphs.append((vl, edges))
+    p = str(tmp_path / "hub.txt")
+    _write(p, graphs)
+    db = gs.Database.load(p, "txt")
+    want = run_oracle(oracle, "txt", p, 4, ["--max-edges", "3"])
+    assert _lines(gs, db, 4, max_edges=3) == want
+    # the same from host arrays converted on the device
+    q = str(tmp_path / "hub.cudabin")
+    db.write(q, "cudabin")
+    import numpy as np
+    raw = np.fromfile(q, dtype=np.int32)
+    n, esz, maxv = (int(x) for x in raw[:3])
+    cuts = np.cumsum([4, esz, esz, n * maxv, n * maxv + 1])
+    e, el, vl, vo = (raw[a:b] for a, b in zip(cuts[:-1], cuts[1:]))
+    dev = gs.Database.from_arrays(n, maxv, e, el, vl, vo, device=True)
+    assert _lines(gs, dev, 4, max_edges=3) == want
+
+
+def _random_graphs(r, count, nv, vlabels, elabels):
+    graphs = []
+    for _ in range(count):
+        n = r.randint(*nv)
+        edges = {(r.randrange(v), v) for v in range(1, n)}
+        for _ in range(n // 4):
+            a, b = sorted(r.sample(range(n), 2))
+            edges.add((a, b))
+        graphs.append(([r.randrange(vlabels) for _ in range(n)], [(a, b, r.randrange(elabels)) for a, b in sorted(edges)]))
+    return graphs
+
+
+# one label (no label bits), alphabets of powers of two and one more, and one whose label pairs
+# are too many for the 4-byte entries and items (mined on columns)
+@pytest.mark.parametrize("vlabels,elabels,count", [(1, 1, 30), (2, 4, 60), (32, 3, 200), (33, 3, 200), (300, 40, 2500)])
+def test_alphabets(gs, oracle, tmp_path, vlabels, elabels, count):
+    r = random.Random(vlabels)
+    p = str(tmp_path / "db.txt")
+    _write(p, _random_graphs(r, count, (3, 24), vlabels, elabels))
+    s = max(2, count // 10) if vlabels <= 33 else 3
+    want = run_oracle(oracle, "txt", p, s, ["--max-edges", "4"])
+    assert _lines(gs, gs.Database.load(p, "txt"), s, max_edges=4) == want
+
+
+def test_batch_of_both_formats(gs, tmp_path):
+    r = random.Random(3)
+    dbs = []
+    for i, nv in enumerate([(4, 20), (60, 64), (60, 90), (4, 30), (66, 70)]):
+        p = str(tmp_path / ("b%d.txt" % i))
+        _write(p, _random_graphs(r, 40, nv, 3, 2))
+        dbs.append(gs.Database.load(p, "txt"))
+    sups = [12, 25, 25, 10, 25]
+    got, _ = gs.mine_batch(dbs, sups, max_edges=4)
+    for db, s, pats in zip(dbs, sups, got):
+        assert pats == gs.mine(db, s, max_edges=4)[0]
+        # the lists strategy mines every database on columns
+        assert pats == gs.mine(db, s, max_edges=4, extension="lists")[0]
+
+
+def test_record_overflow(gs):
+    # the first waves of a fresh engine write more extension items than its
+    # record buffer holds (they are enumerated again); small waves never do
+    db = gs.Database.generate(5, scale=0.25)
+    s = int(0.01 * len(db))
+    gs.engine_reset()
+    first, _ = gs.mine_collect(db, s)
+    again, _ = gs.mine_collect(db, s)
+    small, _ = gs.mine_collect(db, s, wave_rows=1 << 20)
+    assert first == again == small
+    gs.engine_reset()
