@@ -172,4 +172,31 @@ struct alignas(16) ChildOut {
   int32_t *gord;  // the child's graph ranks
 };
 
+// A wave's (or root group's) results header, 8-byte words in device memory,
+// written to pinned host memory by the wave's last kernel.  The time stamps are
+// the device's nanosecond clock, taken by the first thread of a kernel: kernels
+// of one stream start when the one before has finished.
+enum HeadWord {
+  kHeadRecords = 0,   // extension records written by the count pass (packed rows: most blocks of a region)
+  kHeadFlags = 1,     // consistency flags
+  kHeadSelected = 2,  // selected candidates   } counters of
+  kHeadExt = 3,       // embeddings of all keys } the support
+  kHeadListed = 4,    // keys counted          } selection
+  kHeadSelBytes = 5,  // algorithmic bytes     }
+  kHeadDone = 6,      // blocks of the last kernel that have finished
+  kHeadCount0 = 7,    // stamps: count,
+  kHeadSel0 = 8,      //   selection,
+  kHeadMin0 = 9,      //   canonicality,
+  kHeadEnd = 10,      //   results written
+  kHeadBytesCount = 11,  // algorithmic bytes so far: column count and materialise kernels
+  kHeadBytesMat = 12,
+  kHeadMat = 13,      // per wave context, the stamps of its last materialise pass: start, end
+  kHeadSeq = 29,      // the wave's number, written last
+  kHeadWords = 32,
+};
+constexpr int kMaxWaveCtx = 8;
+// A context's materialise stamps: the start, and the ends of the blocks spread
+// over kMatSlots cache lines (their maximum is the end).
+constexpr int kMatSlots = 32, kMatStampWords = 16 * (kMatSlots + 1);
+
 }  // namespace gsgb

@@ -670,43 +670,22 @@ struct NodeLayout {
   std::vector<SlotDesc> slots;
 };
 
-// The device work of one wave up to its results copy: descriptor upload,
-// scratch clears, count, selection, canonicality, results download, with the
-// context's events between them.
+// The device work of one wave up to its results in host memory: tables in and
+// scratch cleared (begin), count, selection, canonicality and results out.
+constexpr int kWaveKernels = 5;
 struct WaveSeq {
-  void *desc_dst = nullptr;
-  const void *desc_src = nullptr;
   size_t desc_bytes = 0;
-  void *zero = nullptr;
-  size_t zero_bytes = 0;
-  void *head = nullptr;
-  void *head_host = nullptr;
-  size_t d2h_bytes = 0;
-  KernelCall count, screen, listed, ismin;
-  bool with_min = false;
+  KernelCall k[kWaveKernels];  // begin, count, screen, listed, is_min
 };
 
 // WaveSeq as an instantiated CUDA graph, one per count-kernel variant and
 // context: each wave updates the nodes' parameters and launches the graph.
 struct WaveGraph {
   const void *count_func = nullptr;
-  bool with_min = false;
   cudaGraph_t g = nullptr;
   cudaGraphExec_t x = nullptr;
-  cudaGraphNode_t h2d, mz, mh, count, screen, listed, ismin, d2h;
+  cudaGraphNode_t node[kWaveKernels];
 };
-
-inline cudaMemsetParams clear_params(void *dst, size_t bytes)
-{
-  cudaMemsetParams m{};
-  m.dst = dst;
-  m.pitch = 0;
-  m.value = 0;
-  m.elementSize = 1;
-  m.width = bytes;
-  m.height = 1;
-  return m;
-}
 
 inline cudaKernelNodeParams kernel_params(KernelCall &c)
 {
@@ -720,14 +699,7 @@ inline cudaKernelNodeParams kernel_params(KernelCall &c)
   return k;
 }
 
-// Header slots of a wave's results (unsigned long long each).
-constexpr int kHeadRecords = 0;   // extension records written by the count pass
-constexpr int kHeadFlags = 1;     // consistency flags after the count pass
-constexpr int kHeadSelected = 2;  // selected candidates   } counters of
-constexpr int kHeadExt = 3;       // embeddings of all keys } the support
-constexpr int kHeadListed = 4;    // keys counted          } selection
-constexpr int kHeadSelBytes = 5;  // algorithmic bytes     }
-constexpr size_t kHeadBytes = 64;
+constexpr size_t kHeadBytes = sizeof(unsigned long long) * kHeadWords;
 // A record block of packed rows in int4 units of the record buffer: 32 items
 // of 4 bytes and a 16-byte header.
 constexpr long long kRecBlockInt4 = 9;
@@ -744,15 +716,15 @@ struct WaveCtx {
   DBuf<unsigned long long> d_recn;
   DBuf<long long> d_keyword;
   DBuf<int32_t> d_lnode;   // lists strategy: the node of each frequent forward key
-  // A wave's results, copied back in one piece: a 64-byte header (kHead*
-  // slots) followed by the selected candidates {key, support, embeddings,
-  // node << 2 | verdict}.  The zeroed region holds the embedding counts and the support
+  // A wave's results, written to pinned host memory by its last kernel: the
+  // header (HeadWord) followed by the selected candidates {key, support,
+  // embeddings, node << 2 | verdict}.  The zeroed region holds the embedding counts and the support
   // bitmaps (one memset).  The child table holds the children's outputs and
   // (key, child) pairs (one upload).
   DBuf<char> d_head, d_zero, d_mat;
   HBuf<char> h_head, h_mat;
   DBuf<int2> d_listed;               // keys with enough embeddings to be counted
-  int64_t sel_hint = 4096;           // selected entries copied back with the wave's results
+  int64_t sel_hint = 4096;           // selected entries there is room for in the pinned results
   bool rec_enabled = true;
   long long wanted_rec = 0;    // record capacity to have before the next wave (after an overflow)
   // pinned host mirrors
@@ -760,44 +732,36 @@ struct WaveCtx {
   HBuf<int32_t> h_sup, h_cnt, h_childmap;
   HBuf<ChildOut> h_outs;
   HBuf<long long> h_keyword;
-  HBuf<unsigned long long> h_misc;  // [0] records written, [1] consistency flags, [2..3] = d_selc
-  // 0/1 count, 1/6 selection, 6/2 canonicality, 3 results copied, 4/5 materialise
-  // (the root context: 0/1 a group's count and support, 3 read back, 5 first
-  // embeddings)
-  cudaEvent_t ev[7] = {};
-  bool have_events = false;
+  cudaEvent_t ev_mat = nullptr;  // after the last materialise pass (the root context: after the first embeddings)
   std::vector<WaveGraph> graphs;
   // the context's stream (wave contexts; the root context uses the engine's)
   cudaStream_t stream = nullptr;
-  // records of ev[5] (materialise passes), and the records of the engine's
-  // ev_main and of the other contexts' ev[5] this context's stream already waits for
+  // records of ev_mat, and the records of the engine's ev_main and of the other
+  // contexts' ev_mat this context's stream already waits for
   uint64_t mat_gen = 0, seen_main = 0;
   uint64_t seen_mat[8] = {};
 
   void init(bool own_stream)
   {
-    if(!have_events) {
-      for(auto &e : ev) CK(cudaEventCreate(&e));
-      have_events = true;
-    }
+    if(!ev_mat) CK(cudaEventCreateWithFlags(&ev_mat, cudaEventDisableTiming));
     if(own_stream && !stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    h_misc.ensure(4);
   }
   void free()
   {
     d_desc.free(); d_bm.free(); d_bmx.free(); d_cnt.free(); d_sup.free(); d_childmap.free(); d_cursor.free();
     d_outs.free(); d_rec.free(); d_recn.free(); d_keyword.free(); d_listed.free(); d_lnode.free();
     d_head.free(); d_zero.free(); d_mat.free(); h_head.free(); h_mat.free();
-    h_desc.free(); h_sup.free(); h_cnt.free(); h_childmap.free(); h_outs.free(); h_keyword.free(); h_misc.free();
+    h_desc.free(); h_sup.free(); h_cnt.free(); h_childmap.free(); h_outs.free(); h_keyword.free();
     sel_hint = 4096;
     for(auto &g : graphs) {
       if(g.x) cudaGraphExecDestroy(g.x);
       if(g.g) cudaGraphDestroy(g.g);
     }
     graphs.clear();
-    if(have_events)
-      for(auto &e : ev) cudaEventDestroy(e);
-    have_events = false;
+    if(ev_mat) cudaEventDestroy(ev_mat);
+    ev_mat = nullptr;
+    mat_gen = seen_main = 0;
+    for(auto &m : seen_mat) m = 0;
     if(stream) {
       cudaStreamSynchronize(stream);
       cudaStreamDestroy(stream);
@@ -833,7 +797,7 @@ int64_t rule_skip_adj_bytes()
 #define GS_WAVE_CTX 3
 #endif
 constexpr int kWaveCtx = GS_WAVE_CTX;
-static_assert(kWaveCtx <= 8, "WaveCtx::seen_mat holds 8 contexts");
+static_assert(kWaveCtx <= kMaxWaveCtx, "WaveCtx::seen_mat and the header hold 8 contexts");
 
 struct Engine {
   // Streams: the engine's (database table, root phases) and one per wave
@@ -853,6 +817,10 @@ struct Engine {
   int64_t pool_limit = 0;
   DBuf<DevDB> d_dbs;
   DBuf<unsigned long long> d_bytes;   // [0] count bytes, [1] materialise bytes (column kernels), [3] flags
+  DBuf<unsigned long long> d_stamps;  // every wave context's materialise stamps
+  uint64_t seq = 0;                   // number of the last wave or root group
+  int64_t bytes_seen[2] = { 0, 0 };   // d_bytes[0..1] as last read
+  unsigned long long mat_counted[kWaveCtx] = {};  // start stamp of each context's last pass met in the statistics
   WaveCtx ctx[kWaveCtx];
   // root phases: the root level of a group of jobs, one launch per kernel
   WaveCtx rootx;
@@ -865,8 +833,8 @@ struct Engine {
   // are the materialise passes queued for its wave (the record-driven pass
   // reads records, the enumerating fallback the wave's columns); counts read
   // live nodes only, root phases write new blocks only.  Each context's
-  // event 5 follows its latest materialise pass, so when every context's
-  // event 5 has completed, every block released so far is free (a later
+  // ev_mat follows its latest materialise pass, so when every context's
+  // ev_mat has completed, every block released so far is free (a later
   // record of an event only makes the wait longer).
   std::vector<void *> released;
   uint64_t main_gen = 0;          // records of ev_main
@@ -879,10 +847,15 @@ struct Engine {
       CK(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
       CK(cudaEventCreateWithFlags(&ev_main, cudaEventDisableTiming));
       d_bytes.ensure(4);
+      d_stamps.ensure((size_t)kWaveCtx * kMatStampWords);
+      CK(cudaMemsetAsync(d_stamps.p, 0, sizeof(unsigned long long) * kWaveCtx * kMatStampWords, stream));
       d_dbs.ensure(kMaxDbSlots);
       CK(cudaMemsetAsync(d_bytes.p, 0, sizeof(unsigned long long) * 4, stream));
+      bytes_seen[0] = bytes_seen[1] = 0;
       for(auto &c : ctx) c.init(true);
       rootx.init(false);
+      CK(cudaStreamSynchronize(stream));
+      main_gen = 0;
       ready = true;
     }
     pool.set_limit(pool_limit);
@@ -902,6 +875,7 @@ struct Engine {
     pool.destroy();
     d_dbs.free();
     d_bytes.free();
+    d_stamps.free();
     for(auto &c : ctx) c.free();
     rootx.free();
     cudaStreamSynchronize(aux);
@@ -938,11 +912,11 @@ struct Engine {
   {
     if(released.empty()) return false;
     for(auto &c : ctx) {
-      if(!c.have_events) continue;
-      const cudaError_t q = cudaEventQuery(c.ev[5]);
+      if(!c.ev_mat) continue;
+      const cudaError_t q = cudaEventQuery(c.ev_mat);
       if(q == cudaErrorNotReady) {
         if(!wait) return false;
-        CK(cudaEventSynchronize(c.ev[5]));
+        CK(cudaEventSynchronize(c.ev_mat));
       } else {
         CK(q);
       }
@@ -1123,15 +1097,8 @@ template <class T> T *carve(char *base, size_t &off, size_t n)
   return p;
 }
 
-double ms_between(cudaEvent_t a, cudaEvent_t b)
-{
-  float ms = 0;
-  if(cudaEventElapsedTime(&ms, a, b) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return ms;
-}
+// milliseconds between two of the device's time stamps
+double ms_between(unsigned long long a, unsigned long long b) { return b > a ? 1e-6 * (double)(b - a) : 0.0; }
 
 // adds the wall time of a scope to a millisecond counter
 struct ScopeMs {
@@ -1148,7 +1115,6 @@ double ms_since(clk::time_point t0) { return std::chrono::duration<double, std::
 // One wave in flight: its nodes and where their descriptors live.
 struct Flight {
   bool busy = false;
-  bool mat_pending = false;  // the ctx's materialise events still to be read
   uint64_t seq = 0;
   std::vector<int32_t> nodes;  // node pool ids
   std::vector<NodeLayout> lays;
@@ -1170,7 +1136,9 @@ struct Flight {
   int64_t tb = 0;
   int4 *rec = nullptr;
   long long rec_cap = 0;
-  int64_t sel_copied = 0;    // selected entries copied back with the results
+  int64_t sel_copied = 0;    // selected entries there is room for with the results
+  uint64_t res_seq = 0;      // the results' sequence number
+  uint64_t main_gen = 0, mat_gen[kWaveCtx] = {};  // passes ahead of the wave when it was launched
   uint32_t *bm = nullptr;    // the wave's support bitmaps (in the zeroed region)
   int32_t *cnt = nullptr;    // its counter copies, cstride apart (cursors of the records materialise)
   long long cstride = 0;
@@ -1193,7 +1161,7 @@ public:
   {
     nctx_ = wo_.wave_nodes > 1 ? kWaveCtx : 1;
     E.pool.reset_peak();
-    CK(cudaMemsetAsync(E.d_bytes.p, 0, sizeof(unsigned long long) * 4, E.stream));
+    for(int i = 0; i < 2; i++) seen_bytes_[i] = E.bytes_seen[i];
   }
 
   // Validates the job, makes its database resident, mines its root level and
@@ -1312,29 +1280,35 @@ public:
     if(job(id) && jobs_[id]->done) jobs_[id].reset();
   }
 
-  // Waits for the last materialise passes and folds the device counters into
-  // the statistics; checks the kernels' consistency flags.
+  // Folds the device counters into the statistics and checks the kernels'
+  // consistency flags.  They came with the last wave's results when every
+  // materialise pass was ahead of it; otherwise the device is read.
   void sync_stats()
   {
-    for(int c = 0; c < nctx_; c++) {
-      if(fl_[c].mat_pending) {
-        CK(cudaEventSynchronize(E.ctx[c].ev[5]));
-        st_.mat_ms += ms_between(E.ctx[c].ev[4], E.ctx[c].ev[5]);
-        fl_[c].mat_pending = false;
+    bool seen = main_seen_ == E.main_gen;
+    for(int c = 0; c < kWaveCtx; c++) seen = seen && mat_seen_[c] == E.ctx[c].mat_gen;
+    if(!seen) {
+      for(auto &c : E.ctx) CK(cudaStreamSynchronize(c.stream));
+      // (on the engine's stream: its own passes are ahead)
+      unsigned long long bytes[4] = { 0, 0, 0, 0 };
+      std::vector<unsigned long long> st((size_t)kWaveCtx * kMatStampWords);
+      d2h(bytes, E.d_bytes.p, sizeof(bytes));
+      d2h(st.data(), E.d_stamps.p, sizeof(unsigned long long) * st.size());
+      CK(cudaStreamSynchronize(E.stream));
+      CK(cudaGetLastError());
+      check_flags(bytes[3]);
+      fold_bytes(bytes[0], bytes[1]);
+      for(int c = 0; c < kWaveCtx; c++) {
+        const unsigned long long *x = st.data() + (size_t)c * kMatStampWords;
+        unsigned long long end = 0;
+        for(int q = 1; q <= kMatSlots; q++) end = std::max(end, x[16 * q]);
+        fold_mat(c, x[0], end);
       }
+      main_seen_ = E.main_gen;
+      for(int c = 0; c < kWaveCtx; c++) mat_seen_[c] = E.ctx[c].mat_gen;
     }
-    // every context's passes done before the counters are read
-    for(auto &c : E.ctx) CK(cudaStreamSynchronize(c.stream));
-    unsigned long long bytes[4] = { 0, 0, 0, 0 };
-    d2h(bytes, E.d_bytes.p, sizeof(bytes));
-    CK(cudaStreamSynchronize(E.stream));
-    E.reap(false);
     CK(cudaGetLastError());
-    check_flags(bytes[3]);
-    st_.count_bytes += (int64_t)bytes[0] - seen_bytes_[0];
-    st_.mat_bytes += (int64_t)bytes[1] - seen_bytes_[1];
-    seen_bytes_[0] = (int64_t)bytes[0];
-    seen_bytes_[1] = (int64_t)bytes[1];
+    E.reap(false);
     st_.peak_pool_bytes = std::max<int64_t>(st_.peak_pool_bytes, (int64_t)E.pool.peak());
   }
 
@@ -1358,6 +1332,12 @@ private:
   int64_t active_ = 0;
   int64_t stacked_ = 0;          // nodes on all jobs' stacks
   int64_t seen_bytes_[2] = { 0, 0 };
+  // the engine's root phases and every context's materialise passes whose flags
+  // and byte counters have been read
+  uint64_t main_seen_ = 0, mat_seen_[kWaveCtx] = {};
+  // per context, the materialise pass whose time is being added up
+  unsigned long long mat_start_[kWaveCtx] = {};
+  double mat_ms_[kWaveCtx] = {};
   bool defer_emit_ = false;
   // per-wave scratch of finish(), reused
   struct Mat { int32_t node, cand, pid; };
@@ -1378,6 +1358,49 @@ private:
   {
     CK(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, s ? s : E.stream));
     st_.d2h_bytes += (int64_t)n;
+  }
+  // Waits until the results header's sequence word is seq: polls the pinned
+  // word, and the stream now and then for an error.
+  void wait_results(const volatile unsigned long long *hhead, uint64_t seq, cudaStream_t s)
+  {
+    const clk::time_point t0 = clk::now();
+    const unsigned long long *w = const_cast<const unsigned long long *>(hhead) + kHeadSeq;
+    double next = 0.2;
+    while(__atomic_load_n(w, __ATOMIC_ACQUIRE) != seq) {
+      for(int i = 0; i < 64 && __atomic_load_n(w, __ATOMIC_RELAXED) != seq; i++) {
+      }
+      if(ms_since(t0) < next) continue;
+      next = ms_since(t0) + 0.2;
+      const cudaError_t q = cudaStreamQuery(s);
+      if(q == cudaErrorNotReady) continue;
+      CK(q);
+      // finished: the word must be there
+      if(__atomic_load_n(w, __ATOMIC_ACQUIRE) != seq) throw Error(ST_ERR_STATE, "a wave ended without its results");
+    }
+    st_.host_wait_ms += ms_since(t0);
+  }
+  void fold_bytes(unsigned long long count, unsigned long long mat)
+  {
+    st_.count_bytes += (int64_t)count - seen_bytes_[0];
+    st_.mat_bytes += (int64_t)mat - seen_bytes_[1];
+    E.bytes_seen[0] = seen_bytes_[0] = (int64_t)count;
+    E.bytes_seen[1] = seen_bytes_[1] = (int64_t)mat;
+  }
+  // context c's materialise pass that began at `start` has lasted until `end`
+  // (a pass still running is added up as its blocks finish)
+  void fold_mat(int c, unsigned long long start, unsigned long long end)
+  {
+    if(start == 0 || E.ctx[c].mat_gen == 0) return;
+    if(mat_start_[c] != start) {
+      mat_start_[c] = start;
+      mat_ms_[c] = start == E.mat_counted[c] ? 1e300 : 0;  // (an earlier scheduler's pass)
+      E.mat_counted[c] = start;
+    }
+    const double ms = ms_between(start, end);
+    if(ms > mat_ms_[c]) {
+      st_.mat_ms += ms - mat_ms_[c];
+      mat_ms_[c] = ms;
+    }
   }
   // device consistency flags (slot 3 of the counters)
   unsigned int *err_flag() { return reinterpret_cast<unsigned int *>(E.d_bytes.p + 3); }
@@ -1537,54 +1560,46 @@ private:
   {
     WaveCtx &X = E.rootx;
     const int32_t n = (int32_t)rj.size();
-    // the pinned mirrors below were last read by the previous group's copies
-    CK(cudaEventSynchronize(X.ev[5]));
-    X.d_bm.ensure(bmw);
+    // the pinned mirrors below were last read by the previous group's kernels
+    CK(cudaEventSynchronize(X.ev_mat));
+    const size_t cnt_bytes = Carver::round((size_t)cntn * 4);
+    X.d_zero.ensure(cnt_bytes + Carver::round((size_t)bmw * 4));
+    int32_t *const cnt = (int32_t *)X.d_zero.p;
+    uint32_t *const bm = (uint32_t *)(X.d_zero.p + cnt_bytes);
     X.d_bmx.ensure(bmw);
-    X.d_cnt.ensure(cntn);
-    X.d_sup.ensure(2 * (size_t)keys);  // supports, then embeddings
-    X.d_childmap.ensure(keys);
-    // pseudo nodes spanning each job's root keys (for the support kernel), then the job table
-    const size_t nd_bytes = sizeof(NodeDesc) * n, tab_bytes = nd_bytes + sizeof(RootJob) * n;
+    const size_t res_n = (2 * (size_t)keys + 3) & ~(size_t)3;  // supports, then embeddings
+    X.d_sup.ensure(res_n);
+    X.h_sup.ensure(res_n);
+    X.d_head.ensure(kHeadBytes);
+    X.h_head.ensure(kHeadBytes);
+    // the job table, and the device table of the databases that joined
+    const size_t tab_bytes = Carver::round(sizeof(RootJob) * n);
     X.d_desc.ensure(tab_bytes);
     X.h_desc.ensure(tab_bytes);
-    NodeDesc *hn = (NodeDesc *)X.h_desc.p;
-    for(int32_t q = 0; q < n; q++) {
-      NodeDesc nd{};
-      nd.words = rj[q].words;
-      nd.nkeys = rj[q].R;
-      nd.key_base = rj[q].key_base;
-      nd.bm_base = rj[q].bm_base;
-      hn[q] = nd;
-    }
-    std::memcpy(X.h_desc.p + nd_bytes, rj.data(), sizeof(RootJob) * n);
-    h2d(X.d_desc.p, X.h_desc.p, tab_bytes);
-    const NodeDesc *d_nd = (const NodeDesc *)X.d_desc.p;
-    const RootJob *d_rj = (const RootJob *)(X.d_desc.p + nd_bytes);
-    CK(cudaMemsetAsync(X.d_bm.p, 0, (size_t)bmw * 4, E.stream));
-    CK(cudaMemsetAsync(X.d_cnt.p, 0, (size_t)cntn * 4, E.stream));
-    CK(cudaEventRecord(X.ev[0], E.stream));
-    launch_root_count(d_rj, n, tiles, E.d_dbs.p, X.d_bm.p, X.d_cnt.p, X.d_sup.p + keys, keys, E.stream);
-    launch_support(d_nd, n, keys, X.d_bm.p, X.d_bmx.p, X.d_sup.p, E.stream);
-    CK(cudaEventRecord(X.ev[1], E.stream));
-    st_.launches += 3;
-    X.h_sup.ensure(2 * (size_t)keys);
-    d2h(X.h_sup.p, X.d_sup.p, (size_t)keys * 8);
-    d2h(X.h_misc.p + 1, E.d_bytes.p + 3, sizeof(unsigned long long));
-    CK(cudaEventRecord(X.ev[3], E.stream));
-    {
-      const clk::time_point t0 = clk::now();
-      CK(cudaEventSynchronize(X.ev[3]));
-      st_.host_wait_ms += ms_since(t0);
-    }
+    std::memcpy(X.h_desc.p, rj.data(), sizeof(RootJob) * n);
+    st_.h2d_bytes += (int64_t)tab_bytes;
+    const RootJob *d_rj = (const RootJob *)X.d_desc.p;
+    unsigned long long *const head = (unsigned long long *)X.d_head.p;
+    const volatile unsigned long long *hh = (const volatile unsigned long long *)X.h_head.p;
+    const uint64_t seq = ++E.seq;
+    ((volatile unsigned long long *)X.h_head.p)[kHeadSeq] = 0;
+    KernelCall begin = begin_call(X.d_desc.p, X.h_desc.p, (long long)tab_bytes / 16, X.d_zero.p,
+                                  (long long)(cnt_bytes + Carver::round((size_t)bmw * 4)) / 16, head);
+    CK(begin.run(E.stream));
+    launch_root_count(d_rj, n, tiles, E.d_dbs.p, bm, cnt, head, E.stream);
+    launch_root_support(d_rj, n, keys, bm, X.d_bmx.p, cnt, X.d_sup.p, X.d_sup.p + keys, E.stream);
+    launch_results(X.h_sup.p, X.d_sup.p, (long long)res_n / 4, head, err_flag(), (unsigned long long *)X.h_head.p, seq,
+                   E.stream);
     CK(cudaGetLastError());
-    check_flags(X.h_misc.p[1]);
-    st_.root_ms += ms_between(X.ev[0], X.ev[1]);
+    st_.launches += 4;
+    st_.d2h_bytes += (int64_t)(res_n * 4 + kHeadBytes);
+    wait_results(hh, seq, E.stream);
+    check_flags(hh[kHeadFlags]);
+    st_.root_ms += ms_between(hh[kHeadCount0], hh[kHeadSel0]);
 
     std::vector<ChildOut> outs;
     std::vector<std::vector<int32_t>> made(n);
-    X.h_childmap.ensure(keys);
-    for(int32_t k = 0; k < keys; k++) X.h_childmap.p[k] = -1;
+    std::vector<int32_t> h_map((size_t)keys, -1);
     const int32_t *hsup = X.h_sup.p, *hcnt = X.h_sup.p + keys;
     for(int32_t q = 0; q < n; q++) {
       const int32_t id = gid[q];
@@ -1635,7 +1650,7 @@ private:
           o.col0 = cv.take<int2>(s.n);
           o.gord = cv.take<int32_t>(s.n);
         }
-        X.h_childmap.p[s.key] = (int32_t)outs.size();
+        h_map[s.key] = (int32_t)outs.size();
         outs.push_back(o);
         const int32_t nid = pn_new();
         PNode &nn = pn_[nid];
@@ -1663,17 +1678,24 @@ private:
       S.peak_bytes = std::max(S.peak_bytes, S.live_bytes);
     }
     if(!outs.empty()) {
-      X.d_outs.ensure(outs.size());
-      X.h_outs.ensure(outs.size());
-      std::memcpy(X.h_outs.p, outs.data(), sizeof(ChildOut) * outs.size());
-      h2d(X.d_outs.p, X.h_outs.p, sizeof(ChildOut) * outs.size());
-      h2d(X.d_childmap.p, X.h_childmap.p, (size_t)keys * 4);
+      // the children's outputs and the child map, copied by one kernel
+      const size_t outs_bytes = Carver::round(sizeof(ChildOut) * outs.size());
+      const size_t map_bytes = Carver::round((size_t)keys * 4);
+      X.d_mat.ensure(outs_bytes + map_bytes);
+      X.h_mat.ensure(outs_bytes + map_bytes);
+      std::memcpy(X.h_mat.p, outs.data(), sizeof(ChildOut) * outs.size());
+      std::memcpy(X.h_mat.p + outs_bytes, h_map.data(), (size_t)keys * 4);
+      st_.h2d_bytes += (int64_t)(outs_bytes + map_bytes);
+      KernelCall up = begin_call(X.d_mat.p, X.h_mat.p, (long long)(outs_bytes + map_bytes) / 16, nullptr, 0, head);
+      CK(up.run(E.stream));
       // cursors: the counter copies hold each copy's offset (copy 0 at 0)
-      launch_root_materialize(d_rj, n, tiles, E.d_dbs.p, X.d_bm.p, X.d_bmx.p, X.d_cnt.p, X.d_childmap.p, X.d_outs.p,
-                              err_flag(), E.stream);
-      st_.launches++;
+      launch_root_materialize(d_rj, n, tiles, E.d_dbs.p, bm, X.d_bmx.p, cnt,
+                              (const int32_t *)(X.d_mat.p + outs_bytes), (const ChildOut *)X.d_mat.p, err_flag(),
+                              E.stream);
+      CK(cudaGetLastError());
+      st_.launches += 2;
     }
-    CK(cudaEventRecord(X.ev[5], E.stream));
+    CK(cudaEventRecord(X.ev_mat, E.stream));
     for(int32_t q = 0; q < n; q++) {
       JobState &S = *jobs_[gid[q]];
       S.pending += (int64_t)made[q].size();
@@ -1688,68 +1710,28 @@ private:
   {
     const cudaStream_t st = cs(X);
     st_.h2d_bytes += (int64_t)q.desc_bytes;
-    st_.d2h_bytes += (int64_t)q.d2h_bytes;
     if(wo_.launch_mode != 0) {
-      CK(cudaMemcpyAsync(q.desc_dst, q.desc_src, q.desc_bytes, cudaMemcpyHostToDevice, st));
-      CK(cudaMemsetAsync(q.zero, 0, q.zero_bytes, st));
-      CK(cudaMemsetAsync(q.head, 0, kHeadBytes, st));
-      CK(cudaEventRecord(X.ev[0], st));
-      CK(q.count.run(st));
-      CK(cudaEventRecord(X.ev[1], st));
-      CK(q.screen.run(st));
-      CK(q.listed.run(st));
-      CK(cudaEventRecord(X.ev[6], st));
-      if(q.with_min) CK(q.ismin.run(st));
-      CK(cudaEventRecord(X.ev[2], st));
-      CK(cudaMemcpyAsync(q.head_host, q.head, q.d2h_bytes, cudaMemcpyDeviceToHost, st));
-      CK(cudaEventRecord(X.ev[3], st));
+      for(auto &k : q.k) CK(k.run(st));
       return;
     }
     WaveGraph *G = nullptr;
     for(auto &g : X.graphs)
-      if(g.count_func == q.count.func && g.with_min == q.with_min) G = &g;
-    const cudaMemsetParams mz = clear_params(q.zero, q.zero_bytes), mh = clear_params(q.head, kHeadBytes);
-    cudaKernelNodeParams kc = kernel_params(q.count), ks = kernel_params(q.screen), kl = kernel_params(q.listed);
-    cudaKernelNodeParams km{};
-    if(q.with_min) km = kernel_params(q.ismin);
+      if(g.count_func == q.k[1].func) G = &g;
     if(!G) {
       X.graphs.emplace_back();
       G = &X.graphs.back();
-      G->count_func = q.count.func;
-      G->with_min = q.with_min;
-      cudaGraph_t g;
-      CK(cudaGraphCreate(&g, 0));
-      G->g = g;
-      cudaGraphNode_t e0, e1, e2, e3, e6, last;
-      CK(cudaGraphAddMemcpyNode1D(&G->h2d, g, nullptr, 0, q.desc_dst, q.desc_src, q.desc_bytes,
-                                  cudaMemcpyHostToDevice));
-      CK(cudaGraphAddMemsetNode(&G->mz, g, &G->h2d, 1, &mz));
-      CK(cudaGraphAddMemsetNode(&G->mh, g, &G->mz, 1, &mh));
-      CK(cudaGraphAddEventRecordNode(&e0, g, &G->mh, 1, X.ev[0]));
-      CK(cudaGraphAddKernelNode(&G->count, g, &e0, 1, &kc));
-      CK(cudaGraphAddEventRecordNode(&e1, g, &G->count, 1, X.ev[1]));
-      CK(cudaGraphAddKernelNode(&G->screen, g, &e1, 1, &ks));
-      CK(cudaGraphAddKernelNode(&G->listed, g, &G->screen, 1, &kl));
-      CK(cudaGraphAddEventRecordNode(&e6, g, &G->listed, 1, X.ev[6]));
-      last = e6;
-      if(q.with_min) {
-        CK(cudaGraphAddKernelNode(&G->ismin, g, &last, 1, &km));
-        last = G->ismin;
+      G->count_func = q.k[1].func;
+      CK(cudaGraphCreate(&G->g, 0));
+      for(int i = 0; i < kWaveKernels; i++) {
+        const cudaKernelNodeParams kp = kernel_params(q.k[i]);
+        CK(cudaGraphAddKernelNode(&G->node[i], G->g, i ? &G->node[i - 1] : nullptr, i ? 1 : 0, &kp));
       }
-      CK(cudaGraphAddEventRecordNode(&e2, g, &last, 1, X.ev[2]));
-      CK(cudaGraphAddMemcpyNode1D(&G->d2h, g, &e2, 1, q.head_host, q.head, q.d2h_bytes, cudaMemcpyDeviceToHost));
-      CK(cudaGraphAddEventRecordNode(&e3, g, &G->d2h, 1, X.ev[3]));
-      CK(cudaGraphInstantiate(&G->x, g, 0));
+      CK(cudaGraphInstantiate(&G->x, G->g, 0));
     } else {
-      CK(cudaGraphExecMemcpyNodeSetParams1D(G->x, G->h2d, q.desc_dst, q.desc_src, q.desc_bytes,
-                                            cudaMemcpyHostToDevice));
-      CK(cudaGraphExecMemsetNodeSetParams(G->x, G->mz, &mz));
-      CK(cudaGraphExecMemsetNodeSetParams(G->x, G->mh, &mh));
-      CK(cudaGraphExecKernelNodeSetParams(G->x, G->count, &kc));
-      CK(cudaGraphExecKernelNodeSetParams(G->x, G->screen, &ks));
-      CK(cudaGraphExecKernelNodeSetParams(G->x, G->listed, &kl));
-      if(q.with_min) CK(cudaGraphExecKernelNodeSetParams(G->x, G->ismin, &km));
-      CK(cudaGraphExecMemcpyNodeSetParams1D(G->x, G->d2h, q.head_host, q.head, q.d2h_bytes, cudaMemcpyDeviceToHost));
+      for(int i = 0; i < kWaveKernels; i++) {
+        const cudaKernelNodeParams kp = kernel_params(q.k[i]);
+        CK(cudaGraphExecKernelNodeSetParams(G->x, G->node[i], &kp));
+      }
     }
     CK(cudaGraphLaunch(G->x, st));
   }
@@ -1829,7 +1811,7 @@ private:
     int32_t *hl = carve<int32_t>(hb, off, tot_cols);
     int32_t *hcode = carve<int32_t>(hb, off, 5 * (size_t)tot_edges);
     int32_t *ht = carve<int32_t>(hb, off, packed ? W : 0);
-    const size_t desc_bytes = off;
+    const size_t desc_bytes = Carver::round(off);
     int32_t planes = 1;
     int32_t eo = 0;
     int32_t co = 0, so = 0, kmax = 1;
@@ -1955,7 +1937,7 @@ private:
     const size_t cnt_bytes = sizeof(int32_t) * (size_t)cstride * ccopies;
     // packed rows: the record regions' counters, behind the embedding counters
     const size_t reg_bytes = packed ? sizeof(uint32_t) * kRecRegions * kRecRegionStride : 0;
-    const size_t zero_bytes = cnt_bytes + reg_bytes + sizeof(uint32_t) * (size_t)std::max<int64_t>(bb, 1);
+    const size_t zero_bytes = Carver::round(cnt_bytes + reg_bytes + sizeof(uint32_t) * (size_t)std::max<int64_t>(bb, 1));
     X.d_zero.ensure(zero_bytes);
     X.d_head.ensure(kHeadBytes + sizeof(int4) * (size_t)std::max(kb, 1));
     X.d_bmx.ensure(std::max<int64_t>(bb, 1));
@@ -1997,38 +1979,39 @@ private:
         f.rec = X.d_rec.p + f.rec_cap * kRecRegions;
       }
     }
-    // the frequent candidates come back compacted: a prefix sized from earlier
-    // waves, the rest (rarely) by a second copy
+    // the frequent candidates come back compacted, as many as there was need of
+    // room for in earlier waves (the rest, rarely, by a second copy)
     f.sel_copied = std::min<int64_t>(kb, X.sel_hint);
     X.h_head.ensure(kHeadBytes + sizeof(int4) * (size_t)std::max<int64_t>(f.sel_copied, 1));
     WaveSeq q;
-    q.desc_dst = X.d_desc.p;
-    q.desc_src = hb;
     q.desc_bytes = desc_bytes;
-    q.zero = X.d_zero.p;
-    q.zero_bytes = zero_bytes;
-    q.head = X.d_head.p;
-    q.head_host = X.h_head.p;
-    q.d2h_bytes = kHeadBytes + sizeof(int4) * (size_t)f.sel_copied;
+    q.k[0] = begin_call(X.d_desc.p, hb, (long long)desc_bytes / 16, X.d_zero.p, (long long)zero_bytes / 16, head);
     if(packed)
-      q.count = rows_count_call(f.dn, f.dt, W, (int32_t)tb, planes, f.ds, f.bm, cnt, ccopies, cstride,
-                                (uint32_t *)f.rec, f.hdr, (int32_t)f.rec_cap, f.reg, err_flag(), wo_.count_grid);
+      q.k[1] = rows_count_call(f.dn, f.dt, W, (int32_t)tb, planes, f.ds, f.bm, cnt, ccopies, cstride,
+                                (uint32_t *)f.rec, f.hdr, (int32_t)f.rec_cap, f.reg, head, err_flag(), wo_.count_grid);
     else
-      q.count = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
-                              err_flag(), f.rec, f.rec_cap, f.rec ? head + kHeadRecords : nullptr,
+      q.k[1] = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
+                              err_flag(), f.rec, f.rec_cap, head,
                               wo_.count_grid, ccopies, cstride, f.join, f.rule_skip);
     int32_t *lnode = nullptr;
     if(f.lists) {
       X.d_lnode.ensure(std::max(kb, 1));
       lnode = X.d_lnode.p;
     }
-    q.screen = screen_keys_call(f.dn, W, kb, cnt, ccopies, cstride, X.d_childmap.p, X.d_listed.p,
-                                head + kHeadSelected, err_flag(), head + kHeadFlags, lnode,
-                                f.rec ? f.reg : nullptr, head + kHeadRecords);
-    q.listed = count_listed_call(f.dn, X.d_listed.p, f.bm, cnt, X.d_bmx.p, X.d_keyword.p, sel, kb,
-                                 head + kHeadSelected, lnode);
-    q.with_min = wo_.min_check == 0;
-    if(q.with_min) q.ismin = is_min_call(f.dn, W, f.ds, E.d_dbs.p, dcode, sel, kb, head + kHeadSelected);
+    q.k[2] = screen_keys_call(f.dn, W, kb, cnt, ccopies, cstride, X.d_childmap.p, X.d_listed.p, head, err_flag(), lnode,
+                              f.rec ? f.reg : nullptr);
+    q.k[3] = count_listed_call(f.dn, X.d_listed.p, f.bm, cnt, X.d_bmx.p, X.d_keyword.p, sel, kb, head, lnode);
+    f.res_seq = ++E.seq;
+    ((volatile unsigned long long *)X.h_head.p)[kHeadSeq] = 0;
+    ResultsOut ro{};
+    ro.hsel = (int4 *)(X.h_head.p + kHeadBytes);
+    ro.hcap = f.sel_copied;
+    ro.hhead = (unsigned long long *)X.h_head.p;
+    ro.seq = f.res_seq;
+    ro.bytes = E.d_bytes.p;
+    ro.stamps = E.d_stamps.p;
+    ro.nctx = kWaveCtx;
+    q.k[4] = is_min_call(f.dn, W, f.ds, E.d_dbs.p, dcode, sel, kb, head, wo_.min_check == 0, ro);
     // the wave's nodes were made by the root phases (engine stream) or by
     // other contexts' materialise passes (their last ones cover every node
     // made so far; this context's own are ahead on its stream)
@@ -2039,12 +2022,15 @@ private:
       }
       for(int d = 0; d < kWaveCtx; d++)
         if(d != c && X.seen_mat[d] != E.ctx[d].mat_gen) {
-          CK(cudaStreamWaitEvent(X.stream, E.ctx[d].ev[5], 0));
+          CK(cudaStreamWaitEvent(X.stream, E.ctx[d].ev_mat, 0));
           X.seen_mat[d] = E.ctx[d].mat_gen;
         }
     }
+    // the passes that are ahead of this wave (their flags come with its results)
+    f.main_gen = E.main_gen;
+    for(int d = 0; d < kWaveCtx; d++) f.mat_gen[d] = E.ctx[d].mat_gen;
     issue(X, q);
-    st_.launches += q.with_min ? 4 : 3;
+    st_.launches += kWaveKernels;
     f.busy = true;
     f.seq = ++seq_;
     st_.host_build_ms += ms_since(t_begin);
@@ -2056,25 +2042,19 @@ private:
     WaveCtx &X = E.ctx[c];
     const cudaStream_t st = cs(X);
     Flight &f = fl_[c];
-    {
-      const clk::time_point t0 = clk::now();
-      CK(cudaEventSynchronize(X.ev[3]));
-      st_.host_wait_ms += ms_since(t0);
-    }
-    CK(cudaGetLastError());
+    wait_results((const volatile unsigned long long *)X.h_head.p, f.res_seq, st);
     const unsigned long long *hh = (const unsigned long long *)X.h_head.p;
     check_flags(hh[kHeadFlags]);
     const clk::time_point t_ready = clk::now();
     const double min_before = st_.host_min_ms;
-    if(f.mat_pending) {
-      // this context's previous materialise ran before the count just read
-      st_.mat_ms += ms_between(X.ev[4], X.ev[5]);
-      f.mat_pending = false;
-    }
-    st_.count_ms += ms_between(X.ev[0], X.ev[1]);
-    st_.support_ms += ms_between(X.ev[1], X.ev[2]);
-    st_.sel_ms += ms_between(X.ev[1], X.ev[6]);
-    st_.min_ms += ms_between(X.ev[6], X.ev[2]);
+    st_.count_ms += ms_between(hh[kHeadCount0], hh[kHeadSel0]);
+    st_.support_ms += ms_between(hh[kHeadSel0], hh[kHeadEnd]);
+    st_.sel_ms += ms_between(hh[kHeadSel0], hh[kHeadMin0]);
+    st_.min_ms += ms_between(hh[kHeadMin0], hh[kHeadEnd]);
+    for(int d = 0; d < kWaveCtx; d++) fold_mat(d, hh[kHeadMat + 2 * d], hh[kHeadMat + 2 * d + 1]);
+    fold_bytes(hh[kHeadBytesCount], hh[kHeadBytesMat]);
+    main_seen_ = std::max(main_seen_, f.main_gen);
+    for(int d = 0; d < kWaveCtx; d++) mat_seen_[d] = std::max(mat_seen_[d], f.mat_gen[d]);
     std::vector<int32_t> &nodes = f.nodes;
     std::vector<NodeLayout> &lays = f.lays;
     const NodeDesc *hn = f.hn;
@@ -2083,12 +2063,14 @@ private:
     // frequent candidates (compacted on the device)
     const int64_t nsel = (int64_t)hh[kHeadSelected];
     const long long nrec = f.rec ? (long long)hh[kHeadRecords] : -1;
-    st_.extensions += (int64_t)hh[kHeadExt];
+    const int64_t n_ext = (int64_t)hh[kHeadExt];
+    st_.extensions += n_ext;
     st_.sel_bytes += (int64_t)hh[kHeadSelBytes];
     // the count kernel's bytes per extension (bitmap word and counter, and the
     // record when records are on), counted here rather than in its inner loop
-    st_.count_bytes += (int64_t)hh[kHeadExt] * (8 + (f.rec ? (f.packed ? 4 : 16) : 0));
+    st_.count_bytes += n_ext * (8 + (f.rec ? (f.packed ? 4 : 16) : 0));
     if(nsel > kb) throw Error(ST_ERR_STATE, "candidate selection overflow");
+    st_.d2h_bytes += (int64_t)kHeadBytes + (int64_t)sizeof(int4) * std::min<int64_t>(nsel, f.sel_copied);
     if(nsel > f.sel_copied) {
       // copies the whole list again (growing the pinned buffer drops its
       // contents) on the side stream: the wave's results are complete, and the
@@ -2335,32 +2317,32 @@ private:
     }
     if(!outs.empty()) {
       // an item and its child map entry per extension
-      if(f.packed) st_.mat_bytes += 8 * (int64_t)hh[kHeadExt];
-      // one upload: children's outputs, then the (key, child) pairs
+      if(f.packed) st_.mat_bytes += 8 * n_ext;
+      // one table: children's outputs, then the (key, child) pairs
       const size_t outs_bytes = Carver::round(sizeof(ChildOut) * outs.size());
       const size_t pairs_bytes = Carver::round(sizeof(int2) * pairs.size());
-      const size_t mat_bytes = outs_bytes + pairs_bytes + (list_blk >= 0 ? sizeof(int32_t) * (size_t)W : 0);
+      const size_t mat_bytes = outs_bytes + pairs_bytes + (list_blk >= 0 ? Carver::round(sizeof(int32_t) * (size_t)W) : 0);
       X.d_mat.ensure(mat_bytes);
       X.h_mat.ensure(mat_bytes);
       std::memcpy(X.h_mat.p, outs.data(), sizeof(ChildOut) * outs.size());
       std::memcpy(X.h_mat.p + outs_bytes, pairs.data(), sizeof(int2) * pairs.size());
       if(list_blk >= 0) std::memcpy(X.h_mat.p + outs_bytes + pairs_bytes, list_rb.data(), sizeof(int32_t) * W);
-      h2d(X.d_mat.p, X.h_mat.p, mat_bytes, st);
       const ChildOut *douts = (const ChildOut *)X.d_mat.p;
       X.d_cursor.ensure(outs.size());
-      CK(cudaEventRecord(X.ev[4], st));
-      launch_scatter_childmap((const int2 *)(X.d_mat.p + outs_bytes), (int32_t)pairs.size(), X.d_childmap.p,
-                              X.d_cursor.p, (int32_t)outs.size(), st);
+      st_.h2d_bytes += (int64_t)mat_bytes;
+      unsigned long long *const stamps = E.d_stamps.p + (size_t)c * kMatStampWords;
+      launch_children(X.d_mat.p, X.h_mat.p, (long long)mat_bytes / 16, (const int2 *)(X.h_mat.p + outs_bytes),
+                      (int32_t)pairs.size(), X.d_childmap.p, X.d_cursor.p, (int32_t)outs.size(), stamps, st);
       // lists strategy: the records pass also counts the list rows
       ListBuild lb{ X.d_lnode.p, f.dn, (const int32_t *)(X.d_mat.p + outs_bytes + pairs_bytes) };
       if(list_blk >= 0) CK(cudaMemsetAsync(list_off, 0, sizeof(int32_t) * (size_t)(list_rows + 1), st));
       if(f.packed) {
         if(f.rec && nrec <= f.rec_cap) {
           launch_rows_records((const uint32_t *)f.rec, f.hdr, f.reg, (int32_t)f.rec_cap, (int32_t)nrec, f.planes,
-                              f.dn, X.d_childmap.p, f.bm, X.d_bmx.p, f.cnt, f.cstride, douts, err_flag(), st);
+                              f.dn, X.d_childmap.p, f.bm, X.d_bmx.p, f.cnt, f.cstride, douts, err_flag(), stamps, st);
         } else {
           launch_rows_materialize(f.dn, f.dt, W, (int32_t)f.tb, f.planes, f.ds, f.bm, X.d_bmx.p, X.d_childmap.p,
-                                  X.d_cursor.p, douts, err_flag(), st);
+                                  X.d_cursor.p, douts, err_flag(), stamps, st);
           if(f.rec)
             X.wanted_rec = std::max<long long>(X.wanted_rec, (nrec + nrec / 4) * kRecBlockInt4 * kRecRegions);
         }
@@ -2368,12 +2350,12 @@ private:
         // record-driven: one thread per extension record, no graph access
         launch_materialize_records(f.rec, nrec, X.d_childmap.p, X.d_keyword.p, f.bm, X.d_bmx.p, f.cnt, f.cstride,
                                    douts, E.d_bytes.p + 1, err_flag(), list_blk >= 0 ? &lb : nullptr,
-                                   list_off + 1, st);
+                                   list_off + 1, stamps, st);
       } else {
         // records overflowed (or are disabled): enumerate again
         launch_wave_materialize(f.dn, W, f.tb, f.kmax, f.small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, X.d_bmx.p,
                                 X.d_childmap.p, X.d_cursor.p, douts, E.d_bytes.p + 1, err_flag(), f.join,
-                                f.rule_skip, st);
+                                f.rule_skip, stamps, st);
         if(f.rec) X.wanted_rec = std::max<long long>(X.wanted_rec, nrec + nrec / 4);
       }
       if(list_blk >= 0) {
@@ -2381,10 +2363,10 @@ private:
         st_.list_entries += list_n;
         st_.launches += 2;
       }
-      CK(cudaEventRecord(X.ev[5], st));
+      CK(cudaGetLastError());
+      CK(cudaEventRecord(X.ev_mat, st));
       X.mat_gen++;
       st_.launches += 2;
-      f.mat_pending = true;
     }
     // the parents are done: drop their column references and graph ranks
     // (stream order keeps the materialise kernel ahead of any reuse)
@@ -2820,23 +2802,23 @@ int support_count_host(const int32_t *keys, const int32_t *gids, int64_t n, int3
     const size_t o_k = 0, o_g = o_k + al(4 * (size_t)std::max<int64_t>(n, 1));
     const size_t o_bm = o_g + al(4 * (size_t)std::max<int64_t>(n, 1));
     const size_t o_bmx = o_bm + al(4 * nw), o_sup = o_bmx + al(4 * nw);
-    const size_t o_nd = o_sup + al(4 * (size_t)n_keys), total = o_nd + al(sizeof(NodeDesc));
+    const size_t o_rj = o_sup + al(4 * (size_t)n_keys), total = o_rj + al(sizeof(RootJob));
     CK(cudaSetDevice(0));
     CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     CK(cudaMalloc(&blk, total));
-    NodeDesc nd{};
-    nd.words = words;
-    nd.nkeys = n_keys;
+    RootJob rj{};  // one job without counter copies: supports only
+    rj.words = words;
+    rj.R = n_keys;
     if(n > 0) {
       CK(cudaMemcpyAsync(blk + o_k, keys, 4 * (size_t)n, cudaMemcpyHostToDevice, s));
       CK(cudaMemcpyAsync(blk + o_g, gids, 4 * (size_t)n, cudaMemcpyHostToDevice, s));
     }
-    CK(cudaMemcpyAsync(blk + o_nd, &nd, sizeof(nd), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(blk + o_rj, &rj, sizeof(rj), cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(blk + o_bm, 0, 4 * nw, s));
     launch_records_bitmap((const int32_t *)(blk + o_k), (const int32_t *)(blk + o_g), n, words,
                           (uint32_t *)(blk + o_bm), s);
-    launch_support((const NodeDesc *)(blk + o_nd), 1, n_keys, (const uint32_t *)(blk + o_bm),
-                   (int32_t *)(blk + o_bmx), (int32_t *)(blk + o_sup), s);
+    launch_root_support((const RootJob *)(blk + o_rj), 1, n_keys, (const uint32_t *)(blk + o_bm),
+                        (int32_t *)(blk + o_bmx), nullptr, (int32_t *)(blk + o_sup), nullptr, s);
     CK(cudaMemcpyAsync(support, blk + o_sup, 4 * (size_t)n_keys, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     CK(cudaGetLastError());

@@ -21,6 +21,7 @@
 // A candidate whose pattern is larger, or whose embeddings outgrow the
 // buffer, is left to the host checker (verdict 2).
 #include "gs_kernels.hpp"
+#include "gs_stamp.cuh"
 
 namespace gsgb {
 
@@ -340,15 +341,17 @@ __global__ void __launch_bounds__(kMinWarps * 32) k_is_min(const NodeDesc *__res
                                                            const SlotDesc *__restrict__ slots,
                                                            const DevDB *__restrict__ dbs,
                                                            const int32_t *__restrict__ codes, int4 *sel,
-                                                           int sel_cap, const unsigned long long *counters)
+                                                           int sel_cap, unsigned long long *head, int check,
+                                                           const ResultsOut out)
 {
+  stamp_start(head + kHeadMin0);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   MinSmem &S = reinterpret_cast<MinSmem *>(smem_raw)[warp];
-  const long long nsel = min((long long)counters[0], (long long)sel_cap);
+  const long long nsel = min((long long)head[kHeadSelected], (long long)sel_cap);
   const long long nwarps = (long long)gridDim.x * kMinWarps;
   for(long long i = (long long)blockIdx.x * kMinWarps + warp; i < nsel; i += nwarps) {
-    const int4 x = sel[i];
+    int4 x = sel[i];
     // the node the selection recorded, or (out of range) the search by key
     int ni = x.w >> 2;
     if(ni < 0 || ni >= nnodes || x.x < nodes[ni].key_base || x.x >= nodes[ni].key_base + nodes[ni].nkeys)
@@ -356,7 +359,7 @@ __global__ void __launch_bounds__(kMinWarps * 32) k_is_min(const NodeDesc *__res
     const NodeDesc &nd = nodes[ni];
     const int len = nd.code_len, n = len + 1;
     int verdict = 2;
-    if(n <= kMinE) {
+    if(check && n <= kMinE) {
       // the parent's code, then the candidate edge decoded from its key
       for(int t = lane; t < len; t += 32) {
         const int32_t *c = codes + 5 * ((long long)nd.code_off + t);
@@ -399,14 +402,52 @@ __global__ void __launch_bounds__(kMinWarps * 32) k_is_min(const NodeDesc *__res
       if(nd.k + 1 <= kMinV) verdict = warp_is_min(S, n, lane);
       __syncwarp();
     }
-    if(lane == 0) sel[i].w = (x.w & ~3) | verdict;
+    if(lane == 0) {
+      x.w = (x.w & ~3) | verdict;
+      sel[i].w = x.w;
+      if(i < out.hcap) out.hsel[i] = x;
+    }
+  }
+  // the block that finishes last writes the header, its sequence word last
+  __syncthreads();
+  __shared__ int last;
+  if(threadIdx.x == 0) {
+    __threadfence_system();
+    last = atomicAdd(&head[kHeadDone], 1ull) == gridDim.x - 1 ? 1 : 0;
+  }
+  __syncthreads();
+  if(!last) return;
+  __threadfence();
+  volatile unsigned long long *const o = out.hhead;
+  const volatile unsigned long long *const h = head;
+  const int t = threadIdx.x;
+  if(t < kHeadEnd && t != kHeadDone && t != kHeadFlags) o[t] = h[t];
+  if(t == kHeadFlags) o[t] = ((const volatile unsigned long long *)out.bytes)[3];
+  if(t == kHeadEnd) o[t] = now_ns();
+  if(t == kHeadBytesCount || t == kHeadBytesMat) o[t] = ((const volatile unsigned long long *)out.bytes)[t - kHeadBytesCount];
+  for(int c = warp; c < out.nctx; c += kMinWarps) {
+    const volatile unsigned long long *st = out.stamps + (long long)c * kMatStampWords;
+    unsigned long long end = 0;
+    for(int q = lane; q < kMatSlots; q += 32) end = max(end, (unsigned long long)st[16 * (1 + q)]);
+    for(int d = 16; d > 0; d >>= 1) end = max(end, __shfl_xor_sync(kFull, end, d));
+    if(lane == 0) {
+      o[kHeadMat + 2 * c] = st[0];
+      o[kHeadMat + 2 * c + 1] = end;
+    }
+  }
+  __threadfence_system();
+  __syncthreads();
+  if(t == 0) {
+    __threadfence_system();
+    o[kHeadSeq] = out.seq;
   }
 }
 
 }  // namespace
 
 KernelCall is_min_call(const NodeDesc *nodes, int32_t nnodes, const SlotDesc *slots, const DevDB *dbs,
-                       const int32_t *codes, int4 *sel, int32_t sel_cap, const unsigned long long *counters)
+                       const int32_t *codes, int4 *sel, int32_t sel_cap, unsigned long long *head, bool check,
+                       const ResultsOut &out)
 {
   const size_t smem = sizeof(MinSmem) * kMinWarps;
   static const bool configured = [smem] {
@@ -426,7 +467,9 @@ KernelCall is_min_call(const NodeDesc *nodes, int32_t nnodes, const SlotDesc *sl
   c.arg(codes);
   c.arg(sel);
   c.arg(sel_cap);
-  c.arg(counters);
+  c.arg(head);
+  c.arg(check ? 1 : 0);
+  c.arg(out);
   return c;
 }
 

@@ -6,8 +6,11 @@
 // its parent node, so support = popcount.  The reference instead sorts or
 // flags 32-byte extension records per candidate (compute_support.cpp:146-257,
 // 805-960).
+#include <algorithm>
+
 #include "gs_kernels.hpp"
 #include "gs_lists.cuh"
+#include "gs_stamp.cuh"
 
 namespace gsgb {
 
@@ -157,42 +160,185 @@ __device__ __forceinline__ void root_tiles(const RootJob *__restrict__ jobs, int
 }
 
 __global__ void __launch_bounds__(kBlock) k_root_count(const RootJob *__restrict__ jobs, int njobs, long long tiles,
-                                                        const DevDB *__restrict__ dbs, uint32_t *bm, int32_t *cnt)
+                                                        const DevDB *__restrict__ dbs, uint32_t *bm, int32_t *cnt,
+                                                        unsigned long long *head)
 {
+  stamp_start(head ? head + kHeadCount0 : nullptr);
   root_tiles<false>(jobs, njobs, tiles, dbs, bm, nullptr, cnt, nullptr, nullptr, nullptr);
 }
 
-// Per key of the group, one warp: the job's counter copies turn into the
-// offsets of each copy's share (copy q: the count of copies 0..q-1, a warp
-// scan over the copies; copy 0 starts at 0 as the materialise pass's cursor)
-// and the total goes to tot[key].
-__global__ void __launch_bounds__(kBlock) k_sum_copies(const RootJob *__restrict__ jobs, int njobs, int total_keys,
-                                                        int32_t *cnt, int32_t *tot)
+// A key of at most kBigWords bitmap words is taken by one warp, a larger one (a
+// key present in up to a million graphs has 31,250 words) by a whole block, so
+// that its words are not read by one warp in a long chain of dependent steps.
+constexpr int kBigWords = 1024;
+
+// Popcounts of a key's words with their exclusive prefixes (bmx), 4 words per
+// lane per step; returns the total (all lanes).
+__device__ __forceinline__ int warp_prefix_words(const uint32_t *__restrict__ bm, int32_t *bmx, int words)
+{
+  const int lane = threadIdx.x & 31;
+  int running = 0;
+  for(int w0 = 0; w0 < words; w0 += 128) {
+    const int w = w0 + 4 * lane;
+    int c[4], t = 0;
+#pragma unroll
+    for(int q = 0; q < 4; q++) {
+      c[q] = (w + q < words) ? __popc(bm[w + q]) : 0;
+      t += c[q];
+    }
+    int incl = t;
+    for(int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if(lane >= o) incl += u;
+    }
+    int at = running + incl - t;
+#pragma unroll
+    for(int q = 0; q < 4; q++) {
+      if(w + q < words) bmx[w + q] = at;
+      at += c[q];
+    }
+    running += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  return running;
+}
+
+// The same by a whole block, 8 words per thread per step (all threads call it;
+// wtot: kBlock / 32 ints).
+__device__ __forceinline__ int block_prefix_words(const uint32_t *__restrict__ bm, int32_t *bmx, int words, int *wtot)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kPer = 8, kStep = kBlock * kPer;
+  int running = 0;
+  for(int w0 = 0; w0 < words; w0 += kStep) {
+    const int w = w0 + kPer * threadIdx.x;
+    int c[kPer], t = 0;
+#pragma unroll
+    for(int q = 0; q < kPer; q++) {
+      c[q] = (w + q < words) ? __popc(bm[w + q]) : 0;
+      t += c[q];
+    }
+    int incl = t;
+    for(int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if(lane >= o) incl += u;
+    }
+    if(lane == 31) wtot[warp] = incl;
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for(int x = 0; x < kBlock / 32; x++) {
+      const int v = wtot[x];
+      if(x < warp) before += v;
+      total += v;
+    }
+    int at = running + before + incl - t;
+#pragma unroll
+    for(int q = 0; q < kPer; q++) {
+      if(w + q < words) bmx[w + q] = at;
+      at += c[q];
+    }
+    running += total;
+    __syncthreads();  // wtot is rewritten by the next step
+  }
+  return running;
+}
+
+__device__ __forceinline__ int job_of_key(const RootJob *jobs, int njobs, int key)
+{
+  int lo = 0, hi = njobs - 1;
+  while(lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if(jobs[mid].key_base <= key) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// Per key of the group: its support and bitmap prefixes, and its counter
+// copies turned into the offsets of each copy's share (copy q: the count of
+// copies 0..q-1, a warp scan over the copies; copy 0 starts at 0 as the
+// materialise pass's cursor) and their total.
+__global__ void __launch_bounds__(kBlock) k_root_support(const RootJob *__restrict__ jobs, int njobs, int total_keys,
+                                                          const uint32_t *__restrict__ bm, int32_t *bmx, int32_t *cnt,
+                                                          int32_t *sup, int32_t *tot)
 {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for(int kg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; kg < total_keys; kg += warps) {
-    int lo = 0, hi = njobs - 1;
-    while(lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if(jobs[mid].key_base <= kg) lo = mid; else hi = mid - 1;
-    }
-    const RootJob &J = jobs[lo];
-    int32_t *c0 = cnt + J.cnt_base + (kg - J.key_base);
-    int run = 0;
-    for(int q0 = 0; q0 < J.copies; q0 += 32) {
-      const int q = q0 + lane;
-      const int x = q < J.copies ? c0[(long long)q * J.R] : 0;
-      int incl = x;
-      for(int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(full, incl, o);
-        if(lane >= o) incl += t;
+    const RootJob &J = jobs[job_of_key(jobs, njobs, kg)];
+    const int key = kg - J.key_base;
+    if(J.copies > 0) {
+      int32_t *c0 = cnt + J.cnt_base + key;
+      int run = 0;
+      for(int q0 = 0; q0 < J.copies; q0 += 32) {
+        const int q = q0 + lane;
+        const int x = q < J.copies ? c0[(long long)q * J.R] : 0;
+        int incl = x;
+        for(int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(full, incl, o);
+          if(lane >= o) incl += t;
+        }
+        if(q < J.copies) c0[(long long)q * J.R] = run + incl - x;
+        run += __shfl_sync(full, incl, 31);
       }
-      if(q < J.copies) c0[(long long)q * J.R] = run + incl - x;
-      run += __shfl_sync(full, incl, 31);
+      if(lane == 0) tot[kg] = run;
     }
-    if(lane == 0) tot[kg] = run;
+    if(J.words > kBigWords) continue;
+    const long long base = J.bm_base + (long long)key * J.words;
+    const int n = warp_prefix_words(bm + base, bmx + base, J.words);
+    if(lane == 0) sup[kg] = n;
+  }
+  // large keys: one block each (the branch is uniform over the block)
+  __shared__ int wtot[kBlock / 32];
+  for(int kg = blockIdx.x; kg < total_keys; kg += gridDim.x) {
+    const RootJob &J = jobs[job_of_key(jobs, njobs, kg)];
+    if(J.words <= kBigWords) continue;
+    const long long base = J.bm_base + (long long)(kg - J.key_base) * J.words;
+    const int n = block_prefix_words(bm + base, bmx + base, J.words, wtot);
+    if(threadIdx.x == 0) sup[kg] = n;
+  }
+}
+
+// First kernel of a wave or root group (see begin_call).  The tables come
+// straight from pinned host memory: no copy and clear operations between the
+// kernels of the stream.
+__global__ void __launch_bounds__(kBlock) k_begin(int4 *__restrict__ dst, const int4 *__restrict__ src, long long n16,
+                                                  int4 *zero, long long z16, unsigned long long *head)
+{
+  const long long i0 = (long long)blockIdx.x * kBlock + threadIdx.x, stride = (long long)gridDim.x * kBlock;
+  if(i0 < kHeadWords) head[i0] = 0;
+  for(long long i = i0; i < n16; i += 4 * stride) {
+    int4 x[4];
+#pragma unroll
+    for(int q = 0; q < 4; q++)
+      if(i + q * stride < n16) x[q] = src[i + q * stride];
+#pragma unroll
+    for(int q = 0; q < 4; q++)
+      if(i + q * stride < n16) dst[i + q * stride] = x[q];
+  }
+  for(long long i = i0; i < z16; i += stride) zero[i] = make_int4(0, 0, 0, 0);
+}
+
+// Results of a root group to pinned host memory (see launch_results).
+__global__ void __launch_bounds__(kBlock) k_results(int4 *dst, const int4 *__restrict__ src, long long n16,
+                                                    unsigned long long *head, const unsigned int *flags,
+                                                    unsigned long long *hhead, unsigned long long seq)
+{
+  stamp_start(head + kHeadSel0);
+  const long long stride = (long long)gridDim.x * kBlock;
+  for(long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n16; i += stride) dst[i] = src[i];
+  __syncthreads();
+  if(threadIdx.x == 0) {
+    __threadfence_system();
+    if(atomicAdd(&head[kHeadDone], 1ull) == gridDim.x - 1) {
+      __threadfence();
+      volatile unsigned long long *h = head, *o = hhead;
+      o[kHeadCount0] = h[kHeadCount0];
+      o[kHeadSel0] = h[kHeadSel0];
+      o[kHeadFlags] = *(volatile const unsigned int *)flags;
+      __threadfence_system();
+      o[kHeadSeq] = seq;
+    }
   }
 }
 
@@ -204,31 +350,6 @@ __global__ void __launch_bounds__(kBlock) k_root_materialize(const RootJob *__re
                                                               const ChildOut *__restrict__ outs, unsigned int *err)
 {
   root_tiles<true>(jobs, njobs, tiles, dbs, const_cast<uint32_t *>(bm), bmx, cursor, childmap, outs, err);
-}
-
-__global__ void __launch_bounds__(kBlock) k_support(const NodeDesc *__restrict__ nodes, int nnodes, int total_keys,
-                                                     const uint32_t *__restrict__ bm, int32_t *bmx, int32_t *support)
-{
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for(int key = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; key < total_keys; key += warps) {
-    const int n = find_node_by_key(nodes, nnodes, key);
-    const NodeDesc &nd = nodes[n];
-    const long long base = nd.bm_base + (long long)(key - nd.key_base) * nd.words;
-    int running = 0;
-    for(int w0 = 0; w0 < nd.words; w0 += 32) {
-      const int w = w0 + lane;
-      const int c = (w < nd.words) ? __popc(bm[base + w]) : 0;
-      int incl = c;
-      for(int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if(lane >= o) incl += t;
-      }
-      if(w < nd.words) bmx[base + w] = running + incl - c;
-      running += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if(lane == 0) support[key] = running;
-  }
 }
 
 // Support of the candidates of one wave, and their selection, in two passes.
@@ -245,23 +366,20 @@ __global__ void __launch_bounds__(kBlock) k_support(const NodeDesc *__restrict__
 __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restrict__ nodes, int nnodes,
                                                          int total_keys, int32_t *cnt, int cnt_copies,
                                                          long long cnt_stride, int32_t *childmap, int2 *listed,
-                                                         unsigned long long *counters,
-                                                         unsigned int *err, unsigned long long *err_copy,
-                                                         int32_t *lnode, const uint32_t *reg,
-                                                         unsigned long long *reg_max)
+                                                         unsigned long long *head, unsigned int *err,
+                                                         int32_t *lnode, const uint32_t *reg)
 {
+  stamp_start(head + kHeadSel0);
+  unsigned long long *const counters = head + kHeadSelected;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const long long stride = (long long)gridDim.x * blockDim.x;
   unsigned long long ext = 0, bytes = 0;
-  // the consistency flags so far (the count pass has finished) travel back
-  // with the wave's results
-  if(blockIdx.x == 0 && threadIdx.x == 0) *err_copy = *err;
   if(reg && blockIdx.x == 0 && threadIdx.x < 32) {
     uint32_t most = 0;
     for(int r = lane; r < kRecRegions; r += 32) most = max(most, reg[r * kRecRegionStride]);
     most = __reduce_max_sync(full, most);
-    if(lane == 0) *reg_max = most;
+    if(lane == 0) head[kHeadRecords] = most;
   }
   // warp-uniform trip count: the list append below is warp-aggregated
   const long long n32 = ((long long)total_keys + 31) & ~31ll;
@@ -340,20 +458,15 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
 }
 
 // A listed key's support: its bitmap words popcounted, their exclusive
-// prefixes written (bmx), the total compared with minsup.  A key of at most
-// kBigWords words is taken by one warp, 4 words per lane per step; a larger
-// one (a key present in up to a million graphs has 31,250 words) by a whole
-// block, 8 words per thread per step, so that its words are not read by one
-// warp in a long chain of dependent steps.
-constexpr int kBigWords = 1024;
-
+// prefixes written (bmx), the total compared with minsup.
 __device__ __forceinline__ void listed_done(const int2 kn, const NodeDesc &nd, long long wbase, int running,
                                             int32_t *cnt, long long *keyword, int4 *sel, int sel_cap,
-                                            unsigned long long *counters, int32_t *lnode)
+                                            unsigned long long *counters, int32_t *lnode,
+                                            unsigned long long &bytes)
 {
   // algorithmic bytes: the listed entry, each bitmap word read and its
   // prefix written, and for a selected key its word offset, result and counter
-  atomicAdd(&counters[3], 8ull + 8ull * (unsigned)nd.words + (running >= nd.minsup ? 32ull : 0ull));
+  bytes += 8ull + 8ull * (unsigned)nd.words + (running >= nd.minsup ? 32ull : 0ull);
   if(running >= nd.minsup) {
     keyword[kn.x] = wbase;
     const unsigned long long at = atomicAdd(&counters[0], 1ull);
@@ -370,11 +483,12 @@ __global__ void __launch_bounds__(kBlock) k_count_listed(const NodeDesc *__restr
                                                           const uint32_t *__restrict__ bm,
                                                           int32_t *cnt, int32_t *bmx,
                                                           long long *keyword, int4 *sel, int sel_cap,
-                                                          unsigned long long *counters, int32_t *lnode)
+                                                          unsigned long long *head, int32_t *lnode)
 {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  unsigned long long *const counters = head + kHeadSelected;
   const long long nlisted = (long long)counters[2];
+  unsigned long long bytes = 0;
   // small keys: one warp each
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for(long long li = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; li < nlisted; li += warps) {
@@ -383,73 +497,21 @@ __global__ void __launch_bounds__(kBlock) k_count_listed(const NodeDesc *__restr
     const int words = nd.words;
     if(words > kBigWords) continue;
     const long long wbase = nd.bm_base + (long long)(kn.x - nd.key_base) * words;
-    int running = 0;
-    for(int w0 = 0; w0 < words; w0 += 128) {
-      const int w = w0 + 4 * lane;
-      int c[4], t = 0;
-#pragma unroll
-      for(int q = 0; q < 4; q++) {
-        c[q] = (w + q < words) ? __popc(bm[wbase + w + q]) : 0;
-        t += c[q];
-      }
-      int incl = t;
-      for(int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(full, incl, o);
-        if(lane >= o) incl += u;
-      }
-      int at = running + incl - t;
-#pragma unroll
-      for(int q = 0; q < 4; q++) {
-        if(w + q < words) bmx[wbase + w + q] = at;
-        at += c[q];
-      }
-      running += __shfl_sync(full, incl, 31);
-    }
-    if(lane == 0) listed_done(kn, nd, wbase, running, cnt, keyword, sel, sel_cap, counters, lnode);
+    const int running = warp_prefix_words(bm + wbase, bmx + wbase, words);
+    if(lane == 0) listed_done(kn, nd, wbase, running, cnt, keyword, sel, sel_cap, counters, lnode, bytes);
   }
   // large keys: one block each (the branch below is uniform over the block)
   __shared__ int wtot[kBlock / 32];
-  constexpr int kPer = 8, kStep = kBlock * kPer;
   for(long long li = blockIdx.x; li < nlisted; li += gridDim.x) {
     const int2 kn = listed[li];
     const NodeDesc &nd = nodes[kn.y];
     const int words = nd.words;
     if(words <= kBigWords) continue;
     const long long wbase = nd.bm_base + (long long)(kn.x - nd.key_base) * words;
-    int running = 0;
-    for(int w0 = 0; w0 < words; w0 += kStep) {
-      const int w = w0 + kPer * threadIdx.x;
-      int c[kPer], t = 0;
-#pragma unroll
-      for(int q = 0; q < kPer; q++) {
-        c[q] = (w + q < words) ? __popc(bm[wbase + w + q]) : 0;
-        t += c[q];
-      }
-      int incl = t;
-      for(int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(full, incl, o);
-        if(lane >= o) incl += u;
-      }
-      if(lane == 31) wtot[warp] = incl;
-      __syncthreads();
-      int before = 0, total = 0;
-#pragma unroll
-      for(int x = 0; x < kBlock / 32; x++) {
-        const int v = wtot[x];
-        if(x < warp) before += v;
-        total += v;
-      }
-      int at = running + before + incl - t;
-#pragma unroll
-      for(int q = 0; q < kPer; q++) {
-        if(w + q < words) bmx[wbase + w + q] = at;
-        at += c[q];
-      }
-      running += total;
-      __syncthreads();  // wtot is rewritten by the next step
-    }
-    if(threadIdx.x == 0) listed_done(kn, nd, wbase, running, cnt, keyword, sel, sel_cap, counters, lnode);
+    const int running = block_prefix_words(bm + wbase, bmx + wbase, words, wtot);
+    if(threadIdx.x == 0) listed_done(kn, nd, wbase, running, cnt, keyword, sel, sel_cap, counters, lnode, bytes);
   }
+  if(lane == 0 && bytes) atomicAdd(&counters[3], bytes);
 }
 
 // ---- lists strategy: per-row lists of the frequent forward extensions
@@ -541,19 +603,19 @@ void xscan(int32_t *x, long long n, int32_t *scratch, cudaStream_t s)
   }
 }
 
-// childmap[pairs[i].x] = pairs[i].y for the children to materialise, and
-// their output cursors reset
-__global__ void __launch_bounds__(kBlock) k_scatter_childmap(const int2 *__restrict__ pairs, int n, int32_t *childmap,
-                                                              int32_t *cursor, int ncursor)
+// Children to materialise (see launch_children)
+__global__ void __launch_bounds__(kBlock) k_children(int4 *dst, const int4 *__restrict__ src, long long n16,
+                                                     const int2 *__restrict__ pairs, int n, int32_t *childmap,
+                                                     int32_t *cursor, int ncursor, unsigned long long *stamps)
 {
-  const int m = n > ncursor ? n : ncursor;
-  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    if(i < n) {
-      const int2 p = pairs[i];
-      childmap[p.x] = p.y;
-    }
-    if(i < ncursor) cursor[i] = 0;
+  const long long i0 = (long long)blockIdx.x * kBlock + threadIdx.x, stride = (long long)gridDim.x * kBlock;
+  if(i0 <= kMatSlots) stamps[16 * i0] = i0 == 0 ? now_ns() : 0;
+  for(long long i = i0; i < n; i += stride) {
+    const int2 p = pairs[i];
+    childmap[p.x] = p.y;
   }
+  for(long long i = i0; i < n16; i += stride) dst[i] = src[i];
+  for(long long i = i0; i < ncursor; i += stride) cursor[i] = 0;
 }
 
 __global__ void __launch_bounds__(kBlock) k_records_bitmap(const int32_t *__restrict__ keys,
@@ -577,12 +639,40 @@ inline int grid_for(long long n)
 
 }  // namespace
 
-void launch_root_count(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs, uint32_t *bm,
-                       int32_t *cnt, int32_t *tot, int32_t total_keys, cudaStream_t s)
+KernelCall begin_call(void *dst, const void *src, long long n16, void *zero, long long z16, unsigned long long *head)
 {
-  if(tiles > 0) k_root_count<<<grid_for(tiles * 32), kBlock, 0, s>>>(jobs, njobs, tiles, dbs, bm, cnt);
-  if(total_keys > 0)
-    k_sum_copies<<<grid_for((long long)total_keys * 32), kBlock, 0, s>>>(jobs, njobs, total_keys, cnt, tot);
+  KernelCall c;
+  c.func = (const void *)k_begin;
+  c.grid = dim3((unsigned)grid_for(std::max(std::max((n16 + 3) / 4, (z16 + 3) / 4), (long long)kHeadWords)));
+  c.block = dim3(kBlock);
+  c.arg((int4 *)dst);
+  c.arg((const int4 *)src);
+  c.arg(n16);
+  c.arg((int4 *)zero);
+  c.arg(z16);
+  c.arg(head);
+  return c;
+}
+
+void launch_root_count(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs, uint32_t *bm,
+                       int32_t *cnt, unsigned long long *head, cudaStream_t s)
+{
+  k_root_count<<<grid_for(tiles * 32), kBlock, 0, s>>>(jobs, njobs, tiles, dbs, bm, cnt, head);
+}
+
+void launch_root_support(const RootJob *jobs, int32_t njobs, int32_t total_keys, const uint32_t *bm, int32_t *bmx,
+                         int32_t *cnt, int32_t *sup, int32_t *tot, cudaStream_t s)
+{
+  if(total_keys <= 0) return;
+  k_root_support<<<grid_for((long long)total_keys * 32), kBlock, 0, s>>>(jobs, njobs, total_keys, bm, bmx, cnt, sup,
+                                                                          tot);
+}
+
+void launch_results(void *dst, const void *src, long long n16, unsigned long long *head, const unsigned int *flags,
+                    unsigned long long *hhead, unsigned long long seq, cudaStream_t s)
+{
+  const int g = (int)std::max(1ll, std::min(64ll, (n16 + 4 * kBlock - 1) / (4 * kBlock)));
+  k_results<<<g, kBlock, 0, s>>>((int4 *)dst, (const int4 *)src, n16, head, flags, hhead, seq);
 }
 
 void launch_root_materialize(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs,
@@ -605,8 +695,7 @@ void launch_records_bitmap(const int32_t *keys, const int32_t *gids, long long n
 
 KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, int32_t *cnt,
                             int32_t cnt_copies, long long cnt_stride, int32_t *childmap, int2 *listed,
-                            unsigned long long *counters, unsigned int *err, unsigned long long *err_copy,
-                            int32_t *lnode, const uint32_t *reg, unsigned long long *reg_max)
+                            unsigned long long *head, unsigned int *err, int32_t *lnode, const uint32_t *reg)
 {
   KernelCall c;
   c.func = (const void *)k_screen_keys;
@@ -620,18 +709,16 @@ KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total
   c.arg(cnt_stride);
   c.arg(childmap);
   c.arg(listed);
-  c.arg(counters);
+  c.arg(head);
   c.arg(err);
-  c.arg(err_copy);
   c.arg(lnode);
   c.arg(reg);
-  c.arg(reg_max);
   return c;
 }
 
 KernelCall count_listed_call(const NodeDesc *nodes, const int2 *listed, const uint32_t *bm, int32_t *cnt,
                              int32_t *bmx, long long *keyword, int4 *sel, int32_t sel_cap,
-                             unsigned long long *counters, int32_t *lnode)
+                             unsigned long long *head, int32_t *lnode)
 {
   KernelCall c;
   c.func = (const void *)k_count_listed;
@@ -645,7 +732,7 @@ KernelCall count_listed_call(const NodeDesc *nodes, const int2 *listed, const ui
   c.arg(keyword);
   c.arg(sel);
   c.arg(sel_cap);
-  c.arg(counters);
+  c.arg(head);
   c.arg(lnode);
   return c;
 }
@@ -782,19 +869,12 @@ void launch_fill_lists(const int4 *rec, long long nrec, const ListBuild &lb, int
   k_list_fill<<<grid_for(nrec), kBlock, 0, s>>>(rec, nrec, lb, cnt, ent, ent_cap, err);
 }
 
-void launch_scatter_childmap(const int2 *pairs, int32_t n, int32_t *childmap, int32_t *cursor, int32_t ncursor,
-                             cudaStream_t s)
+void launch_children(void *dst, const void *src, long long n16, const int2 *pairs, int32_t n, int32_t *childmap,
+                     int32_t *cursor, int32_t ncursor, unsigned long long *stamps, cudaStream_t s)
 {
-  const int32_t m = n > ncursor ? n : ncursor;
-  if(m <= 0) return;
-  k_scatter_childmap<<<grid_for(m), kBlock, 0, s>>>(pairs, n, childmap, cursor, ncursor);
-}
-
-void launch_support(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, const uint32_t *bm, int32_t *bmx,
-                    int32_t *support, cudaStream_t s)
-{
-  if(total_keys <= 0) return;
-  k_support<<<grid_for((long long)total_keys * 32), kBlock, 0, s>>>(nodes, nnodes, total_keys, bm, bmx, support);
+  const long long m = std::max(std::max((long long)n, n16), (long long)std::max(ncursor, kMatSlots + 1));
+  k_children<<<grid_for(m), kBlock, 0, s>>>((int4 *)dst, (const int4 *)src, n16, pairs, n, childmap, cursor, ncursor,
+                                            stamps);
 }
 
 }  // namespace gsgb

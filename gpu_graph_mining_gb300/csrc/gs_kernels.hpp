@@ -55,15 +55,27 @@ private:
   size_t used_ = 0;
 };
 
+// First kernel of a wave or root group: copies its tables from pinned host
+// memory (n16 16-byte pieces), clears its scratch (z16 pieces) and its header.
+KernelCall begin_call(void *dst, const void *src, long long n16, void *zero, long long z16, unsigned long long *head);
+
 // Root level of a group of jobs: a warp per 32 vertices of a job walks their
 // adjacency; every directed entry (v -> w) with label(v) <= label(w) is a
 // 1-edge embedding (get_forward_root, src/globals/graph_types.cpp:365-375).
 // Sets support-bitmap bit [key][graph] and counts embeddings per key in the
-// warp's counter copy; then per key of the group: tot[key] = its embeddings,
-// copy q >= 1 = the count of copies 0..q-1 and copy 0 = 0 (the materialise
-// pass's cursors).  tiles = the group's warp tiles; total_keys = its keys.
+// warp's counter copy.  tiles = the group's warp tiles.
 void launch_root_count(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs, uint32_t *bm,
-                       int32_t *cnt, int32_t *tot, int32_t total_keys, cudaStream_t s);
+                       int32_t *cnt, unsigned long long *head, cudaStream_t s);
+// Per key of the group: sup[key] = its graphs (popcount of its bitmap words,
+// whose exclusive prefixes go to bmx), tot[key] = its embeddings, counter copy
+// q >= 1 = the count of copies 0..q-1 and copy 0 = 0 (the materialise pass's
+// cursors; a job without copies has none).  total_keys = the group's keys.
+void launch_root_support(const RootJob *jobs, int32_t njobs, int32_t total_keys, const uint32_t *bm, int32_t *bmx,
+                         int32_t *cnt, int32_t *sup, int32_t *tot, cudaStream_t s);
+// Copies n16 16-byte pieces to pinned host memory, then the header, *flags
+// among it, to hhead with its sequence word last.
+void launch_results(void *dst, const void *src, long long n16, unsigned long long *head, const unsigned int *flags,
+                    unsigned long long *hhead, unsigned long long seq, cudaStream_t s);
 // Writes the two columns and graph ranks of every selected root key of the
 // group (childmap over the group's keys), with the counter copies as cursors.
 void launch_root_materialize(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs,
@@ -82,7 +94,7 @@ KernelCall wave_count_call(const NodeDesc *nodes, int32_t nnodes, long long tota
                            bool small_graphs, const int2 *const *coltab, const int32_t *collen, const SlotDesc *slots,
                            const int32_t *vtab, const DevDB *dbs, uint32_t *bm, int32_t *cnt,
                            unsigned long long *bytes, unsigned int *err, int4 *rec, long long rec_cap,
-                           unsigned long long *rec_n, int32_t grid_per_sm, int32_t cnt_copies,
+                           unsigned long long *head, int32_t grid_per_sm, int32_t cnt_copies,
                            long long cnt_stride, bool join, bool rule_skip);
 void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long total_tiles, int32_t kmax,
                              bool small_graphs,
@@ -90,7 +102,7 @@ void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long to
                              const int32_t *vtab, const DevDB *dbs, const uint32_t *bm, const int32_t *bmx,
                              const int32_t *childmap, int32_t *cursor, const ChildOut *outs,
                              unsigned long long *bytes, unsigned int *err, bool join, bool rule_skip,
-                             cudaStream_t s);
+                             unsigned long long *stamps, cudaStream_t s);
 
 // Packed rows (gs_rows.cu).  tile0[] = first 32-row tile of each node; planes =
 // the most planes of the wave's nodes' rows; rec / hdr: record blocks (rec may
@@ -100,18 +112,18 @@ constexpr int kRecRegions = 64, kRecRegionStride = 32;
 KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                            int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, int32_t cnt_copies,
                            long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
-                           unsigned int *err, int32_t grid_per_sm);
+                           unsigned long long *head, unsigned int *err, int32_t grid_per_sm);
 // Materialise by enumerating again, and from the record blocks (cursor and
 // cursor_stride as for launch_materialize_records).
 void launch_rows_materialize(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                              int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
                              const int32_t *childmap, int32_t *cursor, const ChildOut *outs, unsigned int *err,
-                             cudaStream_t s);
+                             unsigned long long *stamps, cudaStream_t s);
 // most: the most blocks of a region
 void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *reg, int32_t blk_cap, int32_t most,
                          int32_t planes, const NodeDesc *nodes, const int32_t *childmap, const uint32_t *bm,
                          const int32_t *bmx, int32_t *cursor, long long cursor_stride, const ChildOut *outs,
-                         unsigned int *err, cudaStream_t s);
+                         unsigned int *err, unsigned long long *stamps, cudaStream_t s);
 // Fills a database's neighbour blocks from its adjacency (db.nb_blocks,
 // db.nb_shift set; *used zeroed: receives the continuation blocks).
 void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStream_t s);
@@ -127,40 +139,51 @@ void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStre
 void launch_materialize_records(const int4 *rec, long long n, const int32_t *childmap, const long long *keyword,
                                 const uint32_t *bm, const int32_t *bmx, int32_t *cursor, long long cursor_stride,
                                 const ChildOut *outs, unsigned long long *bytes, unsigned int *err,
-                                const ListBuild *lists, int32_t *list_cnt, cudaStream_t s);
+                                const ListBuild *lists, int32_t *list_cnt, unsigned long long *stamps,
+                                cudaStream_t s);
 
 // Extension records given as (key, graph id) pairs: sets bit [key][graph].
 // Keys and graph ids must be in range (checked by the caller).
 void launch_records_bitmap(const int32_t *keys, const int32_t *gids, long long n, int32_t words, uint32_t *bm,
                            cudaStream_t s);
 
-// One warp per key: support = popcount of the key's bitmap words; bmx gets
-// the exclusive prefix popcount of each word (for graph-rank lookups).
-// Wave support with candidate selection (k_screen_keys, k_count_listed).
-// counters: [0] selected keys, [1] embeddings of all keys, [2] keys listed for
-// counting; listed and sel hold total_keys entries.  *err_copy = *err (the
-// consistency flags after the count pass).
+// Wave support with candidate selection (k_screen_keys, k_count_listed), into
+// the header's counters; listed and sel hold total_keys entries.  The
+// consistency flags after the count pass go to the header.
 // lnode (lists strategy, may be null): reset to -1 for every key with extensions
-// reg (packed rows, may be null): *reg_max = the most record blocks of a region
+// reg (packed rows, may be null): kHeadRecords = the most record blocks of a region
 KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, int32_t *cnt,
                             int32_t cnt_copies, long long cnt_stride, int32_t *childmap, int2 *listed,
-                            unsigned long long *counters, unsigned int *err, unsigned long long *err_copy,
-                            int32_t *lnode, const uint32_t *reg, unsigned long long *reg_max);
+                            unsigned long long *head, unsigned int *err, int32_t *lnode, const uint32_t *reg);
 // lnode (lists strategy, may be null): lnode[key] = the key's node for every
 // frequent forward key
 KernelCall count_listed_call(const NodeDesc *nodes, const int2 *listed, const uint32_t *bm, int32_t *cnt,
                              int32_t *bmx, long long *keyword, int4 *sel, int32_t sel_cap,
-                             unsigned long long *counters, int32_t *lnode);
-// Canonicality of the selected candidates (gs_ismin.cu): the low two bits of
-// sel[i].w (above them the candidate's node) = 1 minimal, 0 not minimal, 2
-// left to the host.  codes = the wave's code table.
+                             unsigned long long *head, int32_t *lnode);
+// Canonicality of the selected candidates (gs_ismin.cu) and the wave's results:
+// the low two bits of sel[i].w (above them the candidate's node) = 1 minimal, 0
+// not minimal, 2 left to the host (all of them when !check).  codes = the
+// wave's code table.  The first hcap candidates and then the header go to
+// pinned host memory (hsel, hhead), with bytes = the column kernels' byte
+// counters and stamps = every context's materialise stamps, the sequence word
+// last.
+struct ResultsOut {
+  int4 *hsel;
+  long long hcap;
+  unsigned long long *hhead;
+  unsigned long long seq;
+  const unsigned long long *bytes;
+  const unsigned long long *stamps;
+  int nctx;
+};
 KernelCall is_min_call(const NodeDesc *nodes, int32_t nnodes, const SlotDesc *slots, const DevDB *dbs,
-                       const int32_t *codes, int4 *sel, int32_t sel_cap, const unsigned long long *counters);
-// childmap[pairs[i].x] = pairs[i].y, and cursor[0..ncursor) = 0
-void launch_scatter_childmap(const int2 *pairs, int32_t n, int32_t *childmap, int32_t *cursor, int32_t ncursor,
-                             cudaStream_t s);
-void launch_support(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, const uint32_t *bm, int32_t *bmx,
-                    int32_t *support, cudaStream_t s);
+                       const int32_t *codes, int4 *sel, int32_t sel_cap, unsigned long long *head, bool check,
+                       const ResultsOut &out);
+// Children to materialise: their tables (n16 16-byte pieces, in pinned host
+// memory) copied to dst, childmap[pairs[i].x] = pairs[i].y, cursor[0..ncursor)
+// = 0, and the context's materialise stamps started.
+void launch_children(void *dst, const void *src, long long n16, const int2 *pairs, int32_t n, int32_t *childmap,
+                     int32_t *cursor, int32_t ncursor, unsigned long long *stamps, cudaStream_t s);
 
 // Lists strategy: the per-row lists of a wave's nodes' frequent forward
 // extensions, built from the count pass's records (ListBuild, gs_lists.cuh):

@@ -13,6 +13,7 @@
 // and 2.2 -> 0.9 GB of DRAM traffic.  It is bound by issue now (71% of
 // cycles, the integer pipe 69%; 0.24 of the DRAM peak).
 #include "gs_kernels.hpp"
+#include "gs_stamp.cuh"
 
 namespace gsgb {
 
@@ -50,6 +51,7 @@ struct RowsArgs {
   int blk_cap;            // blocks of one region
   uint32_t *reg;          // blocks reserved in each region (may exceed blk_cap: none past it are written)
   unsigned int *err;
+  unsigned long long *stamp;  // count: word for the kernel's start; materialise: the context's stamps
 };
 
 // One warp's shared memory; the right-most path has at most as many slots as
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
   // The warps reserve from kRecRegions counters on as many cache lines: adds
   // to one address complete at about one per 1.6 ns, which bounded the kernel
   // when one counter served all warps.
+  if(!MAT) stamp_start(a.stamp);
   const int region = gwarp % kRecRegions;
   int blk = 0, blk_left = 0, blk_next = 0;  // within the region
   bool ahead = false;
@@ -394,6 +397,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
     const int next = __shfl_sync(kFull, blk_next, 0);
     if(ahead && lane < kRecBlocks && next + lane < a.blk_cap) hdr[next + lane] = make_int4(0, 0, 0, 0);
   }
+  if(MAT) stamp_mat_end(a.stamp);
 }
 
 // Materialise from the record blocks: a warp takes kB blocks (each one tile of
@@ -411,7 +415,8 @@ __global__ void __launch_bounds__(256) k_rows_mat(const uint32_t *__restrict__ r
                                                   const int32_t *__restrict__ childmap,
                                                   const uint32_t *__restrict__ bm, const int32_t *__restrict__ bmx,
                                                   int32_t *cursor, long long cursor_stride,
-                                                  const ChildOut *__restrict__ outs, unsigned int *err)
+                                                  const ChildOut *__restrict__ outs, unsigned int *err,
+                                                  unsigned long long *stamps)
 {
   constexpr int NW = 2 + 4 * (PL - 1);
   const int lane = threadIdx.x & 31;
@@ -524,6 +529,7 @@ __global__ void __launch_bounds__(256) k_rows_mat(const uint32_t *__restrict__ r
       child();
     }
   }
+  stamp_mat_end(stamps);
 }
 
 // Neighbour blocks of a database (a thread per vertex, a warp's continuation
@@ -604,10 +610,10 @@ template <int PL, bool MAT> KernelCall rows_call(const RowsArgs &a, int grid_per
 KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                            int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, int32_t cnt_copies,
                            long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
-                           unsigned int *err, int32_t grid_per_sm)
+                           unsigned long long *head, unsigned int *err, int32_t grid_per_sm)
 {
   const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, bm, nullptr, cnt, cnt_copies, cnt_stride, nullptr,
-                    nullptr, nullptr, rec, hdr, blk_cap, reg, err };
+                    nullptr, nullptr, rec, hdr, blk_cap, reg, err, head + kHeadCount0 };
   if(planes <= 1) return rows_call<1, false>(a, grid_per_sm);
   if(planes <= 2) return rows_call<2, false>(a, grid_per_sm);
   return rows_call<5, false>(a, grid_per_sm);
@@ -616,11 +622,11 @@ KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t 
 void launch_rows_materialize(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                              int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
                              const int32_t *childmap, int32_t *cursor, const ChildOut *outs, unsigned int *err,
-                             cudaStream_t s)
+                             unsigned long long *stamps, cudaStream_t s)
 {
   if(total_tiles <= 0) return;
   const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, const_cast<uint32_t *>(bm), bmx, nullptr, 0, 0, childmap,
-                    cursor, outs, nullptr, nullptr, 0, nullptr, err };
+                    cursor, outs, nullptr, nullptr, 0, nullptr, err, stamps };
   KernelCall c = planes <= 1 ? rows_call<1, true>(a, 0) : planes <= 2 ? rows_call<2, true>(a, 0) : rows_call<5, true>(a, 0);
   c.run(s);
 }
@@ -628,7 +634,7 @@ void launch_rows_materialize(const NodeDesc *nodes, const int32_t *tile0, int32_
 void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *reg, int32_t blk_cap, int32_t most,
                          int32_t planes, const NodeDesc *nodes, const int32_t *childmap, const uint32_t *bm,
                          const int32_t *bmx, int32_t *cursor, long long cursor_stride, const ChildOut *outs,
-                         unsigned int *err, cudaStream_t s)
+                         unsigned int *err, unsigned long long *stamps, cudaStream_t s)
 {
   if(most <= 0) return;
   static_assert(kRecRegions % 8 == 0, "a block of 8 warps per 8 regions");
@@ -638,13 +644,13 @@ void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *r
   const int blocks = (int)(want < cap ? want : cap);
   if(planes <= 1)
     k_rows_mat<1, GS_ROWS_MATB><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
-                                         cursor_stride, outs, err);
+                                         cursor_stride, outs, err, stamps);
   else if(planes <= 2)
     k_rows_mat<2, 1><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
-                                         cursor_stride, outs, err);
+                                         cursor_stride, outs, err, stamps);
   else
     k_rows_mat<5, 1><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
-                                         cursor_stride, outs, err);
+                                         cursor_stride, outs, err, stamps);
 }
 
 void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStream_t s)

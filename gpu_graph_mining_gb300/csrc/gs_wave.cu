@@ -31,6 +31,7 @@
 // selected children's 8-byte column elements and 4-byte graph ranks.
 #include "gs_kernels.hpp"
 #include "gs_lists.cuh"
+#include "gs_stamp.cuh"
 
 namespace gsgb {
 
@@ -82,6 +83,7 @@ struct WaveArgs {
   int cnt_copies;
   long long cnt_stride;
   int rule_skip;  // bisect past forward-rule prefixes of sorted adjacency lists
+  unsigned long long *stamp;   // count: word for the kernel's start; materialise: the context's stamps
 };
 
 template <int KMAX> struct Smem {
@@ -125,6 +127,7 @@ k_wave(const WaveArgs a)
   Smem<KMAX> &S = reinterpret_cast<Smem<KMAX> *>(smem_raw)[warp];
   const long long gwarp = (long long)blockIdx.x * kWarps + warp;
   const long long nwarps = (long long)gridDim.x * kWarps;
+  if(!MAT) stamp_start(a.stamp);
   if(lane == 0) S.bytes = 0;
   // count pass with records: the warp's current reserved chunk (warp-uniform);
   // starts "full" so the first batch reserves a chunk
@@ -446,6 +449,7 @@ k_wave(const WaveArgs a)
   }
   __syncwarp();
   if(a.bytes && lane == 0 && S.bytes) atomicAdd(a.bytes, S.bytes);
+  if(MAT) stamp_mat_end(a.stamp);
 }
 
 template <int KMAX, bool MAT, bool MASK, bool JOIN> void launch_k(const WaveArgs &a, cudaStream_t s)
@@ -518,12 +522,12 @@ KernelCall wave_count_call(const NodeDesc *nodes, int32_t nnodes, long long tota
                            bool small_graphs, const int2 *const *coltab, const int32_t *collen, const SlotDesc *slots,
                            const int32_t *vtab, const DevDB *dbs, uint32_t *bm, int32_t *cnt,
                            unsigned long long *bytes, unsigned int *err, int4 *rec, long long rec_cap,
-                           unsigned long long *rec_n, int32_t grid_per_sm, int32_t cnt_copies,
+                           unsigned long long *head, int32_t grid_per_sm, int32_t cnt_copies,
                            long long cnt_stride, bool join, bool rule_skip)
 {
   WaveArgs a{ nodes, nnodes, total_tiles, coltab, collen, slots, vtab, dbs, bm, nullptr, cnt,
-              nullptr, nullptr, nullptr, bytes, err, rec, rec_cap, rec_n, cnt_copies, cnt_stride,
-              rule_skip ? 1 : 0 };
+              nullptr, nullptr, nullptr, bytes, err, rec, rec_cap, rec ? head + kHeadRecords : nullptr, cnt_copies,
+              cnt_stride, rule_skip ? 1 : 0, head + kHeadCount0 };
   if(small_graphs)
     return join ? count_call<true, true>(kmax, a, grid_per_sm) : count_call<true, false>(kmax, a, grid_per_sm);
   return join ? count_call<false, true>(kmax, a, grid_per_sm) : count_call<false, false>(kmax, a, grid_per_sm);
@@ -535,11 +539,11 @@ void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long to
                              const int32_t *vtab, const DevDB *dbs, const uint32_t *bm, const int32_t *bmx,
                              const int32_t *childmap, int32_t *cursor, const ChildOut *outs,
                              unsigned long long *bytes, unsigned int *err, bool join, bool rule_skip,
-                             cudaStream_t s)
+                             unsigned long long *stamps, cudaStream_t s)
 {
   if(total_tiles <= 0) return;
   WaveArgs a{ nodes, nnodes, total_tiles, coltab, collen, slots, vtab, dbs, const_cast<uint32_t *>(bm), bmx,
-              nullptr, childmap, cursor, outs, bytes, err, nullptr, 0, nullptr, 0, 0, rule_skip ? 1 : 0 };
+              nullptr, childmap, cursor, outs, bytes, err, nullptr, 0, nullptr, 0, 0, rule_skip ? 1 : 0, stamps };
   dispatch<true>(kmax, small_graphs, join, a, s);
 }
 
@@ -553,7 +557,8 @@ __global__ void __launch_bounds__(256) k_mat_records(const int4 *__restrict__ re
                                                      const uint32_t *__restrict__ bm, const int32_t *__restrict__ bmx,
                                                      int32_t *cursor, long long cursor_stride,
                                                      const ChildOut *__restrict__ outs, unsigned long long *bytes,
-                                                     unsigned int *err, const ListBuild lb, int32_t *list_cnt)
+                                                     unsigned int *err, const ListBuild lb, int32_t *list_cnt,
+                                                     unsigned long long *stamps)
 {
   const int lane = threadIdx.x & 31;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -609,6 +614,7 @@ __global__ void __launch_bounds__(256) k_mat_records(const int4 *__restrict__ re
     for(int o = 16; o > 0; o >>= 1) mine += __shfl_down_sync(kFull, mine, o);
     if(lane == 0 && mine) atomicAdd(bytes, mine);
   }
+  stamp_mat_end(stamps);
 }
 
 }  // namespace
@@ -616,14 +622,15 @@ __global__ void __launch_bounds__(256) k_mat_records(const int4 *__restrict__ re
 void launch_materialize_records(const int4 *rec, long long n, const int32_t *childmap, const long long *keyword,
                                 const uint32_t *bm, const int32_t *bmx, int32_t *cursor, long long cursor_stride,
                                 const ChildOut *outs, unsigned long long *bytes, unsigned int *err,
-                                const ListBuild *lists, int32_t *list_cnt, cudaStream_t s)
+                                const ListBuild *lists, int32_t *list_cnt, unsigned long long *stamps,
+                                cudaStream_t s)
 {
   if(n <= 0) return;
   long long blocks = ((n + 31) / 32 * 32 + 255) / 256;
   if(blocks > 16LL * sm_count()) blocks = 16LL * sm_count();
   const ListBuild lb = lists ? *lists : ListBuild{ nullptr, nullptr, nullptr };
   k_mat_records<<<(int)blocks, 256, 0, s>>>(rec, n, childmap, keyword, bm, bmx, cursor, cursor_stride, outs, bytes,
-                                            err, lb, lists ? list_cnt : nullptr);
+                                            err, lb, lists ? list_cnt : nullptr, stamps);
 }
 
 }  // namespace gsgb

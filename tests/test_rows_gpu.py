@@ -103,3 +103,22 @@ def test_record_overflow(gs):
     small, _ = gs.mine_collect(db, s, wave_rows=1 << 20)
     assert first == again == small
     gs.engine_reset()
+
+
+@pytest.mark.parametrize("kw", [{}, {"launch_mode": 1}, {"serial": 1}, {"min_check": 1}, {"extension": "lists"}])
+def test_more_results_than_room(gs, kw):
+    # a fresh engine has room for 4,096 selected candidates per wave in pinned
+    # memory (the rest of a larger wave's come by a second copy); waves of 64
+    # nodes never fill it
+    db = gs.Database.generate(1, scale=1.0)
+    s = 2
+    gs.engine_reset()
+    small, _ = gs.mine_collect(db, s, wave_nodes=64, max_edges=7)
+    gs.engine_reset()
+    large, st = gs.mine_collect(db, s, max_edges=7, **kw)
+    assert st["candidates"] > 4 * 4096 and large == small
+    # one wave after another: the kernels' stamped times fit in the call
+    if kw.get("serial"):
+        parts = [st[k] for k in ("count_ms", "sel_ms", "min_ms", "mat_ms", "root_ms")]
+        assert min(parts) > 0 and sum(parts) <= st["wall_ms"]
+    gs.engine_reset()
