@@ -32,8 +32,8 @@
 // in the last word 2^31 | the block that continues it (again up to 8 entries,
 // or 7 and a link).  A wave's extension records are blocks of 32 four-byte
 // items of one tile, (node's key << 11) | (graph-local new vertex << 5) | row
-// in the tile, each with a header {first row of the tile, node, items |
-// counter copy << 8, the node's first key}.
+// in the tile, each with a header {first row of the tile, node, items,
+// the node's first key}.
 #pragma once
 #include <cstdint>
 
@@ -166,7 +166,9 @@ struct alignas(16) ChildOut {
   int32_t cap;    // rows allocated (the count pass's embedding count for the key)
   int32_t kind;   // 0 forward, 1 backward, 2 root
   int32_t planes; // packed rows: the child's
-  int32_t pad;
+  int32_t k;      // packed rows: the parent's pattern vertices,
+  const uint4 *prows;  // its planes
+  long long pnrows;    //   of so many rows
   int2 *col;      // columns: the child's new last column
   int2 *col0;     // root children only: column 0
   int32_t *gord;  // the child's graph ranks

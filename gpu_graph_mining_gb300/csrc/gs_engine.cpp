@@ -1128,6 +1128,7 @@ struct Flight {
   int32_t planes = 1;        // packed: the most planes of a node's rows
   int4 *hdr = nullptr;       // packed: record headers (rec_cap counts the blocks of one region)
   uint32_t *reg = nullptr;   // packed: the regions' block counters
+  uint32_t *chosen = nullptr;  // packed: a bit per key to materialise
   bool join = false;         // some node joins its parent's lists (lists strategy)
   int32_t W = 0, kb = 0, kmax = 1;
   bool small = true;
@@ -1766,9 +1767,10 @@ private:
         layout_node(top, db, L);
         const int32_t nk = layout_nkeys(L, db);
         const int64_t w = (int64_t)nk * words_for(top.support);
-        // (keys per wave stay below 2^26: records carry a wave key in 27 bits)
+        // (keys per wave stay below 2^26, records carry a wave key in 27 bits; packed
+        // below kRowsKeys, a node having fewer than 2^21)
         if(!nodes.empty() && (rows + top.nrows > wo_.wave_rows || words + w > wo_.wave_words ||
-                              wkeys + nk >= ((int64_t)1 << 26))) {
+                              wkeys + nk >= (S.packed ? kRowsKeys - (1 << 21) : 1 << 26))) {
           full = true;
           break;
         }
@@ -1932,12 +1934,16 @@ private:
     // node's few counters; copies spread them over L2 slices (summed by screening)
     // (records hold a key in 27 bits next to the copy: one copy beyond that)
     const int32_t ccopies =
-        kb >= (1 << 27) ? 1 : (int32_t)std::max<int64_t>(1, std::min<int64_t>(packed ? 4 : 16, ((int64_t)1 << 22) / std::max(kb, 1)));
+        packed             ? kRowsCopies
+        : kb >= (1 << 27) ? 1
+                          : (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, ((int64_t)1 << 22) / std::max(kb, 1)));
     const long long cstride = (long long)Carver::round(sizeof(int32_t) * (size_t)std::max(kb, 1)) / 4;
     const size_t cnt_bytes = sizeof(int32_t) * (size_t)cstride * ccopies;
     // packed rows: the record regions' counters, behind the embedding counters
     const size_t reg_bytes = packed ? sizeof(uint32_t) * kRecRegions * kRecRegionStride : 0;
-    const size_t zero_bytes = Carver::round(cnt_bytes + reg_bytes + sizeof(uint32_t) * (size_t)std::max<int64_t>(bb, 1));
+    // and a bit per key to materialise
+    const size_t sel_bytes = packed ? Carver::round((size_t)(kb + 31) / 32 * 4) : 0;
+    const size_t zero_bytes = Carver::round(cnt_bytes + reg_bytes + sel_bytes + sizeof(uint32_t) * (size_t)std::max<int64_t>(bb, 1));
     X.d_zero.ensure(zero_bytes);
     X.d_head.ensure(kHeadBytes + sizeof(int4) * (size_t)std::max(kb, 1));
     X.d_bmx.ensure(std::max<int64_t>(bb, 1));
@@ -1948,7 +1954,8 @@ private:
     f.cnt = cnt;
     f.cstride = cstride;
     f.reg = packed ? (uint32_t *)(X.d_zero.p + cnt_bytes) : nullptr;
-    f.bm = (uint32_t *)(X.d_zero.p + cnt_bytes + reg_bytes);
+    f.chosen = packed ? (uint32_t *)(X.d_zero.p + cnt_bytes + reg_bytes) : nullptr;
+    f.bm = (uint32_t *)(X.d_zero.p + cnt_bytes + reg_bytes + sel_bytes);
     unsigned long long *head = (unsigned long long *)X.d_head.p;
     int4 *sel = (int4 *)(X.d_head.p + kHeadBytes);
     // records: how many the wave appends is not known up front, so keep the
@@ -1987,7 +1994,7 @@ private:
     q.desc_bytes = desc_bytes;
     q.k[0] = begin_call(X.d_desc.p, hb, (long long)desc_bytes / 16, X.d_zero.p, (long long)zero_bytes / 16, head);
     if(packed)
-      q.k[1] = rows_count_call(f.dn, f.dt, W, (int32_t)tb, planes, f.ds, f.bm, cnt, ccopies, cstride,
+      q.k[1] = rows_count_call(f.dn, f.dt, W, (int32_t)tb, planes, f.ds, f.bm, cnt, cstride,
                                 (uint32_t *)f.rec, f.hdr, (int32_t)f.rec_cap, f.reg, head, err_flag(), wo_.count_grid);
     else
       q.k[1] = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
@@ -1998,7 +2005,7 @@ private:
       X.d_lnode.ensure(std::max(kb, 1));
       lnode = X.d_lnode.p;
     }
-    q.k[2] = screen_keys_call(f.dn, W, kb, cnt, ccopies, cstride, X.d_childmap.p, X.d_listed.p, head, err_flag(), lnode,
+    q.k[2] = screen_keys_call(f.dn, W, kb, cnt, ccopies, cstride, packed ? nullptr : X.d_childmap.p, X.d_listed.p, head, err_flag(), lnode,
                               f.rec ? f.reg : nullptr);
     q.k[3] = count_listed_call(f.dn, X.d_listed.p, f.bm, cnt, X.d_bmx.p, X.d_keyword.p, sel, kb, head, lnode);
     f.res_seq = ++E.seq;
@@ -2254,6 +2261,9 @@ private:
             // word and prefix, the row written
             st_.mat_bytes += rowsn * (16 * packed_planes(p.nv) + 8 + 16 * packed_planes(nv));
             o.planes = packed_planes(nv);
+            o.k = p.nv;
+            o.prows = p.rows;
+            o.pnrows = p.nrows;
             o.rows = cv.take<uint4>((size_t)rowsn * o.planes);
             o.word = hn[m.node].bm_base + (int64_t)cd.key * hn[m.node].words;
           } else {
@@ -2332,17 +2342,18 @@ private:
       st_.h2d_bytes += (int64_t)mat_bytes;
       unsigned long long *const stamps = E.d_stamps.p + (size_t)c * kMatStampWords;
       launch_children(X.d_mat.p, X.h_mat.p, (long long)mat_bytes / 16, (const int2 *)(X.h_mat.p + outs_bytes),
-                      (int32_t)pairs.size(), X.d_childmap.p, X.d_cursor.p, (int32_t)outs.size(), stamps, st);
+                      (int32_t)pairs.size(), X.d_childmap.p, f.chosen, X.d_cursor.p, (int32_t)outs.size(), stamps, st);
       // lists strategy: the records pass also counts the list rows
       ListBuild lb{ X.d_lnode.p, f.dn, (const int32_t *)(X.d_mat.p + outs_bytes + pairs_bytes) };
       if(list_blk >= 0) CK(cudaMemsetAsync(list_off, 0, sizeof(int32_t) * (size_t)(list_rows + 1), st));
       if(f.packed) {
         if(f.rec && nrec <= f.rec_cap) {
           launch_rows_records((const uint32_t *)f.rec, f.hdr, f.reg, (int32_t)f.rec_cap, (int32_t)nrec, f.planes,
-                              f.dn, X.d_childmap.p, f.bm, X.d_bmx.p, f.cnt, f.cstride, douts, err_flag(), stamps, st);
+                              f.chosen, X.d_childmap.p, f.bm, X.d_bmx.p, f.cnt, f.cstride, douts, err_flag(), stamps,
+                              st);
         } else {
-          launch_rows_materialize(f.dn, f.dt, W, (int32_t)f.tb, f.planes, f.ds, f.bm, X.d_bmx.p, X.d_childmap.p,
-                                  X.d_cursor.p, douts, err_flag(), stamps, st);
+          launch_rows_materialize(f.dn, f.dt, W, (int32_t)f.tb, f.planes, f.ds, f.bm, X.d_bmx.p, f.chosen,
+                                  X.d_childmap.p, X.d_cursor.p, douts, err_flag(), stamps, st);
           if(f.rec)
             X.wanted_rec = std::max<long long>(X.wanted_rec, (nrec + nrec / 4) * kRecBlockInt4 * kRecRegions);
         }

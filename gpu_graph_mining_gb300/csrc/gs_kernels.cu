@@ -356,7 +356,8 @@ __global__ void __launch_bounds__(kBlock) k_root_materialize(const RootJob *__re
 // Screening, one thread per key: a key with fewer embeddings than its node's
 // minsup cannot be found in that many graphs, so only keys with cnt >= minsup
 // are listed for counting; every key with embeddings gets childmap -1
-// (overwritten afterwards for the children that are materialised).
+// (overwritten afterwards for the children that are materialised; null for
+// packed rows, which mark those in a bit set).
 // Counting, one warp per listed key: popcount of its bitmap with prefix
 // counts for the materialise pass; the frequent keys are appended to sel as
 // {key, support, embeddings, node << 2} (order unspecified; the low two bits
@@ -408,12 +409,12 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
     int n = 0;
     bool cand = false;
     if(c > 0) {
-      childmap[key] = -1;
+      if(childmap) childmap[key] = -1;
       if(lnode) lnode[key] = -1;
       ext += (unsigned long long)c;
       n = find_node_by_key(nodes, nnodes, key);
       cand = c >= nodes[n].minsup;
-      bytes += lnode ? 8 : 4;  // child map (and list node) reset
+      bytes += (childmap ? 4 : 0) + (lnode ? 4 : 0);  // child map and list node reset
     }
     if(cand && cnt_copies > 1) {
       // a key that may be materialised: copy 0 keeps the total, copy q >= 1
@@ -606,13 +607,14 @@ void xscan(int32_t *x, long long n, int32_t *scratch, cudaStream_t s)
 // Children to materialise (see launch_children)
 __global__ void __launch_bounds__(kBlock) k_children(int4 *dst, const int4 *__restrict__ src, long long n16,
                                                      const int2 *__restrict__ pairs, int n, int32_t *childmap,
-                                                     int32_t *cursor, int ncursor, unsigned long long *stamps)
+                                                     uint32_t *chosen, int32_t *cursor, int ncursor, unsigned long long *stamps)
 {
   const long long i0 = (long long)blockIdx.x * kBlock + threadIdx.x, stride = (long long)gridDim.x * kBlock;
   if(i0 <= kMatSlots) stamps[16 * i0] = i0 == 0 ? now_ns() : 0;
   for(long long i = i0; i < n; i += stride) {
     const int2 p = pairs[i];
     childmap[p.x] = p.y;
+    if(chosen) atomicOr(&chosen[p.x >> 5], 1u << (p.x & 31));
   }
   for(long long i = i0; i < n16; i += stride) dst[i] = src[i];
   for(long long i = i0; i < ncursor; i += stride) cursor[i] = 0;
@@ -870,11 +872,11 @@ void launch_fill_lists(const int4 *rec, long long nrec, const ListBuild &lb, int
 }
 
 void launch_children(void *dst, const void *src, long long n16, const int2 *pairs, int32_t n, int32_t *childmap,
-                     int32_t *cursor, int32_t ncursor, unsigned long long *stamps, cudaStream_t s)
+                     uint32_t *chosen, int32_t *cursor, int32_t ncursor, unsigned long long *stamps, cudaStream_t s)
 {
   const long long m = std::max(std::max((long long)n, n16), (long long)std::max(ncursor, kMatSlots + 1));
-  k_children<<<grid_for(m), kBlock, 0, s>>>((int4 *)dst, (const int4 *)src, n16, pairs, n, childmap, cursor, ncursor,
-                                            stamps);
+  k_children<<<grid_for(m), kBlock, 0, s>>>((int4 *)dst, (const int4 *)src, n16, pairs, n, childmap, chosen, cursor,
+                                            ncursor, stamps);
 }
 
 }  // namespace gsgb

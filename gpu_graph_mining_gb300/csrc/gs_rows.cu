@@ -40,10 +40,10 @@ struct RowsArgs {
   const SlotDesc *slots;
   uint32_t *bm;           // count: bitmaps to set; materialise: read
   const int32_t *bmx;     // materialise: prefix popcounts
-  int32_t *cnt;           // count: embeddings per key, cnt_copies copies cnt_stride apart
-  int cnt_copies;
+  int32_t *cnt;           // count: embeddings per key, kRowsCopies copies cnt_stride apart
   long long cnt_stride;
-  const int32_t *childmap;  // materialise
+  const uint32_t *chosen;   // materialise: a bit per key to materialise,
+  const int32_t *childmap;  //   and such a key's child
   int32_t *cursor;
   const ChildOut *outs;
   uint32_t *rec;          // count, optional: record blocks
@@ -95,22 +95,27 @@ template <int NW> __device__ __forceinline__ unsigned id_of(const unsigned (&w)[
   return (x >> ((t & 3) * 8)) & 0xffu;
 }
 
-// The packed-row part of a child's outputs (two 16-byte loads).
+// The packed-row part of a child's outputs (three 16-byte loads).
 struct RowsOut {
   uint4 *rows;
   long long word;
-  int cap, kind, planes;
+  int cap, kind, planes, k;
+  const uint4 *prows;
+  long long pnrows;
 };
 __device__ __forceinline__ RowsOut load_out(const ChildOut *o)
 {
   const int4 *p = reinterpret_cast<const int4 *>(o);
-  const int4 x = __ldg(p), y = __ldg(p + 1);
+  const int4 x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2);
   RowsOut r;
   r.rows = reinterpret_cast<uint4 *>(((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x);
   r.word = (long long)(((unsigned long long)(unsigned)x.w << 32) | (unsigned)x.z);
   r.cap = y.x;
   r.kind = y.y;
   r.planes = y.z;
+  r.k = y.w;
+  r.prows = reinterpret_cast<const uint4 *>(((unsigned long long)(unsigned)z.y << 32) | (unsigned)z.x);
+  r.pnrows = (long long)(((unsigned long long)(unsigned)z.w << 32) | (unsigned)z.z);
   return r;
 }
 
@@ -151,7 +156,6 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   RowsSmem<PL> &S = smem[warp];
   const int gwarp = blockIdx.x * kWarps + warp, nwarps = gridDim.x * kWarps;
-  const int copy = gwarp % (a.cnt_copies > 0 ? a.cnt_copies : 1);
   // the warp's reserved record blocks, and (lane 0) those reserved ahead: a
   // reservation made at the start of a tile arrives while its rows are loaded.
   // The warps reserve from kRecRegions counters on as many cache lines: adds
@@ -343,16 +347,14 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
         const int key_base = S.key_base;
         if(!MAT) {
           // one counter add per distinct key, into this warp's copy of the
-          // counters (copies spread a node's hot counters over L2 slices); one
-          // bitmap OR per distinct key unless a lane's graph differs from its key
-          // group leader's (a tile's rows mostly share a graph).  Their bytes and
-          // the items' are added on the host from the wave's extension total.
+          // counters, and one bitmap OR unless a lane's graph differs from its key
+          // group leader's (a tile's rows mostly share a graph)
           const unsigned peers = __match_any_sync(kFull, key);
           const int leader = __ffs(peers) - 1;
           const int g_lead = __shfl_sync(kFull, g_o, leader);
           if(key >= 0 && (lane == leader || g_o != g_lead))
             atomicOr(&a.bm[S.bm_base + (long long)key * S.words + (g_o >> 5)], 1u << (g_o & 31));
-          if(key >= 0 && lane == leader) atomicAdd(&a.cnt[copy * a.cnt_stride + key_base + key], __popc(peers));
+          if(key >= 0 && lane == leader) atomicAdd(&a.cnt[(gwarp % kRowsCopies) * a.cnt_stride + key_base + key], __popc(peers));
           if(a.rec) {
             if(blk_left == 0) {
               if(!ahead) reserve();
@@ -363,13 +365,14 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
             if(blk < a.blk_cap) {  // past the region's end nothing is written
               const long long b = (long long)region * a.blk_cap + blk;
               a.rec[b * 32 + lane] = it;
-              if(lane == 0) a.hdr[b] = make_int4(row0, n, m | (copy << 8), key_base);
+              if(lane == 0) a.hdr[b] = make_int4(row0, n, m | (gwarp % kRowsCopies) << 8, key_base);
             }
             blk++;
             blk_left--;
           }
         } else {
-          const int c = key >= 0 ? a.childmap[key_base + key] : -1;
+          const int wkey = key_base + key;
+          const int c = key >= 0 && ((a.chosen[wkey >> 5] >> (wkey & 31)) & 1u) ? a.childmap[wkey] : -1;
           const unsigned peers = __match_any_sync(kFull, c);
           const int leader = __ffs(peers) - 1;
           int pos = 0;
@@ -400,133 +403,116 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
   if(MAT) stamp_mat_end(a.stamp);
 }
 
-// Materialise from the record blocks: a warp takes kB blocks (each one tile of
-// one node) side by side, an item of each per lane.  A key's cursor copies
-// start where the counts of the copies before end.  The chain per item is
-// child map, child, bitmap word and cursor: several blocks per warp and the
-// next ones' items and child map entries loaded ahead keep it in flight.
-#ifndef GS_ROWS_MATB
-#define GS_ROWS_MATB 1
-#endif
-template <int PL, int kB>
-__global__ void __launch_bounds__(256) k_rows_mat(const uint32_t *__restrict__ rec, const int4 *__restrict__ hdr,
-                                                  const uint32_t *__restrict__ reg, int blk_cap, int nblk,
-                                                  const NodeDesc *__restrict__ nodes,
-                                                  const int32_t *__restrict__ childmap,
-                                                  const uint32_t *__restrict__ bm, const int32_t *__restrict__ bmx,
-                                                  int32_t *cursor, long long cursor_stride,
-                                                  const ChildOut *__restrict__ outs, unsigned int *err,
-                                                  unsigned long long *stamps)
+// Materialise from the record blocks.  A warp takes kMatBlocks consecutive
+// blocks of a region, their loads in flight together, tests the items' keys in
+// the bit set of the chosen ones (a node's keys are a few words, one sector)
+// and queues the items that are; 32 queued ones are then placed together:
+// child map, child, and from there the parent's row, the graph rank's bitmap
+// word and the cursor side by side.  A third of the items are chosen on
+// 250,000 graphs of 40 edges, a tenth in the deep waves.  An item per lane
+// with a child map entry gathered for every item took 5.7 ms a pass there,
+// this 3.8 (100,000 graphs at 1%: 0.63 -> 0.46); latency and issue bound (60%),
+// 0.22 of the DRAM peak.  The child map gather was 13 to 15 sectors a block.
+constexpr int kMatWarps = 8, kMatBlocks = 4;
+constexpr int kMatGrid = 16;  // thread blocks per SM: 8 are resident
+
+template <int PL>
+__global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__restrict__ rec,
+                                                             const int4 *__restrict__ hdr,
+                                                             const uint32_t *__restrict__ reg, int blk_cap,
+                                                             const uint32_t *__restrict__ chosen,
+                                                             const int32_t *__restrict__ childmap,
+                                                             const uint32_t *__restrict__ bm,
+                                                             const int32_t *__restrict__ bmx, int32_t *cursor,
+                                                             long long cursor_stride,
+                                                             const ChildOut *__restrict__ outs, unsigned int *err,
+                                                             unsigned long long *stamps)
 {
   constexpr int NW = 2 + 4 * (PL - 1);
+  // queue entries: wave key (25 bits), counter copy (2), graph-local new vertex
+  // (6), parent row (31)
+  __shared__ unsigned long long queue[kMatWarps][32 * (kMatBlocks + 1)];
+  unsigned long long *const q = queue[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  // Block b is block b / kRecRegions of region b % kRecRegions; a warp stays in
-  // one region (nwarps is a multiple of their number).
-  const int b0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // a warp stays in one region (the number of warps is a multiple of theirs)
+  const int b0 = blockIdx.x * kMatWarps + (threadIdx.x >> 5);
   const int region = b0 % kRecRegions;
+  const int step = gridDim.x * kMatWarps / kRecRegions * kMatBlocks;
   const int used = min((int)min(__ldg(&reg[region * kRecRegionStride]), 0x7fffff00u), blk_cap);
-  int4 h1[kB];
-  unsigned it1[kB];
-  int c1[kB];
-  auto load = [&](int b) {
+  const int4 *const rh = hdr + (long long)region * blk_cap;
+  const uint32_t *const ri = rec + (long long)region * blk_cap * 32 + lane;
+  int qn = 0;
+  for(int i = b0 / kRecRegions * kMatBlocks; i < used || qn > 0; i += step) {
+    if(i < used) {
+      int4 h = make_int4(0, 0, 0, 0);  // lane t: the header of block i + t
+      if(lane < kMatBlocks && i + lane < used) h = __ldg(&rh[i + lane]);
+      unsigned it[kMatBlocks];
+      uint32_t w[kMatBlocks];
 #pragma unroll
-    for(int q = 0; q < kB; q++) {
-      h1[q] = make_int4(0, 0, 0, 0);
-      it1[q] = 0;
-      const int bq = b + q * nwarps, i = bq / kRecRegions;
-      if(bq < nblk && i < used) {
-        const long long at = (long long)region * blk_cap + i;
-        h1[q] = __ldg(&hdr[at]);
-        it1[q] = __ldg(&rec[at * 32 + lane]);
+      for(int t = 0; t < kMatBlocks; t++) it[t] = i + t < used ? __ldg(&ri[(long long)(i + t) * 32]) : 0u;
+#pragma unroll
+      for(int t = 0; t < kMatBlocks; t++) {
+        const int m = __shfl_sync(kFull, h.z, t) & 0xff, key = __shfl_sync(kFull, h.w, t) + (int)(it[t] >> 11);
+        w[t] = lane < m ? chosen[key >> 5] : 0u;
+      }
+#pragma unroll
+      for(int t = 0; t < kMatBlocks; t++) {
+        const int key = __shfl_sync(kFull, h.w, t) + (int)(it[t] >> 11);
+        const bool on = (w[t] >> (key & 31)) & 1u;
+        const unsigned m = __ballot_sync(kFull, on);
+        if(m) {
+          const int row0 = __shfl_sync(kFull, h.x, t), copy = __shfl_sync(kFull, h.z, t) >> 8;
+          if(on)
+            q[qn + __popc(m & lanemask_lt())] = ((unsigned long long)(unsigned)(key * kRowsCopies + copy) << 37) |
+                                                ((unsigned long long)((it[t] >> 5) & 63u) << 31) |
+                                                (unsigned)(row0 + (int)(it[t] & 31u));
+          qn += __popc(m);
+        }
       }
     }
-  };
-  auto child = [&]() {
+    const bool last = i + step >= used;
+    while(qn >= 32 || (last && qn > 0)) {
+      __syncwarp();
+      const int m = min(qn, 32);
+      const bool has = lane < m;
+      const unsigned long long e = has ? q[qn - m + lane] : 0ull;
+      qn -= m;
+      __syncwarp();
+      const int kc = has ? (int)(e >> 37) : -1, key = kc / kRowsCopies, row = (int)(e & 0x7fffffffull);
+      const unsigned lv = (unsigned)(e >> 31) & 63u;
+      RowsOut out{};
+      if(has) out = load_out(&outs[childmap[key]]);
+      uint4 r = make_uint4(0, 0, 0, 0);
+      unsigned w[NW];
 #pragma unroll
-    for(int q = 0; q < kB; q++)
-      c1[q] = lane < (h1[q].z & 0xff) ? childmap[h1[q].w + (int)(it1[q] >> 11)] : -1;
-  };
-  load(b0);
-  child();
-  for(int b = b0; b < nblk; b += kB * nwarps) {
-    int4 h[kB];
-    unsigned it[kB];
-    int c[kB];
-    bool any = false;
+      for(int t = 0; t < NW; t++) w[t] = 0;
+      if(has) {
+        r = __ldg(&out.prows[row]);
+        w[0] = r.z;
+        w[1] = r.w;
+        const int planes = out.k <= 8 ? 1 : 1 + (out.k + 7) / 16;
 #pragma unroll
-    for(int q = 0; q < kB; q++) {
-      h[q] = h1[q];
-      it[q] = it1[q];
-      c[q] = c1[q];
-      any = any || c[q] >= 0;
-    }
-    load(b + kB * nwarps);
-    if(__ballot_sync(kFull, any)) {
-      RowsOut out[kB];
-      uint4 r[kB];
-      unsigned w[kB][NW];
-      int nrows[kB];
-#pragma unroll
-      for(int q = 0; q < kB; q++) {
-        out[q] = RowsOut{};
-        if(c[q] >= 0) out[q] = load_out(&outs[c[q]]);
-        // an empty block's header names node 0: its rows are not used
-        const NodeDesc &nd = nodes[h[q].y];
-        nrows[q] = nd.nrows;
-        const int row = h[q].x + lane;
-        r[q] = make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for(int t = 0; t < NW; t++) w[q][t] = 0;
-        if(row < nrows[q]) {
-          r[q] = __ldg(&nd.rows[row]);
-          w[q][0] = r[q].z;
-          w[q][1] = r[q].w;
-#pragma unroll
-          for(int p = 1; p < PL; p++)
-            if(p < nd.planes) {
-              const uint4 x = __ldg(&nd.rows[(long long)p * nrows[q] + row]);
-              w[q][4 * p - 2] = x.x;
-              w[q][4 * p - 1] = x.y;
-              w[q][4 * p] = x.z;
-              w[q][4 * p + 1] = x.w;
-            }
-        }
+        for(int p = 1; p < PL; p++)
+          if(p < planes) {
+            const uint4 x = __ldg(&out.prows[p * out.pnrows + row]);
+            w[4 * p - 2] = x.x;
+            w[4 * p - 1] = x.y;
+            w[4 * p] = x.z;
+            w[4 * p + 1] = x.w;
+          }
       }
-      int gb[kB], g[kB], pos[kB], bpre[kB];
-      uint32_t bword[kB];
-#pragma unroll
-      for(int q = 0; q < kB; q++) {
-        const int o = (int)(it[q] & 31u);
-        gb[q] = (int)__shfl_sync(kFull, r[q].x, o);
-        g[q] = (int)__shfl_sync(kFull, r[q].y, o);
-#pragma unroll
-        for(int t = 0; t < NW; t++) w[q][t] = __shfl_sync(kFull, w[q][t], o);
-        // the bitmap word and its prefix are loaded before the cursor add, so
-        // that their latencies overlap
-        bword[q] = 0;
-        bpre[q] = 0;
-        if(c[q] >= 0) {
-          bword[q] = bm[out[q].word + (g[q] >> 5)];
-          bpre[q] = bmx[out[q].word + (g[q] >> 5)];
-        }
-        const unsigned peers = __match_any_sync(kFull, c[q]);
-        const int leader = __ffs(peers) - 1;
-        pos[q] = 0;
-        if(c[q] >= 0 && lane == leader)
-          pos[q] = atomicAdd(&cursor[(h[q].z >> 8) * cursor_stride + h[q].w + (int)(it[q] >> 11)], __popc(peers));
-        pos[q] = __shfl_sync(kFull, pos[q], leader) + __popc(peers & lanemask_lt());
+      const unsigned peers = __match_any_sync(kFull, kc);
+      const int leader = __ffs(peers) - 1;
+      int pos = 0;
+      if(has && lane == leader) pos = atomicAdd(&cursor[(kc % kRowsCopies) * cursor_stride + key], __popc(peers));
+      pos = __shfl_sync(kFull, pos, leader) + __popc(peers & lanemask_lt());
+      if(has) {
+        const int g = (int)r.y;
+        const long long wi = out.word + (g >> 5);
+        const int rank = bmx[wi] + __popc(bm[wi] & ((1u << (g & 31)) - 1u));
+        if(pos < out.cap) store_row<PL>(out, pos, (int)r.x, rank, w, out.k, lv);
+        else atomicOr(err, 4u);
       }
-      child();
-#pragma unroll
-      for(int q = 0; q < kB; q++)
-        if(c[q] >= 0) {
-          const int rank = bpre[q] + __popc(bword[q] & ((1u << (g[q] & 31)) - 1u));
-          if(pos[q] < out[q].cap) store_row<PL>(out[q], pos[q], gb[q], rank, w[q], nodes[h[q].y].k, (it[q] >> 5) & 63u);
-          else atomicOr(err, 4u);
-        }
-    } else {
-      child();
     }
   }
   stamp_mat_end(stamps);
@@ -608,11 +594,11 @@ template <int PL, bool MAT> KernelCall rows_call(const RowsArgs &a, int grid_per
 }  // namespace
 
 KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
-                           int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, int32_t cnt_copies,
-                           long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
+                           int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, long long cnt_stride,
+                           uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
                            unsigned long long *head, unsigned int *err, int32_t grid_per_sm)
 {
-  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, bm, nullptr, cnt, cnt_copies, cnt_stride, nullptr,
+  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, bm, nullptr, cnt, cnt_stride, nullptr, nullptr,
                     nullptr, nullptr, rec, hdr, blk_cap, reg, err, head + kHeadCount0 };
   if(planes <= 1) return rows_call<1, false>(a, grid_per_sm);
   if(planes <= 2) return rows_call<2, false>(a, grid_per_sm);
@@ -621,36 +607,30 @@ KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t 
 
 void launch_rows_materialize(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                              int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
-                             const int32_t *childmap, int32_t *cursor, const ChildOut *outs, unsigned int *err,
-                             unsigned long long *stamps, cudaStream_t s)
+                             const uint32_t *chosen, const int32_t *childmap, int32_t *cursor, const ChildOut *outs,
+                             unsigned int *err, unsigned long long *stamps, cudaStream_t s)
 {
   if(total_tiles <= 0) return;
-  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, const_cast<uint32_t *>(bm), bmx, nullptr, 0, 0, childmap,
-                    cursor, outs, nullptr, nullptr, 0, nullptr, err, stamps };
+  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, const_cast<uint32_t *>(bm), bmx, nullptr, 0, chosen,
+                    childmap, cursor, outs, nullptr, nullptr, 0, nullptr, err, stamps };
   KernelCall c = planes <= 1 ? rows_call<1, true>(a, 0) : planes <= 2 ? rows_call<2, true>(a, 0) : rows_call<5, true>(a, 0);
   c.run(s);
 }
 
 void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *reg, int32_t blk_cap, int32_t most,
-                         int32_t planes, const NodeDesc *nodes, const int32_t *childmap, const uint32_t *bm,
+                         int32_t planes, const uint32_t *chosen, const int32_t *childmap, const uint32_t *bm,
                          const int32_t *bmx, int32_t *cursor, long long cursor_stride, const ChildOut *outs,
                          unsigned int *err, unsigned long long *stamps, cudaStream_t s)
 {
   if(most <= 0) return;
-  static_assert(kRecRegions % 8 == 0, "a block of 8 warps per 8 regions");
-  const int nblk = most * kRecRegions;
-  // a multiple of kRecRegions warps
-  const long long want = nblk / 8, cap = 32LL * sm_count() / (kRecRegions / 8) * (kRecRegions / 8);
+  static_assert(kRecRegions % kMatWarps == 0, "thread blocks per set of regions");
+  constexpr int kPer = kRecRegions / kMatWarps;
+  const long long want = ((long long)most + kMatBlocks - 1) / kMatBlocks * kPer;
+  const long long cap = (long long)kMatGrid * sm_count() / kPer * kPer;
   const int blocks = (int)(want < cap ? want : cap);
-  if(planes <= 1)
-    k_rows_mat<1, GS_ROWS_MATB><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
-                                         cursor_stride, outs, err, stamps);
-  else if(planes <= 2)
-    k_rows_mat<2, 1><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
-                                         cursor_stride, outs, err, stamps);
-  else
-    k_rows_mat<5, 1><<<blocks, 256, 0, s>>>(rec, hdr, reg, blk_cap, nblk, nodes, childmap, bm, bmx, cursor,
-                                         cursor_stride, outs, err, stamps);
+  auto *f = planes <= 1 ? k_rows_mat<1> : planes <= 2 ? k_rows_mat<2> : k_rows_mat<5>;
+  f<<<blocks, kMatWarps * 32, 0, s>>>(rec, hdr, reg, blk_cap, chosen, childmap, bm, bmx, cursor, cursor_stride, outs, err,
+                                      stamps);
 }
 
 void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStream_t s)
