@@ -114,7 +114,7 @@ struct NodeDesc {
   int32_t db;            // index into the resident-database table
   int32_t minsup;        // the node's job's minimum support (candidate selection)
   int32_t code_off;      // the node's DFS code: edges code_off.. of the wave's code table
-  int32_t code_len;      //   (5 int32 per edge: from, to, fromlabel, elabel, tolabel)
+  int32_t code_len;      //   (a uint2 per edge)
   int32_t nfwd;          // keys below nfwd are forward extensions
   // Lists strategy (extension by intersection): a forward child's extensions
   // from right-most-path vertices other than its new right-most vertex are

@@ -94,6 +94,10 @@ int32_t Database::pair_index(int32_t a, int32_t el, int32_t tl) const
 void Database::index_pairs()
 {
   const int64_t tab = (int64_t)VL * EL * VL;
+  pair_code.assign((size_t)root_keys, 0);
+  for(int32_t a = 0; a < VL; a++)
+    for(size_t i = 0; i < pairs[a].size(); i++)
+      pair_code[root_off[a] + i] = (int32_t)(((uint32_t)pairs[a][i].first << 16) | (uint32_t)pairs[a][i].second);
   pair_tab.clear();
   if(tab > 1 << 20) return;
   pair_tab.assign((size_t)tab, -1);
@@ -191,10 +195,8 @@ void Database::upload()
   CK(cudaMemcpy(b + o_pi, pidx.data(), sizeof(int32_t) * tab, cudaMemcpyHostToDevice));
   std::vector<int32_t> ro(root_off);
   ro.push_back(root_keys);
-  std::vector<int32_t> pc(root_keys + 1, 0);
-  for(int32_t a = 0; a < VL; a++)
-    for(size_t i = 0; i < pairs[a].size(); i++)
-      pc[root_off[a] + i] = (pairs[a][i].first << 16) | pairs[a][i].second;
+  std::vector<int32_t> pc(pair_code);
+  pc.push_back(0);
   CK(cudaMemcpy(b + o_ro, ro.data(), sizeof(int32_t) * (VL + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b + o_pc, pc.data(), sizeof(int32_t) * (root_keys + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b + o_vb, vb.data(), sizeof(int32_t) * (host.n_graphs + 1), cudaMemcpyHostToDevice));
@@ -522,12 +524,31 @@ struct ColRef {
   int64_t n;
 };
 
+// A DFS edge in 8 bytes (dense labels): the codes of nodes and patterns, and of
+// the canonicality kernel's code table.
+struct CEdge {
+  uint8_t from, to;
+  uint16_t el, fl, tl;
+  bool is_forward() const { return from < to; }
+  DFS dfs() const { return DFS{ from, to, fl, el, tl }; }
+};
+static_assert(sizeof(CEdge) == 8, "the canonicality kernel reads a code edge as two words");
+
+// A right-most-path vertex of a node, from the root to the right-most vertex.
+struct RmSlot {
+  uint8_t vertex;   // pattern vertex
+  uint8_t joined;   // the code has an edge from the right-most vertex to it already
+  uint16_t vlab;
+  uint16_t el, tl;  // the path edge that leaves it (not the right-most vertex)
+  int32_t pair;     // and its index among the pairs of vlab
+};
+
 // One frequent pattern of a job's output tree; children in traversal order
 // as a linked list.
 struct PatternRec {
-  int32_t parent;
-  DFS edge;
   int64_t support;
+  CEdge edge;
+  int32_t parent;
   int32_t first_child = -1, last_child = -1, next_sibling = -1;
 };
 
@@ -616,15 +637,18 @@ private:
 struct PNode {
   int32_t job;
   int32_t pattern;
-  SmallVec<DFS, 12> code;
-  SmallVec<ColRef, 12> cols;  // column c = pattern vertex c
-  int32_t last_col = -1;      // the node's reference: its last column (the rest by parent links)
-  int32_t *gord = nullptr;
-  int32_t gord_blk;           // packed rows: the block of the rows
+  SmallVec<CEdge, 12> code;
+  SmallVec<RmSlot, 8> slots;  // its right-most path
+  int32_t nfwd, nkeys;        // its forward keys, all its keys
+  int32_t nv = 0;             // pattern vertices
+  int32_t gord_blk;           // the block of the graph ranks; packed rows: of the rows
   int64_t nrows;
   int64_t support;
   uint4 *rows = nullptr;      // packed rows: no columns, the whole embeddings in planes of nrows
-  int32_t nv = 0;             // packed rows: pattern vertices
+  // columns (kept allocated when a packed node takes this one's place)
+  std::unique_ptr<SmallVec<ColRef, 12>> cols;  // column c = pattern vertex c
+  int32_t last_col = -1;      // the node's reference: its last column (the rest by parent links)
+  int32_t *gord = nullptr;
   // lists strategy (forward children whose parent kept its per-row lists):
   // the parent's lists (a pool block shared by the parent's wave) and the
   // join rule (NodeDesc::join_lo / join_key / join_hi)
@@ -633,6 +657,46 @@ struct PNode {
   const int2 *list_ent = nullptr;
   int64_t list_rows = 0;
   int32_t join_lo = 0, join_key = 0, join_hi = 0;
+};
+
+// DFS-tree nodes of one scheduler after another: nodes stay in place while the
+// pool grows, and stacks and waves pass their ids around.  The engine keeps
+// up to kKeep of them allocated between runs (their first touch is most of
+// what a node costs the host otherwise).
+class NodePool {
+public:
+  PNode &operator[](int32_t id) { return chunks_[id >> kShift][id & ((1 << kShift) - 1)]; }
+  int32_t take()
+  {
+    if(!free_.empty()) {
+      const int32_t id = free_.back();
+      free_.pop_back();
+      return id;
+    }
+    if((used_ >> kShift) == (int32_t)chunks_.size()) chunks_.emplace_back(new PNode[1 << kShift]);
+    return used_++;
+  }
+  void put(int32_t id) { free_.push_back(id); }
+  // all nodes free again
+  void restart()
+  {
+    used_ = 0;
+    free_.clear();
+    if(chunks_.size() > (kKeep >> kShift)) chunks_.resize(kKeep >> kShift);
+  }
+  void clear()
+  {
+    used_ = 0;
+    std::vector<int32_t>().swap(free_);
+    chunks_.clear();
+  }
+
+private:
+  static constexpr int kShift = 8;
+  static constexpr size_t kKeep = 1 << 16;
+  std::vector<std::unique_ptr<PNode[]>> chunks_;
+  std::vector<int32_t> free_;
+  int32_t used_ = 0;
 };
 
 // One mining job inside a scheduler.
@@ -655,19 +719,13 @@ struct JobState {
 struct Candidate {
   int32_t node;
   int32_t key;
-  DFS dfs;
+  CEdge edge;
+  int32_t slot;     // forward: the slot it leaves from, and its pair there;
+  int32_t pair;     // backward: the slot it goes to
   int32_t support;
   int32_t cnt;
   int32_t verdict;  // canonicality from the GPU: 1 / 0, or 2 = check on the host
   bool ok;
-};
-
-struct NodeLayout {
-  int32_t nrm;
-  int32_t maxtoc;
-  int32_t nfwd;
-  std::vector<int32_t> vlab;   // per pattern vertex
-  std::vector<SlotDesc> slots;
 };
 
 // The device work of one wave up to its results in host memory: tables in and
@@ -799,6 +857,65 @@ int64_t rule_skip_adj_bytes()
 constexpr int kWaveCtx = GS_WAVE_CTX;
 static_assert(kWaveCtx <= kMaxWaveCtx, "WaveCtx::seen_mat and the header hold 8 contexts");
 
+// One wave in flight: its nodes and where their descriptors live.
+struct Flight {
+  bool busy = false;
+  uint64_t seq = 0;
+  std::vector<int32_t> nodes;  // node pool ids
+  NodeDesc *hn = nullptr;    // in the ctx's pinned descriptor mirror
+  const NodeDesc *dn = nullptr;
+  const int2 *const *dc = nullptr;
+  const SlotDesc *ds = nullptr;
+  const int32_t *dv = nullptr, *dl = nullptr;
+  bool packed = false;       // the wave's nodes have packed rows
+  const int32_t *dt = nullptr;  // packed: first tile of each node
+  int32_t planes = 1;        // packed: the most planes of a node's rows
+  int4 *hdr = nullptr;       // packed: record headers (rec_cap counts the blocks of one region)
+  uint32_t *reg = nullptr;   // packed: the regions' block counters
+  uint32_t *chosen = nullptr;  // packed: a bit per key to materialise
+  bool join = false;         // some node joins its parent's lists (lists strategy)
+  int32_t W = 0, kb = 0, kmax = 1;
+  bool small = true;
+  bool rule_skip = false;    // the count kernel bisects past forward-rule prefixes
+  bool lists = false;        // the wave builds its children's parent-row lists (lists strategy)
+  int64_t tb = 0;
+  int4 *rec = nullptr;
+  long long rec_cap = 0;
+  int64_t sel_copied = 0;    // selected entries there is room for with the results
+  uint64_t res_seq = 0;      // the results' sequence number
+  uint64_t main_gen = 0, mat_gen[kWaveCtx] = {};  // passes ahead of the wave when it was launched
+  uint32_t *bm = nullptr;    // the wave's support bitmaps (in the zeroed region)
+  int32_t *cnt = nullptr;    // its counter copies, cstride apart (cursors of the records materialise)
+  long long cstride = 0;
+  std::vector<int32_t> sel_at, sel_order;  // the candidates' counting sort by node
+};
+
+// A scheduler's nodes and per-wave scratch, kept by the engine between runs.
+struct Scratch {
+  struct Mat { int32_t node, cand, pid; };
+  NodePool nodes;
+  Flight fl[kWaveCtx];
+  std::vector<Candidate> cands;
+  std::vector<int32_t> todo, made, made_at, acc, touched;
+  std::vector<Mat> mats;
+  // pattern arrays of finished jobs, for the next ones
+  std::vector<std::vector<PatternRec>> spare;
+  void give(std::vector<PatternRec> &v)
+  {
+    if(spare.size() < 64 && v.capacity() > 0 && v.capacity() <= (1 << 16)) {
+      v.clear();
+      spare.emplace_back(std::move(v));
+    }
+    std::vector<PatternRec>().swap(v);
+  }
+  // ready for a new scheduler
+  void restart()
+  {
+    nodes.restart();
+    for(Flight &f : fl) f.busy = false;
+  }
+};
+
 struct Engine {
   // Streams: the engine's (database table, root phases) and one per wave
   // context, so that one wave's selection and materialise passes run beside
@@ -817,6 +934,7 @@ struct Engine {
   int64_t pool_limit = 0;
   DBuf<DevDB> d_dbs;
   DBuf<unsigned long long> d_bytes;   // [0] count bytes, [1] materialise bytes (column kernels), [3] flags
+  Scratch scratch;
   DBuf<unsigned long long> d_stamps;  // every wave context's materialise stamps
   uint64_t seq = 0;                   // number of the last wave or root group
   int64_t bytes_seen[2] = { 0, 0 };   // d_bytes[0..1] as last read
@@ -886,6 +1004,7 @@ struct Engine {
     blocks.clear();
     free_blocks.clear();
     workers.reset();
+    scratch = Scratch();
     ready = false;
   }
   // a pool block of `bytes`; starts with no references
@@ -998,95 +1117,117 @@ int64_t g_pool_limit = 0;
 
 inline int32_t words_for(int64_t support) { return (int32_t)((support + 31) / 32); }
 
-// Right-most-path slots and key layout of one node (see NodeDesc/SlotDesc).
-void layout_node(const PNode &n, const Database &db, NodeLayout &L)
+// A root node's right-most path and keys.
+void root_layout(PNode &n, const Database &db)
 {
-  const auto &c = n.code;
-  int rm[kMaxPatternEdges];
-  L.nrm = build_rmpath(c.data(), (int)c.size(), rm);
-  L.maxtoc = c[rm[0]].to;
-  const int k = L.maxtoc + 1;
-  L.vlab.assign(k, 0);
-  L.vlab[0] = c[0].fromlabel;
-  for(const DFS &d : c)
-    if(d.is_forward()) L.vlab[d.to] = d.tolabel;
-  L.slots.assign(L.nrm + 1, SlotDesc{});
-  int32_t fk = 0;
-  for(int s = 0; s <= L.nrm; s++) {
-    SlotDesc &sd = L.slots[s];
-    // (el_u, tl_u) <= (el, tl) lexicographically <=> (el_u << 16 | tl_u) <= (el << 16 | tl)
-    int32_t el = -1, tl = 0;  // the right-most-path edge's labels
-    if(s < L.nrm) {
-      const DFS &e = c[rm[L.nrm - 1 - s]];
-      sd.vertex = e.from;
-      el = e.elabel;
-      tl = e.tolabel;
-    } else {
-      sd.vertex = L.maxtoc;
-    }
-    sd.frule = s < L.nrm ? (int32_t)(((uint32_t)el << 16) | (uint32_t)tl) : INT32_MIN;
-    sd.vlab = L.vlab[sd.vertex];
-    sd.fkey_off = fk;
-    fk += db.pair_cnt[sd.vlab];
-    sd.bkey_off = -1;
-    sd.bmin = INT32_MAX;
-    sd.pbase = db.root_off[sd.vlab];
-    // the path edge is in the database: its pair is the first that the rule allows
-    if(db.dev.nb) sd.prule = ((s < L.nrm ? db.pair_index(sd.vlab, el, tl) : 0) + 1) << db.dev.nb_shift;
-  }
-  L.nfwd = fk;
-  const int32_t rlab = L.vlab[L.maxtoc];
-  // backward targets: from-vertices of rmpath edges other than the deepest
-  // (slots 0..nrm-2), unless the code already joins them to the right-most vertex
-  for(int s = 0; s + 1 < L.nrm; s++) {
-    SlotDesc &sd = L.slots[s];
-    const DFS &e = c[rm[L.nrm - 1 - s]];
-    bool joined = false;
-    for(const DFS &d : c)
-      if((d.from == L.maxtoc && d.to == sd.vertex) || (d.to == L.maxtoc && d.from == sd.vertex)) joined = true;
-    sd.bkey_off = joined ? -1 : fk + s * db.EL;
-    // el_u < el || (el_u == el && tl_u <= label(r))  <=>  el >= el_u + (tl_u > label(r))
-    sd.bmin = joined ? INT32_MAX : e.elabel + (e.tolabel > rlab ? 1 : 0);
-  }
+  const CEdge &e = n.code[0];
+  n.slots.push_back(RmSlot{ 0, 0, e.fl, e.el, e.tl, db.pair_index(e.fl, e.el, e.tl) });
+  n.slots.push_back(RmSlot{ 1, 0, e.tl, 0, 0, -1 });
+  n.nv = 2;
+  n.nfwd = n.nkeys = db.pair_cnt[e.fl] + db.pair_cnt[e.tl];
 }
 
-int32_t layout_nkeys(const NodeLayout &L, const Database &db) { return L.nfwd + std::max(0, L.nrm - 1) * db.EL; }
-
-// key -> candidate DFS edge (full labels)
-bool decode_key(const NodeLayout &L, const Database &db, int32_t key, DFS &d)
+// A child's, from its parent's: a forward edge leaves the path at its slot and
+// makes its new vertex the right-most one, a backward edge joins the
+// right-most vertex to its slot's.
+void child_layout(PNode &n, const PNode &p, const Candidate &cd, const Database &db)
 {
-  if(key < L.nfwd) {
-    for(int s = 0; s <= L.nrm; s++) {
-      const SlotDesc &sd = L.slots[s];
-      const int32_t cnt = db.pair_cnt[sd.vlab];
-      if(key >= sd.fkey_off && key < sd.fkey_off + cnt) {
-        const auto &p = db.pairs[sd.vlab][key - sd.fkey_off];
-        d = DFS{ sd.vertex, L.maxtoc + 1, sd.vlab, p.first, p.second };
+  const CEdge &e = cd.edge;
+  if(!e.is_forward()) {
+    n.slots.assign(p.slots.data(), p.slots.size());
+    n.slots[cd.slot].joined = 1;
+    n.nv = p.nv;
+    n.nfwd = p.nfwd;
+    n.nkeys = p.nkeys;
+    return;
+  }
+  n.slots.assign(p.slots.data(), (size_t)cd.slot + 1);
+  int32_t fk = 0;
+  for(RmSlot &s : n.slots) {
+    s.joined = 0;
+    fk += db.pair_cnt[s.vlab];
+  }
+  RmSlot &u = n.slots[cd.slot];
+  u.el = e.el;
+  u.tl = e.tl;
+  u.pair = cd.pair;
+  n.slots.push_back(RmSlot{ (uint8_t)p.nv, 0, e.tl, 0, 0, -1 });
+  n.nv = p.nv + 1;
+  n.nfwd = fk + db.pair_cnt[e.tl];
+  n.nkeys = n.nfwd + cd.slot * db.EL;
+}
+
+// A node's slots for the kernels (NodeDesc / SlotDesc); returns whether one
+// takes a backward edge.
+bool fill_slots(const PNode &n, const Database &db, SlotDesc *out)
+{
+  const int nrm = (int)n.slots.size() - 1;
+  const int32_t rlab = n.slots[nrm].vlab;
+  bool back = false;
+  int32_t fk = 0;
+  for(int s = 0; s <= nrm; s++) {
+    const RmSlot &r = n.slots[s];
+    SlotDesc &d = out[s];
+    d.vertex = r.vertex;
+    d.vlab = r.vlab;
+    d.fkey_off = fk;
+    fk += db.pair_cnt[r.vlab];
+    // (el_u, tl_u) <= (el, tl) lexicographically <=> (el_u << 16 | tl_u) <= (el << 16 | tl);
+    // the path edge is in the database: its pair is the first that the rule allows
+    d.frule = s < nrm ? (int32_t)(((uint32_t)r.el << 16) | r.tl) : INT32_MIN;
+    d.prule = (s < nrm ? r.pair + 1 : 1) << db.dev.nb_shift;
+    d.pbase = db.root_off[r.vlab];
+    // backward targets: all but the last two of the path, unless joined already;
+    // el_u < el || (el_u == el && tl_u <= label(r))  <=>  el >= el_u + (tl_u > label(r))
+    const bool b = s + 1 < nrm && !r.joined;
+    d.bkey_off = b ? n.nfwd + s * db.EL : -1;
+    d.bmin = b ? r.el + (r.tl > rlab ? 1 : 0) : INT32_MAX;
+    back = back || b;
+  }
+  return back;
+}
+
+// key -> the candidate's edge, slot and pair
+bool decode_key(const PNode &n, const Database &db, Candidate &cd)
+{
+  const int nrm = (int)n.slots.size() - 1;
+  if(cd.key < n.nfwd) {
+    int32_t at = cd.key;
+    for(int s = 0; s <= nrm; s++) {
+      const RmSlot &r = n.slots[s];
+      const int32_t cnt = db.pair_cnt[r.vlab];
+      if(at < cnt) {
+        const uint32_t pc = (uint32_t)db.pair_code[db.root_off[r.vlab] + at];
+        cd.edge = CEdge{ r.vertex, (uint8_t)n.nv, (uint16_t)(pc >> 16), r.vlab, (uint16_t)pc };
+        cd.slot = s;
+        cd.pair = at;
         return true;
       }
+      at -= cnt;
     }
     return false;
   }
-  const int32_t b = (key - L.nfwd) / db.EL, el = (key - L.nfwd) % db.EL;
-  if(b < 0 || b + 1 >= L.nrm) return false;
-  const SlotDesc &sd = L.slots[b];
-  if(sd.bkey_off < 0) return false;
-  d = DFS{ L.maxtoc, sd.vertex, L.vlab[L.maxtoc], el, sd.vlab };
+  const int32_t b = (cd.key - n.nfwd) / db.EL, el = (cd.key - n.nfwd) % db.EL;
+  if(b < 0 || b + 1 >= nrm || n.slots[b].joined) return false;
+  const RmSlot &r = n.slots[b];
+  cd.edge = CEdge{ n.slots[nrm].vertex, r.vertex, (uint16_t)el, n.slots[nrm].vlab, r.vlab };
+  cd.slot = b;
+  cd.pair = -1;
   return true;
 }
 
 // order of children in the sequential miner's traversal (gspan.cpp:250-271)
-bool seq_before(const DFS &a, const DFS &b)
+bool seq_before(const CEdge &a, const CEdge &b)
 {
   const bool fa = a.is_forward(), fb = b.is_forward();
   if(fa != fb) return !fa;
   if(!fa) {
     if(a.to != b.to) return a.to < b.to;
-    return a.elabel < b.elabel;
+    return a.el < b.el;
   }
   if(a.from != b.from) return a.from > b.from;
-  if(a.elabel != b.elabel) return a.elabel < b.elabel;
-  return a.tolabel < b.tolabel;
+  if(a.el != b.el) return a.el < b.el;
+  return a.tl < b.tl;
 }
 
 template <class T> T *carve(char *base, size_t &off, size_t n)
@@ -1112,40 +1253,6 @@ using clk = std::chrono::steady_clock;
 
 double ms_since(clk::time_point t0) { return std::chrono::duration<double, std::milli>(clk::now() - t0).count(); }
 
-// One wave in flight: its nodes and where their descriptors live.
-struct Flight {
-  bool busy = false;
-  uint64_t seq = 0;
-  std::vector<int32_t> nodes;  // node pool ids
-  std::vector<NodeLayout> lays;
-  NodeDesc *hn = nullptr;    // in the ctx's pinned descriptor mirror
-  const NodeDesc *dn = nullptr;
-  const int2 *const *dc = nullptr;
-  const SlotDesc *ds = nullptr;
-  const int32_t *dv = nullptr, *dl = nullptr;
-  bool packed = false;       // the wave's nodes have packed rows
-  const int32_t *dt = nullptr;  // packed: first tile of each node
-  int32_t planes = 1;        // packed: the most planes of a node's rows
-  int4 *hdr = nullptr;       // packed: record headers (rec_cap counts the blocks of one region)
-  uint32_t *reg = nullptr;   // packed: the regions' block counters
-  uint32_t *chosen = nullptr;  // packed: a bit per key to materialise
-  bool join = false;         // some node joins its parent's lists (lists strategy)
-  int32_t W = 0, kb = 0, kmax = 1;
-  bool small = true;
-  bool rule_skip = false;    // the count kernel bisects past forward-rule prefixes
-  bool lists = false;        // the wave builds its children's parent-row lists (lists strategy)
-  int64_t tb = 0;
-  int4 *rec = nullptr;
-  long long rec_cap = 0;
-  int64_t sel_copied = 0;    // selected entries there is room for with the results
-  uint64_t res_seq = 0;      // the results' sequence number
-  uint64_t main_gen = 0, mat_gen[kWaveCtx] = {};  // passes ahead of the wave when it was launched
-  uint32_t *bm = nullptr;    // the wave's support bitmaps (in the zeroed region)
-  int32_t *cnt = nullptr;    // its counter copies, cstride apart (cursors of the records materialise)
-  long long cstride = 0;
-  std::vector<int32_t> sel_at, sel_order;  // the candidates' counting sort by node
-};
-
 // The wave scheduler.  Jobs join at any time (add) and leave when their last
 // DFS-tree node is done; each step launches waves into the idle contexts and
 // completes the oldest wave in flight.  With two contexts the host decodes
@@ -1158,11 +1265,13 @@ struct Flight {
 // completed (Engine::reap).
 class Sched {
 public:
-  Sched(Engine &e, const MineOptions &wo, MineStats &st) : E(e), wo_(wo), st_(st)
+  Sched(Engine &e, const MineOptions &wo, MineStats &st)
+      : E(e), wo_(wo), st_(st), pn_(e.scratch.nodes), fl_(e.scratch.fl)
   {
     nctx_ = wo_.wave_nodes > 1 ? kWaveCtx : 1;
     E.pool.reset_peak();
     for(int i = 0; i < 2; i++) seen_bytes_[i] = E.bytes_seen[i];
+    E.scratch.restart();
   }
 
   // Validates the job, makes its database resident, mines its root level and
@@ -1227,6 +1336,10 @@ public:
     JobState &S = *jobs_.back();
     S.job = j;
     S.db_slot = slot;
+    if(!E.scratch.spare.empty()) {
+      S.pats.swap(E.scratch.spare.back());
+      E.scratch.spare.pop_back();
+    }
     // the lists strategy joins on parent rows: columns
     S.packed = db->dev.nb != nullptr && wo_.extension == 0;
     active_++;
@@ -1320,9 +1433,8 @@ private:
   const MineOptions &wo_;
   MineStats &st_;
   int nctx_ = kWaveCtx;
-  std::deque<PNode> pn_;          // DFS-tree nodes (stacks and waves hold their ids)
-  std::vector<int32_t> pn_free_;
-  Flight fl_[kWaveCtx];
+  NodePool &pn_;                  // DFS-tree nodes (stacks and waves hold their ids)
+  Flight (&fl_)[kWaveCtx];
   uint64_t seq_ = 0;
   std::vector<std::unique_ptr<JobState>> jobs_;
   std::vector<int32_t> order_;   // unfinished jobs, oldest first
@@ -1340,14 +1452,6 @@ private:
   unsigned long long mat_start_[kWaveCtx] = {};
   double mat_ms_[kWaveCtx] = {};
   bool defer_emit_ = false;
-  // per-wave scratch of finish(), reused
-  struct Mat { int32_t node, cand, pid; };
-  std::vector<Candidate> w_cands_;
-  std::vector<int32_t> w_todo_, w_made_, w_made_at_, w_acc_, w_touched_;
-  std::vector<ChildOut> w_outs_;
-  std::vector<int2> w_pairs_;
-  std::vector<Mat> w_mats_;
-
   // a wave context's stream (all on the engine's with the serial option)
   cudaStream_t cs(const WaveCtx &X) const { return wo_.serial ? E.stream : X.stream; }
   void h2d(void *dst, const void *src, size_t n, cudaStream_t s = nullptr)
@@ -1411,33 +1515,26 @@ private:
     if(v) throw Error(ST_ERR_STATE, "kernel consistency check failed (flags " + std::to_string(v) + ")");
   }
 
-  // DFS-tree node pool: nodes stay in place (a deque keeps references valid
-  // while it grows) and stacks and waves pass their ids around
   int32_t pn_new()
   {
-    int32_t id;
-    if(!pn_free_.empty()) {
-      id = pn_free_.back();
-      pn_free_.pop_back();
-    } else {
-      id = (int32_t)pn_.size();
-      pn_.emplace_back();
-    }
+    const int32_t id = pn_.take();
     PNode &p = pn_[id];
     p.code.assign(nullptr, 0);
-    p.cols.assign(nullptr, 0);
+    p.slots.assign(nullptr, 0);
+    if(p.cols) p.cols->assign(nullptr, 0);
     p.last_col = -1;
     p.gord = nullptr;
     p.rows = nullptr;
-    p.nv = 0;
     p.list_blk = -1;
     p.list_off = nullptr;
-    p.list_ent = nullptr;
-    p.list_rows = 0;
-    p.join_lo = p.join_key = p.join_hi = 0;
     return id;
   }
-  void pn_free(int32_t id) { pn_free_.push_back(id); }
+  void pn_free(int32_t id) { pn_.put(id); }
+  static SmallVec<ColRef, 12> &cols_of(PNode &p)
+  {
+    if(!p.cols) p.cols.reset(new SmallVec<ColRef, 12>());
+    return *p.cols;
+  }
 
   // releases a node's columns and graph ranks
   void drop_node(JobState &S, PNode &p)
@@ -1469,7 +1566,7 @@ private:
       ScopeMs t(st_.host_emit_ms);
       emit(S);
     }
-    std::vector<PatternRec>().swap(S.pats);
+    E.scratch.give(S.pats);
     std::vector<int32_t>().swap(S.roots);
     std::vector<int32_t>().swap(S.root_keys);
   }
@@ -1501,7 +1598,7 @@ public:
   void release_patterns(int32_t id)
   {
     JobState &S = *jobs_[id];
-    std::vector<PatternRec>().swap(S.pats);
+    E.scratch.give(S.pats);
     std::vector<int32_t>().swap(S.roots);
     std::vector<int32_t>().swap(S.root_keys);
   }
@@ -1609,7 +1706,7 @@ private:
       const int32_t kb = rj[q].key_base;
       const bool extend = S.job.opt.max_edges != 1;
       // frequent roots of this job (and partition), in the reference's order
-      struct Sel { int32_t key, pid; DFS d; int32_t sup; int64_t n; };
+      struct Sel { int32_t key, pid; CEdge d; int32_t sup; int64_t n; };
       std::vector<Sel> sel;
       int32_t root_index = 0;
       size_t bytes = 0;
@@ -1623,7 +1720,7 @@ private:
           // root-subtree partition: independent subtrees, no exchange between parts
           const int32_t ri = root_index++;
           if(S.job.opt.root_parts > 1 && ri % S.job.opt.root_parts != S.job.opt.root_part) continue;
-          PatternRec pr{ -1, DFS{ 0, 1, fl, el, tl }, sup };
+          PatternRec pr{ sup, CEdge{ 0, 1, (uint16_t)el, (uint16_t)fl, (uint16_t)tl }, -1 };
           S.pats.push_back(pr);
           const int32_t pid = (int32_t)S.pats.size() - 1;
           S.roots.push_back(pid);
@@ -1658,15 +1755,15 @@ private:
         nn.job = id;
         nn.pattern = s.pid;
         nn.code.push_back(s.d);
-        nn.nv = 2;
+        root_layout(nn, db);
         if(S.packed) {
           nn.rows = o.rows;
           S.live_bytes += s.n * 16;
         } else {
           const int32_t id0 = E.new_col(o.col0, s.n, blk, -1);
           nn.last_col = E.new_col(o.col, s.n, blk, id0, true);
-          nn.cols.push_back(ColRef{ o.col0, s.n });
-          nn.cols.push_back(ColRef{ o.col, s.n });
+          cols_of(nn).push_back(ColRef{ o.col0, s.n });
+          cols_of(nn).push_back(ColRef{ o.col, s.n });
           nn.gord = o.gord;
           S.live_bytes += s.n * (int64_t)(2 * sizeof(int2) + sizeof(int32_t));
         }
@@ -1749,23 +1846,18 @@ private:
     int64_t limit = std::max(1, wo_.wave_nodes);
     if(nctx_ > 1 && idle > 1) limit = std::max<int64_t>(1, std::min<int64_t>(limit, (stacked_ + idle - 1) / idle));
     std::vector<int32_t> &nodes = f.nodes;
-    std::vector<NodeLayout> &lays = f.lays;  // kept between waves: layouts reuse their vectors
     nodes.clear();
     int64_t rows = 0, words = 0, wkeys = 0;
     bool full = false;
     int format = -1;  // a wave's nodes all have packed rows or all have columns
     for(size_t oi = 0; oi < order_.size() && !full; oi++) {
       JobState &S = *jobs_[order_[oi]];
-      const Database &db = *S.job.db;
       if(S.stack.empty()) continue;
       if(format < 0) format = S.packed ? 1 : 0;
       if(format != (S.packed ? 1 : 0)) continue;
       while(!S.stack.empty() && (int64_t)nodes.size() < limit) {
         const PNode &top = pn_[S.stack.back()];
-        if(lays.size() <= nodes.size()) lays.emplace_back();
-        NodeLayout &L = lays[nodes.size()];
-        layout_node(top, db, L);
-        const int32_t nk = layout_nkeys(L, db);
+        const int32_t nk = top.nkeys;
         const int64_t w = (int64_t)nk * words_for(top.support);
         // (keys per wave stay below 2^26, records carry a wave key in 27 bits; packed
         // below kRowsKeys, a node having fewer than 2^21)
@@ -1794,15 +1886,15 @@ private:
     bool any_join = false;
     for(int32_t n = 0; n < W; n++) {
       const PNode &p = pn_[nodes[n]];
-      tot_cols += (int32_t)p.cols.size();
-      tot_slots += (int32_t)lays[n].slots.size();
+      tot_cols += p.rows ? 0 : p.nv;
+      tot_slots += (int32_t)p.slots.size();
       tot_edges += (int32_t)p.code.size();
       any_join = any_join || p.list_off != nullptr;
     }
     size_t off = 0;
     const bool packed = format == 1;
     size_t need = 256 * 8 + sizeof(NodeDesc) * W + sizeof(int2 *) * tot_cols + sizeof(SlotDesc) * tot_slots +
-                  2 * sizeof(int32_t) * tot_cols + 5 * sizeof(int32_t) * tot_edges + sizeof(int32_t) * W;
+                  2 * sizeof(int32_t) * tot_cols + sizeof(CEdge) * tot_edges + sizeof(int32_t) * W;
     X.h_desc.ensure(need);
     X.d_desc.ensure(need);
     char *hb = X.h_desc.p;
@@ -1811,7 +1903,7 @@ private:
     SlotDesc *hs = carve<SlotDesc>(hb, off, tot_slots);
     int32_t *hv = carve<int32_t>(hb, off, tot_cols);
     int32_t *hl = carve<int32_t>(hb, off, tot_cols);
-    int32_t *hcode = carve<int32_t>(hb, off, 5 * (size_t)tot_edges);
+    CEdge *hcode = carve<CEdge>(hb, off, (size_t)tot_edges);
     int32_t *ht = carve<int32_t>(hb, off, packed ? W : 0);
     const size_t desc_bytes = Carver::round(off);
     int32_t planes = 1;
@@ -1825,7 +1917,6 @@ private:
     int32_t kb = 0;
     for(int32_t n = 0; n < W; n++) {
       const PNode &p = pn_[nodes[n]];
-      const NodeLayout &L = lays[n];
       const JobState &S = *jobs_[p.job];
       const Database &db = *S.job.db;
       NodeDesc &d = hn[n];
@@ -1834,20 +1925,20 @@ private:
       d.bm_base = bb;
       d.gord = p.gord;
       d.nrows = (int32_t)p.nrows;
-      d.k = packed ? p.nv : (int32_t)p.cols.size();
+      d.k = p.nv;
       d.col_off = co;
       d.slot_off = so;
       d.vtab_off = co;
-      d.nslot = (int32_t)L.slots.size();
-      d.minlabel = p.code[0].fromlabel;
+      d.nslot = (int32_t)p.slots.size();
+      d.minlabel = p.code[0].fl;
       d.words = words_for(p.support);
       d.key_base = kb;
-      d.nkeys = layout_nkeys(L, db);
+      d.nkeys = p.nkeys;
       d.db = S.db_slot;
       d.minsup = S.job.minsup;
       d.code_off = eo;
       d.code_len = (int32_t)p.code.size();
-      d.nfwd = L.nfwd;
+      d.nfwd = p.nfwd;
       if(p.list_off) {
         // lists strategy: join the parent's per-row lists
         d.csr_off = p.list_off;
@@ -1858,27 +1949,22 @@ private:
         d.join_hi = p.join_hi;
         st_.join_nodes++;
       }
-      for(const DFS &e : p.code) {
-        int32_t *c = hcode + 5 * (size_t)eo++;
-        c[0] = e.from;
-        c[1] = e.to;
-        c[2] = e.fromlabel;
-        c[3] = e.elabel;
-        c[4] = e.tolabel;
-      }
-      for(size_t cc = 0; cc < p.cols.size(); cc++) {
-        hc[co + cc] = p.cols[cc].ptr;
-        hl[co + cc] = (int32_t)p.cols[cc].n;
-        hv[co + cc] = -1;
-      }
-      for(size_t s = 0; s < L.slots.size(); s++) {
-        hs[so + s] = L.slots[s];
-        if(L.slots[s].bkey_off < 0) continue;
-        if(packed) d.back = 1;
-        else hv[co + L.slots[s].vertex] = (int32_t)s;
+      std::copy(p.code.begin(), p.code.end(), hcode + eo);
+      eo += (int32_t)p.code.size();
+      const bool back = fill_slots(p, db, hs + so);
+      if(!packed) {
+        const SmallVec<ColRef, 12> &cols = *p.cols;
+        for(size_t cc = 0; cc < cols.size(); cc++) {
+          hc[co + cc] = cols[cc].ptr;
+          hl[co + cc] = (int32_t)cols[cc].n;
+          hv[co + cc] = -1;
+        }
+        for(int32_t s = 0; s < d.nslot; s++)
+          if(hs[so + s].bkey_off >= 0) hv[co + hs[so + s].vertex] = s;
       }
       if(packed) {
         ht[n] = (int32_t)tb;
+        d.back = back ? 1 : 0;
         d.rows = p.rows;
         d.nb = db.dev.nb;
         d.pair_code = db.dev.pair_code;
@@ -1915,7 +2001,7 @@ private:
     f.packed = packed;
     f.planes = planes;
     if(tb >= INT32_MAX) throw Error(ST_ERR_LIMIT, "a wave has 2^36 or more embedding rows");
-    const int32_t *dcode = (const int32_t *)(db_ + ((char *)hcode - hb));
+    const uint2 *dcode = (const uint2 *)(db_ + ((char *)hcode - hb));
     f.join = any_join;
     f.W = W;
     f.kb = kb;
@@ -2063,7 +2149,6 @@ private:
     main_seen_ = std::max(main_seen_, f.main_gen);
     for(int d = 0; d < kWaveCtx; d++) mat_seen_[d] = std::max(mat_seen_[d], f.mat_gen[d]);
     std::vector<int32_t> &nodes = f.nodes;
-    std::vector<NodeLayout> &lays = f.lays;
     const NodeDesc *hn = f.hn;
     const int32_t W = f.W, kb = f.kb;
 
@@ -2103,13 +2188,15 @@ private:
     std::vector<int32_t> &order = f.sel_order;
     order.resize((size_t)nsel);
     for(int64_t i = 0; i < nsel; i++) order[at[hsel[i].w >> 2]++] = (int32_t)i;
-    std::vector<Candidate> &cands = w_cands_;
+    std::vector<Candidate> &cands = E.scratch.cands;
     cands.clear();
     cands.reserve((size_t)nsel);
+    int64_t n_cands = 0;
     for(int64_t oi = 0; oi < nsel; oi++) {
       const int4 e = hsel[order[oi]];
       const int32_t n = e.w >> 2;
-      const JobState &S = *jobs_[pn_[nodes[n]].job];
+      const PNode &p = pn_[nodes[n]];
+      const JobState &S = *jobs_[p.job];
       if(S.cancelled) continue;
       Candidate cd;
       cd.node = n;
@@ -2118,26 +2205,26 @@ private:
       cd.cnt = e.z;
       cd.verdict = wo_.min_check == 0 ? (e.w & 3) : 2;
       cd.ok = cd.verdict == 1;
-      if(cd.key < 0 || cd.key >= hn[n].nkeys) throw Error(ST_ERR_STATE, "selected key outside its node");
-      // the kernels emit keys of valid extensions only: one that does not
-      // decode is an inconsistency, not a pattern to skip
-      if(!decode_key(lays[n], *S.job.db, cd.key, cd.dfs))
-        throw Error(ST_ERR_STATE, "selected key does not decode to an extension");
+      if(cd.key < 0 || cd.key >= p.nkeys) throw Error(ST_ERR_STATE, "selected key outside its node");
       // a frequent pattern beyond what the embedding store and the checkers
       // take (64 vertices, 127 edges) is refused, never dropped: its
       // canonical form is frequent too, so the output would need it
       if(cd.cnt < 0 || cd.cnt == INT32_MAX)
         throw Error(ST_ERR_LIMIT, "a pattern has 2^31 or more embeddings in one wave");
-      const size_t pe = pn_[nodes[n]].code.size() + 1;
-      if(pe >= (size_t)kMaxPatternEdges || (cd.dfs.is_forward() && cd.dfs.to + 1 > kMaxPatternVertices))
+      if(p.code.size() + 1 >= (size_t)kMaxPatternEdges || (cd.key < p.nfwd && p.nv + 1 > kMaxPatternVertices))
         throw Error(ST_ERR_LIMIT, "frequent pattern exceeds 64 vertices or 127 edges; cap max_edges");
+      n_cands++;
+      if(cd.verdict == 0 && !f.lists) continue;  // (the lists keep them)
+      // the kernels emit keys of valid extensions only: one that does not
+      // decode is an inconsistency, not a pattern to skip
+      if(!decode_key(p, *S.job.db, cd)) throw Error(ST_ERR_STATE, "selected key does not decode to an extension");
       cands.push_back(cd);
     }
-    st_.candidates += (int64_t)cands.size();
+    st_.candidates += n_cands;
     // canonicality: the GPU's verdicts; the rest on the host, in parallel
     {
       const clk::time_point t0 = clk::now();
-      std::vector<int32_t> &todo = w_todo_;
+      std::vector<int32_t> &todo = E.scratch.todo;
       todo.clear();
       for(int32_t i = 0; i < (int32_t)cands.size(); i++)
         if(cands[i].verdict != 0 && cands[i].verdict != 1) todo.push_back(i);
@@ -2148,21 +2235,22 @@ private:
         DFS buf[kMaxPatternEdges + 1];
         const size_t n = code.size();
         if(n + 1 > (size_t)kMaxPatternEdges) { cd.ok = false; return; }
-        std::copy(code.begin(), code.end(), buf);
-        buf[n] = cd.dfs;
+        for(size_t i = 0; i < n; i++) buf[i] = code[i].dfs();
+        buf[n] = cd.edge.dfs();
         cd.ok = E.checkers[w].is_min(buf, (int)n + 1);
       });
       st_.host_min_ms += ms_since(t0);
     }
 
     // accepted children: output tree, materialisation slots
-    std::vector<ChildOut> &outs = w_outs_;
-    std::vector<int2> &pairs = w_pairs_;
-    outs.clear();
-    pairs.clear();
+    // the children's table is written in its pinned place: outputs, then (key,
+    // child) pairs
+    ChildOut *outs = nullptr;
+    int2 *pairs = nullptr;
+    size_t nout = 0, outs_bytes = 0, pairs_bytes = 0;
     // children in node order (a node's children are contiguous, from made_at[n])
-    std::vector<int32_t> &made = w_made_;
-    std::vector<int32_t> &made_at = w_made_at_;
+    std::vector<int32_t> &made = E.scratch.made;
+    std::vector<int32_t> &made_at = E.scratch.made_at;
     made.clear();
     made_at.assign((size_t)W + 1, 0);
     // lists strategy: every node with a forward child to materialise keeps
@@ -2175,13 +2263,13 @@ private:
     std::vector<int32_t> list_rb;  // per node: its first list row, or -1
     {
       // accepted candidates; cands is grouped by node, so each node's are contiguous
-      std::vector<int32_t> &acc = w_acc_;
+      std::vector<int32_t> &acc = E.scratch.acc;
       acc.clear();
       acc.reserve(cands.size());
       for(int32_t i = 0; i < (int32_t)cands.size(); i++)
         if(cands[i].ok) acc.push_back(i);
       // pass 1: output tree (reference order) and which children to materialise
-      std::vector<Mat> &mats = w_mats_;
+      std::vector<Scratch::Mat> &mats = E.scratch.mats;
       mats.clear();
       mats.reserve(acc.size());
       size_t bytes = 0;
@@ -2189,15 +2277,16 @@ private:
         const int32_t n = cands[acc[a0]].node;
         size_t a1 = a0;
         while(a1 < acc.size() && cands[acc[a1]].node == n) a1++;
-        std::sort(acc.begin() + a0, acc.begin() + a1,
-                  [&](int32_t a, int32_t b) { return seq_before(cands[a].dfs, cands[b].dfs); });
+        if(a1 - a0 > 1)
+          std::sort(acc.begin() + a0, acc.begin() + a1,
+                    [&](int32_t a, int32_t b) { return seq_before(cands[a].edge, cands[b].edge); });
         PNode &p = pn_[nodes[n]];
         JobState &S = *jobs_[p.job];
         const int32_t max_edges = S.job.opt.max_edges;
         for(size_t ai = a0; ai < a1; ai++) {
           const int32_t ci = acc[ai];
           const Candidate &cd = cands[ci];
-          S.pats.push_back(PatternRec{ p.pattern, cd.dfs, cd.support });
+          S.pats.push_back(PatternRec{ cd.support, cd.edge, p.pattern });
           const int32_t pid = (int32_t)S.pats.size() - 1;
           PatternRec &par = S.pats[p.pattern];
           if(par.last_child < 0) par.first_child = pid;
@@ -2205,11 +2294,11 @@ private:
           par.last_child = pid;
           const int32_t child_edges = (int32_t)p.code.size() + 1;
           if(max_edges > 0 && child_edges >= max_edges) continue;
-          if(child_edges >= kMaxPatternEdges || (cd.dfs.is_forward() && cd.dfs.to + 1 > 64))
+          if(child_edges >= kMaxPatternEdges || (cd.edge.is_forward() && cd.edge.to + 1 > 64))
             throw Error(ST_ERR_LIMIT, "pattern exceeds 64 vertices or 127 edges");
-          mats.push_back(Mat{ n, ci, pid });
+          mats.push_back(Scratch::Mat{ n, ci, pid });
           bytes += f.packed ? Carver::round((size_t)cd.cnt * 16 *
-                                            packed_planes(p.nv + (cd.dfs.is_forward() ? 1 : 0)))
+                                            packed_planes(p.nv + (cd.edge.is_forward() ? 1 : 0)))
                             : Carver::round((size_t)cd.cnt * 8) + Carver::round((size_t)cd.cnt * 4);
         }
         a0 = a1;
@@ -2217,15 +2306,15 @@ private:
       if(f.lists && f.rec && nrec >= 0 && nrec <= f.rec_cap) {
         list_rb.assign(W, -1);
         std::vector<char> need(W, 0);
-        for(const Mat &m : mats)
-          if(cands[m.cand].dfs.is_forward()) need[m.node] = 1;
+        for(const Scratch::Mat &m : mats)
+          if(cands[m.cand].edge.is_forward()) need[m.node] = 1;
         for(int32_t n = 0; n < W; n++)
           if(need[n]) {
             list_rb[n] = (int32_t)list_rows;
             list_rows += pn_[nodes[n]].nrows;
           }
         for(const Candidate &cd : cands)
-          if(need[cd.node] && cd.key < lays[cd.node].nfwd) list_n += cd.cnt;
+          if(need[cd.node] && cd.key < pn_[nodes[cd.node]].nfwd) list_n += cd.cnt;
         if(list_rows > 0 && list_rows + 1 < INT32_MAX && list_n < INT32_MAX) {
           const size_t lb = Carver::round(sizeof(int32_t) * (size_t)(list_rows + 1)) +
                             Carver::round(sizeof(int2) * (size_t)std::max<int64_t>(list_n, 1)) +
@@ -2244,9 +2333,12 @@ private:
         const int32_t blk = E.new_block(bytes);
         Carver cv{ (char *)E.blocks[blk].base };
         made.reserve(mats.size());
-        outs.reserve(mats.size());
-        pairs.reserve(mats.size());
-        for(const Mat &m : mats) {
+        outs_bytes = Carver::round(sizeof(ChildOut) * mats.size());
+        pairs_bytes = Carver::round(sizeof(int2) * mats.size());
+        X.h_mat.ensure(outs_bytes + pairs_bytes + (list_blk >= 0 ? Carver::round(sizeof(int32_t) * (size_t)W) : 0));
+        outs = (ChildOut *)X.h_mat.p;
+        pairs = (int2 *)(X.h_mat.p + outs_bytes);
+        for(const Scratch::Mat &m : mats) {
           made_at[m.node + 1]++;
           const Candidate &cd = cands[m.cand];
           PNode &p = pn_[nodes[m.node]];
@@ -2254,8 +2346,8 @@ private:
           const int64_t rowsn = cd.cnt;
           ChildOut o{};
           o.cap = (int32_t)rowsn;
-          o.kind = cd.dfs.is_forward() ? 0 : 1;
-          const int32_t nv = p.nv + (cd.dfs.is_forward() ? 1 : 0);
+          o.kind = cd.edge.is_forward() ? 0 : 1;
+          const int32_t nv = p.nv + (cd.edge.is_forward() ? 1 : 0);
           if(f.packed) {
             // algorithmic bytes of a child row: its parent's, the rank's bitmap
             // word and prefix, the row written
@@ -2270,26 +2362,27 @@ private:
             o.col = cv.take<int2>(rowsn);
             o.gord = cv.take<int32_t>(rowsn);
           }
-          pairs.push_back(make_int2(hn[m.node].key_base + cd.key, (int32_t)outs.size()));
-          outs.push_back(o);
+          pairs[nout] = make_int2(hn[m.node].key_base + cd.key, (int32_t)nout);
+          outs[nout++] = o;
           const int32_t nid = pn_new();
           PNode &nn = pn_[nid];
           nn.job = p.job;
           nn.pattern = m.pid;
           nn.code.reserve(p.code.size() + 1);
           nn.code.assign(p.code.data(), p.code.size());
-          nn.code.push_back(cd.dfs);
-          nn.nv = nv;
+          nn.code.push_back(cd.edge);
+          child_layout(nn, p, cd, *S.job.db);
           if(f.packed) {
             nn.rows = o.rows;
             S.live_bytes += rowsn * 16 * o.planes;
           } else {
             // forward children append a column, backward children replace the last
-            const size_t keep = cd.dfs.is_forward() ? p.cols.size() : p.cols.size() - 1;
-            nn.cols.reserve(keep + 1);
-            nn.cols.assign(p.cols.data(), keep);
-            nn.cols.push_back(ColRef{ o.col, rowsn });
-            nn.last_col = E.new_col(o.col, rowsn, blk, cd.dfs.is_forward() ? p.last_col : E.cols[p.last_col].parent);
+            const size_t keep = cd.edge.is_forward() ? p.cols->size() : p.cols->size() - 1;
+            SmallVec<ColRef, 12> &nc = cols_of(nn);
+            nc.reserve(keep + 1);
+            nc.assign(p.cols->data(), keep);
+            nc.push_back(ColRef{ o.col, rowsn });
+            nn.last_col = E.new_col(o.col, rowsn, blk, cd.edge.is_forward() ? p.last_col : E.cols[p.last_col].parent);
             nn.gord = o.gord;
             S.live_bytes += rowsn * (int64_t)(sizeof(int2) + sizeof(int32_t));
           }
@@ -2297,27 +2390,24 @@ private:
           E.block_ref(blk);
           nn.nrows = rowsn;
           nn.support = cd.support;
-          if(list_blk >= 0 && cd.dfs.is_forward() && list_rb[m.node] >= 0) {
+          if(list_blk >= 0 && cd.edge.is_forward() && list_rb[m.node] >= 0) {
             nn.list_blk = list_blk;
             E.block_ref(list_blk);
             nn.list_off = list_off + list_rb[m.node];
             nn.list_ent = list_ent;
             nn.list_rows = p.nrows;
+            nn.join_lo = nn.join_hi = 0;
             // the child's right-most path up to the new edge's source u is
             // the parent's, with the same forward keys: the parent's keys
             // from u's slot and the slots before it stay keys of the child
             // (from u only those at or after the new edge's pair)
             // (gspan_cuda_lists.cpp:327-369 possible_extension, 372-443 the
             // forward-forward joins)
-            const NodeLayout &Lp = lays[m.node];
-            for(const SlotDesc &sd : Lp.slots) {
-              const int32_t hi = sd.fkey_off + S.job.db->pair_cnt[sd.vlab];
-              if(cd.key >= sd.fkey_off && cd.key < hi) {
-                nn.join_lo = sd.fkey_off;
-                nn.join_key = cd.key;
-                nn.join_hi = hi;
-              }
+            for(int32_t q = 0; q <= cd.slot; q++) {
+              nn.join_lo = nn.join_hi;
+              nn.join_hi += S.job.db->pair_cnt[p.slots[q].vlab];
             }
+            nn.join_key = cd.key;
           }
           S.peak_bytes = std::max(S.peak_bytes, S.live_bytes);
           made.push_back(nid);
@@ -2325,24 +2415,18 @@ private:
       }
       for(int32_t n = 0; n < W; n++) made_at[n + 1] += made_at[n];
     }
-    if(!outs.empty()) {
+    if(nout > 0) {
       // an item and its child map entry per extension
       if(f.packed) st_.mat_bytes += 8 * n_ext;
-      // one table: children's outputs, then the (key, child) pairs
-      const size_t outs_bytes = Carver::round(sizeof(ChildOut) * outs.size());
-      const size_t pairs_bytes = Carver::round(sizeof(int2) * pairs.size());
       const size_t mat_bytes = outs_bytes + pairs_bytes + (list_blk >= 0 ? Carver::round(sizeof(int32_t) * (size_t)W) : 0);
       X.d_mat.ensure(mat_bytes);
-      X.h_mat.ensure(mat_bytes);
-      std::memcpy(X.h_mat.p, outs.data(), sizeof(ChildOut) * outs.size());
-      std::memcpy(X.h_mat.p + outs_bytes, pairs.data(), sizeof(int2) * pairs.size());
       if(list_blk >= 0) std::memcpy(X.h_mat.p + outs_bytes + pairs_bytes, list_rb.data(), sizeof(int32_t) * W);
       const ChildOut *douts = (const ChildOut *)X.d_mat.p;
-      X.d_cursor.ensure(outs.size());
+      X.d_cursor.ensure(nout);
       st_.h2d_bytes += (int64_t)mat_bytes;
       unsigned long long *const stamps = E.d_stamps.p + (size_t)c * kMatStampWords;
-      launch_children(X.d_mat.p, X.h_mat.p, (long long)mat_bytes / 16, (const int2 *)(X.h_mat.p + outs_bytes),
-                      (int32_t)pairs.size(), X.d_childmap.p, f.chosen, X.d_cursor.p, (int32_t)outs.size(), stamps, st);
+      launch_children(X.d_mat.p, X.h_mat.p, (long long)mat_bytes / 16, pairs, (int32_t)nout, X.d_childmap.p, f.chosen,
+                      X.d_cursor.p, (int32_t)nout, stamps, st);
       // lists strategy: the records pass also counts the list rows
       ListBuild lb{ X.d_lnode.p, f.dn, (const int32_t *)(X.d_mat.p + outs_bytes + pairs_bytes) };
       if(list_blk >= 0) CK(cudaMemsetAsync(list_off, 0, sizeof(int32_t) * (size_t)(list_rows + 1), st));
@@ -2381,7 +2465,7 @@ private:
     }
     // the parents are done: drop their column references and graph ranks
     // (stream order keeps the materialise kernel ahead of any reuse)
-    std::vector<int32_t> &touched = w_touched_;
+    std::vector<int32_t> &touched = E.scratch.touched;
     touched.clear();
     for(int32_t n = W - 1; n >= 0; n--) {
       JobState &S = *jobs_[pn_[nodes[n]].job];
@@ -2413,7 +2497,8 @@ private:
     if(!j.emit) return;
     r1 = std::min(r1, S.roots.size());
     const LabelMap &lm = j.db->labels;
-    std::vector<DFS> path, styled, orig;
+    std::vector<CEdge> path;
+    std::vector<DFS> styled, orig;
     std::vector<int32_t> flat;
     struct Frame { int32_t pat; int32_t next; };
     std::vector<Frame> st;
@@ -2422,10 +2507,8 @@ private:
       styled.resize(n);
       orig.resize(n);
       for(size_t i = 0; i < n; i++) {
-        orig[i] = path[i];
-        orig[i].fromlabel = lm.vlabel_of[path[i].fromlabel];
-        orig[i].tolabel = lm.vlabel_of[path[i].tolabel];
-        orig[i].elabel = lm.elabel_of[path[i].elabel];
+        orig[i] = DFS{ path[i].from, path[i].to, lm.vlabel_of[path[i].fl], lm.elabel_of[path[i].el],
+                       lm.vlabel_of[path[i].tl] };
       }
       to_style(orig.data(), (int)n, (LabelStyle)j.opt.label_style, styled.data());
       flat.resize(n * 5);

@@ -71,6 +71,7 @@ struct Database {
   // pairs[a] = sorted (elabel, tolabel) pairs occurring next to label-a vertices
   std::vector<std::vector<std::pair<int32_t, int32_t>>> pairs;
   std::vector<int32_t> pair_cnt, root_off;
+  std::vector<int32_t> pair_code;  // [root_keys] (elabel << 16) | tolabel of each label's pairs, from root_off
   std::vector<int32_t> pair_tab;  // [VL * EL * VL] index of a label's (elabel, tolabel) in pairs, small alphabets only
   int32_t root_keys = 0;
   // device copy

@@ -340,7 +340,7 @@ __device__ int warp_is_min(MinSmem &S, int n, int lane)
 __global__ void __launch_bounds__(kMinWarps * 32) k_is_min(const NodeDesc *__restrict__ nodes, int nnodes,
                                                            const SlotDesc *__restrict__ slots,
                                                            const DevDB *__restrict__ dbs,
-                                                           const int32_t *__restrict__ codes, int4 *sel,
+                                                           const uint2 *__restrict__ codes, int4 *sel,
                                                            int sel_cap, unsigned long long *head, int check,
                                                            const ResultsOut out)
 {
@@ -362,14 +362,16 @@ __global__ void __launch_bounds__(kMinWarps * 32) k_is_min(const NodeDesc *__res
     if(check && n <= kMinE) {
       // the parent's code, then the candidate edge decoded from its key
       for(int t = lane; t < len; t += 32) {
-        const int32_t *c = codes + 5 * ((long long)nd.code_off + t);
-        const bool fwd = c[0] < c[1];
-        S.cf[t] = c[0];
-        S.ct[t] = c[1];
-        S.cel[t] = c[3];
-        S.ctl[t] = fwd ? c[4] : -1;
-        if(t == 0) S.vlab[c[0]] = c[2];
-        if(fwd && c[1] < kMinV) S.vlab[c[1]] = c[4];
+        // a code edge: from, to (bytes), edge label | from label, to label
+        const uint2 c = codes[(long long)nd.code_off + t];
+        const int f = (int)(c.x & 0xffu), to = (int)((c.x >> 8) & 0xffu);
+        const bool fwd = f < to;
+        S.cf[t] = f;
+        S.ct[t] = to;
+        S.cel[t] = (int)(c.x >> 16);
+        S.ctl[t] = fwd ? (int)(c.y >> 16) : -1;
+        if(t == 0) S.vlab[f] = (int)(c.y & 0xffffu);
+        if(fwd && to < kMinV) S.vlab[to] = (int)(c.y >> 16);
       }
       const DevDB &db = dbs[nd.db];
       const int kl = x.x - nd.key_base, maxtoc = nd.k - 1;
@@ -446,7 +448,7 @@ __global__ void __launch_bounds__(kMinWarps * 32) k_is_min(const NodeDesc *__res
 }  // namespace
 
 KernelCall is_min_call(const NodeDesc *nodes, int32_t nnodes, const SlotDesc *slots, const DevDB *dbs,
-                       const int32_t *codes, int4 *sel, int32_t sel_cap, unsigned long long *head, bool check,
+                       const uint2 *codes, int4 *sel, int32_t sel_cap, unsigned long long *head, bool check,
                        const ResultsOut &out)
 {
   const size_t smem = sizeof(MinSmem) * kMinWarps;

@@ -168,7 +168,8 @@ KernelCall count_listed_call(const NodeDesc *nodes, const int2 *listed, const ui
 // Canonicality of the selected candidates (gs_ismin.cu) and the wave's results:
 // the low two bits of sel[i].w (above them the candidate's node) = 1 minimal, 0
 // not minimal, 2 left to the host (all of them when !check).  codes = the
-// wave's code table.  The first hcap candidates and then the header go to
+// wave's code table (a uint2 per edge: from | to << 8 | edge label << 16, from
+// label | to label << 16).  The first hcap candidates and then the header go to
 // pinned host memory (hsel, hhead), with bytes = the column kernels' byte
 // counters and stamps = every context's materialise stamps, the sequence word
 // last.
@@ -182,7 +183,7 @@ struct ResultsOut {
   int nctx;
 };
 KernelCall is_min_call(const NodeDesc *nodes, int32_t nnodes, const SlotDesc *slots, const DevDB *dbs,
-                       const int32_t *codes, int4 *sel, int32_t sel_cap, unsigned long long *head, bool check,
+                       const uint2 *codes, int4 *sel, int32_t sel_cap, unsigned long long *head, bool check,
                        const ResultsOut &out);
 // Children to materialise: their tables (n16 16-byte pieces, in pinned host
 // memory) copied to dst, childmap[pairs[i].x] = pairs[i].y, cursor[0..ncursor)

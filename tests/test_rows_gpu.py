@@ -122,3 +122,20 @@ def test_more_results_than_room(gs, kw):
         parts = [st[k] for k in ("count_ms", "sel_ms", "min_ms", "mat_ms", "root_ms")]
         assert min(parts) > 0 and sum(parts) <= st["wall_ms"]
     gs.engine_reset()
+
+
+def test_nodes_reused_across_formats(gs, tmp_path):
+    # the engine keeps its DFS-tree nodes between runs: packed and column runs
+    # of different depth, one after the other, take each other's nodes
+    r = random.Random(11)
+    small, large = str(tmp_path / "s.txt"), str(tmp_path / "l.txt")
+    _write(small, _random_graphs(r, 60, (10, 40), 2, 2))
+    _write(large, _random_graphs(r, 40, (66, 80), 2, 2))
+    a, b = gs.Database.load(small, "txt"), gs.Database.load(large, "txt")
+    runs = [(a, 30, {"max_edges": 6}), (b, 30, {"max_edges": 4}), (a, 30, {"max_edges": 6, "extension": "lists"}),
+            (a, 20, {"max_edges": 4, "wave_nodes": 7})]
+    gs.engine_reset()
+    want = [gs.mine(d, s, **kw)[0] for d, s, kw in runs]
+    for (d, s, kw), pats in list(zip(runs, want))[::-1]:
+        assert gs.mine(d, s, **kw)[0] == pats
+    assert want[0] == want[2]
