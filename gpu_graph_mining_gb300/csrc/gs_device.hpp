@@ -132,13 +132,6 @@ struct NodeDesc {
   int32_t join_lo;         // first forward key of u
   int32_t join_key;        // the new edge's key (in the parent)
   int32_t join_hi;         // one past u's forward keys
-  // packed rows (rows == nullptr: the node has columns)
-  const uint4 *rows;         // planes of nrows
-  const uint4 *nb;           // its database's neighbour blocks,
-  const int32_t *pair_code;  //   pair codes,
-  int32_t nb_blocks, nb_shift, n_vertices;
-  int32_t planes;
-  int32_t back;              // 1: some slot takes a backward edge
 };
 
 // One right-most-path vertex of a node.  The order rules of the
@@ -149,14 +142,30 @@ struct NodeDesc {
 //   backward allowed iff el_u < el || (el_u == el && tl_u <= label(right-most))
 //     <=>  el >= bmin
 struct alignas(16) SlotDesc {
-  int32_t vertex;    // pattern vertex id
-  int32_t vlab;      // its (dense) label
-  int32_t fkey_off;  // forward keys of this slot: fkey_off + pair_idx(vlab, el, tl)
-  int32_t bkey_off;  // backward keys to this vertex: bkey_off + el; -1 if not a target
-  int32_t frule;
-  int32_t bmin;
   int32_t prule;     // packed rows: the least neighbour entry that the forward rule allows
+  int32_t fkey_off;  // forward keys of this slot: fkey_off + pair_idx(vlab, el, tl)
+  int32_t vertex;    // pattern vertex id
+  int32_t bkey_off;  // backward keys to this vertex: bkey_off + el; -1 if not a target
+  int32_t bmin;
   int32_t pbase;     // the first pair code of the vertex's label
+  int32_t frule;
+  int32_t vlab;      // its (dense) label
+};
+
+// What the packed-row count needs of a node, copied to shared memory whole.
+struct alignas(16) PackedNode {
+  const uint4 *rows;         // planes of nrows
+  const uint4 *nb;           // its database's neighbour blocks
+  int32_t nrows, k, nslot, planes;
+  int32_t nb_shift;
+  uint32_t minl;             // forward targets: entry label field >= minl
+  int32_t back;              // 1: some slot takes a backward edge
+  int32_t words;             // bitmap words per key
+  long long bm_base;
+  int32_t key_base;
+  int32_t n_vertices;
+  const int32_t *pair_code;
+  int32_t nb_blocks, slot_off;
 };
 
 // Output slots of a child node selected for materialisation.

@@ -868,7 +868,8 @@ struct Flight {
   const SlotDesc *ds = nullptr;
   const int32_t *dv = nullptr, *dl = nullptr;
   bool packed = false;       // the wave's nodes have packed rows
-  const int32_t *dt = nullptr;  // packed: first tile of each node
+  const int32_t *dt = nullptr;  // packed: first tile of each node,
+  const PackedNode *dp = nullptr;  //   and what the count needs of it
   int32_t planes = 1;        // packed: the most planes of a node's rows
   int4 *hdr = nullptr;       // packed: record headers (rec_cap counts the blocks of one region)
   uint32_t *reg = nullptr;   // packed: the regions' block counters
@@ -1893,8 +1894,8 @@ private:
     }
     size_t off = 0;
     const bool packed = format == 1;
-    size_t need = 256 * 8 + sizeof(NodeDesc) * W + sizeof(int2 *) * tot_cols + sizeof(SlotDesc) * tot_slots +
-                  2 * sizeof(int32_t) * tot_cols + sizeof(CEdge) * tot_edges + sizeof(int32_t) * W;
+    size_t need = 256 * 9 + sizeof(NodeDesc) * W + sizeof(int2 *) * tot_cols + sizeof(SlotDesc) * tot_slots +
+                  2 * sizeof(int32_t) * tot_cols + sizeof(CEdge) * tot_edges + (sizeof(int32_t) + sizeof(PackedNode)) * W;
     X.h_desc.ensure(need);
     X.d_desc.ensure(need);
     char *hb = X.h_desc.p;
@@ -1905,6 +1906,7 @@ private:
     int32_t *hl = carve<int32_t>(hb, off, tot_cols);
     CEdge *hcode = carve<CEdge>(hb, off, (size_t)tot_edges);
     int32_t *ht = carve<int32_t>(hb, off, packed ? W : 0);
+    PackedNode *hp = carve<PackedNode>(hb, off, packed ? W : 0);
     const size_t desc_bytes = Carver::round(off);
     int32_t planes = 1;
     int32_t eo = 0;
@@ -1964,18 +1966,27 @@ private:
       }
       if(packed) {
         ht[n] = (int32_t)tb;
-        d.back = back ? 1 : 0;
-        d.rows = p.rows;
-        d.nb = db.dev.nb;
-        d.pair_code = db.dev.pair_code;
-        d.nb_blocks = db.dev.nb_blocks;
-        d.nb_shift = db.dev.nb_shift;
-        d.n_vertices = db.dev.n_vertices;
-        d.planes = packed_planes(p.nv);
-        planes = std::max(planes, d.planes);
+        PackedNode &g = hp[n];
+        g.rows = p.rows;
+        g.nb = db.dev.nb;
+        g.nrows = d.nrows;
+        g.k = d.k;
+        g.nslot = d.nslot;
+        g.planes = packed_planes(p.nv);
+        g.nb_shift = db.dev.nb_shift;
+        g.minl = (uint32_t)d.minlabel << 6;
+        g.back = back ? 1 : 0;
+        g.words = d.words;
+        g.bm_base = bb;
+        g.key_base = kb;
+        g.n_vertices = db.dev.n_vertices;
+        g.pair_code = db.dev.pair_code;
+        g.nb_blocks = db.dev.nb_blocks;
+        g.slot_off = so;
+        planes = std::max(planes, g.planes);
         // algorithmic bytes: the row and one neighbour block per slot (an
         // extension's bitmap word, counter and record are added with the results)
-        st_.count_bytes += p.nrows * (16 * d.planes + 32 * d.nslot);
+        st_.count_bytes += p.nrows * (16 * g.planes + 32 * d.nslot);
       } else {
         co += d.k;
       }
@@ -1998,6 +2009,7 @@ private:
     f.dv = (const int32_t *)(db_ + ((char *)hv - hb));
     f.dl = (const int32_t *)(db_ + ((char *)hl - hb));
     f.dt = (const int32_t *)(db_ + ((char *)ht - hb));
+    f.dp = (const PackedNode *)(db_ + ((char *)hp - hb));
     f.packed = packed;
     f.planes = planes;
     if(tb >= INT32_MAX) throw Error(ST_ERR_LIMIT, "a wave has 2^36 or more embedding rows");
@@ -2080,7 +2092,7 @@ private:
     q.desc_bytes = desc_bytes;
     q.k[0] = begin_call(X.d_desc.p, hb, (long long)desc_bytes / 16, X.d_zero.p, (long long)zero_bytes / 16, head);
     if(packed)
-      q.k[1] = rows_count_call(f.dn, f.dt, W, (int32_t)tb, planes, f.ds, f.bm, cnt, cstride,
+      q.k[1] = rows_count_call(f.dp, f.dt, W, (int32_t)tb, planes, f.ds, f.bm, cnt, cstride,
                                 (uint32_t *)f.rec, f.hdr, (int32_t)f.rec_cap, f.reg, head, err_flag(), wo_.count_grid);
     else
       q.k[1] = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
@@ -2436,7 +2448,7 @@ private:
                               f.chosen, X.d_childmap.p, f.bm, X.d_bmx.p, f.cnt, f.cstride, douts, err_flag(), stamps,
                               st);
         } else {
-          launch_rows_materialize(f.dn, f.dt, W, (int32_t)f.tb, f.planes, f.ds, f.bm, X.d_bmx.p, f.chosen,
+          launch_rows_materialize(f.dp, f.dt, W, (int32_t)f.tb, f.planes, f.ds, f.bm, X.d_bmx.p, f.chosen,
                                   X.d_childmap.p, X.d_cursor.p, douts, err_flag(), stamps, st);
           if(f.rec)
             X.wanted_rec = std::max<long long>(X.wanted_rec, (nrec + nrec / 4) * kRecBlockInt4 * kRecRegions);

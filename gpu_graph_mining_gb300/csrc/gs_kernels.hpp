@@ -104,7 +104,8 @@ void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long to
                              unsigned long long *bytes, unsigned int *err, bool join, bool rule_skip,
                              unsigned long long *stamps, cudaStream_t s);
 
-// Packed rows (gs_rows.cu).  tile0[] = first 32-row tile of each node; planes =
+// Packed rows (gs_rows.cu).  nodes, tile0: every node's PackedNode and first
+// 32-row tile; planes =
 // the most planes of the wave's nodes' rows; rec / hdr: record blocks (rec may
 // be null) in kRecRegions regions of blk_cap blocks, reg[r * kRecRegionStride]
 // counts the blocks reserved in region r (zeroed before).  cnt: kRowsCopies
@@ -113,14 +114,14 @@ void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long to
 // 14% slower); the wave's keys stay below kRowsKeys.
 constexpr int kRecRegions = 64, kRecRegionStride = 32;
 constexpr int kRowsCopies = 4, kRowsKeys = 1 << 25;
-KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
+KernelCall rows_count_call(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                            int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, long long cnt_stride,
                            uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
                            unsigned long long *head, unsigned int *err, int32_t grid_per_sm);
 // Materialise by enumerating again (cursor per child), and from the record
 // blocks (cursor: the counter copies after selection, as for
 // launch_materialize_records).
-void launch_rows_materialize(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
+void launch_rows_materialize(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                              int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
                              const uint32_t *chosen, const int32_t *childmap, int32_t *cursor, const ChildOut *outs,
                              unsigned int *err, unsigned long long *stamps, cudaStream_t s);

@@ -8,10 +8,12 @@
 // loads (a sector each), then two offsets and about 21 bytes of entries per
 // right-most-path vertex, and every step of 32 entries searched owners and
 // emitted few extensions.  250,000 graphs of 40 edges at minsup 0.5% (192 M
-// rows, 760 M extensions, one stream): count kernels 33.3 ms on columns, 12.4
+// rows, 760 M extensions, one stream): count kernels 33.3 ms on columns, 11.4
 // here; a large launch 1.30 -> 0.46 ms with 989 M -> 402 M warp instructions
 // and 2.2 -> 0.9 GB of DRAM traffic.  It is bound by issue now (71% of
 // cycles, the integer pipe 69%; 0.24 of the DRAM peak).
+#include <algorithm>
+
 #include "gs_kernels.hpp"
 #include "gs_stamp.cuh"
 
@@ -30,13 +32,17 @@ namespace {
 #endif
 constexpr int kWarps = GS_ROWS_WARPS;
 constexpr unsigned kFull = 0xffffffffu;
+#ifndef GS_ROWS_GROUP
+#define GS_ROWS_GROUP 4  // tiles
+#endif
 constexpr int kRecBlocks = 4;  // record blocks a warp reserves at a time
 
 struct RowsArgs {
-  const NodeDesc *nodes;
+  const PackedNode *nodes;
   const int32_t *tile0;   // first 32-row tile of each node
   int nnodes;
   int total_tiles;
+  int group;              // consecutive tiles a warp takes at a time
   const SlotDesc *slots;
   uint32_t *bm;           // count: bitmaps to set; materialise: read
   const int32_t *bmx;     // materialise: prefix popcounts
@@ -60,10 +66,8 @@ template <int PL> struct RowsSmem {
   static constexpr int kSlots = PL == 1 ? 8 : PL == 2 ? 24 : 64;
   uint2 q[32 * 9];      // accepted items waiting for emission (31 and one block per lane):
                         // {entry, or backward key << 11; owner row | slot << 5 | kBackItem}
-  int4 slot[kSlots];    // {least entry allowed, key of entry 1 << shift, pattern vertex, backward keys or -1}
-  int2 slotb[kSlots];   // {least backward edge label, first pair code}
-  long long bm_base;    // the tile's node, for emission
-  int words, key_base;
+  PackedNode nd;        // the tile's node and its right-most path
+  SlotDesc slot[kSlots];
 };
 
 __device__ __forceinline__ unsigned lanemask_lt()
@@ -83,6 +87,14 @@ __device__ __forceinline__ int warp_incl(int x)
     asm volatile("{ .reg .s32 t; .reg .pred p; shfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff; @p add.s32 %0, %0, t; }"
                  : "+r"(x)
                  : "r"(o));
+  return x;
+}
+
+// 1 << n, 0 for n of 32 and more
+__device__ __forceinline__ unsigned shl_one(unsigned n)
+{
+  unsigned x;
+  asm("shl.b32 %0, 1, %1;" : "=r"(x) : "r"(n));
   return x;
 }
 
@@ -170,84 +182,92 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
     ahead = true;
   };
 
-  for(int tile = gwarp; tile < a.total_tiles; tile += nwarps) {
-    // ---- the tile's node (tiles never span nodes): a 32-way search
-    int lo = 0, hi = a.nnodes;  // the node is the last in [lo, hi) with tile0 <= tile
-    while(hi - lo > 1) {
-      const int step = (hi - lo + 31) >> 5;
-      const int probe = lo + lane * step;
-      const unsigned ok = __ballot_sync(kFull, probe < hi && __ldg(&a.tile0[probe]) <= tile);
-      lo += (31 - __clz(ok | 1u)) * step;
-      hi = min(hi, lo + step);
-    }
-    const int n = lo;
+  // Groups of consecutive tiles: while the node stays the same, so do its
+  // tables in shared memory (250,000 graphs: 12.3 ms in ones, 11.7 in twos,
+  // 11.4 in fours, 11.5 in eights).
+  int n = 0, n_first = 0, n_end = 0;  // the tables' node and its tiles
+  for(int t0 = gwarp * a.group; t0 < a.total_tiles; t0 += nwarps * a.group)
+  for(int tile = t0; tile < min(t0 + a.group, a.total_tiles); tile++) {
     if(!MAT && a.rec && blk_left < kRecBlocks && !ahead) reserve();
-    const NodeDesc &nd = a.nodes[n];
-    const int k = nd.k, nslot = nd.nslot, sh = nd.nb_shift;
-    if(k > RowsSmem<PL>::kSlots || nslot > RowsSmem<PL>::kSlots || k < 2 || nslot < 2 || nd.planes > PL) {
+    // ---- the tile's node (tiles never span nodes): a 32-way search
+    if(tile < n_first || tile >= n_end) {
+      int lo = 0, hi = a.nnodes;  // the node is the last in [lo, hi) with tile0 <= tile
+      while(hi - lo > 1) {
+        const int step = (hi - lo + 31) >> 5;
+        const int probe = lo + lane * step;
+        const unsigned ok = __ballot_sync(kFull, probe < hi && __ldg(&a.tile0[probe]) <= tile);
+        lo += (31 - __clz(ok | 1u)) * step;
+        hi = min(hi, lo + step);
+      }
+      n = lo;
+      n_first = __ldg(&a.tile0[n]);
+      n_end = n + 1 < a.nnodes ? __ldg(&a.tile0[n + 1]) : a.total_tiles;
+      __syncwarp();  // the previous node's tables have been read
+      constexpr int kNd = sizeof(PackedNode) / 16;
+      if(lane < kNd) reinterpret_cast<int4 *>(&S.nd)[lane] = __ldg(reinterpret_cast<const int4 *>(&a.nodes[n]) + lane);
+      __syncwarp();
+      const int4 *sd = reinterpret_cast<const int4 *>(a.slots + S.nd.slot_off);
+      for(int t = lane; t < 2 * min(S.nd.nslot, RowsSmem<PL>::kSlots); t += 32) reinterpret_cast<int4 *>(S.slot)[t] = __ldg(&sd[t]);
+      __syncwarp();
+    }
+    const int k = S.nd.k, nslot = S.nd.nslot, sh = S.nd.nb_shift;
+    if(k > RowsSmem<PL>::kSlots || nslot > RowsSmem<PL>::kSlots || k < 2 || nslot < 2 || S.nd.planes > PL) {
       if(lane == 0) atomicOr(a.err, 2u);
       continue;
     }
-    const int row0 = (tile - __ldg(&a.tile0[n])) * 32;
+    const int row0 = (tile - n_first) * 32;
     const int i = row0 + lane;
-    bool valid = i < nd.nrows;
+    bool valid = i < S.nd.nrows;
     unsigned w[NW];
 #pragma unroll
     for(int q = 0; q < NW; q++) w[q] = 0;
     int gb = 0, g = 0;
     if(valid) {
-      const uint4 r = __ldg(&nd.rows[i]);
+      const uint4 r = __ldg(&S.nd.rows[i]);
       gb = (int)r.x;
       g = (int)r.y;
       w[0] = r.z;
       w[1] = r.w;
 #pragma unroll
       for(int p = 1; p < PL; p++)
-        if(p < nd.planes) {
-          const uint4 x = __ldg(&nd.rows[(long long)p * nd.nrows + i]);
+        if(p < S.nd.planes) {
+          const uint4 x = __ldg(&S.nd.rows[(long long)p * S.nd.nrows + i]);
           w[4 * p - 2] = x.x;
           w[4 * p - 1] = x.y;
           w[4 * p] = x.z;
           w[4 * p + 1] = x.w;
         }
     }
-    __syncwarp();  // the previous tile's reads of the tables are done
-    for(int t = lane; t < nslot; t += 32) {
-      const SlotDesc &sd = a.slots[nd.slot_off + t];
-      S.slot[t] = make_int4(sd.prule, sd.fkey_off - 1, sd.vertex, sd.bkey_off);
-      S.slotb[t] = make_int2(sd.bmin, sd.pbase);
-    }
-    if(lane == 0) {
-      S.bm_base = nd.bm_base;
-      S.words = nd.words;
-      S.key_base = nd.key_base;
-    }
-    if(valid && (unsigned)g >= (unsigned)nd.words * 32u) {
-      atomicOr(a.err, 1u);
+    if(valid && ((unsigned)g >= (unsigned)S.nd.words * 32u || (unsigned)gb >= (unsigned)S.nd.n_vertices)) {
+      atomicOr(a.err, (unsigned)g >= (unsigned)S.nd.words * 32u ? 1u : 2u);
       valid = false;
     }
-    if(valid && (unsigned)gb >= (unsigned)nd.n_vertices) {
-      atomicOr(a.err, 2u);
-      valid = false;
-    }
-    unsigned long long mask = 0;  // the row's vertices
+    unsigned m_lo = 0, m_hi = 0;  // the row's vertices
     if(PL == 1) {
 #pragma unroll
       for(int t = 0; t < 8; t++)
-        if(t < k) mask |= 1ull << ((w[t >> 2] >> ((t & 3) * 8)) & 63u);
+        if(t < k) {
+          const unsigned lv = (w[t >> 2] >> ((t & 3) * 8)) & 0xffu;
+          m_lo |= shl_one(lv);
+          m_hi |= shl_one(lv - 32u);
+        }
     } else {
-      for(int t = 0; t < k; t++) mask |= 1ull << (id_of(w, t) & 63u);
+      for(int t = 0; t < k; t++) {
+        const unsigned lv = id_of(w, t);
+        m_lo |= shl_one(lv);
+        m_hi |= shl_one(lv - 32u);
+      }
     }
-    __syncwarp();
-    const bool back = nd.back != 0;
-    const uint4 *__restrict__ nb = nd.nb;
-    const unsigned wlm = (1u << sh) - 64u;           // the label field
-    const unsigned minl = (unsigned)nd.minlabel << 6;  // forward targets: label >= minlabel
+    const unsigned long long mask = ((unsigned long long)m_hi << 32) | m_lo;
+    const bool back = S.nd.back != 0;
+    const uint4 *__restrict__ nb = S.nd.nb;
+    const unsigned wlm = (1u << sh) - 64u;  // the label field
+    const unsigned minl = S.nd.minl;
 
     uint4 xa = make_uint4(0, 0, 0, 0), xb = xa;
     auto fetch = [&](int s) {
       if(valid) {
-        const long long v = (long long)gb + id_of(w, S.slot[s].z);
+        const long long v = (long long)gb + id_of(w, S.slot[s].vertex);
         xa = __ldg(&nb[2 * v]);
         xb = __ldg(&nb[2 * v + 1]);
       }
@@ -263,7 +283,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       if(cont && hops < 16) {  // (a list of 63 entries has 9 blocks)
         hops++;
         const unsigned b = x[7] & 0x7fffffffu;
-        const bool ok = (int)x[7] < 0 && b < (unsigned)nd.nb_blocks;
+        const bool ok = (int)x[7] < 0 && b < (unsigned)S.nd.nb_blocks;
         xa = xb = make_uint4(0, 0, 0, 0);
         if(ok) {
           xa = __ldg(&nb[2ll * b]);
@@ -276,16 +296,16 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
         more = false;
       }
       // ---- this block's entries that are forward extensions
-      const int4 sl = S.slot[s];
+      const int rule = S.slot[s].prule;
       unsigned acc = 0;
       if(minl == 0) {
 #pragma unroll
         for(int u = 0; u < 8; u++)
-          acc |= (int)x[u] >= sl.x && !((unsigned)(mask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
+          acc |= (int)x[u] >= rule && !((unsigned)(mask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
       } else {
 #pragma unroll
         for(int u = 0; u < 8; u++)
-          acc |= (int)x[u] >= sl.x && (x[u] & wlm) >= minl && !((unsigned)(mask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
+          acc |= (int)x[u] >= rule && (x[u] & wlm) >= minl && !((unsigned)(mask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
       }
       const int c = __popc(acc);
       const int incl = warp_incl(c);
@@ -301,7 +321,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       if(back && s == nslot - 1) {
         unsigned long long bmask = 0;  // the row's vertices that a backward edge may go to
         for(int t = 0; t + 2 < nslot; t++)
-          if(S.slot[t].w >= 0) bmask |= 1ull << (id_of(w, S.slot[t].z) & 63u);
+          if(S.slot[t].bkey_off >= 0) bmask |= 1ull << (id_of(w, S.slot[t].vertex) & 63u);
         unsigned bb = 0;
 #pragma unroll
         for(int u = 0; u < 8; u++)
@@ -315,10 +335,10 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
 #pragma unroll
             for(int q = 1; q < 8; q++) y = u == q ? x[q] : y;
             bb &= bb - 1;
-            const int el = __ldg(&nd.pair_code[S.slotb[s].y + (int)(y >> sh) - 1]) >> 16;
+            const int el = __ldg(&S.nd.pair_code[S.slot[s].pbase + (int)(y >> sh) - 1]) >> 16;
             for(int t = 0; t + 2 < nslot; t++)
-              if(S.slot[t].w >= 0 && id_of(w, S.slot[t].z) == (y & 63u) && el >= S.slotb[t].x) {
-                item = (unsigned)(S.slot[t].w + el) << 11;
+              if(S.slot[t].bkey_off >= 0 && id_of(w, S.slot[t].vertex) == (y & 63u) && el >= S.slot[t].bmin) {
+                item = (unsigned)(S.slot[t].bkey_off + el) << 11;
                 ok = true;
               }
           }
@@ -337,14 +357,14 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
           const uint2 e = S.q[qn - m + lane];
           it = e.y & 31u;
           if(e.y & kBackItem) it |= e.x;
-          else it |= ((unsigned)S.slot[e.y >> 5].y + (e.x >> sh)) << 11 | (e.x & 63u) << 5;
+          else it |= ((unsigned)S.slot[e.y >> 5].fkey_off - 1u + (e.x >> sh)) << 11 | (e.x & 63u) << 5;
         }
         qn -= m;
         __syncwarp();
         const int key = lane < m ? (int)(it >> 11) : -1;
         const int o = (int)(it & 31u);
         const int g_o = __shfl_sync(kFull, g, o);
-        const int key_base = S.key_base;
+        const int key_base = S.nd.key_base;
         if(!MAT) {
           // one counter add per distinct key, into this warp's copy of the
           // counters, and one bitmap OR unless a lane's graph differs from its key
@@ -353,7 +373,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
           const int leader = __ffs(peers) - 1;
           const int g_lead = __shfl_sync(kFull, g_o, leader);
           if(key >= 0 && (lane == leader || g_o != g_lead))
-            atomicOr(&a.bm[S.bm_base + (long long)key * S.words + (g_o >> 5)], 1u << (g_o & 31));
+            atomicOr(&a.bm[S.nd.bm_base + (long long)key * S.nd.words + (g_o >> 5)], 1u << (g_o & 31));
           if(key >= 0 && lane == leader) atomicAdd(&a.cnt[(gwarp % kRowsCopies) * a.cnt_stride + key_base + key], __popc(peers));
           if(a.rec) {
             if(blk_left == 0) {
@@ -363,8 +383,8 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
               ahead = false;
             }
             if(blk < a.blk_cap) {  // past the region's end nothing is written
-              const long long b = (long long)region * a.blk_cap + blk;
-              a.rec[b * 32 + lane] = it;
+              const unsigned b = (unsigned)region * (unsigned)a.blk_cap + (unsigned)blk;  // (below 2^26 blocks)
+              a.rec[b * 32u + (unsigned)lane] = it;
               if(lane == 0) a.hdr[b] = make_int4(row0, n, m | (gwarp % kRowsCopies) << 8, key_base);
             }
             blk++;
@@ -578,10 +598,12 @@ __global__ void __launch_bounds__(256) k_neighbour_blocks(const int32_t *__restr
   }
 }
 
-template <int PL, bool MAT> KernelCall rows_call(const RowsArgs &a, int grid_per_sm)
+template <int PL, bool MAT> KernelCall rows_call(RowsArgs a, int grid_per_sm)
 {
-  long long blocks = ((long long)a.total_tiles + kWarps - 1) / kWarps;
   const long long cap = (long long)sm_count() * (grid_per_sm > 0 ? grid_per_sm : GS_ROWS_GRID);
+  // in groups once every warp of a full grid has one: below that the chip would idle
+  a.group = (int)std::max(1ll, std::min((long long)GS_ROWS_GROUP, a.total_tiles / (cap * kWarps)));
+  long long blocks = ((long long)a.total_tiles + kWarps * a.group - 1) / (kWarps * a.group);
   blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
   KernelCall c;
   c.func = (const void *)k_rows<PL, MAT>;
@@ -593,25 +615,25 @@ template <int PL, bool MAT> KernelCall rows_call(const RowsArgs &a, int grid_per
 
 }  // namespace
 
-KernelCall rows_count_call(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
+KernelCall rows_count_call(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                            int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, long long cnt_stride,
                            uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
                            unsigned long long *head, unsigned int *err, int32_t grid_per_sm)
 {
-  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, bm, nullptr, cnt, cnt_stride, nullptr, nullptr,
+  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, 1, slots, bm, nullptr, cnt, cnt_stride, nullptr, nullptr,
                     nullptr, nullptr, rec, hdr, blk_cap, reg, err, head + kHeadCount0 };
   if(planes <= 1) return rows_call<1, false>(a, grid_per_sm);
   if(planes <= 2) return rows_call<2, false>(a, grid_per_sm);
   return rows_call<5, false>(a, grid_per_sm);
 }
 
-void launch_rows_materialize(const NodeDesc *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
+void launch_rows_materialize(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                              int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
                              const uint32_t *chosen, const int32_t *childmap, int32_t *cursor, const ChildOut *outs,
                              unsigned int *err, unsigned long long *stamps, cudaStream_t s)
 {
   if(total_tiles <= 0) return;
-  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, slots, const_cast<uint32_t *>(bm), bmx, nullptr, 0, chosen,
+  const RowsArgs a{ nodes, tile0, nnodes, total_tiles, 1, slots, const_cast<uint32_t *>(bm), bmx, nullptr, 0, chosen,
                     childmap, cursor, outs, nullptr, nullptr, 0, nullptr, err, stamps };
   KernelCall c = planes <= 1 ? rows_call<1, true>(a, 0) : planes <= 2 ? rows_call<2, true>(a, 0) : rows_call<5, true>(a, 0);
   c.run(s);
