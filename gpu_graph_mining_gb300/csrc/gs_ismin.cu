@@ -9,17 +9,30 @@
 // minimum code in the pattern, and compare each new edge with the
 // candidate's edge at the same position (from the second edge on).
 //
-// Warp-parallel form.  The pattern (at most 32 vertices and 64 edges here)
-// lives in shared memory as an adjacency list in code order.  The lanes split
-// the embeddings of the partial minimum code; each step takes the
-// lexicographic minimum of the lanes' best extensions with one warp
-// reduction (backward: by edge label; forward: by (edge label, to label)
-// packed into one integer), and the embeddings of the chosen edge are
-// appended to the other buffer with warp-aggregated positions.  An
-// embedding records only its vertex map and used-vertex / used-edge bit
-// sets: the labels of the minimum code's edges are the minimum code's own.
-// A candidate whose pattern is larger, or whose embeddings outgrow the
-// buffer, is left to the host checker (verdict 2).
+// Warp-parallel form.  The pattern (at most 32 vertices and 64 edges here, a
+// simple graph) lives in shared memory as its directed edges.  An embedding of
+// the partial minimum code is the inverse map, pattern vertex -> minimum-code
+// vertex, and the set of pattern edges used.  One pass looks at every
+// (embedding, directed edge) pair, a pair per lane: it is a backward edge to a
+// right-most-path vertex, a forward edge from one, or nothing, which two map
+// bytes, the edge bit and one compare with the path edge that leaves that
+// vertex decide.  The path itself is a bit mask, and its edges (edge label, to
+// label, one word) are a register of the lane numbered like the vertex they
+// leave.  The next minimum-code edge is two warp reductions over the pairs
+// (backward before forward, backward nearest the root first, forward deepest
+// first; then the labels), is compared with the candidate's, and only then are
+// the pairs that match it appended to the other buffer.  Typically one
+// embedding and fewer than 32 directed edges: a step is one pass.  A candidate
+// whose pattern is larger, or whose embeddings outgrow the buffer, is left to
+// the host checker (verdict 2).
+//
+// What bounds it is the latency of one candidate's chain of steps: a wave has
+// hundreds of candidates, the chip a thousand warps and more.  A lane per
+// embedding that walked path and adjacency serially took 26 us a wave on 64
+// small databases mined as a batch (2.2 ms a mine, one stream), this 9.8 (0.81
+// ms); 250,000 graphs at 0.5%: 0.85 -> 0.31 ms; 100,000 at 1%: 0.25 -> 0.11.
+#include <algorithm>
+
 #include "gs_kernels.hpp"
 #include "gs_stamp.cuh"
 
@@ -29,30 +42,22 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMinWarps = 4;
+constexpr int kMinGrid = 4;   // thread blocks per SM
 constexpr int kMinV = 32;     // pattern vertices checked on the GPU
 constexpr int kMinE = 64;     // pattern edges checked on the GPU
 constexpr int kMinCap = 128;  // embeddings per buffer
 
-struct MEmb {
-  uint8_t map[kMinV];  // minimum-code vertex -> pattern vertex
-  uint32_t vmask;      // pattern vertices used
-  uint32_t pad;
+struct alignas(16) MEmb {
+  uint8_t inv[kMinV];  // pattern vertex -> minimum-code vertex + 1, 0 = not used
   uint64_t emask;      // pattern edges used
+  uint64_t pad;
 };
 
 struct MinSmem {
   MEmb buf[2][kMinCap];
-  uint32_t adj[2 * kMinE];  // (edge label << 16) | (edge id << 8) | neighbour
-  int32_t aoff[kMinV + 1];
+  uint2 de[2 * kMinE];  // directed edges: {from | to << 8 | edge << 16, edge label << 16 | to's label}
+  uint2 code[kMinE];    // the candidate's code: {from | to << 8, edge label << 16 | to label, 0 if backward}
   int32_t vlab[kMinV];
-  // the candidate code, sequential-reference style: to label -1 for backward edges
-  int32_t cf[kMinE], ct[kMinE], cel[kMinE], ctl[kMinE];
-  // the minimum code built so far
-  int32_t mf[kMinE], mt[kMinE], mel[kMinE];
-  int32_t rm[kMinE];
-  int32_t nrm;
-  int32_t ncur;
-  int32_t nnext;
 };
 
 __device__ __forceinline__ unsigned lanemask_lt()
@@ -72,266 +77,142 @@ __device__ __forceinline__ int node_of_key(const NodeDesc *nodes, int n, int key
   return lo;
 }
 
-// appends a copy of `src` (extended as given) to the next buffer; the warp
-// calls it converged, `take` says which lanes append.  Returns false if the
-// buffer overflowed.
-__device__ __forceinline__ bool append(MinSmem &S, int nb, bool take, const MEmb &src, int newv, int pv, int eid,
-                                       int lane)
-{
-  const unsigned m = __ballot_sync(kFull, take);
-  const int base = S.nnext;
-  const int pos = base + __popc(m & lanemask_lt());
-  if(take && pos < kMinCap) {
-    MEmb &d = S.buf[nb][pos];
-    d = src;
-    if(newv >= 0) {
-      d.map[newv] = (uint8_t)pv;
-      d.vmask |= 1u << pv;
-    }
-    d.emask |= 1ull << eid;
-  }
-  __syncwarp();
-  if(lane == 0) S.nnext = base + __popc(m);
-  __syncwarp();
-  return base + __popc(m) <= kMinCap;
-}
-
 // 1 minimal, 0 not minimal, 2 left to the host
 __device__ int warp_is_min(MinSmem &S, int n, int lane)
 {
-  // ---- pattern graph: labels and adjacency in code order
-  int nv = 0;
-  for(int i = 0; i < n; i++) nv = max(nv, max(S.cf[i], S.ct[i]) + 1);
-  if(nv > kMinV) return 2;
-  if(lane == 0) {
-    for(int v = 0; v <= nv; v++) S.aoff[v] = 0;
-    for(int i = 0; i < n; i++) {
-      S.aoff[S.cf[i] + 1]++;
-      S.aoff[S.ct[i] + 1]++;
-    }
-    for(int v = 0; v < nv; v++) S.aoff[v + 1] += S.aoff[v];
-    int fill[kMinV];
-    for(int v = 0; v < nv; v++) fill[v] = S.aoff[v];
-    for(int i = 0; i < n; i++) {
-      const uint32_t e = ((uint32_t)S.cel[i] << 16) | ((uint32_t)i << 8);
-      S.adj[fill[S.cf[i]]++] = e | (uint32_t)S.ct[i];
-      S.adj[fill[S.ct[i]]++] = e | (uint32_t)S.cf[i];
-    }
-  }
-  __syncwarp();
   const int na = 2 * n;
-  int maxdeg = 0;
-  for(int v = 0; v < nv; v++) maxdeg = max(maxdeg, S.aoff[v + 1] - S.aoff[v]);
-
-  // ---- first edge: minimum (from label, edge label, to label) with from label <= to label
-  unsigned long long best = ~0ull;
+  const unsigned by_na = 0xffffffffu / (unsigned)na + 1u;  // i / na == umulhi(i, by_na): i < kMinCap * na
   for(int t = lane; t < na; t += 32) {
-    int v = 0;
-    while(S.aoff[v + 1] <= t) v++;
-    const uint32_t a = S.adj[t];
-    const int to = a & 0xff, el = a >> 16;
-    if(S.vlab[v] > S.vlab[to]) continue;
-    const unsigned long long k = ((unsigned long long)S.vlab[v] << 32) | ((unsigned long long)el << 16) | S.vlab[to];
-    best = min(best, k);
+    const uint2 c = S.code[t >> 1];
+    const int f = c.x & 0xff, w = (c.x >> 8) & 0xff, from = t & 1 ? w : f, to = t & 1 ? f : w;
+    S.de[t] = make_uint2((unsigned)(from | to << 8 | (t >> 1) << 16), (c.y & 0xffff0000u) | (unsigned)S.vlab[to]);
   }
-  for(int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(kFull, best, o));
-  if(best == ~0ull) return 2;
-  const int b0 = (int)(best >> 32), b1 = (int)((best >> 16) & 0xffff), b2 = (int)(best & 0xffff);
-  if(lane == 0) S.nnext = 0;
-  __syncwarp();
+  // ---- first edge: minimum (from label, edge label, to label) with from label <= to label
+  unsigned bf = ~0u, bl = ~0u;
+  for(int t = lane; t < na; t += 32) {
+    const uint2 d = S.de[t];
+    const unsigned fl = (unsigned)S.vlab[d.x & 0xff];
+    if(fl <= (d.y & 0xffffu) && (fl < bf || (fl == bf && d.y < bl))) {
+      bf = fl;
+      bl = d.y;
+    }
+  }
+  const unsigned minlabel = __reduce_min_sync(kFull, bf);
+  if(minlabel == ~0u) return 2;
+  const unsigned first = __reduce_min_sync(kFull, bf == minlabel ? bl : ~0u);
+  int ncur = 0;
   for(int t0 = 0; t0 < na; t0 += 32) {
     const int t = t0 + lane;
-    bool take = false;
-    int v = 0, to = 0, id = 0;
-    if(t < na) {
-      while(S.aoff[v + 1] <= t) v++;
-      const uint32_t a = S.adj[t];
-      to = a & 0xff;
-      id = (a >> 8) & 0xff;
-      take = S.vlab[v] <= S.vlab[to] && S.vlab[v] == b0 && (int)(a >> 16) == b1 && S.vlab[to] == b2;
+    uint2 d = make_uint2(0, 0);
+    if(t < na) d = S.de[t];
+    const int v = d.x & 0xff, w = (d.x >> 8) & 0xff;
+    const bool take = t < na && d.y == first && (unsigned)S.vlab[v] == minlabel;
+    const unsigned m = __ballot_sync(kFull, take);
+    const int pos = ncur + __popc(m & lanemask_lt());
+    ncur += __popc(m);
+    if(ncur > kMinCap) return 2;
+    if(take) {
+      MEmb &e = S.buf[0][pos];
+      reinterpret_cast<uint4 *>(e.inv)[0] = reinterpret_cast<uint4 *>(e.inv)[1] = make_uint4(0, 0, 0, 0);
+      e.inv[v] = 1;
+      e.inv[w] = 2;
+      e.emask = 1ull << (d.x >> 16);
     }
-    MEmb e;
-    e.map[0] = (uint8_t)v;
-    e.vmask = 1u << v;
-    e.pad = 0;
-    e.emask = 0;
-    if(!append(S, 0, take, e, 1, to, id, lane)) return 2;
-  }
-  if(lane == 0) {
-    S.ncur = S.nnext;
-    S.mf[0] = 0;
-    S.mt[0] = 1;
-    S.mel[0] = b1;
   }
   __syncwarp();
-  const int minlabel = b0;
-  int cb = 0;  // the buffer holding the current embeddings
 
+  // the minimum code's right-most path: its vertices, the right-most one and
+  // that one's label; lane v: the path edge that leaves vertex v
+  unsigned path = 3u, leave = first, rlab = first & 0xffffu;
+  int rm = 1, cb = 0;
   for(int m = 1;; m++) {
     // every pattern edge is in the minimum code
     if(m >= n) return 1;
-    if(lane == 0) {
-      // right-most path of the minimum code (forward edges, deepest first)
-      int cnt = 0, old_from = -1;
-      for(int i = m - 1; i >= 0; i--)
-        if(S.mf[i] < S.mt[i] && (cnt == 0 || old_from == S.mt[i])) {
-          S.rm[cnt++] = i;
-          old_from = S.mf[i];
-        }
-      S.nrm = cnt;
-      S.nnext = 0;
-    }
-    __syncwarp();
-    const int nrm = S.nrm, ncur = S.ncur;
-    const int maxtoc = S.mt[S.rm[0]];
     const MEmb *cur = S.buf[cb];
-
-    // ---- backward edges from the right-most vertex: the right-most-path
-    // index nearest the root with any wins; per embedding the first matching
-    // adjacency entry counts (get_backward)
-    int found = -1, bel = 0;
-    for(int i = nrm - 1; i >= 1 && found < 0; --i) {
-      const int v1f = S.mf[S.rm[i]], v1t = S.mt[S.rm[i]], e1el = S.mel[S.rm[i]];
-      unsigned lb = 0xffffffffu;
-      for(int j = lane; j < ncur; j += 32) {
-        const MEmb &e = cur[j];
-        const int r = e.map[maxtoc], e1from = e.map[v1f], e1to = e.map[v1t];
-        for(int t = S.aoff[r]; t < S.aoff[r + 1]; t++) {
-          const uint32_t a = S.adj[t];
-          const int to = a & 0xff, id = (a >> 8) & 0xff, el = a >> 16;
-          if((e.emask >> id) & 1ull) continue;
-          if(to == e1from && (e1el < el || (e1el == el && S.vlab[e1to] <= S.vlab[r]))) {
-            lb = min(lb, (unsigned)el);
-            break;
+    const int items = ncur * na;
+    // backward edges go to the path's vertices but the last two
+    const unsigned inner = path & ~(1u << rm);
+    const unsigned targets = inner & ~(1u << (31 - __clz(inner)));
+    // the pair i: its edge, embedding, and its place in the order of the
+    // extensions (kNone: not one), then its labels
+    constexpr unsigned kNone = 255u;
+    auto look = [&](int i, uint2 &d, int &j, unsigned &prio, unsigned &key) {
+      const bool in = i < items;
+      j = (int)__umulhi((unsigned)i, by_na);
+      d = make_uint2(0, 0);
+      unsigned iv = 0, iw = 0;
+      bool used = false;
+      if(in) {
+        d = S.de[i - j * na];
+        iv = cur[j].inv[d.x & 0xff];
+        iw = cur[j].inv[(d.x >> 8) & 0xff];
+        used = (cur[j].emask >> (d.x >> 16)) & 1ull;
+      }
+      const int c = (int)iv - 1, q = iw ? (int)iw - 1 : c;
+      const unsigned rule = __shfl_sync(kFull, leave, q & 31);
+      prio = kNone;
+      key = ~0u;
+      if(iv) {
+        if(iw) {
+          const unsigned el = d.y >> 16;
+          if(c == rm && ((targets >> q) & 1u) && !used &&
+             ((rule >> 16) < el || ((rule >> 16) == el && (rule & 0xffffu) <= rlab))) {
+            prio = (unsigned)q;
+            key = el << 16;
           }
+        } else if(((path >> c) & 1u) && (d.y & 0xffffu) >= minlabel && (c == rm || d.y >= rule)) {
+          prio = 64u + 31u - (unsigned)c;
+          key = d.y;
         }
       }
-      lb = __reduce_min_sync(kFull, lb);
-      if(lb != 0xffffffffu) {
-        found = i;
-        bel = (int)lb;
+    };
+    uint2 d;
+    int j;
+    unsigned prio, key;
+    look(lane, d, j, prio, key);
+    unsigned bp = prio, bk = key;
+    for(int i0 = 32; i0 < items; i0 += 32) {
+      look(i0 + lane, d, j, prio, key);
+      if(prio < bp || (prio == bp && key < bk)) {
+        bp = prio;
+        bk = key;
       }
     }
-    if(found >= 0) {
-      const int v1f = S.mf[S.rm[found]], v1t = S.mt[S.rm[found]], e1el = S.mel[S.rm[found]];
-      for(int j0 = 0; j0 < ncur; j0 += 32) {
-        const int j = j0 + lane;
-        bool take = false;
-        int id = 0;
-        MEmb e;
-        if(j < ncur) {
-          e = cur[j];
-          const int r = e.map[maxtoc], e1from = e.map[v1f], e1to = e.map[v1t];
-          for(int t = S.aoff[r]; t < S.aoff[r + 1]; t++) {
-            const uint32_t a = S.adj[t];
-            const int to = a & 0xff, aid = (a >> 8) & 0xff, el = a >> 16;
-            if((e.emask >> aid) & 1ull) continue;
-            if(to == e1from && (e1el < el || (e1el == el && S.vlab[e1to] <= S.vlab[r]))) {
-              take = el == bel;
-              id = aid;
-              break;
-            }
-          }
-        }
-        if(!append(S, cb ^ 1, take, e, -1, 0, id, lane)) return 2;
-      }
-      const int nf = maxtoc, nt = S.mf[S.rm[found]];
-      if(S.cf[m] != nf || S.ct[m] != nt || S.cel[m] != bel || S.ctl[m] != -1) return 0;
-      if(lane == 0) {
-        S.mf[m] = nf;
-        S.mt[m] = nt;
-        S.mel[m] = bel;
-        S.ncur = S.nnext;
-      }
-      cb ^= 1;
-      __syncwarp();
-      continue;
-    }
-
-    // ---- forward: pure from the right-most vertex, else from the right-most
-    // path, deepest first; minimum (edge label, to label)
-    if(maxtoc + 1 >= kMinV) return 2;
-    int which = -2;
-    unsigned fb = 0xffffffffu;
-    {
-      unsigned lb = 0xffffffffu;
-      for(int j = lane; j < ncur; j += 32) {
+    const unsigned mp = __reduce_min_sync(kFull, bp);
+    if(mp == kNone) return 1;
+    const unsigned mk = __reduce_min_sync(kFull, bp == mp ? bk : ~0u);
+    const bool fwd = mp >= 64u;
+    const int nf = fwd ? 95 - (int)mp : rm, nt = fwd ? rm + 1 : (int)mp;
+    const uint2 want = S.code[m];
+    if(want.x != (unsigned)(nf | nt << 8) || want.y != mk) return 0;
+    if(m + 1 == n) return 1;
+    // ---- the embeddings of the longer code
+    int nnext = 0;
+    for(int i0 = 0; i0 < items; i0 += 32) {
+      if(items > 32) look(i0 + lane, d, j, prio, key);
+      const bool take = prio == mp && key == mk;
+      const unsigned tm = __ballot_sync(kFull, take);
+      const int pos = nnext + __popc(tm & lanemask_lt());
+      nnext += __popc(tm);
+      if(nnext > kMinCap) return 2;
+      if(take) {
         const MEmb &e = cur[j];
-        const int r = e.map[maxtoc];
-        for(int t = S.aoff[r]; t < S.aoff[r + 1]; t++) {
-          const uint32_t a = S.adj[t];
-          const int to = a & 0xff, el = a >> 16;
-          if(minlabel > S.vlab[to] || ((e.vmask >> to) & 1u)) continue;
-          lb = min(lb, ((unsigned)el << 16) | (unsigned)S.vlab[to]);
-        }
-      }
-      lb = __reduce_min_sync(kFull, lb);
-      if(lb != 0xffffffffu) {
-        which = -1;
-        fb = lb;
+        MEmb &o = S.buf[cb ^ 1][pos];
+        const uint4 x = reinterpret_cast<const uint4 *>(e.inv)[0], y = reinterpret_cast<const uint4 *>(e.inv)[1];
+        const uint64_t em = e.emask | 1ull << (d.x >> 16);
+        reinterpret_cast<uint4 *>(o.inv)[0] = x;
+        reinterpret_cast<uint4 *>(o.inv)[1] = y;
+        o.emask = em;
+        if(fwd) o.inv[(d.x >> 8) & 0xff] = (uint8_t)(rm + 2);
       }
     }
-    for(int i = 0; which == -2 && i < nrm; ++i) {
-      const int vf = S.mf[S.rm[i]], vt = S.mt[S.rm[i]], eel = S.mel[S.rm[i]];
-      unsigned lb = 0xffffffffu;
-      for(int j = lane; j < ncur; j += 32) {
-        const MEmb &e = cur[j];
-        const int efrom = e.map[vf], eto = e.map[vt], tolabel = S.vlab[eto];
-        for(int t = S.aoff[efrom]; t < S.aoff[efrom + 1]; t++) {
-          const uint32_t a = S.adj[t];
-          const int to = a & 0xff, el = a >> 16, tl2 = S.vlab[to];
-          if(eto == to || minlabel > tl2 || ((e.vmask >> to) & 1u)) continue;
-          if(eel < el || (eel == el && tolabel <= tl2)) lb = min(lb, ((unsigned)el << 16) | (unsigned)tl2);
-        }
-      }
-      lb = __reduce_min_sync(kFull, lb);
-      if(lb != 0xffffffffu) {
-        which = i;
-        fb = lb;
-      }
+    if(fwd) {
+      path = (path & ((2u << nf) - 1u)) | 1u << nt;
+      if(lane == nf) leave = mk;
+      rm = nt;
+      rlab = mk & 0xffffu;
     }
-    if(which == -2) return 1;
-    const int fel = (int)(fb >> 16), ftl = (int)(fb & 0xffff);
-    const int vf = which == -1 ? maxtoc : S.mf[S.rm[which]];
-    const int vt = which == -1 ? -1 : S.mt[S.rm[which]];
-    const int eel = which == -1 ? 0 : S.mel[S.rm[which]];
-    for(int j0 = 0; j0 < ncur; j0 += 32) {
-      const int j = j0 + lane;
-      const bool live = j < ncur;
-      MEmb e;
-      int x = 0, deg = 0, eto = -1, tolabel = 0;
-      if(live) {
-        e = cur[j];
-        x = e.map[vf];
-        deg = S.aoff[x + 1] - S.aoff[x];
-        if(which >= 0) {
-          eto = e.map[vt];
-          tolabel = S.vlab[eto];
-        }
-      }
-      for(int t = 0; t < maxdeg; t++) {
-        bool take = false;
-        int to = 0, id = 0;
-        if(live && t < deg) {
-          const uint32_t a = S.adj[S.aoff[x] + t];
-          to = a & 0xff;
-          id = (a >> 8) & 0xff;
-          const int el = a >> 16, tl2 = S.vlab[to];
-          if(!(minlabel > tl2 || ((e.vmask >> to) & 1u)) && el == fel && tl2 == ftl) {
-            if(which == -1) take = true;
-            else take = eto != to && (eel < el || (eel == el && tolabel <= tl2));
-          }
-        }
-        if(!append(S, cb ^ 1, take, e, maxtoc + 1, to, id, lane)) return 2;
-      }
-    }
-    if(S.cf[m] != vf || S.ct[m] != maxtoc + 1 || S.cel[m] != fel || S.ctl[m] != ftl) return 0;
-    if(lane == 0) {
-      S.mf[m] = vf;
-      S.mt[m] = maxtoc + 1;
-      S.mel[m] = fel;
-      S.ncur = S.nnext;
-    }
+    ncur = nnext;
     cb ^= 1;
     __syncwarp();
   }
@@ -359,49 +240,40 @@ __global__ void __launch_bounds__(kMinWarps * 32) k_is_min(const NodeDesc *__res
     const NodeDesc &nd = nodes[ni];
     const int len = nd.code_len, n = len + 1;
     int verdict = 2;
-    if(check && n <= kMinE) {
+    if(check && n <= kMinE && nd.k + 1 <= kMinV) {
       // the parent's code, then the candidate edge decoded from its key
       for(int t = lane; t < len; t += 32) {
         // a code edge: from, to (bytes), edge label | from label, to label
         const uint2 c = codes[(long long)nd.code_off + t];
-        const int f = (int)(c.x & 0xffu), to = (int)((c.x >> 8) & 0xffu);
+        const unsigned f = c.x & 0xffu, to = (c.x >> 8) & 0xffu;
         const bool fwd = f < to;
-        S.cf[t] = f;
-        S.ct[t] = to;
-        S.cel[t] = (int)(c.x >> 16);
-        S.ctl[t] = fwd ? (int)(c.y >> 16) : -1;
+        S.code[t] = make_uint2(c.x & 0xffffu, (c.x & 0xffff0000u) | (fwd ? c.y >> 16 : 0u));
         if(t == 0) S.vlab[f] = (int)(c.y & 0xffffu);
-        if(fwd && to < kMinV) S.vlab[to] = (int)(c.y >> 16);
+        if(fwd) S.vlab[to] = (int)(c.y >> 16);
       }
+      const int kl = x.x - nd.key_base, rmv = nd.k - 1, nslot = nd.nslot;
       const DevDB &db = dbs[nd.db];
-      const int kl = x.x - nd.key_base, maxtoc = nd.k - 1;
-      const SlotDesc *sl = slots + nd.slot_off;
-      int f, t, el, tl;
-      if(kl < nd.nfwd) {
-        int s = 0;
-        for(int q = 1; q < nd.nslot; q++)
-          if(sl[q].fkey_off <= kl) s = q;
-        const int pc = db.pair_code[db.root_off[sl[s].vlab] + (kl - sl[s].fkey_off)];
-        f = sl[s].vertex;
-        t = maxtoc + 1;
-        el = pc >> 16;
-        tl = pc & 0xffff;
-      } else {
-        const int b = (kl - nd.nfwd) / db.EL;
-        f = maxtoc;
-        t = sl[b].vertex;
-        el = (kl - nd.nfwd) % db.EL;
-        tl = -1;
+      // a slot of the right-most path per lane (at most k <= 31)
+      int4 s0 = make_int4(0, INT32_MAX, 0, 0), s1 = s0;
+      if(lane < nslot) {
+        const int4 *sl = reinterpret_cast<const int4 *>(slots + nd.slot_off + lane);
+        s0 = __ldg(sl);
+        s1 = __ldg(sl + 1);
       }
+      const bool fwd = kl < nd.nfwd;
+      const int EL = db.EL;
+      // forward: the last slot whose keys begin at or before the key
+      const int s = fwd ? 31 - __clz(__ballot_sync(kFull, s0.y <= kl) | 1u) : (kl - nd.nfwd) / EL;
+      const int sv = __shfl_sync(kFull, s0.z, s & 31), sf = __shfl_sync(kFull, s0.y, s & 31);
+      const int sp = __shfl_sync(kFull, s1.y, s & 31);
+      const int pc = fwd ? db.pair_code[sp + (kl - sf)] : ((kl - nd.nfwd) % EL) << 16;
       if(lane == 0) {
-        S.cf[len] = f;
-        S.ct[len] = t;
-        S.cel[len] = el;
-        S.ctl[len] = tl;
-        if(tl >= 0 && t < kMinV) S.vlab[t] = tl;
+        const int f = fwd ? sv : rmv, t = fwd ? rmv + 1 : sv;
+        S.code[len] = make_uint2((unsigned)(f | t << 8), (unsigned)pc);
+        if(fwd) S.vlab[t] = pc & 0xffff;
       }
       __syncwarp();
-      if(nd.k + 1 <= kMinV) verdict = warp_is_min(S, n, lane);
+      verdict = warp_is_min(S, n, lane);
       __syncwarp();
     }
     if(lane == 0) {
@@ -459,7 +331,9 @@ KernelCall is_min_call(const NodeDesc *nodes, int32_t nnodes, const SlotDesc *sl
   (void)configured;
   KernelCall c;
   c.func = (const void *)k_is_min;
-  c.grid = dim3((unsigned)(2 * sm_count()));
+  // a warp per key at most (sel_cap is the wave's keys); up to the resident
+  // blocks (250,000 graphs: 0.31 ms with 4 an SM, 0.36 with 2, 0.32 with 8)
+  c.grid = dim3((unsigned)std::max(1, std::min((sel_cap + kMinWarps - 1) / kMinWarps, kMinGrid * sm_count())));
   c.block = dim3(kMinWarps * 32);
   c.smem = (unsigned)smem;
   c.arg(nodes);

@@ -139,3 +139,29 @@ def test_nodes_reused_across_formats(gs, tmp_path):
     for (d, s, kw), pats in list(zip(runs, want))[::-1]:
         assert gs.mine(d, s, **kw)[0] == pats
     assert want[0] == want[2]
+
+
+def _shape(name):
+    """One pattern family per graph: its edges, and a label per vertex."""
+    kind, n, labels = name
+    if kind == "path":
+        e = [(i, i + 1) for i in range(n - 1)]
+    elif kind == "cycle":
+        e = [(i, (i + 1) % n) for i in range(n)]
+    else:
+        e = [(i, j) for i in range(n) for j in range(i + 1, n)]
+    return [i % labels for i in range(n)], [(a, b, 0) for a, b in e]
+
+
+# the canonicality kernel's edges: one pass of 32 directed edges and several (past 16 edges),
+# up to its 32 vertices and past them, backward edges, and embeddings that outgrow its buffer
+# (6 vertices all joined, one label: 720), each against the host's check and the oracle
+@pytest.mark.parametrize("shape", [("path", 17, 1), ("path", 18, 3), ("path", 32, 2), ("path", 34, 1), ("cycle", 9, 3),
+                                   ("cycle", 32, 1), ("cycle", 33, 1), ("complete", 5, 1), ("complete", 6, 1)])
+def test_canonicality(gs, oracle, tmp_path, shape):
+    p = str(tmp_path / "shape.txt")
+    _write(p, [_shape(shape)] * 3)
+    db = gs.Database.load(p, "txt")
+    got = _lines(gs, db, 2)
+    assert got == _lines(gs, db, 2, min_check=1)
+    assert got == run_oracle(oracle, "txt", p, 2)
