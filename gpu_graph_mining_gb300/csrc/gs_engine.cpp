@@ -1823,7 +1823,14 @@ private:
       CK(cudaGraphCreate(&G->g, 0));
       for(int i = 0; i < kWaveKernels; i++) {
         const cudaKernelNodeParams kp = kernel_params(q.k[i]);
-        CK(cudaGraphAddKernelNode(&G->node[i], G->g, i ? &G->node[i - 1] : nullptr, i ? 1 : 0, &kp));
+        CK(cudaGraphAddKernelNode(&G->node[i], G->g, nullptr, 0, &kp));
+        if(i == 0) continue;
+        cudaGraphEdgeData e{};
+        if(q.k[i].early) {
+          e.from_port = cudaGraphKernelNodePortProgrammatic;
+          e.type = cudaGraphDependencyTypeProgrammatic;
+        }
+        CK(cudaGraphAddDependencies(G->g, &G->node[i - 1], &G->node[i], &e, 1));
       }
       CK(cudaGraphInstantiate(&G->x, G->g, 0));
     } else {

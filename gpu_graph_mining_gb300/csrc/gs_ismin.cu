@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(kMinWarps * 32) k_is_min(const NodeDesc *__res
                                                            int sel_cap, unsigned long long *head, int check,
                                                            const ResultsOut out)
 {
+  after_previous();
   stamp_start(head + kHeadMin0);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -331,6 +332,7 @@ KernelCall is_min_call(const NodeDesc *nodes, int32_t nnodes, const SlotDesc *sl
   (void)configured;
   KernelCall c;
   c.func = (const void *)k_is_min;
+  c.early = true;
   // a warp per key at most (sel_cap is the wave's keys); up to the resident
   // blocks (250,000 graphs: 0.31 ms with 4 an SM, 0.36 with 2, 0.32 with 8)
   c.grid = dim3((unsigned)std::max(1, std::min((sel_cap + kMinWarps - 1) / kMinWarps, kMinGrid * sm_count())));

@@ -174,7 +174,7 @@ constexpr int kBigWords = 1024;
 
 // Popcounts of a key's words with their exclusive prefixes (bmx), 4 words per
 // lane per step; returns the total (all lanes).
-__device__ __forceinline__ int warp_prefix_words(const uint32_t *__restrict__ bm, int32_t *bmx, int words)
+__device__ __forceinline__ int warp_prefix_words(const uint32_t *bm, int32_t *bmx, int words)
 {
   const int lane = threadIdx.x & 31;
   int running = 0;
@@ -204,7 +204,7 @@ __device__ __forceinline__ int warp_prefix_words(const uint32_t *__restrict__ bm
 
 // The same by a whole block, 8 words per thread per step (all threads call it;
 // wtot: kBlock / 32 ints).
-__device__ __forceinline__ int block_prefix_words(const uint32_t *__restrict__ bm, int32_t *bmx, int words, int *wtot)
+__device__ __forceinline__ int block_prefix_words(const uint32_t *bm, int32_t *bmx, int words, int *wtot)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kPer = 8, kStep = kBlock * kPer;
@@ -258,9 +258,10 @@ __device__ __forceinline__ int job_of_key(const RootJob *jobs, int njobs, int ke
 // copies 0..q-1, a warp scan over the copies; copy 0 starts at 0 as the
 // materialise pass's cursor) and their total.
 __global__ void __launch_bounds__(kBlock) k_root_support(const RootJob *__restrict__ jobs, int njobs, int total_keys,
-                                                          const uint32_t *__restrict__ bm, int32_t *bmx, int32_t *cnt,
+                                                          const uint32_t *bm, int32_t *bmx, int32_t *cnt,
                                                           int32_t *sup, int32_t *tot)
 {
+  after_previous();
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -320,10 +321,11 @@ __global__ void __launch_bounds__(kBlock) k_begin(int4 *__restrict__ dst, const 
 }
 
 // Results of a root group to pinned host memory (see launch_results).
-__global__ void __launch_bounds__(kBlock) k_results(int4 *dst, const int4 *__restrict__ src, long long n16,
+__global__ void __launch_bounds__(kBlock) k_results(int4 *dst, const int4 *src, long long n16,
                                                     unsigned long long *head, const unsigned int *flags,
                                                     unsigned long long *hhead, unsigned long long seq)
 {
+  after_previous();
   stamp_start(head + kHeadSel0);
   const long long stride = (long long)gridDim.x * kBlock;
   for(long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n16; i += stride) dst[i] = src[i];
@@ -368,8 +370,9 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
                                                          int total_keys, int32_t *cnt, int cnt_copies,
                                                          long long cnt_stride, int32_t *childmap, int2 *listed,
                                                          unsigned long long *head, unsigned int *err,
-                                                         int32_t *lnode, const uint32_t *reg)
+                                                         int32_t *lnode, const volatile uint32_t *reg)
 {
+  after_previous();
   stamp_start(head + kHeadSel0);
   unsigned long long *const counters = head + kHeadSelected;
   const unsigned full = 0xffffffffu;
@@ -480,12 +483,12 @@ __device__ __forceinline__ void listed_done(const int2 kn, const NodeDesc &nd, l
 }
 
 __global__ void __launch_bounds__(kBlock) k_count_listed(const NodeDesc *__restrict__ nodes,
-                                                          const int2 *__restrict__ listed,
-                                                          const uint32_t *__restrict__ bm,
+                                                          const int2 *listed, const uint32_t *__restrict__ bm,
                                                           int32_t *cnt, int32_t *bmx,
                                                           long long *keyword, int4 *sel, int sel_cap,
                                                           unsigned long long *head, int32_t *lnode)
 {
+  after_previous();
   const int lane = threadIdx.x & 31;
   unsigned long long *const counters = head + kHeadSelected;
   const long long nlisted = (long long)counters[2];
@@ -666,15 +669,39 @@ void launch_root_support(const RootJob *jobs, int32_t njobs, int32_t total_keys,
                          int32_t *cnt, int32_t *sup, int32_t *tot, cudaStream_t s)
 {
   if(total_keys <= 0) return;
-  k_root_support<<<grid_for((long long)total_keys * 32), kBlock, 0, s>>>(jobs, njobs, total_keys, bm, bmx, cnt, sup,
-                                                                          tot);
+  KernelCall c;
+  c.func = (const void *)k_root_support;
+  c.early = true;
+  c.grid = dim3((unsigned)grid_for((long long)total_keys * 32));
+  c.block = dim3(kBlock);
+  c.arg(jobs);
+  c.arg(njobs);
+  c.arg(total_keys);
+  c.arg(bm);
+  c.arg(bmx);
+  c.arg(cnt);
+  c.arg(sup);
+  c.arg(tot);
+  c.run(s);
 }
 
 void launch_results(void *dst, const void *src, long long n16, unsigned long long *head, const unsigned int *flags,
                     unsigned long long *hhead, unsigned long long seq, cudaStream_t s)
 {
   const int g = (int)std::max(1ll, std::min(64ll, (n16 + 4 * kBlock - 1) / (4 * kBlock)));
-  k_results<<<g, kBlock, 0, s>>>((int4 *)dst, (const int4 *)src, n16, head, flags, hhead, seq);
+  KernelCall c;
+  c.func = (const void *)k_results;
+  c.early = true;
+  c.grid = dim3((unsigned)g);
+  c.block = dim3(kBlock);
+  c.arg((int4 *)dst);
+  c.arg((const int4 *)src);
+  c.arg(n16);
+  c.arg(head);
+  c.arg(flags);
+  c.arg(hhead);
+  c.arg(seq);
+  c.run(s);
 }
 
 void launch_root_materialize(const RootJob *jobs, int32_t njobs, long long tiles, const DevDB *dbs,
@@ -701,6 +728,7 @@ KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total
 {
   KernelCall c;
   c.func = (const void *)k_screen_keys;
+  c.early = true;
   c.grid = dim3((unsigned)grid_for(((long long)total_keys + 31) / 32 * 32));
   c.block = dim3(kBlock);
   c.arg(nodes);
@@ -724,7 +752,10 @@ KernelCall count_listed_call(const NodeDesc *nodes, const int2 *listed, const ui
 {
   KernelCall c;
   c.func = (const void *)k_count_listed;
-  c.grid = dim3((unsigned)(8 * sm_count()));
+  c.early = true;
+  // a warp per key, or a block where a key has many words: at most one of
+  // either per key of the wave (sel_cap)
+  c.grid = dim3((unsigned)std::max(1, std::min(sel_cap, 8 * sm_count())));
   c.block = dim3(kBlock);
   c.arg(nodes);
   c.arg(listed);

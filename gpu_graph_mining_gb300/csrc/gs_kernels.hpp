@@ -33,6 +33,7 @@ struct KernelCall {
   const void *func = nullptr;
   dim3 grid, block;
   unsigned smem = 0;
+  bool early = false;  // may start before the kernel ahead of it has finished (after_previous())
   template <class T> void arg(const T &v)
   {
     used_ = (used_ + alignof(T) - 1) & ~(alignof(T) - 1);
@@ -45,7 +46,21 @@ struct KernelCall {
     for(int i = 0; i < n_; i++) ptr_[i] = store_ + off_[i];
     return ptr_;
   }
-  cudaError_t run(cudaStream_t s) { return cudaLaunchKernel(func, grid, block, params(), smem, s); }
+  cudaError_t run(cudaStream_t s)
+  {
+    if(!early) return cudaLaunchKernel(func, grid, block, params(), smem, s);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelExC(&c, func, params());
+  }
 
 private:
   alignas(16) unsigned char store_[384];

@@ -118,7 +118,7 @@ struct RowsOut {
 __device__ __forceinline__ RowsOut load_out(const ChildOut *o)
 {
   const int4 *p = reinterpret_cast<const int4 *>(o);
-  const int4 x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2);
+  const int4 x = p[0], y = p[1], z = p[2];
   RowsOut r;
   r.rows = reinterpret_cast<uint4 *>(((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x);
   r.word = (long long)(((unsigned long long)(unsigned)x.w << 32) | (unsigned)x.z);
@@ -163,6 +163,7 @@ __device__ __forceinline__ void store_row(const RowsOut &out, int pos, int gb, i
 template <int PL, bool MAT>
 __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_rows(const RowsArgs a)
 {
+  if(!MAT) after_previous();
   constexpr int NW = 2 + 4 * (PL - 1);
   __shared__ RowsSmem<PL> smem[kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -195,19 +196,19 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       while(hi - lo > 1) {
         const int step = (hi - lo + 31) >> 5;
         const int probe = lo + lane * step;
-        const unsigned ok = __ballot_sync(kFull, probe < hi && __ldg(&a.tile0[probe]) <= tile);
+        const unsigned ok = __ballot_sync(kFull, probe < hi && a.tile0[probe] <= tile);
         lo += (31 - __clz(ok | 1u)) * step;
         hi = min(hi, lo + step);
       }
       n = lo;
-      n_first = __ldg(&a.tile0[n]);
-      n_end = n + 1 < a.nnodes ? __ldg(&a.tile0[n + 1]) : a.total_tiles;
+      n_first = a.tile0[n];
+      n_end = n + 1 < a.nnodes ? a.tile0[n + 1] : a.total_tiles;
       __syncwarp();  // the previous node's tables have been read
       constexpr int kNd = sizeof(PackedNode) / 16;
-      if(lane < kNd) reinterpret_cast<int4 *>(&S.nd)[lane] = __ldg(reinterpret_cast<const int4 *>(&a.nodes[n]) + lane);
+      if(lane < kNd) reinterpret_cast<int4 *>(&S.nd)[lane] = reinterpret_cast<const int4 *>(&a.nodes[n])[lane];
       __syncwarp();
       const int4 *sd = reinterpret_cast<const int4 *>(a.slots + S.nd.slot_off);
-      for(int t = lane; t < 2 * min(S.nd.nslot, RowsSmem<PL>::kSlots); t += 32) reinterpret_cast<int4 *>(S.slot)[t] = __ldg(&sd[t]);
+      for(int t = lane; t < 2 * min(S.nd.nslot, RowsSmem<PL>::kSlots); t += 32) reinterpret_cast<int4 *>(S.slot)[t] = sd[t];
       __syncwarp();
     }
     const int k = S.nd.k, nslot = S.nd.nslot, sh = S.nd.nb_shift;
@@ -440,14 +441,14 @@ template <int PL>
 __global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__restrict__ rec,
                                                              const int4 *__restrict__ hdr,
                                                              const uint32_t *__restrict__ reg, int blk_cap,
-                                                             const uint32_t *__restrict__ chosen,
-                                                             const int32_t *__restrict__ childmap,
+                                                             const uint32_t *chosen, const int32_t *childmap,
                                                              const uint32_t *__restrict__ bm,
                                                              const int32_t *__restrict__ bmx, int32_t *cursor,
                                                              long long cursor_stride,
-                                                             const ChildOut *__restrict__ outs, unsigned int *err,
+                                                             const ChildOut *outs, unsigned int *err,
                                                              unsigned long long *stamps)
 {
+  after_previous();
   constexpr int NW = 2 + 4 * (PL - 1);
   // queue entries: wave key (25 bits), counter copy (2), graph-local new vertex
   // (6), parent row (31)
@@ -607,6 +608,7 @@ template <int PL, bool MAT> KernelCall rows_call(RowsArgs a, int grid_per_sm)
   blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
   KernelCall c;
   c.func = (const void *)k_rows<PL, MAT>;
+  c.early = !MAT;
   c.grid = dim3((unsigned)blocks);
   c.block = dim3(kWarps * 32);
   c.arg(a);
@@ -651,8 +653,25 @@ void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *r
   const long long cap = (long long)kMatGrid * sm_count() / kPer * kPer;
   const int blocks = (int)(want < cap ? want : cap);
   auto *f = planes <= 1 ? k_rows_mat<1> : planes <= 2 ? k_rows_mat<2> : k_rows_mat<5>;
-  f<<<blocks, kMatWarps * 32, 0, s>>>(rec, hdr, reg, blk_cap, chosen, childmap, bm, bmx, cursor, cursor_stride, outs, err,
-                                      stamps);
+  KernelCall c;
+  c.func = (const void *)f;
+  c.early = true;
+  c.grid = dim3((unsigned)blocks);
+  c.block = dim3(kMatWarps * 32);
+  c.arg(rec);
+  c.arg(hdr);
+  c.arg(reg);
+  c.arg(blk_cap);
+  c.arg(chosen);
+  c.arg(childmap);
+  c.arg(bm);
+  c.arg(bmx);
+  c.arg(cursor);
+  c.arg(cursor_stride);
+  c.arg(outs);
+  c.arg(err);
+  c.arg(stamps);
+  c.run(s);
 }
 
 void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStream_t s)
