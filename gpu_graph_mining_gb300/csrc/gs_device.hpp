@@ -20,18 +20,18 @@
 // of the row's graph among the graphs that contain the node's pattern
 // (0..support-1), the index into the node's support bitmaps.
 //
-// Packed rows (databases whose graphs have at most 64 vertices): a row is the
+// Packed rows (databases whose graphs have at most 256 vertices): a row is the
 // embedding itself instead of a chain of back-links, the first graph vertex
 // of its graph and one byte per pattern vertex (graph-local ids), with the
 // row's graph rank: 16 bytes up to 8 pattern vertices, 16 more per further 16
 // (planes of nrows uint4: plane 0 = {first vertex, graph rank, ids 0-3,
 // ids 4-7}, plane p = ids 8 + 16(p - 1) ..).  Neighbour lists are 32-byte
 // blocks, block v = vertex v's list, one DRAM sector: up to 8 entries of 4
-// bytes, ((pair index + 1) << nb_shift) | (neighbour label << 6) |
+// bytes, ((pair index + 1) << nb_shift) | (neighbour label << nb_ids) |
 // graph-local neighbour, ascending, 0 = none; a list of more than 8 has 7 and
 // in the last word 2^31 | the block that continues it (again up to 8 entries,
 // or 7 and a link).  A wave's extension records are blocks of 32 four-byte
-// items of one tile, (node's key << 11) | (graph-local new vertex << 5) | row
+// items of one tile, (node's key << (nb_ids + 5)) | (graph-local new vertex << 5) | row
 // in the tile, each with a header {first row of the tile, node, items,
 // the node's first key}.
 #pragma once
@@ -59,25 +59,30 @@ struct DevDB {
   const int32_t *pair_code;  // [root_off[VL]] (elabel << 16) | tolabel of each pair
   const uint4 *nb;           // neighbour blocks (two uint4 each), or nullptr: no packed rows
   int32_t nb_blocks;         // blocks there is room for
-  int32_t nb_shift;          // 6 + bits of a vertex label
+  int32_t nb_shift;          // nb_ids + bits of a vertex label
+  int32_t nb_ids;            // bits of a graph-local vertex: 6, or 8 for graphs of more than 64
 };
 
-// Whether a database takes packed rows: its graphs' vertices as 6-bit ids,
-// neighbour entries below 2^31, and a node's keys (at most 64 slots of pairs
-// and edge labels) below the items' 2^21.
+// Whether a database takes packed rows (nb_shift, else 0): its graphs' vertices
+// as ids of packed_ids bits, neighbour entries below 2^31, and a node's keys (at
+// most 64 slots of pairs and edge labels) in the items' other bits.
+inline int32_t packed_ids(int64_t max_graph_vertices)
+{
+  return max_graph_vertices <= 64 ? 6 : max_graph_vertices <= 256 ? 8 : 0;
+}
 inline int32_t packed_shift(int64_t max_graph_vertices, int64_t VL, int64_t EL, int64_t pairs)
 {
   int32_t bits = 0;
   while(((int64_t)1 << bits) < VL) bits++;
-  const int32_t sh = 6 + bits;
-  if(max_graph_vertices > 64 || sh > 30 || pairs + 1 >= ((int64_t)1 << (31 - sh)) || 64 * (pairs + EL) >= (1 << 21))
+  const int32_t ids = packed_ids(max_graph_vertices), sh = ids + bits;
+  if(!ids || sh > 30 || pairs + 1 >= ((int64_t)1 << (31 - sh)) || 64 * (pairs + EL) >= ((int64_t)1 << (27 - ids)))
     return 0;
   return sh;
 }
 // Neighbour blocks for V vertices and E2 entries: a list of d > 8 entries
-// takes at most d / 7 blocks beside its first; ids of a row address up to 63
+// takes at most d / 7 blocks beside its first; ids of a row address up to 255
 // blocks past its graph's first vertex.
-inline int64_t packed_blocks(int64_t V, int64_t E2) { return V + E2 / 7 + 64; }
+inline int64_t packed_blocks(int64_t V, int64_t E2) { return V + E2 / 7 + 256; }
 // 16-byte planes of a packed row of k pattern vertices.
 inline int32_t packed_planes(int32_t k) { return k <= 8 ? 1 : 1 + (k - 8 + 15) / 16; }
 
@@ -157,7 +162,7 @@ struct alignas(16) PackedNode {
   const uint4 *rows;         // planes of nrows
   const uint4 *nb;           // its database's neighbour blocks
   int32_t nrows, k, nslot, planes;
-  int32_t nb_shift;
+  int32_t nb_shift, nb_ids;
   uint32_t minl;             // forward targets: entry label field >= minl
   int32_t back;              // 1: some slot takes a backward edge
   int32_t words;             // bitmap words per key
@@ -165,7 +170,7 @@ struct alignas(16) PackedNode {
   int32_t key_base;
   int32_t n_vertices;
   const int32_t *pair_code;
-  int32_t nb_blocks, slot_off;
+  int32_t nb_blocks, slot_off, pad[3];
 };
 
 // Output slots of a child node selected for materialisation.

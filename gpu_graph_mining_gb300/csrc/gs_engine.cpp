@@ -220,6 +220,7 @@ void Database::upload()
   dev.pair_code = (const int32_t *)(b + o_pc);
   if(nb_blocks > 0) {
     dev.nb_shift = nb_shift;
+    dev.nb_ids = packed_ids(maxnv);
     dev.nb_blocks = (int32_t)nb_blocks;
     CK(cudaMemsetAsync(b + o_nu, 0, sizeof(int32_t), cudaStreamLegacy));
     launch_neighbour_blocks(dev, (uint4 *)(b + o_nb), (int32_t *)(b + o_nu), cudaStreamLegacy);
@@ -871,6 +872,7 @@ struct Flight {
   const int32_t *dt = nullptr;  // packed: first tile of each node,
   const PackedNode *dp = nullptr;  //   and what the count needs of it
   int32_t planes = 1;        // packed: the most planes of a node's rows
+  bool wide = false;         //   and whether some node's ids have 8 bits
   int4 *hdr = nullptr;       // packed: record headers (rec_cap counts the blocks of one region)
   uint32_t *reg = nullptr;   // packed: the regions' block counters
   uint32_t *chosen = nullptr;  // packed: a bit per key to materialise
@@ -1916,6 +1918,7 @@ private:
     PackedNode *hp = carve<PackedNode>(hb, off, packed ? W : 0);
     const size_t desc_bytes = Carver::round(off);
     int32_t planes = 1;
+    bool wide = false;
     int32_t eo = 0;
     int32_t co = 0, so = 0, kmax = 1;
     bool small = true;  // every database of the wave has graphs of <= 64 vertices
@@ -1981,7 +1984,9 @@ private:
         g.nslot = d.nslot;
         g.planes = packed_planes(p.nv);
         g.nb_shift = db.dev.nb_shift;
-        g.minl = (uint32_t)d.minlabel << 6;
+        g.nb_ids = db.dev.nb_ids;
+        g.minl = (uint32_t)d.minlabel << g.nb_ids;
+        wide = wide || g.nb_ids > 6;
         g.back = back ? 1 : 0;
         g.words = d.words;
         g.bm_base = bb;
@@ -2019,6 +2024,7 @@ private:
     f.dp = (const PackedNode *)(db_ + ((char *)hp - hb));
     f.packed = packed;
     f.planes = planes;
+    f.wide = wide;
     if(tb >= INT32_MAX) throw Error(ST_ERR_LIMIT, "a wave has 2^36 or more embedding rows");
     const uint2 *dcode = (const uint2 *)(db_ + ((char *)hcode - hb));
     f.join = any_join;
@@ -2099,7 +2105,7 @@ private:
     q.desc_bytes = desc_bytes;
     q.k[0] = begin_call(X.d_desc.p, hb, (long long)desc_bytes / 16, X.d_zero.p, (long long)zero_bytes / 16, head);
     if(packed)
-      q.k[1] = rows_count_call(f.dp, f.dt, W, (int32_t)tb, planes, f.ds, f.bm, cnt, cstride,
+      q.k[1] = rows_count_call(f.dp, f.dt, W, (int32_t)tb, planes, wide, f.ds, f.bm, cnt, cstride,
                                 (uint32_t *)f.rec, f.hdr, (int32_t)f.rec_cap, f.reg, head, err_flag(), wo_.count_grid);
     else
       q.k[1] = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
@@ -2451,11 +2457,11 @@ private:
       if(list_blk >= 0) CK(cudaMemsetAsync(list_off, 0, sizeof(int32_t) * (size_t)(list_rows + 1), st));
       if(f.packed) {
         if(f.rec && nrec <= f.rec_cap) {
-          launch_rows_records((const uint32_t *)f.rec, f.hdr, f.reg, (int32_t)f.rec_cap, (int32_t)nrec, f.planes,
+          launch_rows_records((const uint32_t *)f.rec, f.hdr, f.reg, (int32_t)f.rec_cap, (int32_t)nrec, f.planes, f.wide,
                               f.chosen, X.d_childmap.p, f.bm, X.d_bmx.p, f.cnt, f.cstride, douts, err_flag(), stamps,
                               st);
         } else {
-          launch_rows_materialize(f.dp, f.dt, W, (int32_t)f.tb, f.planes, f.ds, f.bm, X.d_bmx.p, f.chosen,
+          launch_rows_materialize(f.dp, f.dt, W, (int32_t)f.tb, f.planes, f.wide, f.ds, f.bm, X.d_bmx.p, f.chosen,
                                   X.d_childmap.p, X.d_cursor.p, douts, err_flag(), stamps, st);
           if(f.rec)
             X.wanted_rec = std::max<long long>(X.wanted_rec, (nrec + nrec / 4) * kRecBlockInt4 * kRecRegions);

@@ -749,6 +749,7 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
       nbd.vgbase = vgbase;
       nbd.n_vertices = (int32_t)V;
       nbd.nb_shift = nb_shift;
+      nbd.nb_ids = packed_ids(mxv);
       nbd.nb_blocks = (int32_t)nb_blocks;
       CK(cudaMemsetAsync(b + o_nu, 0, sizeof(int32_t), s));
       launch_neighbour_blocks(nbd, (uint4 *)(b + o_nb), (int32_t *)(b + o_nu), s);
@@ -813,6 +814,7 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
     db.dev.nb = nbd.nb;
     db.dev.nb_blocks = nbd.nb_blocks;
     db.dev.nb_shift = nbd.nb_shift;
+    db.dev.nb_ids = nbd.nb_ids;
     db.d_root_off = ro;
     db.resident = true;
     db.device_only = true;

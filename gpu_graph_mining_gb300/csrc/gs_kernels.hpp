@@ -121,28 +121,29 @@ void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long to
 
 // Packed rows (gs_rows.cu).  nodes, tile0: every node's PackedNode and first
 // 32-row tile; planes =
-// the most planes of the wave's nodes' rows; rec / hdr: record blocks (rec may
+// the most planes of the wave's nodes' rows; wide: some node's database has
+// nb_ids 8; rec / hdr: record blocks (rec may
 // be null) in kRecRegions regions of blk_cap blocks, reg[r * kRecRegionStride]
 // counts the blocks reserved in region r (zeroed before).  cnt: kRowsCopies
 // copies of the wave's counters, cnt_stride apart (a warp adds into one: 4 take
 // the adds of a large node's few keys as well as 256 would, one makes the count
 // 14% slower); the wave's keys stay below kRowsKeys.
 constexpr int kRecRegions = 64, kRecRegionStride = 32;
-constexpr int kRowsCopies = 4, kRowsKeys = 1 << 25;
+constexpr int kRowsCopies = 4, kRowsKeys = 1 << 23;
 KernelCall rows_count_call(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
-                           int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, long long cnt_stride,
-                           uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
+                           int32_t planes, bool wide, const SlotDesc *slots, uint32_t *bm, int32_t *cnt,
+                           long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
                            unsigned long long *head, unsigned int *err, int32_t grid_per_sm);
 // Materialise by enumerating again (cursor per child), and from the record
 // blocks (cursor: the counter copies after selection, as for
 // launch_materialize_records).
 void launch_rows_materialize(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
-                             int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
+                             int32_t planes, bool wide, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
                              const uint32_t *chosen, const int32_t *childmap, int32_t *cursor, const ChildOut *outs,
                              unsigned int *err, unsigned long long *stamps, cudaStream_t s);
 // most: the most blocks of a region; chosen: a bit per key to materialise
 void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *reg, int32_t blk_cap, int32_t most,
-                         int32_t planes, const uint32_t *chosen, const int32_t *childmap, const uint32_t *bm,
+                         int32_t planes, bool wide, const uint32_t *chosen, const int32_t *childmap, const uint32_t *bm,
                          const int32_t *bmx, int32_t *cursor, long long cursor_stride, const ChildOut *outs,
                          unsigned int *err, unsigned long long *stamps, cudaStream_t s);
 // Fills a database's neighbour blocks from its adjacency (db.nb_blocks,

@@ -1,7 +1,7 @@
 // Extension kernels for packed rows (gs_device.hpp): count (support bitmaps,
 // embedding counts, extension records) and materialise (children's rows), for
 // one wave of DFS-tree nodes.  Same rules and results as the column kernels
-// (gs_wave.cu), which serve graphs of more than 64 vertices, label alphabets
+// (gs_wave.cu), which serve graphs of more than 256 vertices, label alphabets
 // too large for the 4-byte entries and the lists strategy.
 //
 // What the format is for: on columns a row cost a chain of k dependent 8-byte
@@ -62,10 +62,11 @@ struct RowsArgs {
 
 // One warp's shared memory; the right-most path has at most as many slots as
 // the rows have pattern vertices.
-template <int PL> struct RowsSmem {
+template <int PL, bool WIDE> struct RowsSmem {
   static constexpr int kSlots = PL == 1 ? 8 : PL == 2 ? 24 : 64;
+  uint32_t in[WIDE ? 8 * 32 : 1];  // WIDE: the rows' vertices, 8 words a lane (word w of lane l at 32 w + l)
   uint2 q[32 * 9];      // accepted items waiting for emission (31 and one block per lane):
-                        // {entry, or backward key << 11; owner row | slot << 5 | kBackItem}
+                        // {entry, or backward item; owner row | slot << 5 | kBackItem}
   PackedNode nd;        // the tile's node and its right-most path
   SlotDesc slot[kSlots];
 };
@@ -160,14 +161,20 @@ __device__ __forceinline__ void store_row(const RowsOut &out, int pos, int gb, i
 // queue in shared memory, from which full batches of 32 are emitted: one
 // counter add per distinct key, one bitmap OR per (key, graph), and the batch
 // itself as a record block.
-template <int PL, bool MAT>
-__global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_rows(const RowsArgs a)
+//
+// WIDE (some database of the wave has graphs of more than 64 vertices): a node's
+// ids have 6 or 8 bits, and a row's vertex set is 8 words of shared memory (as
+// one 64-bit set in registers it costs less: the narrow kernel stays).  3,000
+// graphs of 60 to 130 vertices, up to 5 edges: count 0.48 ms on columns, 0.33
+// here, materialise 0.12 -> 0.08, the mine 0.86 -> 0.67.
+template <int PL, bool MAT, bool WIDE>
+__global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB : 7) k_rows(const RowsArgs a)
 {
   if(!MAT) after_previous();
   constexpr int NW = 2 + 4 * (PL - 1);
-  __shared__ RowsSmem<PL> smem[kWarps];
+  __shared__ RowsSmem<PL, WIDE> smem[kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  RowsSmem<PL> &S = smem[warp];
+  RowsSmem<PL, WIDE> &S = smem[warp];
   const int gwarp = blockIdx.x * kWarps + warp, nwarps = gridDim.x * kWarps;
   // the warp's reserved record blocks, and (lane 0) those reserved ahead: a
   // reservation made at the start of a tile arrives while its rows are loaded.
@@ -208,11 +215,11 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       if(lane < kNd) reinterpret_cast<int4 *>(&S.nd)[lane] = reinterpret_cast<const int4 *>(&a.nodes[n])[lane];
       __syncwarp();
       const int4 *sd = reinterpret_cast<const int4 *>(a.slots + S.nd.slot_off);
-      for(int t = lane; t < 2 * min(S.nd.nslot, RowsSmem<PL>::kSlots); t += 32) reinterpret_cast<int4 *>(S.slot)[t] = sd[t];
+      for(int t = lane; t < 2 * min(S.nd.nslot, RowsSmem<PL, WIDE>::kSlots); t += 32) reinterpret_cast<int4 *>(S.slot)[t] = sd[t];
       __syncwarp();
     }
     const int k = S.nd.k, nslot = S.nd.nslot, sh = S.nd.nb_shift;
-    if(k > RowsSmem<PL>::kSlots || nslot > RowsSmem<PL>::kSlots || k < 2 || nslot < 2 || S.nd.planes > PL) {
+    if(k > RowsSmem<PL, WIDE>::kSlots || nslot > RowsSmem<PL, WIDE>::kSlots || k < 2 || nslot < 2 || S.nd.planes > PL) {
       if(lane == 0) atomicOr(a.err, 2u);
       continue;
     }
@@ -243,8 +250,18 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       atomicOr(a.err, (unsigned)g >= (unsigned)S.nd.words * 32u ? 1u : 2u);
       valid = false;
     }
+    const int ids = WIDE ? S.nd.nb_ids : 6;
+    const unsigned idm = (1u << ids) - 1u;
     unsigned m_lo = 0, m_hi = 0;  // the row's vertices
-    if(PL == 1) {
+    if(WIDE) {
+      __syncwarp();
+#pragma unroll
+      for(int q = 0; q < 8; q++) S.in[32 * q + lane] = 0;
+      for(int t = 0; t < k; t++) {
+        const unsigned lv = id_of(w, t);
+        S.in[(lv >> 5) * 32 + lane] |= 1u << (lv & 31u);
+      }
+    } else if(PL == 1) {
 #pragma unroll
       for(int t = 0; t < 8; t++)
         if(t < k) {
@@ -260,9 +277,13 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       }
     }
     const unsigned long long mask = ((unsigned long long)m_hi << 32) | m_lo;
+    auto in_row = [&](unsigned y) {  // entry y's vertex
+      if(WIDE) return (S.in[((y & idm) >> 5) * 32 + lane] >> (y & 31u)) & 1u;
+      return (unsigned)(mask >> (y & 63u)) & 1u;
+    };
     const bool back = S.nd.back != 0;
     const uint4 *__restrict__ nb = S.nd.nb;
-    const unsigned wlm = (1u << sh) - 64u;  // the label field
+    const unsigned wlm = (1u << sh) - (1u << ids);  // the label field
     const unsigned minl = S.nd.minl;
 
     uint4 xa = make_uint4(0, 0, 0, 0), xb = xa;
@@ -281,7 +302,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       const unsigned x[8] = { xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w };
       // the next blocks: continuations of this slot's lists, then the next slot
       const unsigned cont = __ballot_sync(kFull, (int)x[7] < 0);
-      if(cont && hops < 16) {  // (a list of 63 entries has 9 blocks)
+      if(cont && hops < (WIDE ? 40 : 16)) {  // (a list of 63 entries has 9 blocks, one of 255 has 37)
         hops++;
         const unsigned b = x[7] & 0x7fffffffu;
         const bool ok = (int)x[7] < 0 && b < (unsigned)S.nd.nb_blocks;
@@ -302,11 +323,11 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       if(minl == 0) {
 #pragma unroll
         for(int u = 0; u < 8; u++)
-          acc |= (int)x[u] >= rule && !((unsigned)(mask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
+          acc |= (int)x[u] >= rule && !in_row(x[u]) ? 1u << u : 0u;
       } else {
 #pragma unroll
         for(int u = 0; u < 8; u++)
-          acc |= (int)x[u] >= rule && (x[u] & wlm) >= minl && !((unsigned)(mask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
+          acc |= (int)x[u] >= rule && (x[u] & wlm) >= minl && !in_row(x[u]) ? 1u << u : 0u;
       }
       const int c = __popc(acc);
       const int incl = warp_incl(c);
@@ -320,13 +341,15 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       // a right-most-path vertex of the row that takes one (not accepted above,
       // so the queue has room: 8 items per lane behind 31)
       if(back && s == nslot - 1) {
-        unsigned long long bmask = 0;  // the row's vertices that a backward edge may go to
-        for(int t = 0; t + 2 < nslot; t++)
-          if(S.slot[t].bkey_off >= 0) bmask |= 1ull << (id_of(w, S.slot[t].vertex) & 63u);
+        // the row's vertices that a backward edge may go to (WIDE: all its vertices)
+        unsigned long long bmask = 0;
+        if(!WIDE)
+          for(int t = 0; t + 2 < nslot; t++)
+            if(S.slot[t].bkey_off >= 0) bmask |= 1ull << (id_of(w, S.slot[t].vertex) & 63u);
         unsigned bb = 0;
 #pragma unroll
         for(int u = 0; u < 8; u++)
-          bb |= (int)x[u] > 0 && ((unsigned)(bmask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
+          bb |= (int)x[u] > 0 && (WIDE ? in_row(x[u]) : (unsigned)(bmask >> (x[u] & 63u)) & 1u) ? 1u << u : 0u;
         while(__ballot_sync(kFull, bb != 0)) {
           unsigned item = 0;
           bool ok = false;
@@ -338,8 +361,8 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
             bb &= bb - 1;
             const int el = __ldg(&S.nd.pair_code[S.slot[s].pbase + (int)(y >> sh) - 1]) >> 16;
             for(int t = 0; t + 2 < nslot; t++)
-              if(S.slot[t].bkey_off >= 0 && id_of(w, S.slot[t].vertex) == (y & 63u) && el >= S.slot[t].bmin) {
-                item = (unsigned)(S.slot[t].bkey_off + el) << 11;
+              if(S.slot[t].bkey_off >= 0 && id_of(w, S.slot[t].vertex) == (y & idm) && el >= S.slot[t].bmin) {
+                item = (unsigned)(S.slot[t].bkey_off + el) << (ids + 5);
                 ok = true;
               }
           }
@@ -353,16 +376,16 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
       while(qn >= 32 || (!more && qn > 0)) {
         __syncwarp();
         const int m = min(qn, 32);
-        unsigned it = 0;  // the record item: (key << 11) | (new vertex << 5) | row
+        unsigned it = 0;  // the record item: (key << (ids + 5)) | (new vertex << 5) | row
         if(lane < m) {
           const uint2 e = S.q[qn - m + lane];
           it = e.y & 31u;
           if(e.y & kBackItem) it |= e.x;
-          else it |= ((unsigned)S.slot[e.y >> 5].fkey_off - 1u + (e.x >> sh)) << 11 | (e.x & 63u) << 5;
+          else it |= ((unsigned)S.slot[e.y >> 5].fkey_off - 1u + (e.x >> sh)) << (ids + 5) | (e.x & idm) << 5;
         }
         qn -= m;
         __syncwarp();
-        const int key = lane < m ? (int)(it >> 11) : -1;
+        const int key = lane < m ? (int)(it >> (ids + 5)) : -1;
         const int o = (int)(it & 31u);
         const int g_o = __shfl_sync(kFull, g, o);
         const int key_base = S.nd.key_base;
@@ -386,7 +409,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
             if(blk < a.blk_cap) {  // past the region's end nothing is written
               const unsigned b = (unsigned)region * (unsigned)a.blk_cap + (unsigned)blk;  // (below 2^26 blocks)
               a.rec[b * 32u + (unsigned)lane] = it;
-              if(lane == 0) a.hdr[b] = make_int4(row0, n, m | (gwarp % kRowsCopies) << 8, key_base);
+              if(lane == 0) a.hdr[b] = make_int4(row0, n, m | (gwarp % kRowsCopies) << 8 | (ids + 5) << 16, key_base);
             }
             blk++;
             blk_left--;
@@ -407,7 +430,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
             const RowsOut out = load_out(&a.outs[c]);
             const long long wi = out.word + (g_o >> 5);
             const int rank = a.bmx[wi] + __popc(a.bm[wi] & ((1u << (g_o & 31)) - 1u));
-            if(pos < out.cap) store_row<PL>(out, pos, gb_o, rank, wo, k, (it >> 5) & 63u);
+            if(pos < out.cap) store_row<PL>(out, pos, gb_o, rank, wo, k, (it >> 5) & idm);
             else atomicOr(a.err, 4u);
           }
         }
@@ -437,7 +460,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 ? GS_ROWS_MINB : 7) k_row
 constexpr int kMatWarps = 8, kMatBlocks = 4;
 constexpr int kMatGrid = 16;  // thread blocks per SM: 8 are resident
 
-template <int PL>
+template <int PL, bool WIDE>
 __global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__restrict__ rec,
                                                              const int4 *__restrict__ hdr,
                                                              const uint32_t *__restrict__ reg, int blk_cap,
@@ -450,8 +473,8 @@ __global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__r
 {
   after_previous();
   constexpr int NW = 2 + 4 * (PL - 1);
-  // queue entries: wave key (25 bits), counter copy (2), graph-local new vertex
-  // (6), parent row (31)
+  // queue entries: wave key (23 bits), counter copy (2), graph-local new vertex
+  // (8), parent row (31)
   __shared__ unsigned long long queue[kMatWarps][32 * (kMatBlocks + 1)];
   unsigned long long *const q = queue[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -473,19 +496,21 @@ __global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__r
       for(int t = 0; t < kMatBlocks; t++) it[t] = i + t < used ? __ldg(&ri[(long long)(i + t) * 32]) : 0u;
 #pragma unroll
       for(int t = 0; t < kMatBlocks; t++) {
-        const int m = __shfl_sync(kFull, h.z, t) & 0xff, key = __shfl_sync(kFull, h.w, t) + (int)(it[t] >> 11);
+        const int hz = __shfl_sync(kFull, h.z, t), m = hz & 0xff;
+        const int key = __shfl_sync(kFull, h.w, t) + (int)(it[t] >> (WIDE ? hz >> 16 : 11));
         w[t] = lane < m ? chosen[key >> 5] : 0u;
       }
 #pragma unroll
       for(int t = 0; t < kMatBlocks; t++) {
-        const int key = __shfl_sync(kFull, h.w, t) + (int)(it[t] >> 11);
+        const int hz = __shfl_sync(kFull, h.z, t), kb = WIDE ? hz >> 16 : 11;
+        const int key = __shfl_sync(kFull, h.w, t) + (int)(it[t] >> kb);
         const bool on = (w[t] >> (key & 31)) & 1u;
         const unsigned m = __ballot_sync(kFull, on);
         if(m) {
-          const int row0 = __shfl_sync(kFull, h.x, t), copy = __shfl_sync(kFull, h.z, t) >> 8;
+          const int row0 = __shfl_sync(kFull, h.x, t), copy = (hz >> 8) & 0xff;
           if(on)
-            q[qn + __popc(m & lanemask_lt())] = ((unsigned long long)(unsigned)(key * kRowsCopies + copy) << 37) |
-                                                ((unsigned long long)((it[t] >> 5) & 63u) << 31) |
+            q[qn + __popc(m & lanemask_lt())] = ((unsigned long long)(unsigned)(key * kRowsCopies + copy) << 39) |
+                                                ((unsigned long long)((it[t] >> 5) & ((1u << (kb - 5)) - 1u)) << 31) |
                                                 (unsigned)(row0 + (int)(it[t] & 31u));
           qn += __popc(m);
         }
@@ -499,8 +524,8 @@ __global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__r
       const unsigned long long e = has ? q[qn - m + lane] : 0ull;
       qn -= m;
       __syncwarp();
-      const int kc = has ? (int)(e >> 37) : -1, key = kc / kRowsCopies, row = (int)(e & 0x7fffffffull);
-      const unsigned lv = (unsigned)(e >> 31) & 63u;
+      const int kc = has ? (int)(e >> 39) : -1, key = kc / kRowsCopies, row = (int)(e & 0x7fffffffull);
+      const unsigned lv = (unsigned)(e >> 31) & 0xffu;
       RowsOut out{};
       if(has) out = load_out(&outs[childmap[key]]);
       uint4 r = make_uint4(0, 0, 0, 0);
@@ -544,7 +569,7 @@ __global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__r
 __global__ void __launch_bounds__(256) k_neighbour_blocks(const int32_t *__restrict__ adj_off, int V,
                                                           const unsigned long long *__restrict__ adj,
                                                           const int32_t *__restrict__ adj_pair,
-                                                          const int32_t *__restrict__ vgbase, int sh, uint4 *nb,
+                                                          const int32_t *__restrict__ vgbase, int sh, int ids, uint4 *nb,
                                                           int nb_blocks, int *used)
 {
   const int lane = threadIdx.x & 31;
@@ -581,8 +606,8 @@ __global__ void __launch_bounds__(256) k_neighbour_blocks(const int32_t *__restr
           x[u] = 0;
           if(u < here) {
             const unsigned long long e = __ldg(&adj[at + u]);
-            x[u] = ((unsigned)(__ldg(&adj_pair[at + u]) + 1) << sh) | ((unsigned)((e >> 32) & 0xffffu) << 6) |
-                   (((unsigned)e - (unsigned)gb) & 63u);
+            x[u] = ((unsigned)(__ldg(&adj_pair[at + u]) + 1) << sh) | ((unsigned)((e >> 32) & 0xffffu) << ids) |
+                   (((unsigned)e - (unsigned)gb) & ((1u << ids) - 1u));
           }
         }
         if(link) x[7] = 0x80000000u | (unsigned)next;
@@ -599,7 +624,7 @@ __global__ void __launch_bounds__(256) k_neighbour_blocks(const int32_t *__restr
   }
 }
 
-template <int PL, bool MAT> KernelCall rows_call(RowsArgs a, int grid_per_sm)
+template <int PL, bool MAT, bool WIDE> KernelCall rows_call(RowsArgs a, int grid_per_sm)
 {
   const long long cap = (long long)sm_count() * (grid_per_sm > 0 ? grid_per_sm : GS_ROWS_GRID);
   // in groups once every warp of a full grid has one: below that the chip would idle
@@ -607,7 +632,7 @@ template <int PL, bool MAT> KernelCall rows_call(RowsArgs a, int grid_per_sm)
   long long blocks = ((long long)a.total_tiles + kWarps * a.group - 1) / (kWarps * a.group);
   blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
   KernelCall c;
-  c.func = (const void *)k_rows<PL, MAT>;
+  c.func = (const void *)k_rows<PL, MAT, WIDE>;
   c.early = !MAT;
   c.grid = dim3((unsigned)blocks);
   c.block = dim3(kWarps * 32);
@@ -615,34 +640,41 @@ template <int PL, bool MAT> KernelCall rows_call(RowsArgs a, int grid_per_sm)
   return c;
 }
 
+template <bool MAT> KernelCall rows_call(const RowsArgs &a, int planes, bool wide, int grid_per_sm)
+{
+  if(wide)
+    return planes <= 1 ? rows_call<1, MAT, true>(a, grid_per_sm)
+         : planes <= 2 ? rows_call<2, MAT, true>(a, grid_per_sm) : rows_call<5, MAT, true>(a, grid_per_sm);
+  return planes <= 1 ? rows_call<1, MAT, false>(a, grid_per_sm)
+       : planes <= 2 ? rows_call<2, MAT, false>(a, grid_per_sm) : rows_call<5, MAT, false>(a, grid_per_sm);
+}
+
 }  // namespace
 
 KernelCall rows_count_call(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
-                           int32_t planes, const SlotDesc *slots, uint32_t *bm, int32_t *cnt, long long cnt_stride,
-                           uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
+                           int32_t planes, bool wide, const SlotDesc *slots, uint32_t *bm, int32_t *cnt,
+                           long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
                            unsigned long long *head, unsigned int *err, int32_t grid_per_sm)
 {
   const RowsArgs a{ nodes, tile0, nnodes, total_tiles, 1, slots, bm, nullptr, cnt, cnt_stride, nullptr, nullptr,
                     nullptr, nullptr, rec, hdr, blk_cap, reg, err, head + kHeadCount0 };
-  if(planes <= 1) return rows_call<1, false>(a, grid_per_sm);
-  if(planes <= 2) return rows_call<2, false>(a, grid_per_sm);
-  return rows_call<5, false>(a, grid_per_sm);
+  return rows_call<false>(a, planes, wide, grid_per_sm);
 }
 
 void launch_rows_materialize(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
-                             int32_t planes, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
+                             int32_t planes, bool wide, const SlotDesc *slots, const uint32_t *bm, const int32_t *bmx,
                              const uint32_t *chosen, const int32_t *childmap, int32_t *cursor, const ChildOut *outs,
                              unsigned int *err, unsigned long long *stamps, cudaStream_t s)
 {
   if(total_tiles <= 0) return;
   const RowsArgs a{ nodes, tile0, nnodes, total_tiles, 1, slots, const_cast<uint32_t *>(bm), bmx, nullptr, 0, chosen,
                     childmap, cursor, outs, nullptr, nullptr, 0, nullptr, err, stamps };
-  KernelCall c = planes <= 1 ? rows_call<1, true>(a, 0) : planes <= 2 ? rows_call<2, true>(a, 0) : rows_call<5, true>(a, 0);
+  KernelCall c = rows_call<true>(a, planes, wide, 0);
   c.run(s);
 }
 
 void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *reg, int32_t blk_cap, int32_t most,
-                         int32_t planes, const uint32_t *chosen, const int32_t *childmap, const uint32_t *bm,
+                         int32_t planes, bool wide, const uint32_t *chosen, const int32_t *childmap, const uint32_t *bm,
                          const int32_t *bmx, int32_t *cursor, long long cursor_stride, const ChildOut *outs,
                          unsigned int *err, unsigned long long *stamps, cudaStream_t s)
 {
@@ -652,7 +684,9 @@ void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *r
   const long long want = ((long long)most + kMatBlocks - 1) / kMatBlocks * kPer;
   const long long cap = (long long)kMatGrid * sm_count() / kPer * kPer;
   const int blocks = (int)(want < cap ? want : cap);
-  auto *f = planes <= 1 ? k_rows_mat<1> : planes <= 2 ? k_rows_mat<2> : k_rows_mat<5>;
+  auto *f = planes <= 1 ? (wide ? k_rows_mat<1, true> : k_rows_mat<1, false>)
+          : planes <= 2 ? (wide ? k_rows_mat<2, true> : k_rows_mat<2, false>)
+                        : (wide ? k_rows_mat<5, true> : k_rows_mat<5, false>);
   KernelCall c;
   c.func = (const void *)f;
   c.early = true;
@@ -679,7 +713,7 @@ void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStre
   if(db.n_vertices <= 0) return;
   const long long want = ((long long)db.n_vertices + 255) / 256, cap = 64LL * sm_count();
   k_neighbour_blocks<<<(int)(want < cap ? want : cap), 256, 0, s>>>(db.adj_off, db.n_vertices, db.adj, db.adj_pair,
-                                                                    db.vgbase, db.nb_shift, nb, db.nb_blocks, used);
+                                                                    db.vgbase, db.nb_shift, db.nb_ids, nb, db.nb_blocks, used);
 }
 
 }  // namespace gsgb

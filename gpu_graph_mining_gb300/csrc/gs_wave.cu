@@ -1,6 +1,6 @@
 // Warp-cooperative extension kernels on columns: count (support bitmaps +
 // embedding counts) and materialise (children's columns), for one wave of
-// DFS-tree nodes.  They serve graphs of more than 64 vertices, label alphabets
+// DFS-tree nodes.  They serve graphs of more than 256 vertices, label alphabets
 // too large for packed rows (packed_shift) and the lists strategy, which joins
 // on the rows' back-links; gs_rows.cu serves the rest.
 //

@@ -1,4 +1,4 @@
-"""Packed rows (graphs of at most 64 vertices) against the oracle and against
+"""Packed rows (graphs of at most 256 vertices) against the oracle and against
 the column kernels: neighbour lists that end at and past their 8-entry blocks,
 databases on either side of the rule that chooses the row format, batches of
 both, and the re-enumerating materialise after a record overflow."""
@@ -165,3 +165,38 @@ def test_canonicality(gs, oracle, tmp_path, shape):
     got = _lines(gs, db, 2)
     assert got == _lines(gs, db, 2, min_check=1)
     assert got == run_oracle(oracle, "txt", p, 2)
+
+
+# graph-local ids of 6 bits (up to 64 vertices), of 8 (up to 256), and columns beyond; rows of one, two
+# and five planes; the hub's list has up to 37 blocks
+@pytest.mark.parametrize("nv", [64, 65, 128, 255, 256, 257])
+def test_graph_sizes(gs, oracle, tmp_path, nv):
+    r = random.Random(nv)
+    p = str(tmp_path / "sizes.txt")
+    hub = [(0, v, r.randrange(3)) for v in range(1, nv)] + [(v, v + 1, 0) for v in range(1, nv - 1, 5)]
+    graphs = _random_graphs(r, 9, (nv - 3, nv), 4, 3) + [([0] + [r.randrange(1, 5) for _ in range(nv - 1)], hub)] * 3
+    _write(p, graphs)
+    db = gs.Database.load(p, "txt")
+    want = run_oracle(oracle, "txt", p, 3, ["--max-edges", "3"])
+    assert _lines(gs, db, 3, max_edges=3) == want
+    # a path of vertices that differ, and edges across it
+    n = nv // 4 * 4
+    path = [(i, i + 1, 0) for i in range(n - 1)] + [(i, i + 3, 1) for i in range(0, n - 3, 40)]
+    _write(p, [(list(range(n)), path)] * 3)
+    want = run_oracle(oracle, "txt", p, 2, ["--max-edges", "26"])
+    assert _lines(gs, gs.Database.load(p, "txt"), 2, max_edges=26) == want
+
+
+def test_batch_of_id_widths(gs, tmp_path):
+    r = random.Random(5)
+    dbs = []
+    for i, nv in enumerate([(4, 20), (60, 64), (65, 90), (250, 256), (257, 260), (4, 30)]):
+        p = str(tmp_path / ("w%d.txt" % i))
+        _write(p, _random_graphs(r, 40, nv, 3, 2))
+        dbs.append(gs.Database.load(p, "txt"))
+    sups = [12, 25, 25, 30, 30, 10]
+    for kw in ({}, {"launch_mode": 1}):
+        got, _ = gs.mine_batch(dbs, sups, max_edges=4, **kw)
+        for db, s, pats in zip(dbs, sups, got):
+            assert pats == gs.mine(db, s, max_edges=4)[0]
+            assert pats == gs.mine(db, s, max_edges=4, extension="lists")[0]
