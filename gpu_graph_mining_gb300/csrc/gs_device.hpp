@@ -193,7 +193,7 @@ struct alignas(16) ChildOut {
 // the device's nanosecond clock, taken by the first thread of a kernel: kernels
 // of one stream start when the one before has finished.
 enum HeadWord {
-  kHeadRecords = 0,   // extension records written by the count pass (packed rows: most blocks of a region)
+  kHeadRecords = 0,   // records (packed rows: blocks) reserved in the fullest region
   kHeadFlags = 1,     // consistency flags
   kHeadSelected = 2,  // selected candidates   } counters of
   kHeadExt = 3,       // embeddings of all keys } the support

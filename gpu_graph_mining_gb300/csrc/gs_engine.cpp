@@ -873,8 +873,8 @@ struct Flight {
   const PackedNode *dp = nullptr;  //   and what the count needs of it
   int32_t planes = 1;        // packed: the most planes of a node's rows
   bool wide = false;         //   and whether some node's ids have 8 bits
-  int4 *hdr = nullptr;       // packed: record headers (rec_cap counts the blocks of one region)
-  uint32_t *reg = nullptr;   // packed: the regions' block counters
+  int4 *hdr = nullptr;       // packed: record headers (rec_cap counts the blocks or records of one region)
+  uint32_t *reg = nullptr;   // the regions' counters
   uint32_t *chosen = nullptr;  // packed: a bit per key to materialise
   bool join = false;         // some node joins its parent's lists (lists strategy)
   int32_t W = 0, kb = 0, kmax = 1;
@@ -2051,7 +2051,7 @@ private:
     const long long cstride = (long long)Carver::round(sizeof(int32_t) * (size_t)std::max(kb, 1)) / 4;
     const size_t cnt_bytes = sizeof(int32_t) * (size_t)cstride * ccopies;
     // packed rows: the record regions' counters, behind the embedding counters
-    const size_t reg_bytes = packed ? sizeof(uint32_t) * kRecRegions * kRecRegionStride : 0;
+    const size_t reg_bytes = sizeof(uint32_t) * kRecRegions * kRecRegionStride;
     // and a bit per key to materialise
     const size_t sel_bytes = packed ? Carver::round((size_t)(kb + 31) / 32 * 4) : 0;
     const size_t zero_bytes = Carver::round(cnt_bytes + reg_bytes + sel_bytes + sizeof(uint32_t) * (size_t)std::max<int64_t>(bb, 1));
@@ -2064,7 +2064,7 @@ private:
     int32_t *cnt = (int32_t *)X.d_zero.p;
     f.cnt = cnt;
     f.cstride = cstride;
-    f.reg = packed ? (uint32_t *)(X.d_zero.p + cnt_bytes) : nullptr;
+    f.reg = (uint32_t *)(X.d_zero.p + cnt_bytes);
     f.chosen = packed ? (uint32_t *)(X.d_zero.p + cnt_bytes + reg_bytes) : nullptr;
     f.bm = (uint32_t *)(X.d_zero.p + cnt_bytes + reg_bytes + sel_bytes);
     unsigned long long *head = (unsigned long long *)X.d_head.p;
@@ -2095,6 +2095,8 @@ private:
         f.rec_cap /= kRecBlockInt4 * kRecRegions;
         f.hdr = X.d_rec.p;
         f.rec = X.d_rec.p + f.rec_cap * kRecRegions;
+      } else {
+        f.rec_cap /= kRecRegions;
       }
     }
     // the frequent candidates come back compacted, as many as there was need of
@@ -2109,7 +2111,7 @@ private:
                                 (uint32_t *)f.rec, f.hdr, (int32_t)f.rec_cap, f.reg, head, err_flag(), wo_.count_grid);
     else
       q.k[1] = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
-                              err_flag(), f.rec, f.rec_cap, head,
+                              err_flag(), f.rec, f.rec_cap, f.reg, head,
                               wo_.count_grid, ccopies, cstride, f.join, f.rule_skip);
     int32_t *lnode = nullptr;
     if(f.lists) {
@@ -2468,7 +2470,7 @@ private:
         }
       } else if(f.rec && nrec <= f.rec_cap) {
         // record-driven: one thread per extension record, no graph access
-        launch_materialize_records(f.rec, nrec, X.d_childmap.p, X.d_keyword.p, f.bm, X.d_bmx.p, f.cnt, f.cstride,
+        launch_materialize_records(f.rec, f.reg, f.rec_cap, nrec, X.d_childmap.p, X.d_keyword.p, f.bm, X.d_bmx.p, f.cnt, f.cstride,
                                    douts, E.d_bytes.p + 1, err_flag(), list_blk >= 0 ? &lb : nullptr,
                                    list_off + 1, stamps, st);
       } else {
@@ -2476,10 +2478,10 @@ private:
         launch_wave_materialize(f.dn, W, f.tb, f.kmax, f.small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, X.d_bmx.p,
                                 X.d_childmap.p, X.d_cursor.p, douts, E.d_bytes.p + 1, err_flag(), f.join,
                                 f.rule_skip, stamps, st);
-        if(f.rec) X.wanted_rec = std::max<long long>(X.wanted_rec, nrec + nrec / 4);
+        if(f.rec) X.wanted_rec = std::max<long long>(X.wanted_rec, (nrec + nrec / 4) * kRecRegions);
       }
       if(list_blk >= 0) {
-        launch_fill_lists(f.rec, nrec, lb, list_off, list_rows, list_ent, list_n, list_scr, err_flag(), st);
+        launch_fill_lists(f.rec, f.reg, f.rec_cap, nrec, lb, list_off, list_rows, list_ent, list_n, list_scr, err_flag(), st);
         st_.list_entries += list_n;
         st_.launches += 2;
       }

@@ -615,13 +615,17 @@ __global__ void __launch_bounds__(kBlock) k_count_listed(const NodeDesc *__restr
 
 // ---- lists strategy: per-row lists of the frequent forward extensions
 
-// cursor[r] starts at list row r's offset and ends at the next row's
-__global__ void __launch_bounds__(kBlock) k_list_fill(const int4 *__restrict__ rec, long long n, const ListBuild lb,
-                                                      int32_t *cursor, int2 *ent, long long ent_cap,
-                                                      unsigned int *err)
+// cursor[r] starts at list row r's offset and ends at the next row's (the grid
+// is a multiple of kRecRegions, a block stays in one region)
+__global__ void __launch_bounds__(kBlock) k_list_fill(const int4 *__restrict__ rec, const uint32_t *__restrict__ reg,
+                                                      long long rec_cap, const ListBuild lb, int32_t *cursor,
+                                                      int2 *ent, long long ent_cap, unsigned int *err)
 {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+  const int region = blockIdx.x % kRecRegions;
+  const long long n = min((long long)__ldg(&reg[region * kRecRegionStride]), rec_cap);
+  rec += region * rec_cap;
+  const long long stride = (long long)(gridDim.x / kRecRegions) * blockDim.x;
+  for(long long i = (long long)(blockIdx.x / kRecRegions) * blockDim.x + threadIdx.x; i < n; i += stride) {
     const int4 x = __ldg(&rec[i]);
     long long row;
     int lk;
@@ -987,16 +991,17 @@ void launch_filter_backward(const int2 *col, int64_t nrows, const int32_t *rec, 
   k_bwd_gather<<<grid_for(nrows), kBlock, 0, s>>>(col, pos, nrows, out);
 }
 
-void launch_fill_lists(const int4 *rec, long long nrec, const ListBuild &lb, int32_t *off, int64_t nrows_total,
+void launch_fill_lists(const int4 *rec, const uint32_t *reg, long long rec_cap, long long most, const ListBuild &lb,
+                       int32_t *off, int64_t nrows_total,
                        int2 *ent, int64_t ent_cap, int32_t *scratch, unsigned int *err, cudaStream_t s)
 {
-  if(nrec <= 0 || nrows_total <= 0) return;
+  if(most <= 0 || nrows_total <= 0) return;
   // the counts of row r are at off[r + 1]; their exclusive scan makes off[r + 1]
   // the start of row r, which the fill's cursor adds carry to the start of
   // row r + 1, with off[0] = 0
   int32_t *cnt = off + 1;
   xscan(cnt, nrows_total, scratch, s);
-  k_list_fill<<<grid_for(nrec), kBlock, 0, s>>>(rec, nrec, lb, cnt, ent, ent_cap, err);
+  k_list_fill<<<region_blocks(most, kBlock), kBlock, 0, s>>>(rec, reg, rec_cap, lb, cnt, ent, ent_cap, err);
 }
 
 void launch_children(void *dst, const void *src, long long n16, const int2 *pairs, int32_t n, int32_t *childmap,

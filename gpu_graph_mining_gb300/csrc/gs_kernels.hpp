@@ -5,6 +5,7 @@
 // embedding count past 2^31 - 1); the offending access is skipped, never
 // performed.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <cuda_runtime.h>
@@ -109,7 +110,7 @@ KernelCall wave_count_call(const NodeDesc *nodes, int32_t nnodes, long long tota
                            bool small_graphs, const int2 *const *coltab, const int32_t *collen, const SlotDesc *slots,
                            const int32_t *vtab, const DevDB *dbs, uint32_t *bm, int32_t *cnt,
                            unsigned long long *bytes, unsigned int *err, int4 *rec, long long rec_cap,
-                           unsigned long long *head, int32_t grid_per_sm, int32_t cnt_copies,
+                           uint32_t *reg, unsigned long long *head, int32_t grid_per_sm, int32_t cnt_copies,
                            long long cnt_stride, bool join, bool rule_skip);
 void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long total_tiles, int32_t kmax,
                              bool small_graphs,
@@ -129,6 +130,13 @@ void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long to
 // the adds of a large node's few keys as well as 256 would, one makes the count
 // 14% slower); the wave's keys stay below kRowsKeys.
 constexpr int kRecRegions = 64, kRecRegionStride = 32;
+// Thread blocks for a kernel whose blocks each stay in one region, an item per
+// thread of threads, the fullest region holding most.
+inline int region_blocks(long long most, int threads)
+{
+  const long long per = std::min((most + threads - 1) / threads, (16ll * sm_count() + kRecRegions - 1) / kRecRegions);
+  return (int)(std::max(per, 1ll) * kRecRegions);
+}
 constexpr int kRowsCopies = 4, kRowsKeys = 1 << 23;
 KernelCall rows_count_call(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                            int32_t planes, bool wide, const SlotDesc *slots, uint32_t *bm, int32_t *cnt,
@@ -155,10 +163,12 @@ void launch_neighbour_blocks(const DevDB &db, uint4 *nb, int32_t *used, cudaStre
 // rank.  keyword[key] = the key's first support-bitmap word.
 // cursor: the wave's counter copies after selection (copy q of a key starts
 // at the count of copies 0..q-1), cursor_stride apart; a record's copy is in
-// bits 27-30 of its key field.
+// bits 27-30 of its key field.  reg, rec_cap: kRecRegions regions of rec_cap
+// records and their fills, as for the packed rows; most: the largest fill.
 // lists (may be null): also counts each list row's entries at list_cnt[row]
 // (lists strategy, launch_fill_lists)
-void launch_materialize_records(const int4 *rec, long long n, const int32_t *childmap, const long long *keyword,
+void launch_materialize_records(const int4 *rec, const uint32_t *reg, long long rec_cap, long long most,
+                                const int32_t *childmap, const long long *keyword,
                                 const uint32_t *bm, const int32_t *bmx, int32_t *cursor, long long cursor_stride,
                                 const ChildOut *outs, unsigned long long *bytes, unsigned int *err,
                                 const ListBuild *lists, int32_t *list_cnt, unsigned long long *stamps,
@@ -248,7 +258,8 @@ void launch_gather_ends(const uint32_t *scanned, int64_t n, const long long *end
 int64_t filter_backward_scratch(int64_t nrows);
 void launch_filter_backward(const int2 *col, int64_t nrows, const int32_t *rec, int64_t nrec, const int32_t *e,
                             int32_t *pos, int32_t *scratch, int2 *out, cudaStream_t s);
-void launch_fill_lists(const int4 *rec, long long nrec, const ListBuild &lb, int32_t *off, int64_t nrows_total,
+void launch_fill_lists(const int4 *rec, const uint32_t *reg, long long rec_cap, long long most, const ListBuild &lb,
+                       int32_t *off, int64_t nrows_total,
                        int2 *ent, int64_t ent_cap, int32_t *scratch, unsigned int *err, cudaStream_t s);
 
 }  // namespace gsgb

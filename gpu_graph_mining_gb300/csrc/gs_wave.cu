@@ -76,8 +76,8 @@ struct WaveArgs {
   // count pass, optional: one record per extension {wave key, child column
   // element x, y, graph rank} for the record-driven materialise pass
   int4 *rec;
-  long long rec_cap;
-  unsigned long long *rec_n;  // records produced (may exceed rec_cap: then none past it are written)
+  long long rec_cap;   // records of one of the kRecRegions regions
+  uint32_t *rec_n;     // records reserved in each region (may exceed rec_cap: none past it are written)
   // count pass: cnt holds cnt_copies copies of the wave's counters, cnt_stride
   // apart; warp w adds into copy w % cnt_copies (summed by the screening pass)
   int cnt_copies;
@@ -130,7 +130,12 @@ k_wave(const WaveArgs a)
   if(!MAT) stamp_start(a.stamp);
   if(lane == 0) S.bytes = 0;
   // count pass with records: the warp's current reserved chunk (warp-uniform);
-  // starts "full" so the first batch reserves a chunk
+  // starts "full" so the first batch reserves a chunk.  The warps reserve from
+  // kRecRegions counters, each with its part of the records: adds to one
+  // address complete at about one per 1.6 ns, which bounded the kernel when one
+  // counter served all warps.
+  const int region = (int)(gwarp % kRecRegions);
+  int4 *const rec = a.rec + region * a.rec_cap;
   long long chunk_base = -1;
   int chunk_fill = kRecChunk;
   const int copy = (int)(gwarp % (a.cnt_copies > 0 ? a.cnt_copies : 1));
@@ -402,17 +407,18 @@ k_wave(const WaveArgs a)
             chunk_fill += cntx;
           } else {
             const int room = kRecChunk - chunk_fill;
-            long long nb = 0;
-            if(lane == 0) nb = (long long)atomicAdd(a.rec_n, (unsigned long long)kRecChunk);
+            int nb = 0;
+            if(lane == 0)
+              nb = (int)min(atomicAdd(&a.rec_n[region * kRecRegionStride], (unsigned)kRecChunk), 0x7fffff00u);
             nb = __shfl_sync(kFull, nb, 0);
-            dst = rank < room ? chunk_base + chunk_fill + rank : nb + (rank - room);
+            dst = rank < room ? chunk_base + chunk_fill + rank : (long long)nb + (rank - room);
             chunk_base = nb;
             chunk_fill = cntx - room;
           }
           if(key >= 0 && dst >= 0 && dst < a.rec_cap) {
             const int i_o = row0 + o;
-            a.rec[dst] = bwd ? make_int4((key_base + key) | rec_tag, S.phi[k - 1][o], S.lp[o], g_o)
-                             : make_int4((key_base + key) | rec_tag, w, i_o, g_o);
+            rec[dst] = bwd ? make_int4((key_base + key) | rec_tag, S.phi[k - 1][o], S.lp[o], g_o)
+                           : make_int4((key_base + key) | rec_tag, w, i_o, g_o);
           }
         }
       } else {
@@ -444,11 +450,16 @@ k_wave(const WaveArgs a)
     // mark the unused tail of the last chunk as holes (key -1)
     for(int f = chunk_fill + lane; f < kRecChunk; f += 32) {
       const long long dst = chunk_base + f;
-      if(dst < a.rec_cap) a.rec[dst] = make_int4(-1, 0, 0, 0);
+      if(dst < a.rec_cap) rec[dst] = make_int4(-1, 0, 0, 0);
     }
   }
-  __syncwarp();
-  if(a.bytes && lane == 0 && S.bytes) atomicAdd(a.bytes, S.bytes);
+  // one add per block: adds to one address complete one after another
+  __syncthreads();
+  if(a.bytes && threadIdx.x == 0) {
+    unsigned long long sum = 0;
+    for(int q = 0; q < kWarps; q++) sum += reinterpret_cast<Smem<KMAX> *>(smem_raw)[q].bytes;
+    if(sum) atomicAdd(a.bytes, sum);
+  }
   if(MAT) stamp_mat_end(a.stamp);
 }
 
@@ -522,11 +533,11 @@ KernelCall wave_count_call(const NodeDesc *nodes, int32_t nnodes, long long tota
                            bool small_graphs, const int2 *const *coltab, const int32_t *collen, const SlotDesc *slots,
                            const int32_t *vtab, const DevDB *dbs, uint32_t *bm, int32_t *cnt,
                            unsigned long long *bytes, unsigned int *err, int4 *rec, long long rec_cap,
-                           unsigned long long *head, int32_t grid_per_sm, int32_t cnt_copies,
+                           uint32_t *reg, unsigned long long *head, int32_t grid_per_sm, int32_t cnt_copies,
                            long long cnt_stride, bool join, bool rule_skip)
 {
   WaveArgs a{ nodes, nnodes, total_tiles, coltab, collen, slots, vtab, dbs, bm, nullptr, cnt,
-              nullptr, nullptr, nullptr, bytes, err, rec, rec_cap, rec ? head + kHeadRecords : nullptr, cnt_copies,
+              nullptr, nullptr, nullptr, bytes, err, rec, rec_cap, reg, cnt_copies,
               cnt_stride, rule_skip ? 1 : 0, head + kHeadCount0 };
   if(small_graphs)
     return join ? count_call<true, true>(kmax, a, grid_per_sm) : count_call<true, false>(kmax, a, grid_per_sm);
@@ -551,7 +562,8 @@ namespace {
 
 // Materialise from the count pass's records: one thread per record, no graph
 // access.  keyword[key] = the key's first bitmap word (node bm_base + key * words).
-__global__ void __launch_bounds__(256) k_mat_records(const int4 *__restrict__ rec, long long n,
+__global__ void __launch_bounds__(256) k_mat_records(const int4 *__restrict__ rec, const uint32_t *__restrict__ reg,
+                                                     long long rec_cap,
                                                      const int32_t *__restrict__ childmap,
                                                      const long long *__restrict__ keyword,
                                                      const uint32_t *__restrict__ bm, const int32_t *__restrict__ bmx,
@@ -561,11 +573,15 @@ __global__ void __launch_bounds__(256) k_mat_records(const int4 *__restrict__ re
                                                      unsigned long long *stamps)
 {
   const int lane = threadIdx.x & 31;
-  const long long stride = (long long)gridDim.x * blockDim.x;
   unsigned long long mine = 0;
+  // a block stays in one region (the grid is a multiple of their number)
+  const int region = blockIdx.x % kRecRegions;
+  const long long n = min((long long)__ldg(&reg[region * kRecRegionStride]), rec_cap);
+  rec += region * rec_cap;
+  const long long stride = (long long)(gridDim.x / kRecRegions) * blockDim.x;
   // the loop runs a warp-uniform number of times: lanes past n carry no record
   const long long n32 = (n + 31) & ~31ll;
-  for(long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n32; r += stride) {
+  for(long long r = (long long)(blockIdx.x / kRecRegions) * blockDim.x + threadIdx.x; r < n32; r += stride) {
     int c = -1, key = 0, cp = 0;
     int4 x = make_int4(0, 0, 0, 0);
     if(r < n) {
@@ -611,25 +627,33 @@ __global__ void __launch_bounds__(256) k_mat_records(const int4 *__restrict__ re
     }
   }
   if(bytes) {
+    // one add per block: adds to one address complete one after another (a warp
+    // each took 31 us of a launch)
+    __shared__ unsigned long long sums[8];
     for(int o = 16; o > 0; o >>= 1) mine += __shfl_down_sync(kFull, mine, o);
-    if(lane == 0 && mine) atomicAdd(bytes, mine);
+    if(lane == 0) sums[threadIdx.x >> 5] = mine;
+    __syncthreads();
+    if(threadIdx.x == 0) {
+      for(int q = 1; q < 8; q++) mine += sums[q];
+      if(mine) atomicAdd(bytes, mine);
+    }
   }
   stamp_mat_end(stamps);
 }
 
 }  // namespace
 
-void launch_materialize_records(const int4 *rec, long long n, const int32_t *childmap, const long long *keyword,
+void launch_materialize_records(const int4 *rec, const uint32_t *reg, long long rec_cap, long long most,
+                                const int32_t *childmap, const long long *keyword,
                                 const uint32_t *bm, const int32_t *bmx, int32_t *cursor, long long cursor_stride,
                                 const ChildOut *outs, unsigned long long *bytes, unsigned int *err,
                                 const ListBuild *lists, int32_t *list_cnt, unsigned long long *stamps,
                                 cudaStream_t s)
 {
-  if(n <= 0) return;
-  long long blocks = ((n + 31) / 32 * 32 + 255) / 256;
-  if(blocks > 16LL * sm_count()) blocks = 16LL * sm_count();
+  if(most <= 0) return;
+  const int blocks = region_blocks(most, 256);
   const ListBuild lb = lists ? *lists : ListBuild{ nullptr, nullptr, nullptr };
-  k_mat_records<<<(int)blocks, 256, 0, s>>>(rec, n, childmap, keyword, bm, bmx, cursor, cursor_stride, outs, bytes,
+  k_mat_records<<<blocks, 256, 0, s>>>(rec, reg, rec_cap, childmap, keyword, bm, bmx, cursor, cursor_stride, outs, bytes,
                                             err, lb, lists ? list_cnt : nullptr, stamps);
 }
 
