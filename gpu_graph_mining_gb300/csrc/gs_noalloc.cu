@@ -17,6 +17,7 @@
 #include <mutex>
 
 #include "../../include/gspan_gb300.h"
+#include "gs_stamp.cuh"
 
 namespace {
 
@@ -42,34 +43,73 @@ struct ErrText {
   void operator=(const char *m) { gsgb::capi_set_error(m); }
 } t_msg;
 
+using gsgb::after_previous;
+
+// The scratch is 16-byte aligned and a multiple of 16 bytes.
 __global__ void k_clear(uint32_t *bm, long long words)
 {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) bm[i] = 0u;
+  const long long stride = (long long)gridDim.x * blockDim.x, n = (words + 3) / 4;
+  for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+    reinterpret_cast<uint4 *>(bm)[i] = make_uint4(0, 0, 0, 0);
 }
 
-// Records outside [0, n_keys) x [0, n_graphs) are skipped.
+__device__ __forceinline__ void mark(uint32_t *bm, int k, int g, int n_keys, int n_graphs, int words)
+{
+  if((unsigned)k >= (unsigned)n_keys || (unsigned)g >= (unsigned)n_graphs) return;
+  atomicOr(&bm[(long long)k * words + (g >> 5)], 1u << (g & 31));
+}
+
+// Records outside [0, n_keys) x [0, n_graphs) are skipped.  vec: both arrays are
+// 16-byte aligned, four records a step and the next four's loads in flight; the
+// first are loaded before the clear is waited for.  Bound by the bitmap ORs:
+// 4 M records into 1,000 keys x 30,011 graphs take 31 us, 126 ORs per ns to
+// words that few share; the loads alone would take 5.  The call: 43.0 -> 34.8 us
+// with one record a step and three launches apart before.
 __global__ void k_mark(uint32_t *bm, const int32_t *__restrict__ keys, const int32_t *__restrict__ gids, long long n,
-                       int n_keys, int n_graphs, int words)
+                       int n_keys, int n_graphs, int words, int vec)
 {
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int k = keys[i], g = gids[i];
-    if((unsigned)k >= (unsigned)n_keys || (unsigned)g >= (unsigned)n_graphs) continue;
-    atomicOr(&bm[(long long)k * words + (g >> 5)], 1u << (g & 31));
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long n4 = vec ? n >> 2 : 0;
+  const int4 *const k4 = reinterpret_cast<const int4 *>(keys), *const g4 = reinterpret_cast<const int4 *>(gids);
+  int4 k_n = make_int4(0, 0, 0, 0), g_n = k_n;
+  if(i0 < n4) {
+    k_n = __ldg(&k4[i0]);
+    g_n = __ldg(&g4[i0]);
   }
+  after_previous();
+  for(long long i = i0; i < n4; i += stride) {
+    const int4 k = k_n, g = g_n;
+    if(i + stride < n4) {
+      k_n = __ldg(&k4[i + stride]);
+      g_n = __ldg(&g4[i + stride]);
+    }
+    mark(bm, k.x, g.x, n_keys, n_graphs, words);
+    mark(bm, k.y, g.y, n_keys, n_graphs, words);
+    mark(bm, k.z, g.z, n_keys, n_graphs, words);
+    mark(bm, k.w, g.w, n_keys, n_graphs, words);
+  }
+  for(long long i = 4 * n4 + i0; i < n; i += stride) mark(bm, __ldg(&keys[i]), __ldg(&gids[i]), n_keys, n_graphs, words);
 }
 
-// One warp per key.
-__global__ void k_count(const uint32_t *__restrict__ bm, int n_keys, int words, int32_t *support)
+// kSupWarps warps per key (1, or the block).
+template <int kSupWarps> __global__ void k_count(const uint32_t *bm, int n_keys, int words, int32_t *support)
 {
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for(int key = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; key < n_keys; key += warps) {
+  after_previous();
+  constexpr int kPer = kSupWarps * 32;
+  const int t = threadIdx.x % kPer;
+  __shared__ int sums[kBlock / 32];
+  for(int key = (blockIdx.x * kBlock + threadIdx.x) / kPer; key < n_keys; key += gridDim.x * (kBlock / kPer)) {
     int c = 0;
-    for(int w = lane; w < words; w += 32) c += __popc(bm[(long long)key * words + w]);
+    for(int w = t; w < words; w += kPer) c += __popc(bm[(long long)key * words + w]);
     for(int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if(lane == 0) support[key] = c;
+    if(kSupWarps > 1) {
+      if((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = c;
+      __syncthreads();
+      for(int q = 1; q < kSupWarps; q++) c += t == 0 ? sums[q] : 0;
+      __syncthreads();
+    }
+    if(t == 0) support[key] = c;
   }
 }
 
@@ -79,6 +119,22 @@ struct DevInfo {
   int sms = 0;
 };
 DevInfo g_dev[kMaxDevices];
+
+// Launch that may begin while the kernel ahead of it in the stream ends (its
+// griddepcontrol.wait holds it until that one's writes are there).
+template <class... P, class... A> cudaError_t launch_early(void (*f)(P...), int grid, cudaStream_t s, A... args)
+{
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3(kBlock);
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, f, P(args)...);
+}
 
 int grid_for(long long n, int sms)
 {
@@ -205,20 +261,27 @@ extern "C" gs_status gs_support_count_noalloc(const int32_t *d_keys, const int32
   if(st != GS_OK) return st;
   uint32_t *bm = di.addr;
   const long long nw = (long long)n_keys * words;
-  k_clear<<<grid_for(nw, di.sms), kBlock, 0, s>>>(bm, nw);
+  k_clear<<<grid_for((nw + 3) / 4, di.sms), kBlock, 0, s>>>(bm, nw);
   if(cudaGetLastError() != cudaSuccess) {
     t_msg = "gs_support_count_noalloc: launch of the scratch clear failed";
     return GS_ERR_CUDA;
   }
   if(n_records > 0) {
-    k_mark<<<grid_for(n_records, di.sms), kBlock, 0, s>>>(bm, d_keys, d_graph_ids, n_records, n_keys, n_graphs,
-                                                          (int)words);
+    const int vec = ((uintptr_t)d_keys | (uintptr_t)d_graph_ids) % 16 == 0 ? 1 : 0;
+    launch_early(k_mark, grid_for(vec ? (n_records + 3) / 4 : n_records, di.sms), s, bm, d_keys, d_graph_ids, n_records,
+                 n_keys, n_graphs, (int)words, vec);
     if(cudaGetLastError() != cudaSuccess) {
       t_msg = "gs_support_count_noalloc: launch of the record marking failed";
       return GS_ERR_CUDA;
     }
   }
-  k_count<<<grid_for((long long)n_keys * 32, di.sms), kBlock, 0, s>>>(bm, n_keys, (int)words, d_support);
+  // a block per key where a warp would take more than 8 rounds
+  if(words > kBlock)
+    launch_early(k_count<kBlock / 32>, grid_for((long long)n_keys * kBlock, di.sms), s, (const uint32_t *)bm, n_keys,
+                 (int)words, d_support);
+  else
+    launch_early(k_count<1>, grid_for((long long)n_keys * 32, di.sms), s, (const uint32_t *)bm, n_keys, (int)words,
+                 d_support);
   if(cudaGetLastError() != cudaSuccess) {
     t_msg = "gs_support_count_noalloc: launch of the popcount failed";
     return GS_ERR_CUDA;
