@@ -480,8 +480,13 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
     most = __reduce_max_sync(full, most);
     if(lane == 0) head[kHeadRecords] = most;
   }
-  // warp-uniform trip count: the list append below is warp-aggregated
-  const long long n32 = ((long long)total_keys + 31) & ~31ll;
+  // block-uniform trip count: the list append below takes one add per block
+  // (adds to one address complete one after another: a wave of a thousand small
+  // nodes has thousands of warps with a listed key)
+  const long long n32 = ((long long)total_keys + kBlock - 1) / kBlock * kBlock;
+  __shared__ int wlist[kBlock / 32];
+  __shared__ unsigned long long list_at;
+  const int warp = threadIdx.x >> 5;
   for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n32; i += stride) {
     const int key = (int)i;
     int c = 0;
@@ -528,12 +533,18 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
     }
     if(cand) bytes += 8;  // the listed entry
     const unsigned m = __ballot_sync(full, cand);
-    if(m) {
-      unsigned long long at = 0;
-      if(lane == 0) at = atomicAdd(&counters[2], (unsigned long long)__popc(m));
-      at = __shfl_sync(full, at, 0);
-      if(cand) listed[at + __popc(m & lanemask_lt())] = make_int2(key, n);
+    if(lane == 0) wlist[warp] = __popc(m);
+    if(!__syncthreads_or(m != 0)) continue;
+    int before = 0, total = 0;
+#pragma unroll
+    for(int w = 0; w < kBlock / 32; w++) {
+      const int x = wlist[w];
+      if(w < warp) before += x;
+      total += x;
     }
+    if(threadIdx.x == 0) list_at = atomicAdd(&counters[2], (unsigned long long)total);
+    __syncthreads();
+    if(cand) listed[list_at + before + __popc(m & lanemask_lt())] = make_int2(key, n);
   }
   for(int o = 16; o > 0; o >>= 1) {
     ext += __shfl_down_sync(full, ext, o);
@@ -610,7 +621,13 @@ __global__ void __launch_bounds__(kBlock) k_count_listed(const NodeDesc *__restr
     const int running = block_prefix_words(bm + wbase, bmx + wbase, words, wtot);
     if(threadIdx.x == 0) listed_done(kn, nd, wbase, running, cnt, keyword, sel, sel_cap, counters, lnode, bytes);
   }
-  if(lane == 0 && bytes) atomicAdd(&counters[3], bytes);
+  __shared__ unsigned long long wbytes[kBlock / 32];
+  if(lane == 0) wbytes[threadIdx.x >> 5] = bytes;
+  __syncthreads();
+  if(threadIdx.x == 0) {
+    for(int w = 1; w < kBlock / 32; w++) bytes += wbytes[w];
+    if(bytes) atomicAdd(&counters[3], bytes);
+  }
 }
 
 // ---- lists strategy: per-row lists of the frequent forward extensions
