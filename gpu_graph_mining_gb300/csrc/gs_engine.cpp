@@ -731,16 +731,18 @@ struct Candidate {
 
 // The device work of one wave up to its results in host memory: tables in and
 // scratch cleared (begin), count, selection, canonicality and results out.
-constexpr int kWaveKernels = 5;
+constexpr int kWaveKernels = 5;  // at most
 struct WaveSeq {
   size_t desc_bytes = 0;
-  KernelCall k[kWaveKernels];  // begin, count, screen, listed, is_min
+  KernelCall k[kWaveKernels];  // begin, count, select (or screen and listed), is_min
+  int n = 0;
 };
 
 // WaveSeq as an instantiated CUDA graph, one per count-kernel variant and
 // context: each wave updates the nodes' parameters and launches the graph.
 struct WaveGraph {
   const void *count_func = nullptr;
+  int n = 0;  // kernels
   cudaGraph_t g = nullptr;
   cudaGraphExec_t x = nullptr;
   cudaGraphNode_t node[kWaveKernels];
@@ -774,6 +776,7 @@ struct WaveCtx {
   DBuf<int4> d_rec;
   DBuf<unsigned long long> d_recn;
   DBuf<long long> d_keyword;
+  DBuf<int2> d_listed;               // keys with enough embeddings to be counted
   DBuf<int32_t> d_lnode;   // lists strategy: the node of each frequent forward key
   // A wave's results, written to pinned host memory by its last kernel: the
   // header (HeadWord) followed by the selected candidates {key, support,
@@ -782,7 +785,6 @@ struct WaveCtx {
   // (key, child) pairs (one upload).
   DBuf<char> d_head, d_zero, d_mat;
   HBuf<char> h_head, h_mat;
-  DBuf<int2> d_listed;               // keys with enough embeddings to be counted
   int64_t sel_hint = 4096;           // selected entries there is room for in the pinned results
   bool rec_enabled = true;
   long long wanted_rec = 0;    // record capacity to have before the next wave (after an overflow)
@@ -1812,18 +1814,19 @@ private:
     const cudaStream_t st = cs(X);
     st_.h2d_bytes += (int64_t)q.desc_bytes;
     if(wo_.launch_mode != 0) {
-      for(auto &k : q.k) CK(k.run(st));
+      for(int i = 0; i < q.n; i++) CK(q.k[i].run(st));
       return;
     }
     WaveGraph *G = nullptr;
     for(auto &g : X.graphs)
-      if(g.count_func == q.k[1].func) G = &g;
+      if(g.count_func == q.k[1].func && g.n == q.n) G = &g;
     if(!G) {
       X.graphs.emplace_back();
       G = &X.graphs.back();
       G->count_func = q.k[1].func;
+      G->n = q.n;
       CK(cudaGraphCreate(&G->g, 0));
-      for(int i = 0; i < kWaveKernels; i++) {
+      for(int i = 0; i < q.n; i++) {
         const cudaKernelNodeParams kp = kernel_params(q.k[i]);
         CK(cudaGraphAddKernelNode(&G->node[i], G->g, nullptr, 0, &kp));
         if(i == 0) continue;
@@ -1836,7 +1839,7 @@ private:
       }
       CK(cudaGraphInstantiate(&G->x, G->g, 0));
     } else {
-      for(int i = 0; i < kWaveKernels; i++) {
+      for(int i = 0; i < q.n; i++) {
         const cudaKernelNodeParams kp = kernel_params(q.k[i]);
         CK(cudaGraphExecKernelNodeSetParams(G->x, G->node[i], &kp));
       }
@@ -2060,7 +2063,6 @@ private:
     X.d_bmx.ensure(std::max<int64_t>(bb, 1));
     X.d_childmap.ensure(std::max(kb, 1));
     X.d_keyword.ensure(std::max(kb, 1));
-    X.d_listed.ensure(std::max(kb, 1));
     int32_t *cnt = (int32_t *)X.d_zero.p;
     f.cnt = cnt;
     f.cstride = cstride;
@@ -2118,9 +2120,17 @@ private:
       X.d_lnode.ensure(std::max(kb, 1));
       lnode = X.d_lnode.p;
     }
-    q.k[2] = screen_keys_call(f.dn, W, kb, cnt, ccopies, cstride, packed ? nullptr : X.d_childmap.p, X.d_listed.p, head, err_flag(), lnode,
-                              f.rec ? f.reg : nullptr);
-    q.k[3] = count_listed_call(f.dn, X.d_listed.p, f.bm, cnt, X.d_bmx.p, X.d_keyword.p, sel, kb, head, lnode);
+    int32_t *const cmap = packed ? nullptr : X.d_childmap.p;
+    uint32_t *const reg = f.rec ? f.reg : nullptr;
+    q.n = 2;
+    if(bb <= kSelectWords) {
+      q.k[q.n++] = select_call(f.dn, W, kb, cnt, ccopies, cstride, cmap, f.bm, X.d_bmx.p, X.d_keyword.p, sel, head,
+                               err_flag(), lnode, reg);
+    } else {
+      X.d_listed.ensure(std::max(kb, 1));
+      q.k[q.n++] = screen_keys_call(f.dn, W, kb, cnt, ccopies, cstride, cmap, X.d_listed.p, head, err_flag(), lnode, reg);
+      q.k[q.n++] = count_listed_call(f.dn, X.d_listed.p, f.bm, cnt, X.d_bmx.p, X.d_keyword.p, sel, kb, head, lnode);
+    }
     f.res_seq = ++E.seq;
     ((volatile unsigned long long *)X.h_head.p)[kHeadSeq] = 0;
     ResultsOut ro{};
@@ -2131,7 +2141,7 @@ private:
     ro.bytes = E.d_bytes.p;
     ro.stamps = E.d_stamps.p;
     ro.nctx = kWaveCtx;
-    q.k[4] = is_min_call(f.dn, W, f.ds, E.d_dbs.p, dcode, sel, kb, head, wo_.min_check == 0, ro);
+    q.k[q.n++] = is_min_call(f.dn, W, f.ds, E.d_dbs.p, dcode, sel, kb, head, wo_.min_check == 0, ro);
     // the wave's nodes were made by the root phases (engine stream) or by
     // other contexts' materialise passes (their last ones cover every node
     // made so far; this context's own are ahead on its stream)
@@ -2150,7 +2160,7 @@ private:
     f.main_gen = E.main_gen;
     for(int d = 0; d < kWaveCtx; d++) f.mat_gen[d] = E.ctx[d].mat_gen;
     issue(X, q);
-    st_.launches += kWaveKernels;
+    st_.launches += q.n;
     f.busy = true;
     f.seq = ++seq_;
     st_.host_build_ms += ms_since(t_begin);

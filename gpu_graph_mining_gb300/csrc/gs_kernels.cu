@@ -449,7 +449,8 @@ __global__ void __launch_bounds__(kBlock) k_root_materialize(const RootJob *__re
   root_tiles<true>(jobs, njobs, tiles, dbs, const_cast<uint32_t *>(bm), bmx, cursor, childmap, outs, err);
 }
 
-// Support of the candidates of one wave, and their selection, in two passes.
+// Support of the candidates of one wave, and their selection, in two kernels
+// (large waves; k_select does it in one).
 // Screening, one thread per key: a key with fewer embeddings than its node's
 // minsup cannot be found in that many graphs, so only keys with cnt >= minsup
 // are listed for counting; every key with embeddings gets childmap -1
@@ -531,7 +532,6 @@ __global__ void __launch_bounds__(kBlock) k_screen_keys(const NodeDesc *__restri
       cnt[key] = c;
       bytes += 4ull * (unsigned)cnt_copies;  // the copies turned into offsets
     }
-    if(cand) bytes += 8;  // the listed entry
     const unsigned m = __ballot_sync(full, cand);
     if(lane == 0) wlist[warp] = __popc(m);
     if(!__syncthreads_or(m != 0)) continue;
@@ -574,9 +574,9 @@ __device__ __forceinline__ void listed_done(const int2 kn, const NodeDesc &nd, l
                                             unsigned long long *counters, int32_t *lnode,
                                             unsigned long long &bytes)
 {
-  // algorithmic bytes: the listed entry, each bitmap word read and its
-  // prefix written, and for a selected key its word offset, result and counter
-  bytes += 8ull + 8ull * (unsigned)nd.words + (running >= nd.minsup ? 32ull : 0ull);
+  // algorithmic bytes: each bitmap word read and its prefix written, and for a
+  // selected key its word offset, result and counter
+  bytes += 8ull * (unsigned)nd.words + (running >= nd.minsup ? 32ull : 0ull);
   if(running >= nd.minsup) {
     keyword[kn.x] = wbase;
     const unsigned long long at = atomicAdd(&counters[0], 1ull);
@@ -626,6 +626,171 @@ __global__ void __launch_bounds__(kBlock) k_count_listed(const NodeDesc *__restr
   __syncthreads();
   if(threadIdx.x == 0) {
     for(int w = 1; w < kBlock / 32; w++) bytes += wbytes[w];
+    if(bytes) atomicAdd(&counters[3], bytes);
+  }
+}
+
+// Support of the candidates of one wave, and their selection.  A block takes
+// chunks of consecutive keys.  Screening, a thread per key: a key with fewer
+// embeddings than its node's minsup cannot be found in that many graphs, so
+// only keys with cnt >= minsup are listed (in shared memory) for counting;
+// every key with embeddings gets childmap -1 (overwritten afterwards for the
+// children that are materialised; null for packed rows, which mark those in a
+// bit set).  Counting, a warp per listed key, or the block where the key has
+// more than kSelWords bitmap words: popcount of its bitmap with prefix counts
+// for the materialise pass; the frequent keys are appended to sel as {key,
+// support, embeddings, node << 2} (order unspecified; the low two bits take the
+// canonicality verdict) and get keyword = their first bitmap word.  counters:
+// [0] selected, [1] embeddings of all keys, [2] listed keys, [3] bytes.
+//
+// A chain of dependent loads bounds it (node, counters, node's bitmap, words).
+constexpr int kSelWords = 256;
+__global__ void __launch_bounds__(kBlock) k_select(const NodeDesc *__restrict__ nodes, int nnodes, int total_keys,
+                                                   int chunk, int32_t *cnt, int cnt_copies, long long cnt_stride,
+                                                   int32_t *childmap, const uint32_t *bm, int32_t *bmx,
+                                                   long long *keyword, int4 *sel, unsigned long long *head,
+                                                   unsigned int *err, int32_t *lnode, const volatile uint32_t *reg)
+{
+  after_previous();
+  stamp_start(head + kHeadSel0);
+  unsigned long long *const counters = head + kHeadSelected;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long ext = 0, bytes = 0;
+  int nlisted = 0;
+  if(reg && blockIdx.x == 0 && threadIdx.x < 32) {
+    uint32_t most = 0;
+    for(int r = lane; r < kRecRegions; r += 32) most = max(most, reg[r * kRecRegionStride]);
+    most = __reduce_max_sync(full, most);
+    if(lane == 0) head[kHeadRecords] = most;
+  }
+  __shared__ int2 list[kBlock];  // {key, node}
+  __shared__ int wlist[kBlock / 32], wtot[kBlock / 32], range[2];
+  for(long long base = (long long)blockIdx.x * chunk; base < total_keys; base += (long long)gridDim.x * chunk) {
+    const int nk = (int)min((long long)chunk, total_keys - base);
+    if(warp < 2) {
+      // the nodes of the chunk's first and last key, 32 probes a round
+      const int k0 = (int)base + (warp ? nk - 1 : 0);
+      int lo = 0, hi = nnodes;
+      while(hi - lo > 1) {
+        const int step = (hi - lo + 31) >> 5;
+        const int probe = lo + lane * step;
+        const unsigned ok = __ballot_sync(full, probe < hi && nodes[probe].key_base <= k0);
+        lo += (31 - __clz(ok | 1u)) * step;
+        hi = min(hi, lo + step);
+      }
+      if(lane == 0) range[warp] = lo;
+    }
+    const int key = (int)base + (int)threadIdx.x;
+    int c = 0, x[4] = { 0, 0, 0, 0 };
+    if((int)threadIdx.x < nk) {
+      // the count pass spread its adds over copies: their total.  A copy that
+      // wrapped (negative) or a total past 2^31 - 1 is clamped to 2^31 - 1
+      // and flagged (bit 8): the host refuses such a key
+#pragma unroll
+      for(int q = 0; q < 4; q++)
+        if(q < cnt_copies) x[q] = cnt[q * cnt_stride + key];
+      bool wrap = (x[0] | x[1] | x[2] | x[3]) < 0;
+      long long c64 = (long long)x[0] + x[1] + x[2] + x[3];
+      for(int q = 4; q < cnt_copies; q++) {
+        const int y = cnt[q * cnt_stride + key];
+        wrap = wrap || y < 0;
+        c64 += y;
+      }
+      if(wrap || c64 > (long long)INT32_MAX) {
+        atomicOr(err, 8u);
+        c = INT32_MAX;
+      } else {
+        c = (int)c64;
+      }
+      bytes += 4ull * (unsigned)cnt_copies;  // the counter copies read
+    }
+    __syncthreads();
+    int n = 0;
+    bool cand = false;
+    if(c > 0) {
+      if(childmap) childmap[key] = -1;
+      if(lnode) lnode[key] = -1;
+      ext += (unsigned long long)c;
+      int hi = range[1];
+      n = range[0];
+      while(n < hi) {
+        const int mid = (n + hi + 1) >> 1;
+        if(nodes[mid].key_base <= key) n = mid; else hi = mid - 1;
+      }
+      cand = c >= nodes[n].minsup;
+      bytes += (childmap ? 4 : 0) + (lnode ? 4 : 0);  // child map and list node reset
+    }
+    if(cand && cnt_copies > 1) {
+      // a key that may be materialised: copy 0 keeps the total, copy q >= 1
+      // becomes the count of copies 0..q-1 (the offset of its share)
+      int run = x[0];
+#pragma unroll
+      for(int q = 1; q < 4; q++)
+        if(q < cnt_copies) {
+          cnt[q * cnt_stride + key] = run;
+          run += x[q];
+        }
+      for(int q = 4; q < cnt_copies; q++) {
+        const int y = cnt[q * cnt_stride + key];
+        cnt[q * cnt_stride + key] = run;
+        run += y;
+      }
+      cnt[key] = c;
+      bytes += 4ull * (unsigned)cnt_copies;  // the copies turned into offsets
+    }
+    const unsigned m = __ballot_sync(full, cand);
+    if(lane == 0) wlist[warp] = __popc(m);
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for(int w = 0; w < kBlock / 32; w++) {
+      const int y = wlist[w];
+      if(w < warp) before += y;
+      total += y;
+    }
+    if(total == 0) continue;
+    if(cand) list[before + __popc(m & lanemask_lt())] = make_int2(key, n);
+    __syncthreads();
+    nlisted += total;
+    for(int li = warp; li < total; li += kBlock / 32) {
+      const int2 kn = list[li];
+      const NodeDesc &nd = nodes[kn.y];
+      const int words = nd.words;
+      if(words > kSelWords) continue;
+      const long long wbase = nd.bm_base + (long long)(kn.x - nd.key_base) * words;
+      const int running = warp_prefix_words(bm + wbase, bmx + wbase, words);
+      if(lane == 0) listed_done(kn, nd, wbase, running, cnt, keyword, sel, total_keys, counters, lnode, bytes);
+    }
+    // the branch is uniform over the block
+    for(int li = 0; li < total; li++) {
+      const int2 kn = list[li];
+      const NodeDesc &nd = nodes[kn.y];
+      const int words = nd.words;
+      if(words <= kSelWords) continue;
+      const long long wbase = nd.bm_base + (long long)(kn.x - nd.key_base) * words;
+      const int running = block_prefix_words(bm + wbase, bmx + wbase, words, wtot);
+      if(threadIdx.x == 0) listed_done(kn, nd, wbase, running, cnt, keyword, sel, total_keys, counters, lnode, bytes);
+    }
+  }
+  for(int o = 16; o > 0; o >>= 1) {
+    ext += __shfl_down_sync(full, ext, o);
+    bytes += __shfl_down_sync(full, bytes, o);
+  }
+  // one add per block: adds to one address complete one after another
+  __shared__ unsigned long long wext[kBlock / 32], wbytes[kBlock / 32];
+  if(lane == 0) {
+    wext[warp] = ext;
+    wbytes[warp] = bytes;
+  }
+  __syncthreads();
+  if(threadIdx.x == 0) {
+    for(int w = 1; w < kBlock / 32; w++) {
+      ext += wext[w];
+      bytes += wbytes[w];
+    }
+    if(ext) atomicAdd(&counters[1], ext);
+    if(nlisted) atomicAdd(&counters[2], (unsigned long long)nlisted);
     if(bytes) atomicAdd(&counters[3], bytes);
   }
 }
@@ -885,6 +1050,37 @@ KernelCall count_listed_call(const NodeDesc *nodes, const int2 *listed, const ui
   c.arg(sel_cap);
   c.arg(head);
   c.arg(lnode);
+  return c;
+}
+
+KernelCall select_call(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, int32_t *cnt, int32_t cnt_copies,
+                       long long cnt_stride, int32_t *childmap, const uint32_t *bm, int32_t *bmx, long long *keyword,
+                       int4 *sel, unsigned long long *head, unsigned int *err, int32_t *lnode, const uint32_t *reg)
+{
+  // as small chunks as the grid allows: a block counts its listed keys in turn
+  const int cap = 8 * sm_count(), per = (total_keys + cap - 1) / cap;
+  const int chunk = std::max(8, std::min(kBlock, per));
+  KernelCall c;
+  c.func = (const void *)k_select;
+  c.early = true;
+  c.grid = dim3((unsigned)std::max(1, std::min((total_keys + chunk - 1) / chunk, cap)));
+  c.block = dim3(kBlock);
+  c.arg(nodes);
+  c.arg(nnodes);
+  c.arg(total_keys);
+  c.arg(chunk);
+  c.arg(cnt);
+  c.arg(cnt_copies);
+  c.arg(cnt_stride);
+  c.arg(childmap);
+  c.arg(bm);
+  c.arg(bmx);
+  c.arg(keyword);
+  c.arg(sel);
+  c.arg(head);
+  c.arg(err);
+  c.arg(lnode);
+  c.arg(reg);
   return c;
 }
 

@@ -183,7 +183,7 @@ void launch_records_bitmap(const int32_t *keys, const int32_t *gids, long long n
 // the header's counters; listed and sel hold total_keys entries.  The
 // consistency flags after the count pass go to the header.
 // lnode (lists strategy, may be null): reset to -1 for every key with extensions
-// reg (packed rows, may be null): kHeadRecords = the most record blocks of a region
+// reg (may be null): kHeadRecords = the fullest region's records or blocks
 KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, int32_t *cnt,
                             int32_t cnt_copies, long long cnt_stride, int32_t *childmap, int2 *listed,
                             unsigned long long *head, unsigned int *err, int32_t *lnode, const uint32_t *reg);
@@ -192,6 +192,17 @@ KernelCall screen_keys_call(const NodeDesc *nodes, int32_t nnodes, int32_t total
 KernelCall count_listed_call(const NodeDesc *nodes, const int2 *listed, const uint32_t *bm, int32_t *cnt,
                              int32_t *bmx, long long *keyword, int4 *sel, int32_t sel_cap,
                              unsigned long long *head, int32_t *lnode);
+// Both in one kernel, for waves of at most kSelectWords bitmap words (8 MiB): a
+// block counts its chunk's listed keys in turn, and keys with many embeddings
+// stand together, so large waves are better spread by a list.  A wave of one
+// node takes 5.0 us in two kernels, 3.0 in one; 250,000 graphs at 0.5% 17 us a
+// wave in two, 50 when every wave takes one.  Selection of a mine with the line
+// at 0, 2^17, 2^19, 2^21, 2^22 words: 100,000 graphs 163, 163, 157, 146, 153 us;
+// 250,000 graphs 571, 560, 566, 553, 554.
+constexpr int64_t kSelectWords = 1 << 21;
+KernelCall select_call(const NodeDesc *nodes, int32_t nnodes, int32_t total_keys, int32_t *cnt, int32_t cnt_copies,
+                       long long cnt_stride, int32_t *childmap, const uint32_t *bm, int32_t *bmx, long long *keyword,
+                       int4 *sel, unsigned long long *head, unsigned int *err, int32_t *lnode, const uint32_t *reg);
 // Canonicality of the selected candidates (gs_ismin.cu) and the wave's results:
 // the low two bits of sel[i].w (above them the candidate's node) = 1 minimal, 0
 // not minimal, 2 left to the host (all of them when !check).  codes = the

@@ -200,3 +200,16 @@ def test_batch_of_id_widths(gs, tmp_path):
         for db, s, pats in zip(dbs, sups, got):
             assert pats == gs.mine(db, s, max_edges=4)[0]
             assert pats == gs.mine(db, s, max_edges=4, extension="lists")[0]
+
+
+# selection in one kernel (waves of up to 2^21 bitmap words) and in two, by graph replay and direct
+# launches; keys of at most 256 words and of more
+@pytest.mark.parametrize("launch_mode", [0, 1])
+def test_selection_forms(gs, launch_mode):
+    db = gs.Database.generate(5, scale=0.2)
+    s = int(0.01 * len(db))
+    large, sl = gs.mine_collect(db, s, launch_mode=launch_mode)
+    small, ss = gs.mine_collect(db, s, launch_mode=launch_mode, wave_words=1 << 20)
+    assert large == small and len(large) > 500
+    # waves limited to 2^20 words take one kernel less each
+    assert sl["launches"] / sl["waves"] > ss["launches"] / ss["waves"]
