@@ -128,7 +128,7 @@ struct MineOptions {
   int32_t root_part = 0;      // mine only the root subtrees with index % root_parts == root_part
   int32_t root_parts = 1;
   int32_t min_check = 0;      // canonicality: 0 on the GPU (host for oversized patterns), 1 on the host
-  int32_t launch_mode = 0;    // a wave's device work: 0 replayed from a CUDA graph, 1 launched directly
+  int32_t launch_mode = 0;    // a wave's device work: 0 replayed from a CUDA graph behind another wave, 1 launched directly
   int32_t count_grid = 0;     // count-kernel grid cap in blocks per SM (0 = the built-in default)
   int32_t extension = 0;      // extension strategy: 0 every right-most-path vertex's adjacency is
                               // scanned; 1 lists: forward children join their parent's per-row

@@ -177,8 +177,9 @@ typedef struct gs_mine_opts {
   int32_t root_parts;  /* order) is root_part modulo root_parts; root_parts <= 1 = all */
   int32_t min_check;   /* canonicality check: 0 = on the GPU (patterns over 32 vertices or 64 edges,
                           or with too many self-embeddings, on the host), 1 = on the host */
-  int32_t launch_mode; /* a wave's device work (uploads, clears, count, selection, check, results
-                          copy): 0 = replayed from a per-variant CUDA graph, 1 = launched directly */
+  int32_t launch_mode; /* a wave's device work (tables in, count, selection, check and results out):
+                          0 = replayed from a per-variant CUDA graph, or launched directly when no
+                          other wave is in flight, 1 = launched directly */
   int32_t count_grid;  /* count-kernel grid cap in blocks per SM; 0 = built-in default (64) */
   int32_t extension;   /* extension strategy: GS_EXTENSION_RMPATH (default) scans the adjacency of every
                           right-most-path vertex of every embedding; GS_EXTENSION_LISTS is the
