@@ -46,6 +46,10 @@ inline unsigned blocks_for(long long n)
   return (unsigned)(b < cap ? b : cap);
 }
 
+// For kernels whose blocks end in an add to one address, which complete one
+// after another at about 1.6 ns: 9,272 blocks took 15 us over 9 MB.
+inline unsigned few_blocks_for(long long n) { return std::min(blocks_for(n), 4u * (unsigned)gsgb::sm_count()); }
+
 // ---- exclusive scan of int64 values, three passes per level
 __global__ void k_scan_blocks(const long long *in, long long *out, long long n, long long *block_sums)
 {
@@ -648,8 +652,8 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
     static const int init[4] = { INT32_MAX, INT32_MIN, INT32_MAX, INT32_MIN };
     CK(cudaMemcpyAsync(mm, init, sizeof(init), cudaMemcpyHostToDevice, s));
   }
-  if(V) k_minmax<<<blocks_for(V), kThreads, 0, s>>>(vl, V, mm, mm + 1);
-  if(E2) k_minmax<<<blocks_for(E2), kThreads, 0, s>>>(el, E2, mm + 2, mm + 3);
+  if(V) k_minmax<<<few_blocks_for(V), kThreads, 0, s>>>(vl, V, mm, mm + 1);
+  if(E2) k_minmax<<<few_blocks_for(E2), kThreads, 0, s>>>(el, E2, mm + 2, mm + 3);
   CK(cudaMemcpyAsync(&rb.flags, flags, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(rb.minmax, mm, sizeof(rb.minmax), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
@@ -684,8 +688,8 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
   scan_exclusive(seen, prank, tab, sc);
   int *d_mx = sc.get<int>(2);
   CK(cudaMemsetAsync(d_mx, 0, 2 * sizeof(int), s));
-  k_max_ll<<<blocks_for(G), kThreads, 0, s>>>(gnv, G, d_mx);
-  if(V) k_max_degree<<<blocks_for(V), kThreads, 0, s>>>(off, V, d_mx + 1);
+  k_max_ll<<<few_blocks_for(G), kThreads, 0, s>>>(gnv, G, d_mx);
+  if(V) k_max_degree<<<few_blocks_for(V), kThreads, 0, s>>>(off, V, d_mx + 1);
   CK(cudaMemcpyAsync(&rb.nkeys, prank + tab, sizeof(long long), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(&rb.max_vertices, d_mx, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
