@@ -13,10 +13,11 @@ e2e        : same metric through the C ABI from host arrays: the reference's
              cudabin arrays copied to the GPU and converted there
              (gs_db_from_arrays_device), mined, every pattern written to the
              host buffer -- all inside the timed step
-roofline   : the count kernel (k_wave count, the dominant kernel): algorithmic
-             bytes / kernel time, both measured inside the library on its own
-             stream with CUDA events, against the measured HBM peak; the
-             materialise and selection kernels beside it
+roofline   : the count kernel ("k_wave count", the dominant kernel; k_rows on
+             packed rows): algorithmic bytes / kernel time, both measured inside
+             the library, the time by stamps of the device's nanosecond clock,
+             against the measured HBM peak; the materialise and selection
+             kernels beside it
 cpu_baseline: the oracle (C restatement of the reference's sequential gSpan) on
              one host core, a time-bounded sample of the same workload
 Nested, same line: configuration 2 (100,000 graphs) at minsup 1/2/5%, the
@@ -314,11 +315,11 @@ class Timer:
 
 def roofline(stats_all, peak, peak_kind, traffic, traffic_note, serial_stats=None):
     """Achieved GB/s of the count, materialise and selection kernels: their
-    algorithmic bytes (counted inside the kernels) / their device time (CUDA
-    events on the wave contexts' streams), averaged over the timed steps.
-    In the timed steps the contexts' streams overlap: one wave's selection and
-    materialise passes share the GPU with another wave's count, so their event
-    spans include time spent sharing it.  serial_stats (untimed passes with
+    algorithmic bytes (counted by the library) / their device time (stamps of
+    the device's clock at the kernels' starts and ends), averaged over the timed
+    steps.  In the timed steps the contexts' streams overlap: one wave's
+    selection and materialise passes share the GPU with another wave's count,
+    so their spans include time spent sharing it.  serial_stats (untimed passes with
     every context on one stream, gs_mine_opts.serial) give each kernel's
     exclusive time: "kernels_one_stream"."""
     n = len(stats_all)
@@ -339,10 +340,10 @@ def roofline(stats_all, peak, peak_kind, traffic, traffic_note, serial_stats=Non
             "frac": count["frac"], "peak_kind": peak_kind, "traffic": traffic, "traffic_source": traffic_note,
             "algorithmic_bytes_per_step": count["algorithmic_bytes_per_step"],
             "kernel_ms_per_step": count["kernel_ms_per_step"], "launches_per_step": waves,
-            "kernels": {"k_wave count": count, "materialise (k_mat_records, k_wave materialise)": mat,
-                        "selection (k_screen_keys + k_count_listed)": sel,
+            "kernels": {"k_wave count": count, "materialise (k_rows_mat; k_mat_records on columns)": mat,
+                        "selection (k_select; k_screen_keys + k_count_listed in large waves)": sel,
                         "k_is_min": {"kernel_ms_per_step": avg("min_ms"), "note": "shared memory only"}},
-            "kernels_note": "event spans on overlapping streams (a pass sharing the GPU with another wave's count)",
+            "kernels_note": "spans on overlapping streams (a pass sharing the GPU with another wave's count)",
             "kernels_one_stream": roofline(serial_stats, peak, peak_kind, None, None)["kernels"] if serial_stats
             else None}
 

@@ -2393,9 +2393,9 @@ private:
           o.kind = cd.edge.is_forward() ? 0 : 1;
           const int32_t nv = p.nv + (cd.edge.is_forward() ? 1 : 0);
           if(f.packed) {
-            // algorithmic bytes of a child row: its parent's, the rank's bitmap
-            // word and prefix, the row written
-            st_.mat_bytes += rowsn * (16 * packed_planes(p.nv) + 8 + 16 * packed_planes(nv));
+            // algorithmic bytes of a child row: its child map entry, its parent's
+            // row, the rank's bitmap word and prefix, the row written
+            st_.mat_bytes += rowsn * (4 + 16 * packed_planes(p.nv) + 8 + 16 * packed_planes(nv));
             o.planes = packed_planes(nv);
             o.k = p.nv;
             o.prows = p.rows;
@@ -2460,8 +2460,8 @@ private:
       for(int32_t n = 0; n < W; n++) made_at[n + 1] += made_at[n];
     }
     if(nout > 0) {
-      // an item and its child map entry per extension
-      if(f.packed) st_.mat_bytes += 8 * n_ext;
+      // an item per extension
+      if(f.packed) st_.mat_bytes += 4 * n_ext;
       const size_t mat_bytes = outs_bytes + pairs_bytes + (list_blk >= 0 ? Carver::round(sizeof(int32_t) * (size_t)W) : 0);
       X.d_mat.ensure(mat_bytes);
       if(list_blk >= 0) std::memcpy(X.h_mat.p + outs_bytes + pairs_bytes, list_rb.data(), sizeof(int32_t) * W);

@@ -8,10 +8,10 @@
 // loads (a sector each), then two offsets and about 21 bytes of entries per
 // right-most-path vertex, and every step of 32 entries searched owners and
 // emitted few extensions.  250,000 graphs of 40 edges at minsup 0.5% (192 M
-// rows, 760 M extensions, one stream): count kernels 33.3 ms on columns, 11.4
-// here; a large launch 1.30 -> 0.46 ms with 989 M -> 402 M warp instructions
-// and 2.2 -> 0.9 GB of DRAM traffic.  It is bound by issue now (71% of
-// cycles, the integer pipe 69%; 0.24 of the DRAM peak).
+// rows, 760 M extensions, one stream): count kernels 33.3 ms on columns, 11.2
+// here; a large launch 1.30 -> 0.45 ms with 989 M -> 390 M warp instructions
+// and 2.2 -> 0.73 GB of DRAM traffic.  It is bound by issue now (70% of
+// cycles, the integer pipe 64%; 0.24 of the DRAM peak).
 #include <algorithm>
 
 #include "gs_kernels.hpp"

@@ -99,7 +99,9 @@ GS_API gs_db *gs_db_from_arrays(int32_t db_size, int32_t edges_sizes, int32_t ma
  * Memory: the scratch and the database come from a stream-ordered pool that
  * keeps up to 16 GiB of device memory between ingests (gs_engine_reset
  * returns it), and such a database holds its adjacency twice (8 more bytes
- * per entry): sorted for mining and in input order for gs_db_write. */
+ * per entry): sorted for mining and in input order for gs_db_write.  Every
+ * database of graphs of at most 256 vertices also holds neighbour blocks when
+ * there is room for them: 32 bytes per vertex and 32/7 per adjacency entry. */
 GS_API gs_db *gs_db_from_arrays_device(int32_t db_size, int32_t edges_sizes, int32_t max_graph_vertex_count,
                                        int32_t vertex_count, const int32_t *edges, const int32_t *edges_labels,
                                        const int32_t *vertex_labels, const int32_t *vertex_offsets,
