@@ -8,7 +8,7 @@
 // loads (a sector each), then two offsets and about 21 bytes of entries per
 // right-most-path vertex, and every step of 32 entries searched owners and
 // emitted few extensions.  250,000 graphs of 40 edges at minsup 0.5% (192 M
-// rows, 760 M extensions, one stream): count kernels 33.3 ms on columns, 11.2
+// rows, 760 M extensions, one stream): count kernels 33.3 ms on columns, 10.7
 // here; a large launch 1.30 -> 0.45 ms with 989 M -> 390 M warp instructions
 // and 2.2 -> 0.73 GB of DRAM traffic.  It is bound by issue now (70% of
 // cycles, the integer pipe 64%; 0.24 of the DRAM peak).
@@ -36,6 +36,7 @@ constexpr unsigned kFull = 0xffffffffu;
 #define GS_ROWS_GROUP 4  // tiles
 #endif
 constexpr int kRecBlocks = 4;  // record blocks a warp reserves at a time
+constexpr int kShort = 6;      // entries of a block that every lane tests
 
 struct RowsArgs {
   const PackedNode *nodes;
@@ -276,10 +277,9 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB :
         m_hi |= shl_one(lv - 32u);
       }
     }
-    const unsigned long long mask = ((unsigned long long)m_hi << 32) | m_lo;
     auto in_row = [&](unsigned y) {  // entry y's vertex
       if(WIDE) return (S.in[((y & idm) >> 5) * 32 + lane] >> (y & 31u)) & 1u;
-      return (unsigned)(mask >> (y & 63u)) & 1u;
+      return __funnelshift_r((y & 32u) ? m_hi : m_lo, 0u, y) & 1u;  // (bit y & 31 of the half)
     };
     const bool back = S.nd.back != 0;
     const uint4 *__restrict__ nb = S.nd.nb;
@@ -320,14 +320,23 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB :
       // ---- this block's entries that are forward extensions
       const int rule = S.slot[s].prule;
       unsigned acc = 0;
+      // lists of more than kShort entries are few: the last words only where a
+      // lane has one (10.91 -> 10.74 ms on 250,000 graphs; at 4 or 5 10.79)
+      const bool tail = __any_sync(kFull, x[kShort] != 0);
       if(minl == 0) {
 #pragma unroll
-        for(int u = 0; u < 8; u++)
-          acc |= (int)x[u] >= rule && !in_row(x[u]) ? 1u << u : 0u;
+        for(int u = 0; u < kShort; u++) acc |= (int)x[u] >= rule && !in_row(x[u]) ? 1u << u : 0u;
+        if(tail)
+#pragma unroll
+          for(int u = kShort; u < 8; u++) acc |= (int)x[u] >= rule && !in_row(x[u]) ? 1u << u : 0u;
       } else {
 #pragma unroll
-        for(int u = 0; u < 8; u++)
+        for(int u = 0; u < kShort; u++)
           acc |= (int)x[u] >= rule && (x[u] & wlm) >= minl && !in_row(x[u]) ? 1u << u : 0u;
+        if(tail)
+#pragma unroll
+          for(int u = kShort; u < 8; u++)
+            acc |= (int)x[u] >= rule && (x[u] & wlm) >= minl && !in_row(x[u]) ? 1u << u : 0u;
       }
       const int c = __popc(acc);
       const int incl = warp_incl(c);
@@ -335,8 +344,12 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB :
       qn += __shfl_sync(kFull, incl, 31);
       const unsigned meta = (unsigned)lane | ((unsigned)s << 5);
 #pragma unroll
-      for(int u = 0; u < 8; u++)
+      for(int u = 0; u < kShort; u++)
         if((acc >> u) & 1u) *at++ = make_uint2(x[u], meta);
+      if(tail)
+#pragma unroll
+        for(int u = kShort; u < 8; u++)
+          if((acc >> u) & 1u) *at++ = make_uint2(x[u], meta);
       // ---- backward edges from the right-most vertex: entries whose vertex is
       // a right-most-path vertex of the row that takes one (not accepted above,
       // so the queue has room: 8 items per lane behind 31)
