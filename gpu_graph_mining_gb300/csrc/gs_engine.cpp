@@ -738,7 +738,7 @@ struct WaveSeq {
   int n = 0;
 };
 
-// WaveSeq as an instantiated CUDA graph, one per count-kernel variant and
+// WaveSeq as an instantiated CUDA graph, one per count-kernel variant, length and
 // context: each wave updates the nodes' parameters and launches the graph.
 struct WaveGraph {
   const void *count_func = nullptr;

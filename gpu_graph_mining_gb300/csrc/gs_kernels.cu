@@ -1,5 +1,5 @@
 // Root-level and support kernels for one GB300 (sm_103a); the wave-level
-// extension kernels are in gs_wave.cu.
+// extension kernels are in gs_rows.cu (packed rows) and gs_wave.cu (columns).
 //
 // Support is counted without extension records: every embedding of a
 // candidate sets one bit in the candidate's bitmap over the graph ranks of
