@@ -474,20 +474,21 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB :
   if(MAT) stamp_mat_end(a.stamp);
 }
 
-// Materialise from the record blocks.  A warp takes kMatBlocks consecutive
-// blocks of a region, their loads in flight together, tests the items' keys in
-// the bit set of the chosen ones (a node's keys are a few words, one sector)
-// and queues the items that are; 32 queued ones are then placed together:
-// child map, child, and from there the parent's row, the graph rank's bitmap
-// word and the cursor side by side.  A third of the items are chosen on
-// 250,000 graphs of 40 edges, a tenth in the deep waves.  An item per lane
-// with a child map entry gathered for every item took 5.7 ms a pass there,
-// this 3.8 (100,000 graphs at 1%: 0.63 -> 0.46); latency and issue bound (60%),
-// 0.22 of the DRAM peak.  The child map gather was 13 to 15 sectors a block.
+// Materialise from the record blocks.  A warp takes B (kMatBlocks, or one in
+// small waves) consecutive blocks of a region, their loads in flight together,
+// tests the items' keys in the bit set of the chosen ones (a node's keys are a
+// few words, one sector) and queues the items that are; 32 queued ones are then
+// placed together: child map, child, and from there the parent's row, the graph
+// rank's bitmap word and the cursor side by side.  A third of the items are
+// chosen on 250,000 graphs of 40 edges, a tenth in the deep waves.  An item per
+// lane with a child map entry gathered for every item took 5.7 ms a pass there,
+// this 3.8 (100,000 graphs at 1%: 0.63 -> 0.43); latency and issue bound (61%),
+// 0.4 of the DRAM peak in a large launch.  The child map gather was 13 to 15
+// sectors a block.
 constexpr int kMatWarps = 8, kMatBlocks = 4;
 constexpr int kMatGrid = 16;  // thread blocks per SM: 8 are resident
 
-template <int PL, bool WIDE>
+template <int PL, bool WIDE, int B>
 __global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__restrict__ rec,
                                                              const int4 *__restrict__ hdr,
                                                              const uint32_t *__restrict__ reg, int blk_cap,
@@ -502,33 +503,33 @@ __global__ void __launch_bounds__(kMatWarps * 32) k_rows_mat(const uint32_t *__r
   constexpr int NW = 2 + 4 * (PL - 1);
   // queue entries: wave key (23 bits), counter copy (2), graph-local new vertex
   // (8), parent row (31)
-  __shared__ unsigned long long queue[kMatWarps][32 * (kMatBlocks + 1)];
+  __shared__ unsigned long long queue[kMatWarps][32 * (B + 1)];
   unsigned long long *const q = queue[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   // a warp stays in one region (the number of warps is a multiple of theirs)
   const int b0 = blockIdx.x * kMatWarps + (threadIdx.x >> 5);
   const int region = b0 % kRecRegions;
-  const int step = gridDim.x * kMatWarps / kRecRegions * kMatBlocks;
+  const int step = gridDim.x * kMatWarps / kRecRegions * B;
   const int used = min((int)min(__ldg(&reg[region * kRecRegionStride]), 0x7fffff00u), blk_cap);
   const int4 *const rh = hdr + (long long)region * blk_cap;
   const uint32_t *const ri = rec + (long long)region * blk_cap * 32 + lane;
   int qn = 0;
-  for(int i = b0 / kRecRegions * kMatBlocks; i < used || qn > 0; i += step) {
+  for(int i = b0 / kRecRegions * B; i < used || qn > 0; i += step) {
     if(i < used) {
       int4 h = make_int4(0, 0, 0, 0);  // lane t: the header of block i + t
-      if(lane < kMatBlocks && i + lane < used) h = __ldg(&rh[i + lane]);
-      unsigned it[kMatBlocks];
-      uint32_t w[kMatBlocks];
+      if(lane < B && i + lane < used) h = __ldg(&rh[i + lane]);
+      unsigned it[B];
+      uint32_t w[B];
 #pragma unroll
-      for(int t = 0; t < kMatBlocks; t++) it[t] = i + t < used ? __ldg(&ri[(long long)(i + t) * 32]) : 0u;
+      for(int t = 0; t < B; t++) it[t] = i + t < used ? __ldg(&ri[(long long)(i + t) * 32]) : 0u;
 #pragma unroll
-      for(int t = 0; t < kMatBlocks; t++) {
+      for(int t = 0; t < B; t++) {
         const int hz = __shfl_sync(kFull, h.z, t), m = hz & 0xff;
         const int key = __shfl_sync(kFull, h.w, t) + (int)(it[t] >> (WIDE ? hz >> 16 : 11));
         w[t] = lane < m ? chosen[key >> 5] : 0u;
       }
 #pragma unroll
-      for(int t = 0; t < kMatBlocks; t++) {
+      for(int t = 0; t < B; t++) {
         const int hz = __shfl_sync(kFull, h.z, t), kb = WIDE ? hz >> 16 : 11;
         const int key = __shfl_sync(kFull, h.w, t) + (int)(it[t] >> kb);
         const bool on = (w[t] >> (key & 31)) & 1u;
@@ -676,6 +677,12 @@ template <bool MAT> KernelCall rows_call(const RowsArgs &a, int planes, bool wid
        : planes <= 2 ? rows_call<2, MAT, false>(a, grid_per_sm) : rows_call<5, MAT, false>(a, grid_per_sm);
 }
 
+template <int B> auto *mat_kernel(int planes, bool wide)
+{
+  if(wide) return planes <= 1 ? k_rows_mat<1, true, B> : planes <= 2 ? k_rows_mat<2, true, B> : k_rows_mat<5, true, B>;
+  return planes <= 1 ? k_rows_mat<1, false, B> : planes <= 2 ? k_rows_mat<2, false, B> : k_rows_mat<5, false, B>;
+}
+
 }  // namespace
 
 KernelCall rows_count_call(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
@@ -708,12 +715,13 @@ void launch_rows_records(const uint32_t *rec, const int4 *hdr, const uint32_t *r
   if(most <= 0) return;
   static_assert(kRecRegions % kMatWarps == 0, "thread blocks per set of regions");
   constexpr int kPer = kRecRegions / kMatWarps;
-  const long long want = ((long long)most + kMatBlocks - 1) / kMatBlocks * kPer;
   const long long cap = (long long)kMatGrid * sm_count() / kPer * kPer;
+  // a block a turn while every block has a warp of its own: four in turn were
+  // 8 to 20% slower there (340 graphs: 33 -> 27 us a mine; larger waves equal)
+  const bool one = (long long)most * kPer <= cap;
+  const long long want = one ? (long long)most * kPer : ((long long)most + kMatBlocks - 1) / kMatBlocks * kPer;
   const int blocks = (int)(want < cap ? want : cap);
-  auto *f = planes <= 1 ? (wide ? k_rows_mat<1, true> : k_rows_mat<1, false>)
-          : planes <= 2 ? (wide ? k_rows_mat<2, true> : k_rows_mat<2, false>)
-                        : (wide ? k_rows_mat<5, true> : k_rows_mat<5, false>);
+  auto *f = one ? mat_kernel<1>(planes, wide) : mat_kernel<kMatBlocks>(planes, wide);
   KernelCall c;
   c.func = (const void *)f;
   c.early = true;
