@@ -274,7 +274,7 @@ namespace {
 
 // First-fit sub-allocator over a few large cudaMalloc chunks.  Memory freed
 // here is handed out again at once: the engine returns a block only after
-// the last passes that may read it have completed (Engine::reap).
+// the last passes that may read or write it have completed (Engine::reap).
 class Pool {
 public:
   void set_limit(int64_t b) { limit_ = b; }
@@ -951,14 +951,15 @@ struct Engine {
   static constexpr int64_t kRootGroupBytes = 1LL << 30;   // bitmap bytes (one job at least)
   bool ready = false;
   // Pool blocks whose last reference was dropped go back to the pool only
-  // after every wave context's last materialise pass has completed: the
-  // only passes that read a node's memory after the host dropped the node
-  // are the materialise passes queued for its wave (the record-driven pass
-  // reads records, the enumerating fallback the wave's columns); counts read
-  // live nodes only, root phases write new blocks only.  Each context's
-  // ev_mat follows its latest materialise pass, so when every context's
-  // ev_mat has completed, every block released so far is free (a later
-  // record of an event only makes the wait longer).
+  // after every wave context's last materialise pass and the last root phase
+  // have completed.  The passes that touch a node's memory after the host
+  // dropped the node are the materialise passes queued for its wave (they read
+  // its rows) and, for a root node of a job cancelled as soon as it was added,
+  // the root phase that is still to write its rows; counts read live nodes
+  // only.  Each context's ev_mat follows its latest materialise pass (the root
+  // context's the latest root phase), so when all of them have completed, every
+  // block released so far is free (a later record of an event only makes the
+  // wait longer).
   std::vector<void *> released;
   uint64_t main_gen = 0;          // records of ev_main
 
@@ -1029,22 +1030,27 @@ struct Engine {
     for(auto &c : ctx)
       if(c.stream) cudaStreamSynchronize(c.stream);
   }
+  // whether the event has completed (wait: waits for it)
+  static bool passed(cudaEvent_t ev, bool wait)
+  {
+    if(!ev) return true;
+    const cudaError_t q = cudaEventQuery(ev);
+    if(q != cudaErrorNotReady) {
+      CK(q);
+      return true;
+    }
+    if(wait) CK(cudaEventSynchronize(ev));
+    return wait;
+  }
   // returns the released blocks to the pool once every context's last
-  // materialise pass has completed (wait: waits for them).  Returns false
-  // when nothing was released.
+  // materialise pass and the last root phase have completed (wait: waits for
+  // them).  Returns false when nothing was released.
   bool reap(bool wait)
   {
     if(released.empty()) return false;
-    for(auto &c : ctx) {
-      if(!c.ev_mat) continue;
-      const cudaError_t q = cudaEventQuery(c.ev_mat);
-      if(q == cudaErrorNotReady) {
-        if(!wait) return false;
-        CK(cudaEventSynchronize(c.ev_mat));
-      } else {
-        CK(q);
-      }
-    }
+    for(auto &c : ctx)
+      if(!passed(c.ev_mat, wait)) return false;
+    if(!passed(rootx.ev_mat, wait)) return false;
     for(void *b : released) pool.release(b);
     released.clear();
     return true;
@@ -1266,8 +1272,8 @@ double ms_since(clk::time_point t0) { return std::chrono::duration<double, std::
 // stream: a wave's count waits for the engine's stream (database table, root
 // levels) and for every other context's last materialise pass, so that its
 // nodes' columns are written before it reads them; pool memory released on
-// the host is reused only after every context's last materialise pass has
-// completed (Engine::reap).
+// the host is reused only after every context's last materialise pass and the
+// last root phase have completed (Engine::reap).
 class Sched {
 public:
   Sched(Engine &e, const MineOptions &wo, MineStats &st)
