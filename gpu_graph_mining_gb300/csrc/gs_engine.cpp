@@ -2066,7 +2066,7 @@ private:
                           : (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, ((int64_t)1 << 22) / std::max(kb, 1)));
     const long long cstride = (long long)Carver::round(sizeof(int32_t) * (size_t)std::max(kb, 1)) / 4;
     const size_t cnt_bytes = sizeof(int32_t) * (size_t)cstride * ccopies;
-    // packed rows: the record regions' counters, behind the embedding counters
+    // the record regions' counters, behind the embedding counters
     const size_t reg_bytes = sizeof(uint32_t) * kRecRegions * kRecRegionStride;
     // and a bit per key to materialise
     const size_t sel_bytes = packed ? Carver::round((size_t)(kb + 31) / 32 * 4) : 0;
@@ -2111,7 +2111,7 @@ private:
         f.hdr = X.d_rec.p;
         f.rec = X.d_rec.p + f.rec_cap * kRecRegions;
       } else {
-        f.rec_cap /= kRecRegions;
+        f.rec_cap = f.rec_cap / (kRecRegions * kRecChunk) * kRecChunk;
       }
     }
     // the frequent candidates come back compacted, as many as there was need of

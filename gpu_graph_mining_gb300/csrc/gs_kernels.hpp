@@ -103,6 +103,8 @@ void launch_root_materialize(const RootJob *jobs, int32_t njobs, long long tiles
 // sized for 8/16/32/64 pattern vertices); collen[] parallels coltab[]: the
 // length of every column.
 // small_graphs: every graph of the wave's databases has <= 64 vertices.
+// rec (may be null): kRecRegions regions of rec_cap records, whole chunks of
+// kRecChunk; reg: their counters, as for the packed rows (zeroed before).
 // rule_skip: in databases with sorted adjacency (DevDB::adj_sorted), a
 // right-most-path vertex's entries below its forward rule are bisected past
 // instead of scanned.
@@ -130,6 +132,10 @@ void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long to
 // the adds of a large node's few keys as well as 256 would, one makes the count
 // 14% slower); the wave's keys stay below kRowsKeys.
 constexpr int kRecRegions = 64, kRecRegionStride = 32;
+#ifndef GS_REC_CHUNK
+#define GS_REC_CHUNK 128
+#endif
+constexpr int kRecChunk = GS_REC_CHUNK;  // column records a warp reserves at a time
 // Thread blocks for a kernel whose blocks each stay in one region, an item per
 // thread of threads, the fullest region holding most.
 inline int region_blocks(long long most, int threads)

@@ -51,10 +51,6 @@ namespace {
 #endif
 constexpr int kWarps = GS_WAVE_WARPS;
 constexpr unsigned kFull = 0xffffffffu;
-#ifndef GS_REC_CHUNK
-#define GS_REC_CHUNK 128
-#endif
-constexpr int kRecChunk = GS_REC_CHUNK;  // records a warp reserves at a time
 
 struct WaveArgs {
   const NodeDesc *nodes;
@@ -76,7 +72,7 @@ struct WaveArgs {
   // count pass, optional: one record per extension {wave key, child column
   // element x, y, graph rank} for the record-driven materialise pass
   int4 *rec;
-  long long rec_cap;   // records of one of the kRecRegions regions
+  int rec_cap;         // records of one of the kRecRegions regions, whole chunks
   uint32_t *rec_n;     // records reserved in each region (may exceed rec_cap: none past it are written)
   // count pass: cnt holds cnt_copies copies of the wave's counters, cnt_stride
   // apart; warp w adds into copy w % cnt_copies (summed by the screening pass)
@@ -108,6 +104,25 @@ __device__ __forceinline__ unsigned lanemask_lt()
   return m;
 }
 
+// A chunk of kRecChunk records (lane 0 of a warp): its first record, or kNoChunk
+// when its region is full.  The warps reserve from kRecRegions counters: adds to
+// one address complete at about one per 1.6 ns, which bounded the kernel when
+// one counter served all warps.  A warp takes its chunks from the regions in
+// turn: one tile of rows at a vertex of thousands of neighbours fills them
+// evenly, where a region per warp needed a buffer of up to 64 times the records.
+// 256 graphs with a vertex of 5,000 neighbours each: a mine 38.1 ms with a region
+// per warp, 33.6 with one counter, 32.4 so; 250,000 graphs of 40 edges at 1%,
+// lists strategy: count kernels 19.9, 21.1 and 18.8 ms.
+static_assert((kRecChunk & (kRecChunk - 1)) == 0, "chunks start at multiples of a power of two");
+constexpr int kNoChunk = -(1 << 30);
+__device__ __forceinline__ int reserve_chunk(uint32_t *reg, int cap, int &region)
+{
+  const int r = region;
+  region = (r + 1) % kRecRegions;
+  const unsigned at = atomicAdd(&reg[r * kRecRegionStride], (unsigned)kRecChunk);
+  return at < (unsigned)cap ? r * cap + (int)at : kNoChunk;
+}
+
 // MASK: every graph of the wave's databases has at most 64 vertices, so
 // "is w already in the embedding" is one bit test of the row's vertex set
 // instead of a loop over its k vertices.  JOIN: some node of the wave joins
@@ -129,15 +144,12 @@ k_wave(const WaveArgs a)
   const long long nwarps = (long long)gridDim.x * kWarps;
   if(!MAT) stamp_start(a.stamp);
   if(lane == 0) S.bytes = 0;
-  // count pass with records: the warp's current reserved chunk (warp-uniform);
-  // starts "full" so the first batch reserves a chunk.  The warps reserve from
-  // kRecRegions counters, each with its part of the records: adds to one
-  // address complete at about one per 1.6 ns, which bounded the kernel when one
-  // counter served all warps.
-  const int region = (int)(gwarp % kRecRegions);
-  int4 *const rec = a.rec + region * a.rec_cap;
-  long long chunk_base = -1;
-  int chunk_fill = kRecChunk;
+  // count pass with records: where the warp's next record goes (warp-uniform).
+  // Chunks start at multiples of kRecChunk: at one, the next record needs a new
+  // chunk.  Negative: the chunk's region was full, the record is dropped.  region
+  // (lane 0): where the warp reserves its next chunk.
+  int region = (int)((gwarp + gwarp / kRecRegions) % kRecRegions);
+  int rec_at = 0;
   const int copy = (int)(gwarp % (a.cnt_copies > 0 ? a.cnt_copies : 1));
   int32_t *const cnt_copy = MAT ? nullptr : a.cnt + copy * a.cnt_stride;
   // records carry the copy their embedding was counted in (bits 27-30 of the
@@ -401,24 +413,20 @@ k_wave(const WaveArgs a)
           // freshly reserved chunk (one global atomic per chunk, not per step)
           const int cntx = __popc(ext);
           const int rank = __popc(ext & lanemask_lt());
-          long long dst = -1;
-          if(chunk_fill + cntx <= kRecChunk) {
-            dst = chunk_base + chunk_fill + rank;
-            chunk_fill += cntx;
-          } else {
-            const int room = kRecChunk - chunk_fill;
-            int nb = 0;
-            if(lane == 0)
-              nb = (int)min(atomicAdd(&a.rec_n[region * kRecRegionStride], (unsigned)kRecChunk), 0x7fffff00u);
-            nb = __shfl_sync(kFull, nb, 0);
-            dst = rank < room ? chunk_base + chunk_fill + rank : (long long)nb + (rank - room);
-            chunk_base = nb;
-            chunk_fill = cntx - room;
+          const int room = -rec_at & (kRecChunk - 1);
+          int dst = rec_at + rank;
+          rec_at += cntx;
+          if(cntx > room) {
+            int chunk = 0;
+            if(lane == 0) chunk = reserve_chunk(a.rec_n, a.rec_cap, region) - room;
+            chunk = __shfl_sync(kFull, chunk, 0);
+            rec_at = chunk + cntx;
+            if(rank >= room) dst = chunk + rank;
           }
-          if(key >= 0 && dst >= 0 && dst < a.rec_cap) {
+          if(key >= 0 && dst >= 0) {
             const int i_o = row0 + o;
-            rec[dst] = bwd ? make_int4((key_base + key) | rec_tag, S.phi[k - 1][o], S.lp[o], g_o)
-                           : make_int4((key_base + key) | rec_tag, w, i_o, g_o);
+            a.rec[dst] = bwd ? make_int4((key_base + key) | rec_tag, S.phi[k - 1][o], S.lp[o], g_o)
+                             : make_int4((key_base + key) | rec_tag, w, i_o, g_o);
           }
         }
       } else {
@@ -446,12 +454,9 @@ k_wave(const WaveArgs a)
     }
     __syncwarp();
   }
-  if(!MAT && a.rec && chunk_base >= 0) {
+  if(!MAT && a.rec && rec_at >= 0) {
     // mark the unused tail of the last chunk as holes (key -1)
-    for(int f = chunk_fill + lane; f < kRecChunk; f += 32) {
-      const long long dst = chunk_base + f;
-      if(dst < a.rec_cap) rec[dst] = make_int4(-1, 0, 0, 0);
-    }
+    for(int f = lane; f < (-rec_at & (kRecChunk - 1)); f += 32) a.rec[rec_at + f] = make_int4(-1, 0, 0, 0);
   }
   // one add per block: adds to one address complete one after another
   __syncthreads();
@@ -537,7 +542,7 @@ KernelCall wave_count_call(const NodeDesc *nodes, int32_t nnodes, long long tota
                            long long cnt_stride, bool join, bool rule_skip)
 {
   WaveArgs a{ nodes, nnodes, total_tiles, coltab, collen, slots, vtab, dbs, bm, nullptr, cnt,
-              nullptr, nullptr, nullptr, bytes, err, rec, rec_cap, reg, cnt_copies,
+              nullptr, nullptr, nullptr, bytes, err, rec, (int)rec_cap, reg, cnt_copies,
               cnt_stride, rule_skip ? 1 : 0, head + kHeadCount0 };
   if(small_graphs)
     return join ? count_call<true, true>(kmax, a, grid_per_sm) : count_call<true, false>(kmax, a, grid_per_sm);
