@@ -34,7 +34,8 @@ namespace gsgb {
 
 void cuda_check(cudaError_t e, const char *what)
 {
-  if(e != cudaSuccess) throw Error(ST_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  if(e != cudaSuccess)
+    throw Error(ST_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e), e == cudaErrorMemoryAllocation);
 }
 
 #define CK(call) cuda_check((call), #call)
@@ -1352,13 +1353,15 @@ public:
       E.scratch.spare.pop_back();
     }
     // the lists strategy joins on parent rows: columns
-    S.packed = db->dev.nb != nullptr && wo_.extension == 0;
+    S.packed = db->dev.nb != nullptr && wo_.extension == 0 && !j.opt.columns;
+    any_packed_ = any_packed_ || S.packed;
     active_++;
     order_.push_back(id);
     return id;
   }
 
   bool idle() const { return active_ == 0; }
+  bool packed() const { return any_packed_; }
 
   void step()
   {
@@ -1439,6 +1442,15 @@ public:
 
   int64_t pool_used() const { return (int64_t)E.pool.used(); }
 
+  // drops from js (the jobs added to this scheduler, in order) those that are done
+  void drop_done(std::vector<MineJob> &js) const
+  {
+    size_t n = 0;
+    for(size_t i = 0; i < js.size(); i++)
+      if(i >= jobs_.size() || !jobs_[i]->done) js[n++] = js[i];
+    js.resize(n);
+  }
+
 private:
   Engine &E;
   const MineOptions &wo_;
@@ -1463,6 +1475,7 @@ private:
   unsigned long long mat_start_[kWaveCtx] = {};
   double mat_ms_[kWaveCtx] = {};
   bool defer_emit_ = false;
+  bool any_packed_ = false;      // some job has packed rows
   // a wave context's stream (all on the engine's with the serial option)
   cudaStream_t cs(const WaveCtx &X) const { return wo_.serial ? E.stream : X.stream; }
   void h2d(void *dst, const void *src, size_t n, cudaStream_t s = nullptr)
@@ -2669,11 +2682,12 @@ int run_jobs_split(std::vector<MineJob> &batch, const MineOptions &wave_opt, Min
     }
   }
   for(auto &v : part) std::sort(v.begin(), v.end());
-  std::vector<MineStats> pst(P);
+  std::vector<MineStats> pst;
   std::vector<std::unique_ptr<Sched>> sch(P);
   std::vector<std::vector<int32_t>> ids(P);
-  std::vector<int> prc(P, ST_OK);
+  std::vector<int> prc;
   std::vector<std::string> perr(P);
+  std::vector<char> pmem;  // parts that device memory was not enough for
   auto engine = [](int p) -> Engine & { return p == 0 ? g_engine : g_extra[p - 1]; };
   auto work = [&](int p) {
     try {
@@ -2691,24 +2705,43 @@ int run_jobs_split(std::vector<MineJob> &batch, const MineOptions &wave_opt, Min
     } catch(const Error &e) {
       prc[p] = e.code;
       perr[p] = e.what();
+      pmem[p] = e.memory;
     } catch(const std::exception &e) {
       prc[p] = ST_ERR_STATE;
       perr[p] = e.what();
     }
   };
-  std::vector<std::thread> th;
-  std::vector<int> inline_parts;  // parts whose thread could not be started run here
-  for(int p = 1; p < P; p++)
-    if(!part[p].empty()) {
-      try {
-        th.emplace_back(work, p);
-      } catch(const std::system_error &) {
-        inline_parts.push_back(p);
+  for(;;) {
+    pst.assign(P, MineStats());
+    prc.assign(P, ST_OK);
+    pmem.assign(P, 0);
+    std::vector<std::thread> th;
+    std::vector<int> inline_parts;  // parts whose thread could not be started run here
+    for(int p = 1; p < P; p++)
+      if(!part[p].empty()) {
+        try {
+          th.emplace_back(work, p);
+        } catch(const std::system_error &) {
+          inline_parts.push_back(p);
+        }
       }
+    if(!part[0].empty()) work(0);
+    for(int p : inline_parts) work(p);
+    for(auto &t : th) t.join();
+    // out of memory with packed rows: all over again on columns (see run_jobs;
+    // nothing has been emitted)
+    bool again = false, packed = false;
+    for(int p = 0; p < P; p++) {
+      again = again || pmem[p];
+      packed = packed || (sch[p] && sch[p]->packed());
     }
-  if(!part[0].empty()) work(0);
-  for(int p : inline_parts) work(p);
-  for(auto &t : th) t.join();
+    if(!again || !packed) break;
+    for(int p = 0; p < P; p++) {
+      sch[p].reset();
+      engine_fail(engine(p));
+    }
+    for(MineJob &j : jobs) j.opt.columns = true;
+  }
   for(int p = 0; p < P; p++)
     if(prc[p] != ST_OK) {
       err = perr[p];
@@ -2773,12 +2806,34 @@ int run_jobs(std::vector<MineJob> &jobs, const MineOptions &wave_opt, MineStats 
     P = std::max(1, std::min<int>({ P, kMaxSchedulers, jobs.size() == 1 ? kMaxSchedulers : (int)jobs.size() }));
     if(P > 1) return run_jobs_split(jobs, wave_opt, st, err, P);
     const clk::time_point t0 = clk::now();
-    g_engine.pool_limit = g_pool_limit;
-    g_engine.init(wave_opt.threads);
-    Sched s(g_engine, wave_opt, st);
-    s.add_all(jobs);
-    while(!s.idle()) s.step();
-    s.sync_stats();
+    // Out of memory with packed rows: the jobs that are not done are mined on
+    // columns.  A packed row takes 16 bytes up to 8 pattern vertices, 32 up to
+    // 24, 80 up to 64; a column row 12, and shares its ancestors' columns with
+    // its siblings: where a pattern of 9 vertices and more has many embeddings,
+    // columns fit in less (64 graphs of a path of 9 with 40 like leaves at its
+    // end: peak 3.28 MB packed, 1.24 MB on columns).
+    std::vector<MineJob> todo(jobs);
+    for(bool again = true; again;) {
+      again = false;
+      g_engine.pool_limit = g_pool_limit;
+      g_engine.init(wave_opt.threads);
+      {
+        Sched s(g_engine, wave_opt, st);
+        try {
+          s.add_all(todo);
+          while(!s.idle()) s.step();
+          s.sync_stats();
+        } catch(const Error &e) {
+          if(!e.memory || !s.packed()) throw;
+          s.drop_done(todo);
+          again = true;
+        }
+      }
+      if(again) {
+        engine_fail(g_engine);
+        for(MineJob &j : todo) j.opt.columns = true;
+      }
+    }
     st.wall_ms += ms_since(t0);
   } catch(const Error &e) {
     err = e.what();
@@ -2825,6 +2880,7 @@ void Scheduler::reset()
 
 int32_t Scheduler::add(const MineJob &job) { return p_->s->add(job); }
 bool Scheduler::idle() const { return p_->s->idle(); }
+bool Scheduler::packed() const { return p_->s->packed(); }
 void Scheduler::step() { p_->s->step(); }
 void Scheduler::cancel(int32_t id) { p_->s->cancel(id); }
 std::vector<int32_t> Scheduler::take_done() { return p_->s->take_done(); }

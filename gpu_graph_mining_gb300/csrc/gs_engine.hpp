@@ -57,7 +57,11 @@ struct DeviceScope {
 
 struct Error : public std::runtime_error {
   int code;
-  Error(int c, const std::string &m) : std::runtime_error(m), code(c) {}
+  bool memory;  // device memory, or the pool's limit, was not enough
+  Error(int c, const std::string &m, bool mem = false)
+      : std::runtime_error(m), code(c), memory(mem || c == ST_ERR_NOMEM)
+  {
+  }
 };
 
 void cuda_check(cudaError_t e, const char *what);
@@ -139,6 +143,7 @@ struct MineOptions {
   int32_t serial = 0;         // 1: every wave context issues on the engine's stream (no kernels overlap)
   int32_t schedulers = 0;     // batches: jobs split over this many schedulers, each with its own engine and
                               // host thread (0 = one per 8 jobs from 16 jobs on, at most 4; else 1)
+  bool columns = false;       // (per job) embeddings in columns although its database takes packed rows
 };
 
 struct MineStats {
@@ -209,6 +214,7 @@ public:
   Scheduler &operator=(const Scheduler &) = delete;
   int32_t add(const MineJob &job);   // validates, mines the root level; returns the job id
   bool idle() const;                 // no unfinished job
+  bool packed() const;               // some job since the last reset has packed rows
   void step();
   void cancel(int32_t id);
   std::vector<int32_t> take_done();  // jobs finished or cancelled since the last call

@@ -229,6 +229,7 @@ private:
   // owned by the server thread
   std::unique_ptr<Scheduler> sched_;
   MineOptions wo_;
+  bool columns_ = false;  // requests are mined on columns (again_on_columns)
   std::unordered_map<int32_t, int64_t> job_req_;  // scheduler job -> request
 
   int64_t estimate(const Request &r) const
@@ -314,6 +315,7 @@ private:
           done_cv_.notify_all();
           break;
         }
+        if(running_.empty()) columns_ = false;
         const clk::time_point now = clk::now();
         // cancellations of queued requests end them now; running ones stop in the scheduler
         for(auto it = queue_.begin(); it != queue_.end();) {
@@ -359,15 +361,7 @@ private:
           r.out.reset(new PatternBuf());
           running_.push_back(r.id);
           max_running_ = std::max<int64_t>(max_running_, (int64_t)running_.size());
-          MineJob j;
-          j.db = dbs_[r.db_id];
-          j.minsup = r.minsup;
-          j.opt = wo_;
-          j.opt.max_edges = r.max_edges;
-          j.opt.label_style = opt_.label_style;
-          j.emit = PatternBuf::emit;
-          j.user = r.out.get();
-          admit.emplace_back(r.id, j);
+          admit.emplace_back(r.id, mine_job(r));
         }
         if(stop_)
           for(int64_t id : running_) {
@@ -379,16 +373,11 @@ private:
       const clk::time_point t0 = clk::now();
       try {
         for(int32_t jid : cancel_jobs) sched_->cancel(jid);
-        for(auto &a : admit) {
-          const int32_t jid = sched_->add(a.second);
-          job_req_[jid] = a.first;
-          std::lock_guard<std::mutex> g(m_);
-          reqs_[a.first]->job = jid;
-        }
+        for(auto &a : admit) add(a);
         if(!sched_->idle()) sched_->step();
         retire();
       } catch(const Error &e) {
-        fail_running(e.code, e.what());
+        if(!e.memory || !again_on_columns()) fail_running(e.code, e.what());
       } catch(const std::exception &e) {
         fail_running(GS_ERR_STATE, e.what());
       }
@@ -396,6 +385,60 @@ private:
       busy_ms_ += ms_between(t0, clk::now());
     }
     sched_.reset();
+  }
+
+  // under m_: a running request's job
+  MineJob mine_job(Request &r) const
+  {
+    MineJob j;
+    j.db = dbs_[r.db_id];
+    j.minsup = r.minsup;
+    j.opt = wo_;
+    j.opt.max_edges = r.max_edges;
+    j.opt.label_style = opt_.label_style;
+    j.opt.columns = columns_;
+    j.emit = PatternBuf::emit;
+    j.user = r.out.get();
+    return j;
+  }
+
+  // Out of memory with packed rows: the requests that are not done start again
+  // on columns, which can need less (run_jobs), and so does what is admitted
+  // until all that runs has ended.  Returns false when they were on columns, or
+  // when they do not fit either.
+  bool again_on_columns()
+  {
+    try {
+      if(!sched_ || !sched_->packed()) return false;
+      retire();  // the requests that were finished before the error
+      sched_->reset();
+      job_req_.clear();
+      std::vector<std::pair<int64_t, MineJob>> jobs;
+      {
+        std::lock_guard<std::mutex> g(m_);
+        columns_ = true;
+        for(int64_t id : running_) {
+          Request &r = *reqs_[id];
+          r.job = -1;
+          r.out.reset(new PatternBuf());
+          jobs.emplace_back(id, mine_job(r));
+        }
+      }
+      for(auto &j : jobs) add(j);
+      return true;
+    } catch(const Error &) {
+      return false;
+    } catch(const std::exception &) {
+      return false;
+    }
+  }
+
+  void add(const std::pair<int64_t, MineJob> &j)
+  {
+    const int32_t jid = sched_->add(j.second);
+    job_req_[jid] = j.first;
+    std::lock_guard<std::mutex> g(m_);
+    reqs_[j.first]->job = jid;
   }
 
   // publishes the jobs the last step finished
