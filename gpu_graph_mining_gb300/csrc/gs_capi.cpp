@@ -234,7 +234,7 @@ gs_status gs_db_get_info(const gs_db *db, gs_db_info *info)
   info->adjacency_entries = db->d.n_adj();
   info->vertex_labels = db->d.VL;
   info->edge_labels = db->d.EL;
-  info->device_bytes = db->d.resident ? (int64_t)db->d.d_bytes : 0;
+  info->device_bytes = db->d.device_bytes();
   return GS_OK;
 }
 

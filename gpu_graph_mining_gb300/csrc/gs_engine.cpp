@@ -35,10 +35,93 @@ namespace gsgb {
 void cuda_check(cudaError_t e, const char *what)
 {
   if(e != cudaSuccess)
-    throw Error(ST_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e), e == cudaErrorMemoryAllocation);
+    throw Error(ST_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e),
+                e == cudaErrorMemoryAllocation ? Error::kMemDevice : Error::kMemNone);
 }
 
 #define CK(call) cuda_check((call), #call)
+
+// ---------------------------------------------------------- neighbour blocks
+
+namespace {
+
+std::mutex g_nb_mu;                             // every Neighbours' fields
+std::vector<std::weak_ptr<Neighbours>> g_nb;    // those that have blocks, and some that had
+
+// cudaMalloc; out of memory, the neighbour blocks that no scheduler uses go first
+cudaError_t device_malloc(void **p, size_t n)
+{
+  const cudaError_t e = cudaMalloc(p, n);
+  if(e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  if(!give_up_neighbours()) return e;
+  return cudaMalloc(p, n);
+}
+
+}  // namespace
+
+NeighboursUse::NeighboursUse(const std::shared_ptr<Neighbours> &n) : n_(n)
+{
+  if(!n_) return;
+  std::lock_guard<std::mutex> g(g_nb_mu);
+  n_->users++;
+  nb_ = n_->nb;
+}
+
+NeighboursUse::~NeighboursUse()
+{
+  if(!n_) return;
+  std::lock_guard<std::mutex> g(g_nb_mu);
+  n_->users--;
+}
+
+std::shared_ptr<Neighbours> own_neighbours(uint4 *nb, size_t bytes, bool pooled)
+{
+  std::shared_ptr<Neighbours> n(new Neighbours());
+  n->nb = nb;
+  n->bytes = bytes;
+  n->pooled = pooled;
+  std::lock_guard<std::mutex> g(g_nb_mu);
+  g_nb.erase(std::remove_if(g_nb.begin(), g_nb.end(), [](const std::weak_ptr<Neighbours> &w) { return w.expired(); }),
+             g_nb.end());
+  g_nb.push_back(n);
+  return n;
+}
+
+std::vector<NeighbourBlock> detach_idle_neighbours()
+{
+  std::vector<NeighbourBlock> out;
+  std::lock_guard<std::mutex> g(g_nb_mu);
+  for(auto &w : g_nb)
+    if(std::shared_ptr<Neighbours> n = w.lock())
+      if(n->nb && n->users == 0) {
+        out.push_back(NeighbourBlock{ n->nb, n->pooled });
+        n->nb = nullptr;
+      }
+  return out;
+}
+
+NeighbourBlock detach_neighbours(const std::shared_ptr<Neighbours> &n)
+{
+  if(!n) return NeighbourBlock{ nullptr, false };
+  std::lock_guard<std::mutex> g(g_nb_mu);
+  const NeighbourBlock b{ n->nb, n->pooled };
+  n->nb = nullptr;
+  return b;
+}
+
+bool give_up_neighbours()
+{
+  const std::vector<NeighbourBlock> v = detach_idle_neighbours();
+  bool pooled = false;
+  for(const NeighbourBlock &b : v) {
+    if(b.pooled) ingest_free_block(b.p);
+    else cudaFree(b.p);
+    pooled = pooled || b.pooled;
+  }
+  if(pooled) ingest_release();
+  return !v.empty();
+}
 
 // ------------------------------------------------------------------ database
 
@@ -110,6 +193,7 @@ void Database::index_pairs()
 void Database::upload()
 {
   if(resident) return;
+  release();  // (of an upload that failed)
   prepare();
   const int64_t V = host.n_vertices(), E2 = host.n_adj();
   const int64_t tab = (int64_t)VL * EL * VL;
@@ -124,15 +208,13 @@ void Database::upload()
   size_t o_vb = o_ro + al(sizeof(int32_t) * (VL + 1));
   size_t o_ap = o_vb + al(sizeof(int32_t) * (host.n_graphs + 1));
   size_t o_pc = o_ap + al(sizeof(int32_t) * (E2 + 1));
-  // neighbour blocks (packed rows), filled by a kernel from the arrays before
   int32_t maxnv = 0;
   for(int32_t g = 0; g < host.n_graphs; g++) maxnv = std::max(maxnv, host.graph_nv(g));
   const int32_t nb_shift = packed_shift(maxnv, VL, EL, root_keys);
   int64_t nb_blocks = nb_shift ? packed_blocks(V, E2) : 0;
   if(nb_blocks >= INT32_MAX) nb_blocks = 0;
   size_t o_nu = o_pc + al(sizeof(int32_t) * (root_keys + 1));
-  size_t o_nb = o_nu + al(sizeof(int32_t));
-  const size_t copied = o_nb;
+  const size_t total = o_nu + al(sizeof(int32_t));
   std::vector<unsigned long long> adj(E2 + 1, 0);
   parallel_ranges(E2, [&](int64_t b, int64_t e, int) {
     for(int64_t k = b; k < e; k++) {
@@ -176,17 +258,8 @@ void Database::upload()
   });
   std::vector<int32_t> vb(host.n_graphs + 1);
   for(int32_t g = 0; g <= host.n_graphs; g++) vb[g] = (int32_t)host.vbase[g];
-  // without room for the neighbour blocks the database is mined on columns
-  size_t total = copied + al(32 * (size_t)nb_blocks);
-  if(nb_blocks > 0 && cudaMalloc(&d_block, total) != cudaSuccess) {
-    cudaGetLastError();
-    d_block = nullptr;
-    nb_blocks = 0;
-    total = copied;
-  }
-  if(!d_block) CK(cudaMalloc(&d_block, total));
-  d_bytes = total;
-  h2d_bytes = copied;
+  CK(device_malloc(&d_block, total));
+  d_bytes = h2d_bytes = total;
   char *b = (char *)d_block;
   CK(cudaMemcpy(b + o_adj, adj.data(), sizeof(unsigned long long) * (E2 + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b + o_off, off.data(), sizeof(int32_t) * (V + 1), cudaMemcpyHostToDevice));
@@ -219,15 +292,24 @@ void Database::upload()
   d_root_off = (int32_t *)(b + o_ro);
   dev.root_off = d_root_off;
   dev.pair_code = (const int32_t *)(b + o_pc);
-  if(nb_blocks > 0) {
+  // neighbour blocks (packed rows), filled by a kernel from the arrays above;
+  // without room for them the database is mined on columns
+  void *nb = nullptr;
+  if(nb_blocks > 0 && cudaMalloc(&nb, 32 * (size_t)nb_blocks) != cudaSuccess) {
+    cudaGetLastError();
+    nb = nullptr;
+  }
+  if(nb) {
     dev.nb_shift = nb_shift;
     dev.nb_ids = packed_ids(maxnv);
     dev.nb_blocks = (int32_t)nb_blocks;
-    CK(cudaMemsetAsync(b + o_nu, 0, sizeof(int32_t), cudaStreamLegacy));
-    launch_neighbour_blocks(dev, (uint4 *)(b + o_nb), (int32_t *)(b + o_nu), cudaStreamLegacy);
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(cudaStreamLegacy));
-    dev.nb = (const uint4 *)(b + o_nb);
+    cudaError_t e = cudaMemsetAsync(b + o_nu, 0, sizeof(int32_t), cudaStreamLegacy);
+    launch_neighbour_blocks(dev, (uint4 *)nb, (int32_t *)(b + o_nu), cudaStreamLegacy);
+    if(e == cudaSuccess) e = cudaGetLastError();
+    if(e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if(e != cudaSuccess) cudaFree(nb);
+    cuda_check(e, "neighbour blocks");
+    neighbours = own_neighbours((uint4 *)nb, 32 * (size_t)nb_blocks, false);
   }
   resident = true;
 }
@@ -255,8 +337,21 @@ void Database::ensure_host()
   }
 }
 
+int64_t Database::device_bytes() const
+{
+  if(!resident) return 0;
+  std::lock_guard<std::mutex> g(g_nb_mu);
+  return (int64_t)(d_bytes + (neighbours && neighbours->nb ? neighbours->bytes : 0));
+}
+
 void Database::release()
 {
+  const NeighbourBlock nb = detach_neighbours(neighbours);
+  if(nb.p) {
+    if(nb.pooled) ingest_free_block(nb.p);
+    else cudaFree(nb.p);
+  }
+  neighbours.reset();
   if(d_block) {
     if(pooled) ingest_free_block(d_block);
     else cudaFree(d_block);
@@ -354,14 +449,19 @@ private:
   }
   void grow(size_t n)
   {
-    size_t freeb = 0, totalb = 0;
-    CK(cudaMemGetInfo(&freeb, &totalb));
-    size_t lim = limit_ > 0 ? (size_t)limit_ : (size_t)(0.7 * (double)(freeb + total_));
-    size_t want = std::max(n, next_);
-    if(total_ + want > lim) want = std::max(n, lim > total_ ? lim - total_ : 0);
-    if(want < n || total_ + want > lim + n) throw Error(ST_ERR_NOMEM, "device pool limit reached");
+    size_t want = 0;
+    for(bool first = true;; first = false) {
+      size_t freeb = 0, totalb = 0;
+      CK(cudaMemGetInfo(&freeb, &totalb));
+      const size_t lim = limit_ > 0 ? (size_t)limit_ : (size_t)(0.7 * (double)(freeb + total_));
+      want = std::max(n, next_);
+      if(total_ + want > lim) want = std::max(n, lim > total_ ? lim - total_ : 0);
+      if(want >= n && total_ + want <= lim + n) break;
+      if(limit_ > 0) throw Error(ST_ERR_NOMEM, "device pool limit reached", Error::kMemLimit);
+      if(!first || !give_up_neighbours()) throw Error(ST_ERR_NOMEM, "device pool limit reached");
+    }
     char *p = nullptr;
-    if(cudaMalloc(&p, want) != cudaSuccess) {
+    if(device_malloc((void **)&p, want) != cudaSuccess) {
       cudaGetLastError();
       throw Error(ST_ERR_NOMEM, "cudaMalloc for the device pool failed");
     }
@@ -388,7 +488,8 @@ template <class T> struct DBuf {
     size_t c = std::max(n, cap * 2);
     if(c < 64) c = 64;
     p = nullptr;
-    CK(cudaMalloc(&p, c * sizeof(T)));
+    cap = 0;
+    CK(device_malloc((void **)&p, c * sizeof(T)));
     cap = c;
   }
   void free()
@@ -1333,7 +1434,9 @@ public:
     if(slot < 0) {
       slot = (int32_t)dbs_.size();
       dbs_.push_back(db);
+      nb_use_.emplace_back(new NeighboursUse(db->neighbours));
       tab_.push_back(db->dev);
+      tab_.back().nb = nb_use_.back()->nb();
       if(tab_.size() > E.d_dbs.cap) {
         // the table is read by waves in flight: let them finish before it moves
         E.sync_all();
@@ -1353,7 +1456,7 @@ public:
       E.scratch.spare.pop_back();
     }
     // the lists strategy joins on parent rows: columns
-    S.packed = db->dev.nb != nullptr && wo_.extension == 0 && !j.opt.columns;
+    S.packed = tab_[slot].nb != nullptr && wo_.extension == 0 && !j.opt.columns;
     any_packed_ = any_packed_ || S.packed;
     active_++;
     order_.push_back(id);
@@ -1465,6 +1568,7 @@ private:
   std::vector<Database *> dbs_;
   std::vector<char> db_seen_;  // wave building: database slots met
   std::vector<DevDB> tab_;
+  std::vector<std::unique_ptr<NeighboursUse>> nb_use_;  // the table's neighbour blocks
   int64_t active_ = 0;
   int64_t stacked_ = 0;          // nodes on all jobs' stacks
   int64_t seen_bytes_[2] = { 0, 0 };
@@ -2007,7 +2111,7 @@ private:
         ht[n] = (int32_t)tb;
         PackedNode &g = hp[n];
         g.rows = p.rows;
-        g.nb = db.dev.nb;
+        g.nb = tab_[S.db_slot].nb;
         g.nrows = d.nrows;
         g.k = d.k;
         g.nslot = d.nslot;
@@ -2687,7 +2791,7 @@ int run_jobs_split(std::vector<MineJob> &batch, const MineOptions &wave_opt, Min
   std::vector<std::vector<int32_t>> ids(P);
   std::vector<int> prc;
   std::vector<std::string> perr(P);
-  std::vector<char> pmem;  // parts that device memory was not enough for
+  std::vector<Error::Memory> pmem;  // what was not enough for a part
   auto engine = [](int p) -> Engine & { return p == 0 ? g_engine : g_extra[p - 1]; };
   auto work = [&](int p) {
     try {
@@ -2714,7 +2818,7 @@ int run_jobs_split(std::vector<MineJob> &batch, const MineOptions &wave_opt, Min
   for(;;) {
     pst.assign(P, MineStats());
     prc.assign(P, ST_OK);
-    pmem.assign(P, 0);
+    pmem.assign(P, Error::kMemNone);
     std::vector<std::thread> th;
     std::vector<int> inline_parts;  // parts whose thread could not be started run here
     for(int p = 1; p < P; p++)
@@ -2730,9 +2834,10 @@ int run_jobs_split(std::vector<MineJob> &batch, const MineOptions &wave_opt, Min
     for(auto &t : th) t.join();
     // out of memory with packed rows: all over again on columns (see run_jobs;
     // nothing has been emitted)
-    bool again = false, packed = false;
+    bool again = false, packed = false, device = false;
     for(int p = 0; p < P; p++) {
-      again = again || pmem[p];
+      again = again || pmem[p] != Error::kMemNone;
+      device = device || pmem[p] == Error::kMemDevice;
       packed = packed || (sch[p] && sch[p]->packed());
     }
     if(!again || !packed) break;
@@ -2740,6 +2845,7 @@ int run_jobs_split(std::vector<MineJob> &batch, const MineOptions &wave_opt, Min
       sch[p].reset();
       engine_fail(engine(p));
     }
+    if(device) give_up_neighbours();
     for(MineJob &j : jobs) j.opt.columns = true;
   }
   for(int p = 0; p < P; p++)
@@ -2814,7 +2920,7 @@ int run_jobs(std::vector<MineJob> &jobs, const MineOptions &wave_opt, MineStats 
     // end: peak 3.28 MB packed, 1.24 MB on columns).
     std::vector<MineJob> todo(jobs);
     for(bool again = true; again;) {
-      again = false;
+      Error::Memory memory = Error::kMemNone;
       g_engine.pool_limit = g_pool_limit;
       g_engine.init(wave_opt.threads);
       {
@@ -2824,13 +2930,15 @@ int run_jobs(std::vector<MineJob> &jobs, const MineOptions &wave_opt, MineStats 
           while(!s.idle()) s.step();
           s.sync_stats();
         } catch(const Error &e) {
-          if(!e.memory || !s.packed()) throw;
+          if(e.memory == Error::kMemNone || !s.packed()) throw;
           s.drop_done(todo);
-          again = true;
+          memory = e.memory;
         }
       }
+      again = memory != Error::kMemNone;
       if(again) {
         engine_fail(g_engine);
+        if(memory == Error::kMemDevice) give_up_neighbours();
         for(MineJob &j : todo) j.opt.columns = true;
       }
     }
@@ -3005,7 +3113,7 @@ int support_count_host(const int32_t *keys, const int32_t *gids, int64_t n, int3
     const size_t o_rj = o_sup + al(4 * (size_t)n_keys), total = o_rj + al(sizeof(RootJob));
     CK(cudaSetDevice(0));
     CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    CK(cudaMalloc(&blk, total));
+    CK(device_malloc((void **)&blk, total));
     RootJob rj{};  // one job without counter copies: supports only
     rj.words = words;
     rj.R = n_keys;
@@ -3072,7 +3180,7 @@ int filter_backward_host(const int32_t *column, int64_t n_rows, const int32_t *r
     const size_t total = o_out + al(8 * (size_t)n_rows);
     CK(cudaSetDevice(0));
     CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    CK(cudaMalloc(&blk, total));
+    CK(device_malloc((void **)&blk, total));
     CK(cudaMemcpyAsync(blk + o_col, column, 8 * (size_t)n_rows, cudaMemcpyHostToDevice, s));
     if(n_records > 0) CK(cudaMemcpyAsync(blk + o_rec, records, 32 * (size_t)n_records, cudaMemcpyHostToDevice, s));
     int32_t *pos = (int32_t *)(blk + o_pos);
@@ -3128,7 +3236,7 @@ int segmented_scan_host(const uint32_t *data, int64_t n, const int64_t *ends, in
     const size_t o_res = o_ends + al(8 * (size_t)std::max<int64_t>(n_ends, 1));
     const size_t o_err = o_res + al(4 * (size_t)std::max<int64_t>(n_ends, 1)), total = o_err + al(4);
     CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    CK(cudaMalloc(&blk, total));
+    CK(device_malloc((void **)&blk, total));
     uint32_t *x = (uint32_t *)(blk + o_x);
     unsigned int *derr = (unsigned int *)(blk + o_err);
     CK(cudaMemcpyAsync(x, data, 4 * (size_t)n, cudaMemcpyHostToDevice, s));

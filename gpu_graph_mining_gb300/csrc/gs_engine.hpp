@@ -57,14 +57,53 @@ struct DeviceScope {
 
 struct Error : public std::runtime_error {
   int code;
-  bool memory;  // device memory, or the pool's limit, was not enough
-  Error(int c, const std::string &m, bool mem = false)
-      : std::runtime_error(m), code(c), memory(mem || c == ST_ERR_NOMEM)
+  // what was not enough: kMemLimit the caller's limit of the embedding pool,
+  // kMemDevice device memory
+  enum Memory { kMemNone, kMemLimit, kMemDevice } memory;
+  Error(int c, const std::string &m, Memory mem = kMemNone)
+      : std::runtime_error(m), code(c), memory(mem == kMemNone && c == ST_ERR_NOMEM ? kMemDevice : mem)
   {
   }
 };
 
 void cuda_check(cudaError_t e, const char *what);
+
+// The neighbour blocks of a resident database (packed rows), an allocation of
+// their own: databases are mined without them too, on columns, so those that no
+// scheduler uses are given up when device memory runs out.  Shared by the
+// database and the schedulers that have mined it.
+struct Neighbours {
+  uint4 *nb = nullptr;  // nullptr: given up
+  size_t bytes = 0;
+  bool pooled = false;  // from the ingest's pool
+  int users = 0;        // schedulers whose database table points to them
+};
+// A scheduler's use of a database's neighbour blocks (nb(): nullptr when there
+// are none, else they stay until the use ends or the database is freed).
+class NeighboursUse {
+public:
+  explicit NeighboursUse(const std::shared_ptr<Neighbours> &n);
+  ~NeighboursUse();
+  NeighboursUse(const NeighboursUse &) = delete;
+  NeighboursUse &operator=(const NeighboursUse &) = delete;
+  const uint4 *nb() const { return nb_; }
+
+private:
+  std::shared_ptr<Neighbours> n_;
+  const uint4 *nb_ = nullptr;
+};
+// New blocks, known to give_up_neighbours.
+std::shared_ptr<Neighbours> own_neighbours(uint4 *nb, size_t bytes, bool pooled);
+// The blocks that no scheduler uses (of one database: used or not), detached from
+// their databases: the caller frees them.
+struct NeighbourBlock {
+  void *p;
+  bool pooled;
+};
+std::vector<NeighbourBlock> detach_idle_neighbours();
+NeighbourBlock detach_neighbours(const std::shared_ptr<Neighbours> &n);
+// Frees every database's blocks that no scheduler uses; false when there are none.
+bool give_up_neighbours();
 
 // Host database plus, once uploaded, its device copy.
 struct Database {
@@ -80,8 +119,9 @@ struct Database {
   int32_t root_keys = 0;
   // device copy
   void *d_block = nullptr;
-  size_t d_bytes = 0;
+  size_t d_bytes = 0;    // neighbour blocks not among them
   size_t h2d_bytes = 0;  // of them copied from the host (upload)
+  std::shared_ptr<Neighbours> neighbours;  // (dev.nb stays null: NeighboursUse)
   DevDB dev{};
   int32_t *d_root_off = nullptr;
   bool resident = false;
@@ -102,6 +142,7 @@ struct Database {
   void ensure_host();  // host arrays of a device-built database (original labels)
   int64_t n_vertices() const { return device_only ? dev_vertices : host.n_vertices(); }
   int64_t n_adj() const { return device_only ? dev_adj : host.n_adj(); }
+  int64_t device_bytes() const;
   ~Database();
 };
 

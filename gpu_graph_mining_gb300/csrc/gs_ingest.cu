@@ -88,6 +88,24 @@ __global__ void k_scan_add(long long *out, long long n, const long long *block_o
 // its memory between ingests (up to kKeepBytes), so that repeated ingests of
 // similar databases allocate and free without driver calls.  Freed in stream
 // order when the ingest returns.
+// An allocation in stream order; out of memory, the neighbour blocks that no
+// scheduler uses go first.
+void *pool_malloc(size_t n, cudaMemPool_t pool, cudaStream_t s)
+{
+  void *p = nullptr;
+  if(cudaMallocFromPoolAsync(&p, n, pool, s) == cudaSuccess) return p;
+  cudaGetLastError();
+  const std::vector<NeighbourBlock> idle = detach_idle_neighbours();
+  if(!idle.empty()) cudaDeviceSynchronize();  // every kernel that read them has finished
+  for(const NeighbourBlock &b : idle) {
+    if(b.pooled) cudaFreeAsync(b.p, s);
+    else cudaFree(b.p);
+  }
+  if(!idle.empty() && cudaMallocFromPoolAsync(&p, n, pool, s) == cudaSuccess) return p;
+  cudaGetLastError();
+  throw Error(ST_ERR_NOMEM, "device ingest: out of device memory");
+}
+
 struct Scratch {
   cudaStream_t s;
   cudaMemPool_t pool;
@@ -100,11 +118,7 @@ struct Scratch {
   }
   template <class T> T *get(size_t n)
   {
-    void *p = nullptr;
-    if(cudaMallocFromPoolAsync(&p, sizeof(T) * std::max<size_t>(n, 1), pool, s) != cudaSuccess) {
-      cudaGetLastError();
-      throw Error(ST_ERR_NOMEM, "device ingest: out of device memory");
-    }
+    void *p = pool_malloc(sizeof(T) * std::max<size_t>(n, 1), pool, s);
     ptrs.push_back(p);
     return (T *)p;
   }
@@ -715,19 +729,13 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
   int64_t nb_blocks = nb_shift ? packed_blocks(V, E2) : 0;
   if(nb_blocks >= INT32_MAX) nb_blocks = 0;
   const size_t o_nu = o_in + al(sizeof(unsigned long long) * (E2 + 1));
-  const size_t o_nb = o_nu + al(sizeof(int32_t));
-  size_t total = o_nb + al(32 * (size_t)nb_blocks);
-  char *b = nullptr;
-  if(nb_blocks > 0 && cudaMallocFromPoolAsync((void **)&b, total, cx.pool, s) != cudaSuccess) {
+  const size_t total = o_nu + al(sizeof(int32_t));
+  char *const b = (char *)pool_malloc(total, cx.pool, s);
+  void *nb = nullptr;
+  if(nb_blocks > 0 && cudaMallocFromPoolAsync(&nb, 32 * (size_t)nb_blocks, cx.pool, s) != cudaSuccess) {
     // without room for them the database is mined on columns
     cudaGetLastError();
-    b = nullptr;
-    nb_blocks = 0;
-    total = o_nb;
-  }
-  if(!b && cudaMallocFromPoolAsync((void **)&b, total, cx.pool, s) != cudaSuccess) {
-    cudaGetLastError();
-    throw Error(ST_ERR_NOMEM, "device ingest: out of device memory");
+    nb = nullptr;
   }
   try {
     int32_t *pidx = (int32_t *)(b + o_pi), *ro = (int32_t *)(b + o_ro), *pc = (int32_t *)(b + o_pc);
@@ -746,7 +754,7 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
     CK(cudaMemcpyAsync(b + o_gb, vgbase, sizeof(int32_t) * V, cudaMemcpyDeviceToDevice, s));
     k_narrow<<<blocks_for(G + 1), kThreads, 0, s>>>(vbase, G + 1, (int32_t *)(b + o_vb));
     DevDB nbd{};
-    if(nb_blocks > 0) {
+    if(nb) {
       nbd.adj = (const unsigned long long *)(b + o_adj);
       nbd.adj_off = off;
       nbd.adj_pair = (const int32_t *)(b + o_ap);
@@ -756,8 +764,7 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
       nbd.nb_ids = packed_ids(mxv);
       nbd.nb_blocks = (int32_t)nb_blocks;
       CK(cudaMemsetAsync(b + o_nu, 0, sizeof(int32_t), s));
-      launch_neighbour_blocks(nbd, (uint4 *)(b + o_nb), (int32_t *)(b + o_nu), s);
-      nbd.nb = (const uint4 *)(b + o_nb);
+      launch_neighbour_blocks(nbd, (uint4 *)nb, (int32_t *)(b + o_nu), s);
     }
     // host metadata (label values, each label's first pair, the pair codes), one read-back
     int32_t *hm = cx.meta_buf((size_t)(nvl + nel + VL + nkeys + 1));
@@ -777,6 +784,8 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
       cudaFreeAsync(db.d_block, s);
       db.d_block = nullptr;
       db.pooled = false;
+      const NeighbourBlock old = detach_neighbours(db.neighbours);
+      if(old.p) cudaFreeAsync(old.p, s);
     }
     db.release();
     db.host = HostDB();
@@ -794,6 +803,7 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
     }
     db.root_keys = (int32_t)nkeys;
     db.index_pairs();
+    db.neighbours = nb ? own_neighbours((uint4 *)nb, 32 * (size_t)nb_blocks, true) : nullptr;
     db.d_block = b;
     db.pooled = true;
     db.d_bytes = total;
@@ -815,7 +825,6 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
     db.dev.n_vertices = (int32_t)V;
     db.dev.root_off = ro;
     db.dev.pair_code = pc;
-    db.dev.nb = nbd.nb;
     db.dev.nb_blocks = nbd.nb_blocks;
     db.dev.nb_shift = nbd.nb_shift;
     db.dev.nb_ids = nbd.nb_ids;
@@ -826,6 +835,7 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
     db.dev_adj = E2;
   } catch(...) {
     cudaFreeAsync(b, s);
+    if(nb) cudaFreeAsync(nb, s);
     throw;
   }
 }

@@ -377,7 +377,7 @@ private:
         if(!sched_->idle()) sched_->step();
         retire();
       } catch(const Error &e) {
-        if(!e.memory || !again_on_columns()) fail_running(e.code, e.what());
+        if(e.memory == Error::kMemNone || !again_on_columns(e.memory)) fail_running(e.code, e.what());
       } catch(const std::exception &e) {
         fail_running(GS_ERR_STATE, e.what());
       }
@@ -406,12 +406,13 @@ private:
   // on columns, which can need less (run_jobs), and so does what is admitted
   // until all that runs has ended.  Returns false when they were on columns, or
   // when they do not fit either.
-  bool again_on_columns()
+  bool again_on_columns(Error::Memory memory)
   {
     try {
       if(!sched_ || !sched_->packed()) return false;
       retire();  // the requests that were finished before the error
       sched_->reset();
+      if(memory == Error::kMemDevice) give_up_neighbours();
       job_req_.clear();
       std::vector<std::pair<int64_t, MineJob>> jobs;
       {

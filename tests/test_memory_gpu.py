@@ -75,3 +75,32 @@ def test_server(gs, tmp_path):
         res = [srv.result(r) for r in rids]
     assert [i["state"] for _, i in res] == [gs.REQ_DONE] * 3
     assert res[1][0] == want and res[0][0] == res[2][0] == other
+
+
+def test_neighbour_blocks_make_room(gs):
+    # a second database fits beside the first one, but not beside its neighbour
+    # blocks: those are given up, and the first is mined on columns
+    torch = pytest.importorskip("torch")
+    gs.engine_reset()
+    a, b, c = (gs.Database.generate(5, seed=s, scale=0.25) for s in (1, 2, 2))
+    s = int(0.02 * len(a))
+    a.upload()
+    want_a, want_b = (gs.mine_collect(d, s, max_edges=4)[0] for d in (a, c))
+    c.free()
+    info = a.info()
+    blocks = 32 * (info["vertices"] + info["adjacency_entries"] // 7 + 256)
+    base = info["device_bytes"] - blocks
+    assert base > 0.5 * blocks > 64 << 20
+    gs.engine_reset()
+    torch.cuda.empty_cache()
+    room = int(base - 0.4 * min(base, blocks))
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+    try:
+        b.upload()
+        assert a.info()["device_bytes"] == base
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    for d, want in ((a, want_a), (b, want_b)):
+        assert gs.mine_collect(d, s, max_edges=4)[0] == want
+    gs.engine_reset()
