@@ -1063,6 +1063,7 @@ struct Engine {
   // block released so far is free (a later record of an event only makes the
   // wait longer).
   std::vector<void *> released;
+  bool root_queued = false;       // a root phase is not known to have completed
   uint64_t main_gen = 0;          // records of ev_main
 
   void init(int threads)
@@ -1096,6 +1097,7 @@ struct Engine {
     if(!ready) return;
     sync_all();
     released.clear();
+    root_queued = false;
     if(ev_main) cudaEventDestroy(ev_main);
     ev_main = nullptr;
     pool.destroy();
@@ -1152,7 +1154,8 @@ struct Engine {
     if(released.empty()) return false;
     for(auto &c : ctx)
       if(!passed(c.ev_mat, wait)) return false;
-    if(!passed(rootx.ev_mat, wait)) return false;
+    if(root_queued && !passed(rootx.ev_mat, wait)) return false;
+    root_queued = false;
     for(void *b : released) pool.release(b);
     released.clear();
     return true;
@@ -1922,6 +1925,7 @@ private:
       st_.launches += 2;
     }
     CK(cudaEventRecord(X.ev_mat, E.stream));
+    E.root_queued = true;
     for(int32_t q = 0; q < n; q++) {
       JobState &S = *jobs_[gid[q]];
       S.pending += (int64_t)made[q].size();
