@@ -866,6 +866,14 @@ constexpr size_t kHeadBytes = sizeof(unsigned long long) * kHeadWords;
 // A record block of packed rows in int4 units of the record buffer: 32 items
 // of 4 bytes and a 16-byte header.
 constexpr long long kRecBlockInt4 = 9;
+// The record buffer of a wave context, int4 (compile-time tunable): what it
+// begins with, and the most it grows to (4 GiB).
+#ifndef GS_REC_INIT
+#define GS_REC_INIT (1ll << 22)
+#endif
+#ifndef GS_REC_MAX
+#define GS_REC_MAX (1ll << 28)
+#endif
 
 // Device scratch and pinned mirrors of one wave in flight.  Two of them let
 // the host prepare one wave's children while the GPU counts the other's.
@@ -2210,9 +2218,9 @@ private:
     f.rec = nullptr;
     f.rec_cap = 0;
     if(X.rec_enabled && X.wanted_rec > (long long)X.d_rec.cap) {
-      // past 2^28 records (4 GiB) or when the device has no room, keep the
+      // past GS_REC_MAX or when the device has no room, keep the
       // enumeration-based materialise instead
-      if(X.wanted_rec > (1ll << 28)) X.rec_enabled = false;
+      if(X.wanted_rec > GS_REC_MAX) X.rec_enabled = false;
       else {
         try {
           X.d_rec.ensure((size_t)X.wanted_rec);
@@ -2223,7 +2231,7 @@ private:
       }
     }
     if(X.rec_enabled) {
-      if(X.d_rec.cap == 0) X.d_rec.ensure((size_t)1 << 22);
+      if(X.d_rec.cap == 0) X.d_rec.ensure((size_t)GS_REC_INIT);
       f.rec = X.d_rec.p;
       f.rec_cap = (long long)X.d_rec.cap;
       if(packed) {
