@@ -32,8 +32,8 @@
 // in the last word 2^31 | the block that continues it (again up to 8 entries,
 // or 7 and a link).  A wave's extension records are blocks of 32 four-byte
 // items of one tile, (node's key << (nb_ids + 5)) | (graph-local new vertex << 5) | row
-// in the tile, each with a header {first row of the tile, node, items,
-// the node's first key}.
+// in the tile, each with a header {first row of the tile, 0, items | counter
+// copy << 8 | (nb_ids + 5) << 16, the node's first key}.
 #pragma once
 #include <cstdint>
 

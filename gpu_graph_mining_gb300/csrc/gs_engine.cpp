@@ -6,8 +6,9 @@
 // 275-489): every node costs ~15-30 kernel launches, each followed by a
 // device synchronise, plus per-node cudaMalloc/cudaFree.  Here a "wave" is a
 // batch of pending tree nodes (possibly of different mining jobs) extended
-// together: per wave there are three kernels (count, support, materialise),
-// one device->host copy of the candidate supports and one synchronise.  With
+// together: four or five kernels (tables in, count, selection, canonicality and
+// results out) and two for its children's rows (tables, materialise), with no
+// copies between them; the host polls a word of the pinned results.  With
 // wave_nodes = 1 the same engine runs the plain one-pattern-at-a-time form.
 //
 // The pattern set, codes and supports follow the sequential miner
@@ -879,20 +880,19 @@ constexpr long long kRecBlockInt4 = 9;
 // the host prepare one wave's children while the GPU counts the other's.
 struct WaveCtx {
   DBuf<char> d_desc;
-  DBuf<uint32_t> d_bm;
-  DBuf<int32_t> d_bmx, d_cnt, d_sup, d_childmap, d_cursor;
-  DBuf<ChildOut> d_outs;
+  DBuf<int32_t> d_bmx, d_sup, d_childmap, d_cursor;
   // extension records of the count pass (record-driven materialise)
   DBuf<int4> d_rec;
-  DBuf<unsigned long long> d_recn;
   DBuf<long long> d_keyword;
   DBuf<int2> d_listed;               // keys with enough embeddings to be counted
   DBuf<int32_t> d_lnode;   // lists strategy: the node of each frequent forward key
   // A wave's results, written to pinned host memory by its last kernel: the
   // header (HeadWord) followed by the selected candidates {key, support,
-  // embeddings, node << 2 | verdict}.  The zeroed region holds the embedding counts and the support
-  // bitmaps (one memset).  The child table holds the children's outputs and
-  // (key, child) pairs (one upload).
+  // embeddings, node << 2 | verdict}.  The zeroed region (cleared by the wave's
+  // first kernel) holds the embedding counts, the record regions' counters and
+  // the support bitmaps.  The child table holds the children's outputs and (key,
+  // child) pairs, copied from its pinned mirror by the kernel ahead of the
+  // materialise pass.
   DBuf<char> d_head, d_zero, d_mat;
   HBuf<char> h_head, h_mat;
   int64_t sel_hint = 4096;           // selected entries there is room for in the pinned results
@@ -900,9 +900,7 @@ struct WaveCtx {
   long long wanted_rec = 0;    // record capacity to have before the next wave (after an overflow)
   // pinned host mirrors
   HBuf<char> h_desc;
-  HBuf<int32_t> h_sup, h_cnt, h_childmap;
-  HBuf<ChildOut> h_outs;
-  HBuf<long long> h_keyword;
+  HBuf<int32_t> h_sup;
   cudaEvent_t ev_mat = nullptr;  // after the last materialise pass (the root context: after the first embeddings)
   std::vector<WaveGraph> graphs;
   // the context's stream (wave contexts; the root context uses the engine's)
@@ -919,10 +917,10 @@ struct WaveCtx {
   }
   void free()
   {
-    d_desc.free(); d_bm.free(); d_bmx.free(); d_cnt.free(); d_sup.free(); d_childmap.free(); d_cursor.free();
-    d_outs.free(); d_rec.free(); d_recn.free(); d_keyword.free(); d_listed.free(); d_lnode.free();
+    d_desc.free(); d_bmx.free(); d_sup.free(); d_childmap.free(); d_cursor.free();
+    d_rec.free(); d_keyword.free(); d_listed.free(); d_lnode.free();
     d_head.free(); d_zero.free(); d_mat.free(); h_head.free(); h_mat.free();
-    h_desc.free(); h_sup.free(); h_cnt.free(); h_childmap.free(); h_outs.free(); h_keyword.free();
+    h_desc.free(); h_sup.free();
     sel_hint = 4096;
     for(auto &g : graphs) {
       if(g.x) cudaGraphExecDestroy(g.x);
@@ -1809,7 +1807,7 @@ private:
     X.h_sup.ensure(res_n);
     X.d_head.ensure(kHeadBytes);
     X.h_head.ensure(kHeadBytes);
-    // the job table, and the device table of the databases that joined
+    // the job table
     const size_t tab_bytes = Carver::round(sizeof(RootJob) * n);
     X.d_desc.ensure(tab_bytes);
     X.h_desc.ensure(tab_bytes);
@@ -2344,8 +2342,8 @@ private:
     st_.d2h_bytes += (int64_t)kHeadBytes + (int64_t)sizeof(int4) * std::min<int64_t>(nsel, f.sel_copied);
     if(nsel > f.sel_copied) {
       // copies the whole list again (growing the pinned buffer drops its
-      // contents) on the side stream: the wave's results are complete, and the
-      // main stream already holds the other context's wave
+      // contents) on the side stream, which no queued wave is ahead on: the
+      // wave's results are complete
       X.h_head.ensure(kHeadBytes + sizeof(int4) * (size_t)nsel);
       CK(cudaMemcpyAsync(X.h_head.p, X.d_head.p, kHeadBytes + sizeof(int4) * (size_t)nsel, cudaMemcpyDeviceToHost,
                          E.aux));

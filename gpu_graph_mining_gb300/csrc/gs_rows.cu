@@ -9,9 +9,9 @@
 // right-most-path vertex, and every step of 32 entries searched owners and
 // emitted few extensions.  250,000 graphs of 40 edges at minsup 0.5% (192 M
 // rows, 760 M extensions, one stream): count kernels 33.3 ms on columns, 10.7
-// here; a large launch 1.30 -> 0.45 ms with 989 M -> 390 M warp instructions
-// and 2.2 -> 0.73 GB of DRAM traffic.  It is bound by issue now (70% of
-// cycles, the integer pipe 64%; 0.24 of the DRAM peak).
+// here.  It is bound by issue now: a large launch of 390 M warp instructions
+// in 0.45 ms issues in 70% of cycles, the integer pipe 64%, at 0.24 of the DRAM
+// peak (0.73 GB).
 #include <algorithm>
 
 #include "gs_kernels.hpp"
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB :
             if(blk < a.blk_cap) {  // past the region's end nothing is written
               const unsigned b = (unsigned)region * (unsigned)a.blk_cap + (unsigned)blk;  // (below 2^26 blocks)
               a.rec[b * 32u + (unsigned)lane] = it;
-              if(lane == 0) a.hdr[b] = make_int4(row0, n, m | (gwarp % kRowsCopies) << 8 | (ids + 5) << 16, key_base);
+              if(lane == 0) a.hdr[b] = make_int4(row0, 0, m | (gwarp % kRowsCopies) << 8 | (ids + 5) << 16, key_base);
             }
             blk++;
             blk_left--;
