@@ -601,9 +601,10 @@ __global__ void __launch_bounds__(256) k_neighbour_blocks(const int32_t *__restr
                                                           int nb_blocks, int *used)
 {
   const int lane = threadIdx.x & 31;
-  const int stride = gridDim.x * blockDim.x;
-  for(int v0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; v0 < V; v0 += stride) {
-    const int v = v0 + lane;
+  // (64 bits: V is below 2^31, the step past the last vertex need not be)
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for(long long v0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll; v0 < V; v0 += stride) {
+    const long long v = v0 + lane;
     int a0 = 0, d = 0, gb = 0;
     if(v < V) {
       a0 = __ldg(&adj_off[v]);
