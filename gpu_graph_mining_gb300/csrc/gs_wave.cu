@@ -1,8 +1,9 @@
 // Warp-cooperative extension kernels on columns: count (support bitmaps +
 // embedding counts) and materialise (children's columns), for one wave of
 // DFS-tree nodes.  They serve graphs of more than 256 vertices, label alphabets
-// too large for packed rows (packed_shift) and the lists strategy, which joins
-// on the rows' back-links; gs_rows.cu serves the rest.
+// too large for packed rows (packed_shift), databases without neighbour blocks,
+// jobs that ran out of memory with packed rows, and the lists strategy, which
+// joins on the rows' back-links; gs_rows.cu serves the rest.
 //
 // gSpan's extension rules, from the sequential reference:
 //   backward  get_backward       src/globals/graph_types.cpp:389-413

@@ -101,7 +101,9 @@ GS_API gs_db *gs_db_from_arrays(int32_t db_size, int32_t edges_sizes, int32_t ma
  * returns it), and such a database holds its adjacency twice (8 more bytes
  * per entry): sorted for mining and in input order for gs_db_write.  Every
  * database of graphs of at most 256 vertices also holds neighbour blocks when
- * there is room for them: 32 bytes per vertex and 32/7 per adjacency entry. */
+ * there is room for them: 32 bytes per vertex and 32/7 per adjacency entry.
+ * They are given up when device memory runs out; the database is then mined
+ * without them (same patterns, slower). */
 GS_API gs_db *gs_db_from_arrays_device(int32_t db_size, int32_t edges_sizes, int32_t max_graph_vertex_count,
                                        int32_t vertex_count, const int32_t *edges, const int32_t *edges_labels,
                                        const int32_t *vertex_labels, const int32_t *vertex_offsets,
@@ -472,7 +474,9 @@ GS_API int32_t gs_dfs_code_is_min(const int32_t *dfs5xN, int32_t n_edges);
 /* Frees the miner's device pool and scratch buffers, and returns the
  * device ingest's cached pool memory. */
 GS_API void gs_engine_reset(void);
-/* Caps the device pool (bytes; 0 = 70% of free device memory). */
+/* Caps the device pool (bytes; 0 = 70% of free device memory).  A call that
+ * runs out of it with packed rows starts its unfinished databases again on
+ * columns, which can need less, before it fails with GS_ERR_NOMEM. */
 GS_API void gs_engine_set_pool_bytes(int64_t bytes);
 
 #ifdef __cplusplus
