@@ -156,39 +156,18 @@ void Database::prepare()
   pairs.assign(VL, {});
   pair_cnt.assign(VL, 0);
   root_off.assign(VL, 0);
-  int32_t acc = 0;
+  pair_code.clear();
   for(int32_t a = 0; a < VL; a++) {
+    root_off[a] = (int32_t)pair_code.size();
     for(int32_t e = 0; e < EL; e++)
       for(int32_t t = 0; t < VL; t++)
-        if(seen[(size_t)(((int64_t)a * EL + e) * VL + t)]) pairs[a].push_back({ e, t });
+        if(seen[(size_t)(((int64_t)a * EL + e) * VL + t)]) {
+          pairs[a].push_back({ e, t });
+          pair_code.push_back((int32_t)(((uint32_t)e << 16) | (uint32_t)t));
+        }
     pair_cnt[a] = (int32_t)pairs[a].size();
-    root_off[a] = acc;
-    acc += pair_cnt[a];
   }
-  root_keys = acc;
-  index_pairs();
-}
-
-int32_t Database::pair_index(int32_t a, int32_t el, int32_t tl) const
-{
-  if(!pair_tab.empty()) return pair_tab[((int64_t)a * EL + el) * VL + tl];
-  const auto &pr = pairs[a];
-  return (int32_t)(std::lower_bound(pr.begin(), pr.end(), std::make_pair(el, tl)) - pr.begin());
-}
-
-void Database::index_pairs()
-{
-  const int64_t tab = (int64_t)VL * EL * VL;
-  pair_code.assign((size_t)root_keys, 0);
-  for(int32_t a = 0; a < VL; a++)
-    for(size_t i = 0; i < pairs[a].size(); i++)
-      pair_code[root_off[a] + i] = (int32_t)(((uint32_t)pairs[a][i].first << 16) | (uint32_t)pairs[a][i].second);
-  pair_tab.clear();
-  if(tab > 1 << 20) return;
-  pair_tab.assign((size_t)tab, -1);
-  for(int32_t a = 0; a < VL; a++)
-    for(size_t i = 0; i < pairs[a].size(); i++)
-      pair_tab[((int64_t)a * EL + pairs[a][i].first) * VL + pairs[a][i].second] = (int32_t)i;
+  root_keys = (int32_t)pair_code.size();
 }
 
 void Database::upload()
@@ -1239,11 +1218,12 @@ int64_t g_pool_limit = 0;
 
 inline int32_t words_for(int64_t support) { return (int32_t)((support + 31) / 32); }
 
-// A root node's right-most path and keys.
-void root_layout(PNode &n, const Database &db)
+// A root node's right-most path and keys (pair: its edge's index among the pairs
+// of its first label).
+void root_layout(PNode &n, const Database &db, int32_t pair)
 {
   const CEdge &e = n.code[0];
-  n.slots.push_back(RmSlot{ 0, 0, e.fl, e.el, e.tl, db.pair_index(e.fl, e.el, e.tl) });
+  n.slots.push_back(RmSlot{ 0, 0, e.fl, e.el, e.tl, pair });
   n.slots.push_back(RmSlot{ 1, 0, e.tl, 0, 0, -1 });
   n.nv = 2;
   n.nfwd = n.nkeys = db.pair_cnt[e.fl] + db.pair_cnt[e.tl];
@@ -1892,7 +1872,7 @@ private:
         nn.job = id;
         nn.pattern = s.pid;
         nn.code.push_back(s.d);
-        root_layout(nn, db);
+        root_layout(nn, db, s.key - kb - db.root_off[s.d.fl]);
         if(S.packed) {
           nn.rows = o.rows;
           S.live_bytes += s.n * 16;

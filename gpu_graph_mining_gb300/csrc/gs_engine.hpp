@@ -115,7 +115,6 @@ struct Database {
   std::vector<std::vector<std::pair<int32_t, int32_t>>> pairs;
   std::vector<int32_t> pair_cnt, root_off;
   std::vector<int32_t> pair_code;  // [root_keys] (elabel << 16) | tolabel of each label's pairs, from root_off
-  std::vector<int32_t> pair_tab;  // [VL * EL * VL] index of a label's (elabel, tolabel) in pairs, small alphabets only
   int32_t root_keys = 0;
   // device copy
   void *d_block = nullptr;
@@ -134,9 +133,6 @@ struct Database {
   const unsigned long long *adj_in = nullptr;
 
   void prepare();   // label compaction and pair tables (host only)
-  void index_pairs();
-  // index of (el, tl) in pairs[a] (it must be there)
-  int32_t pair_index(int32_t a, int32_t el, int32_t tl) const;
   void upload();    // device copy (idempotent)
   void release();   // frees the device copy
   void ensure_host();  // host arrays of a device-built database (original labels)

@@ -802,7 +802,7 @@ void ingest_cudabin_device(Database &db, int32_t G, int32_t esz, int32_t maxv, c
       db.pair_cnt[a] = end - hro[a];
     }
     db.root_keys = (int32_t)nkeys;
-    db.index_pairs();
+    db.pair_code.assign(hpc, hpc + nkeys);
     db.neighbours = nb ? own_neighbours((uint4 *)nb, 32 * (size_t)nb_blocks, true) : nullptr;
     db.d_block = b;
     db.pooled = true;
