@@ -170,7 +170,9 @@ struct alignas(16) PackedNode {
   int32_t key_base;
   int32_t n_vertices;
   const int32_t *pair_code;
-  int32_t nb_blocks, slot_off, pad[3];
+  int32_t nb_blocks, slot_off;
+  int32_t dense;             // 1: many rows a graph (kDenseRows)
+  int32_t pad[2];
 };
 
 // Output slots of a child node selected for materialisation.

@@ -2041,7 +2041,7 @@ private:
     PackedNode *hp = carve<PackedNode>(hb, off, packed ? W : 0);
     const size_t desc_bytes = Carver::round(off);
     int32_t planes = 1;
-    bool wide = false;
+    bool wide = false, dense = false;
     int32_t eo = 0;
     int32_t co = 0, so = 0, kmax = 1;
     bool small = true;  // every database of the wave has graphs of <= 64 vertices
@@ -2118,6 +2118,8 @@ private:
         g.pair_code = db.dev.pair_code;
         g.nb_blocks = db.dev.nb_blocks;
         g.slot_off = so;
+        g.dense = p.nrows >= kDenseRows * p.support ? 1 : 0;
+        dense = dense || g.dense;
         planes = std::max(planes, g.planes);
         // algorithmic bytes: the row and one neighbour block per slot (an
         // extension's bitmap word, counter and record are added with the results)
@@ -2229,7 +2231,7 @@ private:
     q.desc_bytes = desc_bytes;
     q.k[0] = begin_call(X.d_desc.p, hb, (long long)desc_bytes / 16, X.d_zero.p, (long long)zero_bytes / 16, head);
     if(packed)
-      q.k[1] = rows_count_call(f.dp, f.dt, W, (int32_t)tb, planes, wide, f.ds, f.bm, cnt, cstride,
+      q.k[1] = rows_count_call(f.dp, f.dt, W, (int32_t)tb, planes, wide, dense, f.ds, f.bm, cnt, cstride,
                                 (uint32_t *)f.rec, f.hdr, (int32_t)f.rec_cap, f.reg, head, err_flag(), wo_.count_grid);
     else
       q.k[1] = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,

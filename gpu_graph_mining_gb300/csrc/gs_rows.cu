@@ -100,6 +100,14 @@ __device__ __forceinline__ unsigned shl_one(unsigned n)
   return x;
 }
 
+// A bitmap word while other warps set bits of it.
+__device__ __forceinline__ uint32_t word_now(const uint32_t *p)
+{
+  uint32_t x;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p));
+  return x;
+}
+
 // Graph-local id of pattern vertex t (the words' unused bytes are 0).
 template <int NW> __device__ __forceinline__ unsigned id_of(const unsigned (&w)[NW], int t)
 {
@@ -168,7 +176,18 @@ __device__ __forceinline__ void store_row(const RowsOut &out, int pos, int gb, i
 // one 64-bit set in registers it costs less: the narrow kernel stays).  3,000
 // graphs of 60 to 130 vertices, up to 5 edges: count 0.48 ms on columns, 0.33
 // here, materialise 0.12 -> 0.08, the mine 0.86 -> 0.67.
-template <int PL, bool MAT, bool WIDE>
+//
+// DENSE (count; some node of the wave has kDenseRows rows a graph and more): such
+// a node's bitmap words are read before an OR, which is left out where the bit is
+// set.  ORs to one word complete one after another, and when a graph has many
+// rows nearly every OR sets a bit that is there; with few rows a graph the load
+// is a trip to L2 for nothing.  Count kernels of a mine (ms; columns / an OR always /
+// so): 300 stars of 200 leaves of 2 labels 29.5 / 80.9 / 11.5; 300 graphs of 40
+// vertices and 240 edges, 2 labels 11.9 / 21.1 / 3.0; 3,000 trees with hubs, 60
+// vertices, 2 labels 1.48 / 4.33 / 1.19.  With the load for every node 100,000
+// molecule-like graphs at 5% 0.84 -> 1.06, 100,000 of 40 edges at 0.5% 4.37 -> 5.36;
+// a test of the node alone costs those 1%, so it is an instance of its own.
+template <int PL, bool MAT, bool WIDE, bool DENSE>
 __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB : 7) k_rows(const RowsArgs a)
 {
   if(!MAT) after_previous();
@@ -423,8 +442,11 @@ __global__ void __launch_bounds__(kWarps * 32, PL == 1 && !WIDE ? GS_ROWS_MINB :
           const unsigned peers = __match_any_sync(kFull, key);
           const int leader = __ffs(peers) - 1;
           const int g_lead = __shfl_sync(kFull, g_o, leader);
-          if(key >= 0 && (lane == leader || g_o != g_lead))
-            atomicOr(&a.bm[S.nd.bm_base + (long long)key * S.nd.words + (g_o >> 5)], 1u << (g_o & 31));
+          if(key >= 0 && (lane == leader || g_o != g_lead)) {
+            uint32_t *const word = &a.bm[S.nd.bm_base + (long long)key * S.nd.words + (g_o >> 5)];
+            const uint32_t bit = 1u << (g_o & 31);
+            if(!DENSE || !S.nd.dense || !(word_now(word) & bit)) atomicOr(word, bit);
+          }
           if(key >= 0 && lane == leader) atomicAdd(&a.cnt[(gwarp % kRowsCopies) * a.cnt_stride + key_base + key], __popc(peers));
           if(a.rec) {
             if(blk_left == 0) {
@@ -653,7 +675,7 @@ __global__ void __launch_bounds__(256) k_neighbour_blocks(const int32_t *__restr
   }
 }
 
-template <int PL, bool MAT, bool WIDE> KernelCall rows_call(RowsArgs a, int grid_per_sm)
+template <int PL, bool MAT, bool WIDE, bool DENSE> KernelCall rows_call(RowsArgs a, int grid_per_sm)
 {
   const long long cap = (long long)sm_count() * (grid_per_sm > 0 ? grid_per_sm : GS_ROWS_GRID);
   // in groups once every warp of a full grid has one: below that the chip would idle
@@ -661,7 +683,7 @@ template <int PL, bool MAT, bool WIDE> KernelCall rows_call(RowsArgs a, int grid
   long long blocks = ((long long)a.total_tiles + kWarps * a.group - 1) / (kWarps * a.group);
   blocks = blocks > cap ? cap : blocks < 1 ? 1 : blocks;
   KernelCall c;
-  c.func = (const void *)k_rows<PL, MAT, WIDE>;
+  c.func = (const void *)k_rows<PL, MAT, WIDE, DENSE>;
   c.early = !MAT;
   c.grid = dim3((unsigned)blocks);
   c.block = dim3(kWarps * 32);
@@ -669,13 +691,13 @@ template <int PL, bool MAT, bool WIDE> KernelCall rows_call(RowsArgs a, int grid
   return c;
 }
 
-template <bool MAT> KernelCall rows_call(const RowsArgs &a, int planes, bool wide, int grid_per_sm)
+template <bool MAT, bool DENSE> KernelCall rows_call(const RowsArgs &a, int planes, bool wide, int grid_per_sm)
 {
   if(wide)
-    return planes <= 1 ? rows_call<1, MAT, true>(a, grid_per_sm)
-         : planes <= 2 ? rows_call<2, MAT, true>(a, grid_per_sm) : rows_call<5, MAT, true>(a, grid_per_sm);
-  return planes <= 1 ? rows_call<1, MAT, false>(a, grid_per_sm)
-       : planes <= 2 ? rows_call<2, MAT, false>(a, grid_per_sm) : rows_call<5, MAT, false>(a, grid_per_sm);
+    return planes <= 1 ? rows_call<1, MAT, true, DENSE>(a, grid_per_sm)
+         : planes <= 2 ? rows_call<2, MAT, true, DENSE>(a, grid_per_sm) : rows_call<5, MAT, true, DENSE>(a, grid_per_sm);
+  return planes <= 1 ? rows_call<1, MAT, false, DENSE>(a, grid_per_sm)
+       : planes <= 2 ? rows_call<2, MAT, false, DENSE>(a, grid_per_sm) : rows_call<5, MAT, false, DENSE>(a, grid_per_sm);
 }
 
 template <int B> auto *mat_kernel(int planes, bool wide)
@@ -687,13 +709,14 @@ template <int B> auto *mat_kernel(int planes, bool wide)
 }  // namespace
 
 KernelCall rows_count_call(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
-                           int32_t planes, bool wide, const SlotDesc *slots, uint32_t *bm, int32_t *cnt,
+                           int32_t planes, bool wide, bool dense, const SlotDesc *slots, uint32_t *bm, int32_t *cnt,
                            long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,
                            unsigned long long *head, unsigned int *err, int32_t grid_per_sm)
 {
   const RowsArgs a{ nodes, tile0, nnodes, total_tiles, 1, slots, bm, nullptr, cnt, cnt_stride, nullptr, nullptr,
                     nullptr, nullptr, rec, hdr, blk_cap, reg, err, head + kHeadCount0 };
-  return rows_call<false>(a, planes, wide, grid_per_sm);
+  return dense ? rows_call<false, true>(a, planes, wide, grid_per_sm)
+               : rows_call<false, false>(a, planes, wide, grid_per_sm);
 }
 
 void launch_rows_materialize(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
@@ -704,7 +727,7 @@ void launch_rows_materialize(const PackedNode *nodes, const int32_t *tile0, int3
   if(total_tiles <= 0) return;
   const RowsArgs a{ nodes, tile0, nnodes, total_tiles, 1, slots, const_cast<uint32_t *>(bm), bmx, nullptr, 0, chosen,
                     childmap, cursor, outs, nullptr, nullptr, 0, nullptr, err, stamps };
-  KernelCall c = rows_call<true>(a, planes, wide, 0);
+  KernelCall c = rows_call<true, false>(a, planes, wide, 0);
   c.run(s);
 }
 
