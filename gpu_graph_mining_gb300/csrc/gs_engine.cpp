@@ -46,8 +46,9 @@ void cuda_check(cudaError_t e, const char *what)
 
 namespace {
 
-std::mutex g_nb_mu;                             // every Neighbours' fields
+std::mutex g_nb_mu;                             // the list
 std::vector<std::weak_ptr<Neighbours>> g_nb;    // those that have blocks, and some that had
+size_t g_nb_sweep = 64;                         // at this length, those that are gone leave it
 
 // cudaMalloc; out of memory, the neighbour blocks that no scheduler uses go first
 cudaError_t device_malloc(void **p, size_t n)
@@ -61,30 +62,29 @@ cudaError_t device_malloc(void **p, size_t n)
 
 }  // namespace
 
-NeighboursUse::NeighboursUse(const std::shared_ptr<Neighbours> &n) : n_(n)
+NeighboursUse::NeighboursUse(const std::shared_ptr<Neighbours> &n)
 {
-  if(!n_) return;
-  std::lock_guard<std::mutex> g(g_nb_mu);
-  n_->users++;
-  nb_ = n_->nb;
+  if(!n) return;
+  int u = n->users.load();
+  while(u >= 0 && !n->users.compare_exchange_weak(u, u + 1)) {
+  }
+  if(u >= 0) n_ = n;
 }
 
 NeighboursUse::~NeighboursUse()
 {
-  if(!n_) return;
-  std::lock_guard<std::mutex> g(g_nb_mu);
-  n_->users--;
+  if(n_) n_->users--;
 }
 
 std::shared_ptr<Neighbours> own_neighbours(uint4 *nb, size_t bytes, bool pooled)
 {
-  std::shared_ptr<Neighbours> n(new Neighbours());
-  n->nb = nb;
-  n->bytes = bytes;
-  n->pooled = pooled;
+  std::shared_ptr<Neighbours> n = std::make_shared<Neighbours>(nb, bytes, pooled);
   std::lock_guard<std::mutex> g(g_nb_mu);
-  g_nb.erase(std::remove_if(g_nb.begin(), g_nb.end(), [](const std::weak_ptr<Neighbours> &w) { return w.expired(); }),
-             g_nb.end());
+  if(g_nb.size() >= g_nb_sweep) {
+    g_nb.erase(std::remove_if(g_nb.begin(), g_nb.end(), [](const std::weak_ptr<Neighbours> &w) { return w.expired(); }),
+               g_nb.end());
+    g_nb_sweep = 2 * g_nb.size() + 64;
+  }
   g_nb.push_back(n);
   return n;
 }
@@ -94,21 +94,17 @@ std::vector<NeighbourBlock> detach_idle_neighbours()
   std::vector<NeighbourBlock> out;
   std::lock_guard<std::mutex> g(g_nb_mu);
   for(auto &w : g_nb)
-    if(std::shared_ptr<Neighbours> n = w.lock())
-      if(n->nb && n->users == 0) {
-        out.push_back(NeighbourBlock{ n->nb, n->pooled });
-        n->nb = nullptr;
-      }
+    if(std::shared_ptr<Neighbours> n = w.lock()) {
+      int idle = 0;
+      if(n->users.compare_exchange_strong(idle, Neighbours::kGone)) out.push_back(NeighbourBlock{ n->nb, n->pooled });
+    }
   return out;
 }
 
 NeighbourBlock detach_neighbours(const std::shared_ptr<Neighbours> &n)
 {
-  if(!n) return NeighbourBlock{ nullptr, false };
-  std::lock_guard<std::mutex> g(g_nb_mu);
-  const NeighbourBlock b{ n->nb, n->pooled };
-  n->nb = nullptr;
-  return b;
+  if(!n || n->users.exchange(Neighbours::kGone) < 0) return NeighbourBlock{ nullptr, false };
+  return NeighbourBlock{ n->nb, n->pooled };
 }
 
 bool give_up_neighbours()
@@ -320,8 +316,7 @@ void Database::ensure_host()
 int64_t Database::device_bytes() const
 {
   if(!resident) return 0;
-  std::lock_guard<std::mutex> g(g_nb_mu);
-  return (int64_t)(d_bytes + (neighbours && neighbours->nb ? neighbours->bytes : 0));
+  return (int64_t)(d_bytes + (neighbours && neighbours->users.load() >= 0 ? neighbours->bytes : 0));
 }
 
 void Database::release()
@@ -1423,9 +1418,9 @@ public:
     if(slot < 0) {
       slot = (int32_t)dbs_.size();
       dbs_.push_back(db);
-      nb_use_.emplace_back(new NeighboursUse(db->neighbours));
+      nb_use_.emplace_back(db->neighbours);
       tab_.push_back(db->dev);
-      tab_.back().nb = nb_use_.back()->nb();
+      tab_.back().nb = nb_use_.back().nb();
       if(tab_.size() > E.d_dbs.cap) {
         // the table is read by waves in flight: let them finish before it moves
         E.sync_all();
@@ -1557,7 +1552,7 @@ private:
   std::vector<Database *> dbs_;
   std::vector<char> db_seen_;  // wave building: database slots met
   std::vector<DevDB> tab_;
-  std::vector<std::unique_ptr<NeighboursUse>> nb_use_;  // the table's neighbour blocks
+  std::deque<NeighboursUse> nb_use_;  // the table's neighbour blocks
   int64_t active_ = 0;
   int64_t stacked_ = 0;          // nodes on all jobs' stacks
   int64_t seen_bytes_[2] = { 0, 0 };

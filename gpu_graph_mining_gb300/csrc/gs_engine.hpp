@@ -1,6 +1,7 @@
 // The mining engine: resident databases, the device memory pool, and the
 // wave scheduler that extends many DFS-tree nodes per kernel launch.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <memory>
 #include <mutex>
@@ -73,10 +74,12 @@ void cuda_check(cudaError_t e, const char *what);
 // scheduler uses are given up when device memory runs out.  Shared by the
 // database and the schedulers that have mined it.
 struct Neighbours {
-  uint4 *nb = nullptr;  // nullptr: given up
-  size_t bytes = 0;
-  bool pooled = false;  // from the ingest's pool
-  int users = 0;        // schedulers whose database table points to them
+  uint4 *const nb;
+  const size_t bytes;
+  const bool pooled;  // from the ingest's pool
+  static constexpr int kGone = INT32_MIN / 2;
+  std::atomic<int> users{ 0 };  // schedulers whose database table points to them; below 0: given up
+  Neighbours(uint4 *p, size_t n, bool from_pool) : nb(p), bytes(n), pooled(from_pool) {}
 };
 // A scheduler's use of a database's neighbour blocks (nb(): nullptr when there
 // are none, else they stay until the use ends or the database is freed).
@@ -86,11 +89,10 @@ public:
   ~NeighboursUse();
   NeighboursUse(const NeighboursUse &) = delete;
   NeighboursUse &operator=(const NeighboursUse &) = delete;
-  const uint4 *nb() const { return nb_; }
+  const uint4 *nb() const { return n_ ? n_->nb : nullptr; }
 
 private:
   std::shared_ptr<Neighbours> n_;
-  const uint4 *nb_ = nullptr;
 };
 // New blocks, known to give_up_neighbours.
 std::shared_ptr<Neighbours> own_neighbours(uint4 *nb, size_t bytes, bool pooled);
