@@ -144,10 +144,11 @@ inline int region_blocks(long long most, int threads)
   return (int)(std::max(per, 1ll) * kRecRegions);
 }
 constexpr int kRowsCopies = 4, kRowsKeys = 1 << 23;
-// Rows a graph from which a node is dense (PackedNode::dense).  3,000 trees with hubs
-// count 1.19 ms with 8 to 24, 1.24 with 32 and 48, 1.80 with 64; 2,000 graphs of 60 to
-// 130 vertices 0.157 with 8, 0.152 with 12 and more, as without.
-constexpr int kDenseRows = 24;
+// Rows a graph from which a node is dense (PackedNode::dense).  Count of 3,000 trees
+// with hubs 1.19 ms with 8 to 24, 1.24 with 32 and 48, 1.80 with 64; a mine of 5,000
+// stars (17 rows a graph) 0.27 ms with 12 and 16, 0.35 with 24; 2,000 graphs of 60 to 130
+// vertices 0.157 ms with 8, 0.151 with 12 and more, as without.
+constexpr int kDenseRows = 16;
 KernelCall rows_count_call(const PackedNode *nodes, const int32_t *tile0, int32_t nnodes, int32_t total_tiles,
                            int32_t planes, bool wide, bool dense, const SlotDesc *slots, uint32_t *bm, int32_t *cnt,
                            long long cnt_stride, uint32_t *rec, int4 *hdr, int32_t blk_cap, uint32_t *reg,

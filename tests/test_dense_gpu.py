@@ -20,10 +20,10 @@ def _broom(path, leaves, size):
 
 
 # path: rows of one, two and five planes where the leaves begin; leaves: rows a graph of the
-# node that ends in one, the line is at 24
+# node that ends in one, the line is at 16
 @pytest.mark.parametrize("size", [0, 70])
 @pytest.mark.parametrize("path", [2, 8, 24])
-@pytest.mark.parametrize("leaves", [23, 24, 25])
+@pytest.mark.parametrize("leaves", [15, 16, 17])
 def test_rows_a_graph(gs, oracle, tmp_path, path, leaves, size):
     p = str(tmp_path / "brooms.txt")
     graphs = 70
