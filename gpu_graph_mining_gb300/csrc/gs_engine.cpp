@@ -191,7 +191,16 @@ void Database::upload()
   if(nb_blocks >= INT32_MAX) nb_blocks = 0;
   size_t o_nu = o_pc + al(sizeof(int32_t) * (root_keys + 1));
   const size_t total = o_nu + al(sizeof(int32_t));
-  std::vector<unsigned long long> adj(E2 + 1, 0);
+  // all of it in one host block, for one copy
+  const std::unique_ptr<char[]> block(new char[total]);
+  char *const h = block.get();
+  auto ints = [h](size_t o) { return (int32_t *)(h + o); };
+  unsigned long long *const adj = (unsigned long long *)(h + o_adj);
+  int32_t *const off = ints(o_off), *const vl = ints(o_vl), *const vg = ints(o_vg), *const vgb = ints(o_gb);
+  int32_t *const pidx = ints(o_pi), *const ro = ints(o_ro), *const vb = ints(o_vb), *const ap = ints(o_ap);
+  int32_t *const pc = ints(o_pc);
+  adj[E2] = 0;
+  vl[V] = vg[V] = vgb[V] = ap[E2] = pc[root_keys] = *ints(o_nu) = 0;
   parallel_ranges(E2, [&](int64_t b, int64_t e, int) {
     for(int64_t k = b; k < e; k++) {
       const uint32_t w = (uint32_t)host.adj_to[k];
@@ -203,11 +212,11 @@ void Database::upload()
   // order: the entries a right-most-path vertex's forward rule rejects are a
   // prefix the extension kernels skip
   parallel_ranges(V, [&](int64_t v0, int64_t v1, int) {
-    for(int64_t v = v0; v < v1; v++) std::sort(adj.begin() + host.aoff[v], adj.begin() + host.aoff[v + 1]);
+    for(int64_t v = v0; v < v1; v++) std::sort(adj + host.aoff[v], adj + host.aoff[v + 1]);
   }, 1 << 14);
-  std::vector<int32_t> off(V + 1), vg(V + 1, 0), vgb(V + 1, 0), pidx(tab, -1);
   parallel_ranges(V + 1, [&](int64_t b, int64_t e, int) {
     for(int64_t v = b; v < e; v++) off[v] = (int32_t)host.aoff[v];
+    std::copy(vl_dense.begin() + b, vl_dense.begin() + std::min(e, V), vl + b);
   }, 1 << 16);
   parallel_ranges(host.n_graphs, [&](int64_t g0, int64_t g1, int) {
     for(int64_t g = g0; g < g1; g++)
@@ -216,13 +225,13 @@ void Database::upload()
         vgb[v] = (int32_t)host.vbase[g];
       }
   });
+  std::fill(pidx, pidx + tab, -1);
   for(int32_t a = 0; a < VL; a++)
     for(size_t i = 0; i < pairs[a].size(); i++)
       pidx[((int64_t)a * EL + pairs[a][i].first) * VL + pairs[a][i].second] = (int32_t)i;
   // per directed entry: dense index of (elabel, nbr label) among the pairs of
   // the source vertex's label (the forward key offset within a slot, and the
   // root key offset within root_off[label(source)])
-  std::vector<int32_t> ap(E2 + 1, 0);
   parallel_ranges(V, [&](int64_t v0, int64_t v1, int) {
     for(int64_t v = v0; v < v1; v++) {
       const int64_t a = vl_dense[v];
@@ -232,25 +241,14 @@ void Database::upload()
       }
     }
   });
-  std::vector<int32_t> vb(host.n_graphs + 1);
   for(int32_t g = 0; g <= host.n_graphs; g++) vb[g] = (int32_t)host.vbase[g];
+  std::copy(root_off.begin(), root_off.end(), ro);
+  ro[VL] = root_keys;
+  std::copy(pair_code.begin(), pair_code.end(), pc);
   CK(device_malloc(&d_block, total));
   d_bytes = h2d_bytes = total;
   char *b = (char *)d_block;
-  CK(cudaMemcpy(b + o_adj, adj.data(), sizeof(unsigned long long) * (E2 + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b + o_off, off.data(), sizeof(int32_t) * (V + 1), cudaMemcpyHostToDevice));
-  if(V) CK(cudaMemcpy(b + o_vl, vl_dense.data(), sizeof(int32_t) * V, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b + o_vg, vg.data(), sizeof(int32_t) * (V + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b + o_gb, vgb.data(), sizeof(int32_t) * (V + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b + o_pi, pidx.data(), sizeof(int32_t) * tab, cudaMemcpyHostToDevice));
-  std::vector<int32_t> ro(root_off);
-  ro.push_back(root_keys);
-  std::vector<int32_t> pc(pair_code);
-  pc.push_back(0);
-  CK(cudaMemcpy(b + o_ro, ro.data(), sizeof(int32_t) * (VL + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b + o_pc, pc.data(), sizeof(int32_t) * (root_keys + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b + o_vb, vb.data(), sizeof(int32_t) * (host.n_graphs + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b + o_ap, ap.data(), sizeof(int32_t) * (E2 + 1), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(b, h, total, cudaMemcpyHostToDevice));
   dev.adj = (const unsigned long long *)(b + o_adj);
   dev.adj_off = (const int32_t *)(b + o_off);
   dev.vlabel = (const int32_t *)(b + o_vl);
@@ -279,9 +277,8 @@ void Database::upload()
     dev.nb_shift = nb_shift;
     dev.nb_ids = packed_ids(maxnv);
     dev.nb_blocks = (int32_t)nb_blocks;
-    cudaError_t e = cudaMemsetAsync(b + o_nu, 0, sizeof(int32_t), cudaStreamLegacy);
     launch_neighbour_blocks(dev, (uint4 *)nb, (int32_t *)(b + o_nu), cudaStreamLegacy);
-    if(e == cudaSuccess) e = cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
     if(e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if(e != cudaSuccess) cudaFree(nb);
     cuda_check(e, "neighbour blocks");
