@@ -121,6 +121,7 @@ struct NodeDesc {
   int32_t code_off;      // the node's DFS code: edges code_off.. of the wave's code table
   int32_t code_len;      //   (a uint2 per edge)
   int32_t nfwd;          // keys below nfwd are forward extensions
+  int32_t dense;         // 1: many rows a graph (kDenseRows)
   // Lists strategy (extension by intersection): a forward child's extensions
   // from right-most-path vertices other than its new right-most vertex are
   // its parent's frequent forward extensions at the same parent row (minus

@@ -2066,6 +2066,8 @@ private:
       d.code_off = eo;
       d.code_len = (int32_t)p.code.size();
       d.nfwd = p.nfwd;
+      d.dense = p.nrows >= kDenseRows * p.support ? 1 : 0;
+      dense = dense || d.dense;
       if(p.list_off) {
         // lists strategy: join the parent's per-row lists
         d.csr_off = p.list_off;
@@ -2110,8 +2112,7 @@ private:
         g.pair_code = db.dev.pair_code;
         g.nb_blocks = db.dev.nb_blocks;
         g.slot_off = so;
-        g.dense = p.nrows >= kDenseRows * p.support ? 1 : 0;
-        dense = dense || g.dense;
+        g.dense = d.dense;
         planes = std::max(planes, g.planes);
         // algorithmic bytes: the row and one neighbour block per slot (an
         // extension's bitmap word, counter and record are added with the results)
@@ -2228,7 +2229,7 @@ private:
     else
       q.k[1] = wave_count_call(f.dn, W, tb, kmax, small, f.dc, f.dl, f.ds, f.dv, E.d_dbs.p, f.bm, cnt, E.d_bytes.p + 0,
                               err_flag(), f.rec, f.rec_cap, f.reg, head,
-                              wo_.count_grid, ccopies, cstride, f.join, f.rule_skip);
+                              wo_.count_grid, ccopies, cstride, f.join, f.rule_skip, dense);
     int32_t *lnode = nullptr;
     if(f.lists) {
       X.d_lnode.ensure(std::max(kb, 1));

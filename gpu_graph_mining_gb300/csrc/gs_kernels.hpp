@@ -105,6 +105,7 @@ void launch_root_materialize(const RootJob *jobs, int32_t njobs, long long tiles
 // small_graphs: every graph of the wave's databases has <= 64 vertices.
 // rec (may be null): kRecRegions regions of rec_cap records, whole chunks of
 // kRecChunk; reg: their counters, as for the packed rows (zeroed before).
+// dense: some node has kDenseRows rows a graph and more (NodeDesc::dense).
 // rule_skip: in databases with sorted adjacency (DevDB::adj_sorted), a
 // right-most-path vertex's entries below its forward rule are bisected past
 // instead of scanned.
@@ -113,7 +114,7 @@ KernelCall wave_count_call(const NodeDesc *nodes, int32_t nnodes, long long tota
                            const int32_t *vtab, const DevDB *dbs, uint32_t *bm, int32_t *cnt,
                            unsigned long long *bytes, unsigned int *err, int4 *rec, long long rec_cap,
                            uint32_t *reg, unsigned long long *head, int32_t grid_per_sm, int32_t cnt_copies,
-                           long long cnt_stride, bool join, bool rule_skip);
+                           long long cnt_stride, bool join, bool rule_skip, bool dense);
 void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long total_tiles, int32_t kmax,
                              bool small_graphs,
                              const int2 *const *coltab, const int32_t *collen, const SlotDesc *slots,
@@ -144,7 +145,7 @@ inline int region_blocks(long long most, int threads)
   return (int)(std::max(per, 1ll) * kRecRegions);
 }
 constexpr int kRowsCopies = 4, kRowsKeys = 1 << 23;
-// Rows a graph from which a node is dense (PackedNode::dense).  Count of 3,000 trees
+// Rows a graph from which a node is dense (NodeDesc::dense, PackedNode::dense).  Count of 3,000 trees
 // with hubs 1.19 ms with 8 to 24, 1.24 with 32 and 48, 1.80 with 64; a mine of 5,000
 // stars (17 rows a graph) 0.27 ms with 12 and 16, 0.35 with 24; 2,000 graphs of 60 to 130
 // vertices 0.157 ms with 8, 0.151 with 12 and more, as without.

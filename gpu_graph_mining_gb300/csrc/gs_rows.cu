@@ -100,14 +100,6 @@ __device__ __forceinline__ unsigned shl_one(unsigned n)
   return x;
 }
 
-// A bitmap word while other warps set bits of it.
-__device__ __forceinline__ uint32_t word_now(const uint32_t *p)
-{
-  uint32_t x;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p));
-  return x;
-}
-
 // Graph-local id of pattern vertex t (the words' unused bytes are 0).
 template <int NW> __device__ __forceinline__ unsigned id_of(const unsigned (&w)[NW], int t)
 {

@@ -38,4 +38,12 @@ __device__ __forceinline__ void stamp_mat_end(unsigned long long *stamps)
   if(threadIdx.x == 0) atomicMax(&stamps[16 * (1 + blockIdx.x % kMatSlots)], now_ns());
 }
 
+// A bitmap word while other warps set bits of it.
+__device__ __forceinline__ uint32_t word_now(const uint32_t *p)
+{
+  uint32_t x;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p));
+  return x;
+}
+
 }  // namespace gsgb

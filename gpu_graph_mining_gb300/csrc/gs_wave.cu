@@ -128,8 +128,9 @@ __device__ __forceinline__ int reserve_chunk(uint32_t *reg, int cap, int &region
 // "is w already in the embedding" is one bit test of the row's vertex set
 // instead of a loop over its k vertices.  JOIN: some node of the wave joins
 // its parent's per-row lists (lists strategy); without it the join code is
-// compiled out.
-template <int KMAX, bool MAT, bool MASK, bool JOIN>
+// compiled out.  DENSE: some node has kDenseRows rows a graph and more, whose
+// bitmap words are read before an OR, as on packed rows (k_rows).
+template <int KMAX, bool MAT, bool MASK, bool JOIN, bool DENSE>
 __global__ void
 #if GS_WAVE_MINB > 0
 __launch_bounds__(kWarps * 32, GS_WAVE_MINB)
@@ -173,6 +174,7 @@ k_wave(const WaveArgs a)
     const NodeDesc &nd = a.nodes[n];
     const int k = nd.k, nslot = nd.nslot, minlabel = nd.minlabel, words = nd.words, key_base = nd.key_base;
     const long long bm_base = nd.bm_base;
+    const bool dense = DENSE && nd.dense;
     const DevDB &dbr = a.dbs[nd.db];
     const unsigned long long *__restrict__ adj = dbr.adj;
     const int32_t *__restrict__ adj_off = dbr.adj_off;
@@ -404,8 +406,11 @@ k_wave(const WaveArgs a)
         const unsigned peers = __match_any_sync(kFull, key);
         const int leader = __ffs(peers) - 1;
         const int g_lead = __shfl_sync(kFull, g_o, leader);
-        if(key >= 0 && (lane == leader || g_o != g_lead))
-          atomicOr(&a.bm[bm_base + (long long)key * words + (g_o >> 5)], 1u << (g_o & 31));
+        if(key >= 0 && (lane == leader || g_o != g_lead)) {
+          uint32_t *const word = &a.bm[bm_base + (long long)key * words + (g_o >> 5)];
+          const uint32_t bit = 1u << (g_o & 31);
+          if(!dense || !(word_now(word) & bit)) atomicOr(word, bit);
+        }
         if(key >= 0 && lane == leader) atomicAdd(&cnt_copy[key_base + key], __popc(peers));
         const unsigned ext = __ballot_sync(kFull, key >= 0);  // every lane takes part
         if(a.rec && ext) {
@@ -474,7 +479,7 @@ template <int KMAX, bool MAT, bool MASK, bool JOIN> void launch_k(const WaveArgs
   const size_t smem = sizeof(Smem<KMAX>) * kWarps;
   // once per instance (a thread-safe static: schedulers may launch from several threads)
   static const bool configured = [smem] {
-    cudaFuncSetAttribute(k_wave<KMAX, MAT, MASK, JOIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_wave<KMAX, MAT, MASK, JOIN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return true;
   }();
   (void)configured;
@@ -482,7 +487,7 @@ template <int KMAX, bool MAT, bool MASK, bool JOIN> void launch_k(const WaveArgs
   const long long cap = (long long)sm_count() * GS_WAVE_GRID;
   if(blocks > cap) blocks = cap;
   if(blocks < 1) blocks = 1;
-  k_wave<KMAX, MAT, MASK, JOIN><<<(int)blocks, kWarps * 32, smem, s>>>(a);
+  k_wave<KMAX, MAT, MASK, JOIN, false><<<(int)blocks, kWarps * 32, smem, s>>>(a);
 }
 
 template <bool MAT, bool MASK, bool JOIN> void dispatch_k(int kmax, const WaveArgs &a, cudaStream_t s)
@@ -504,11 +509,11 @@ template <bool MAT> void dispatch(int kmax, bool small_graphs, bool join, const 
   }
 }
 
-template <int KMAX, bool MASK, bool JOIN> KernelCall count_call_k(const WaveArgs &a, int grid_per_sm)
+template <int KMAX, bool MASK, bool JOIN, bool DENSE> KernelCall count_call_k(const WaveArgs &a, int grid_per_sm)
 {
   const size_t smem = sizeof(Smem<KMAX>) * kWarps;
   static const bool configured = [smem] {
-    cudaFuncSetAttribute(k_wave<KMAX, false, MASK, JOIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_wave<KMAX, false, MASK, JOIN, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     return true;
   }();
   (void)configured;
@@ -517,7 +522,7 @@ template <int KMAX, bool MASK, bool JOIN> KernelCall count_call_k(const WaveArgs
   if(blocks > cap) blocks = cap;
   if(blocks < 1) blocks = 1;
   KernelCall c;
-  c.func = (const void *)k_wave<KMAX, false, MASK, JOIN>;
+  c.func = (const void *)k_wave<KMAX, false, MASK, JOIN, DENSE>;
   c.grid = dim3((unsigned)blocks);
   c.block = dim3(kWarps * 32);
   c.smem = (unsigned)smem;
@@ -525,12 +530,17 @@ template <int KMAX, bool MASK, bool JOIN> KernelCall count_call_k(const WaveArgs
   return c;
 }
 
-template <bool MASK, bool JOIN> KernelCall count_call(int kmax, const WaveArgs &a, int grid_per_sm)
+template <bool MASK, bool JOIN, bool DENSE> KernelCall count_call(int kmax, const WaveArgs &a, int grid_per_sm)
 {
-  if(kmax <= 8) return count_call_k<8, MASK, JOIN>(a, grid_per_sm);
-  if(kmax <= 16) return count_call_k<16, MASK, JOIN>(a, grid_per_sm);
-  if(kmax <= 32) return count_call_k<32, MASK, JOIN>(a, grid_per_sm);
-  return count_call_k<64, MASK, JOIN>(a, grid_per_sm);
+  if(kmax <= 8) return count_call_k<8, MASK, JOIN, DENSE>(a, grid_per_sm);
+  if(kmax <= 16) return count_call_k<16, MASK, JOIN, DENSE>(a, grid_per_sm);
+  if(kmax <= 32) return count_call_k<32, MASK, JOIN, DENSE>(a, grid_per_sm);
+  return count_call_k<64, MASK, JOIN, DENSE>(a, grid_per_sm);
+}
+
+template <bool MASK, bool JOIN> KernelCall count_call(int kmax, bool dense, const WaveArgs &a, int grid_per_sm)
+{
+  return dense ? count_call<MASK, JOIN, true>(kmax, a, grid_per_sm) : count_call<MASK, JOIN, false>(kmax, a, grid_per_sm);
 }
 
 }  // namespace
@@ -540,14 +550,14 @@ KernelCall wave_count_call(const NodeDesc *nodes, int32_t nnodes, long long tota
                            const int32_t *vtab, const DevDB *dbs, uint32_t *bm, int32_t *cnt,
                            unsigned long long *bytes, unsigned int *err, int4 *rec, long long rec_cap,
                            uint32_t *reg, unsigned long long *head, int32_t grid_per_sm, int32_t cnt_copies,
-                           long long cnt_stride, bool join, bool rule_skip)
+                           long long cnt_stride, bool join, bool rule_skip, bool dense)
 {
   WaveArgs a{ nodes, nnodes, total_tiles, coltab, collen, slots, vtab, dbs, bm, nullptr, cnt,
               nullptr, nullptr, nullptr, bytes, err, rec, (int)rec_cap, reg, cnt_copies,
               cnt_stride, rule_skip ? 1 : 0, head + kHeadCount0 };
   if(small_graphs)
-    return join ? count_call<true, true>(kmax, a, grid_per_sm) : count_call<true, false>(kmax, a, grid_per_sm);
-  return join ? count_call<false, true>(kmax, a, grid_per_sm) : count_call<false, false>(kmax, a, grid_per_sm);
+    return join ? count_call<true, true>(kmax, dense, a, grid_per_sm) : count_call<true, false>(kmax, dense, a, grid_per_sm);
+  return join ? count_call<false, true>(kmax, dense, a, grid_per_sm) : count_call<false, false>(kmax, dense, a, grid_per_sm);
 }
 
 void launch_wave_materialize(const NodeDesc *nodes, int32_t nnodes, long long total_tiles, int32_t kmax,

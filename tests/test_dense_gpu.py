@@ -1,6 +1,6 @@
-"""Counting nodes with many rows a graph (packed rows): their bitmap words are read
-before a bit is set.  Rows around the line of that rule, rows of one, two and five
-planes, 6- and 8-bit ids, graphs over several bitmap words, against the oracle."""
+"""Counting nodes with many rows a graph: their bitmap words are read before a bit is
+set.  Rows around the line of that rule, packed rows of one, two and five planes and
+of 6- and 8-bit ids, columns, graphs over several bitmap words, against the oracle."""
 import pytest
 
 from conftest import run_oracle, to_lines
@@ -21,7 +21,7 @@ def _broom(path, leaves, size):
 
 # path: rows of one, two and five planes where the leaves begin; leaves: rows a graph of the
 # node that ends in one, the line is at 16
-@pytest.mark.parametrize("size", [0, 70])
+@pytest.mark.parametrize("size", [0, 70, 300])
 @pytest.mark.parametrize("path", [2, 8, 24])
 @pytest.mark.parametrize("leaves", [15, 16, 17])
 def test_rows_a_graph(gs, oracle, tmp_path, path, leaves, size):
