@@ -1365,6 +1365,9 @@ public:
     nctx_ = wo_.wave_nodes > 1 ? kWaveCtx : 1;
     E.pool.reset_peak();
     for(int i = 0; i < 2; i++) seen_bytes_[i] = E.bytes_seen[i];
+    // (the schedulers before this one have read what their passes left)
+    main_seen_ = E.main_gen;
+    for(int c = 0; c < kWaveCtx; c++) mat_seen_[c] = E.ctx[c].mat_gen;
     E.scratch.restart();
   }
 
@@ -1374,8 +1377,7 @@ public:
   {
     const int32_t id = enter(j);
     root_phase(std::vector<int32_t>{ id });
-    CK(cudaEventRecord(E.ev_main, E.stream));
-    E.main_gen++;
+    root_phase_queued();
     if(jobs_[id]->pending == 0) complete(id);
     return id;
   }
@@ -1388,8 +1390,7 @@ public:
     ids.reserve(js.size());
     for(const MineJob &j : js) ids.push_back(enter(j));
     root_phase(ids);
-    CK(cudaEventRecord(E.ev_main, E.stream));
-    E.main_gen++;
+    root_phase_queued();
     for(int32_t id : ids)
       if(jobs_[id]->pending == 0) complete(id);
     return ids;
@@ -1556,11 +1557,21 @@ private:
   // the engine's root phases and every context's materialise passes whose flags
   // and byte counters have been read
   uint64_t main_seen_ = 0, mat_seen_[kWaveCtx] = {};
+  bool root_rows_ = false;  // the root phase writes first embeddings
   // per context, the materialise pass whose time is being added up
   unsigned long long mat_start_[kWaveCtx] = {};
   double mat_ms_[kWaveCtx] = {};
   bool defer_emit_ = false;
   bool any_packed_ = false;      // some job has packed rows
+  // A root phase without frequent roots has nothing queued behind the results
+  // that the host has read, the flags among them.
+  void root_phase_queued()
+  {
+    CK(cudaEventRecord(E.ev_main, E.stream));
+    if(main_seen_ == E.main_gen && !root_rows_) main_seen_++;
+    E.main_gen++;
+    root_rows_ = false;
+  }
   // a wave context's stream (all on the engine's with the serial option)
   cudaStream_t cs(const WaveCtx &X) const { return wo_.serial ? E.stream : X.stream; }
   void h2d(void *dst, const void *src, size_t n, cudaStream_t s = nullptr)
@@ -1884,6 +1895,7 @@ private:
       }
       S.peak_bytes = std::max(S.peak_bytes, S.live_bytes);
     }
+    root_rows_ = root_rows_ || !outs.empty();
     if(!outs.empty()) {
       // the children's outputs and the child map, copied by one kernel
       const size_t outs_bytes = Carver::round(sizeof(ChildOut) * outs.size());
