@@ -1,5 +1,6 @@
-// Device time stamps for the per-kernel times of the statistics.  An event
-// between two kernels of a stream costs about 3 us of it; a stamp is one store.
+// Device helpers of several kernels: time stamps for the per-kernel times of the
+// statistics (an event between two kernels of a stream costs about 3 us of it, a
+// stamp is one store), the wait of early launches, a bitmap word in use.
 #pragma once
 #include "gs_device.hpp"
 
